@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "bnsn_constants.h"
+#include "bnsn_fx.cuh"
 
 namespace bnsn {
 namespace fp64 {
@@ -26,20 +27,20 @@ namespace fp64 {
 // to the lower bound.
 BNSN_DI double safe_exp(double x)
 {
-    const double lo = (x > k::ExpLow) ? x : k::ExpLow;
-    return exp((lo < k::ExpUpp) ? lo : k::ExpUpp);
+    if (((uint32_t)__double2hiint(x) & 0x7fffffffu) >= 0x4085e000u) // |x| >= 700 or NaN
+        x = x > 0. ? k::ExpUpp : k::ExpLow;
+    return fx::exp2(fx::exp_arg(x));
 }
 
-// functions.hpp:4376-4396
+// functions.hpp:4376-4396.  The reciprocal is the correctly rounded one: the
+// beta rates take 1 - f where f is within 1e-9 of 1 and multiply it by e^{x}
+// of detailed balance, so an ulp of f shows as 1e-7 of their result.
 BNSN_DI double fermi_distr(double e, double temp, double mu)
 {
     const double arg = (e - mu) / temp;
-    if (arg > 0.)
-    {
-        const double t = safe_exp(-arg);
-        return t / (t + 1.);
-    }
-    return 1. / (safe_exp(arg) + 1.);
+    const double t   = safe_exp(-fabs(arg));
+    const double r   = __drcp_rn(t + 1.);
+    return arg > 0. ? t * r : r;
 }
 
 // functions.hpp:4401-4413 for d1 = w' - w and d2 = w - w' at once (both
@@ -71,7 +72,7 @@ BNSN_DI double bessi1(double x)
         ans = 0.2282967e-1 + y * (-0.2895312e-1 + y * (0.1787654e-1 - y * 0.420059e-2));
         ans = 0.39894228 + y * (-0.3988024e-1 + y * (-0.362018e-2 + y * (0.163801e-2 +
               y * (-0.1031555e-1 + y * ans))));
-        ans *= (exp(ax) / sqrt(ax));
+        ans *= (fx::exp(ax) / sqrt(ax));
     }
     return x < 0. ? -ans : ans;
 }
@@ -89,7 +90,7 @@ BNSN_DI double bessk1(double x)
     else
     {
         y   = 2. / x;
-        ans = (exp(-x) / sqrt(x)) *
+        ans = (fx::exp(-x) / sqrt(x)) *
               (1.25331414 + y * (0.23498619 + y * (-0.3655620e-1 + y * (0.1504268e-1 +
               y * (-0.780353e-2 + y * (0.325614e-2 + y * (-0.68245e-3)))))));
     }
@@ -97,11 +98,17 @@ BNSN_DI double bessk1(double x)
 }
 
 // ---------------------------------------------------------------------------
-// Complete Fermi-Dirac integrals F_k, k = 0..5 (functions.hpp:1550-2838):
-// Fukushima's piecewise minimax rational approximations in x = -|y|
-// (x < -2: series in e^x; -2 <= x <= 0: rational in s = -x/2) with the
-// reflection polynomial for y > 0.  A NaN argument yields 0.
+// Complete Fermi-Dirac integrals F_k, k = 0..5 (functions.hpp:1550-2838), on
+// the integer pipes (bnsn_fx.cuh): within one ulp, as the reference's
+// rational approximations (1.4e-16).  A NaN argument yields 0.
 // ---------------------------------------------------------------------------
+
+// F_K(y) for K = KLO..KHI at one argument; out[K - KLO].
+template <int KLO, int KHI>
+BNSN_DI void fdi_orders(double y, double* out)
+{
+    fx::fd_orders<KLO, KHI>(y, out);
+}
 
 template <int N>
 BNSN_DI double horner(const double (&c)[N], double t)
@@ -223,10 +230,14 @@ template <> struct FdiCoef<5>
 };
 
 
-// F_K(y) for K = KLO..KHI at one argument; out[K - KLO].  The regime test and
-// the exponential are shared by all orders.
+// The same integrals from the reference's own approximations in its operation
+// order (Fukushima's piecewise minimax rational forms in x = -|y|: x < -2 a
+// series in e^x, -2 <= x <= 0 rational in s = -x/2, the reflection polynomial
+// for y > 0).  Six times the cost of fdi_orders, with which it agrees to an
+// ulp; for the cells of the pair kernel whose cancellation magnifies an ulp of
+// a Fermi integral by 10^8 and more (pair_low_energy).
 template <int KLO, int KHI>
-BNSN_DI void fdi_orders(double y, double* out)
+__device__ __noinline__ void fdi_rational(double y, double* out)
 {
     const double x = -fabs(y);
     if (x < -2.)
@@ -332,7 +343,7 @@ BNSN_DI void distr_species(double n_in, double J_in, double chi, double gamma36,
             y * (y * (y * (y * (y * (y + 255.936658313629) + 9.42360945627147e-5) -
                            81.2467063138386) - 180.100197053091) - 89.0343496217014) +
             143.849128123195;
-        eta = exp(num / den);
+        eta = fx::exp(num / den);
     }
     else
     {
@@ -348,21 +359,21 @@ BNSN_DI void distr_species(double n_in, double J_in, double chi, double gamma36,
     *c_f             = k::CF;
     const double Tnu = J / (n * (k::CF + 3.));
     *temp_f          = Tnu;
-    *beta_f          = n / (k::FourPiHc3 * gamma36 * pow(Tnu, k::CF + 3.));
+    *beta_f          = n / (k::FourPiHc3 * gamma36 * fx::pow(Tnu, k::CF + 3.));
 }
 
 // distribution.hpp:298-315 (TotalNuF) for the 4 species at one energy;
-// pow(omega, c_f) is evaluated once when the species share c_f.
+// fx::pow(omega, c_f) is evaluated once when the species share c_f.
 BNSN_DI void total_nu_f4(double omega, const Distr& d, bool same_cf, double* g)
 {
-    double pw = same_cf ? pow(omega, d.c_f[0]) : 0.;
+    double pw = same_cf ? fx::pow(omega, d.c_f[0]) : 0.;
 #pragma unroll
     for (int s = 0; s < 4; ++s)
     {
         const double T_t = d.temp_t[s];
         const double ft  = fermi_distr(omega, T_t, d.temp_t[s] * d.eta_t[s]);
-        const double p   = same_cf ? pw : pow(omega, d.c_f[s]);
-        const double fn  = d.beta_f[s] * p * exp(-omega / d.temp_f[s]);
+        const double p   = same_cf ? pw : fx::pow(omega, d.c_f[s]);
+        const double fn  = d.beta_f[s] * p * fx::exp(-omega / d.temp_f[s]);
         g[s]             = d.w_t[s] * ft + d.w_f[s] * fn;
     }
 }
@@ -532,7 +543,7 @@ BNSN_DI double eta_nn_sc(double nb, double temp, double yN)
     const double nN = yN * nb;
     if (nN <= 0.)
         return 0.;
-    const double eFN = k::IsoEf * pow(nN, 2. / 3.);
+    const double eFN = k::IsoEf * fx::pow(nN, 2. / 3.);
     const double aux = 1.5 * temp / eFN;
     return nN * aux / sqrt(1. + aux * aux);
 }
@@ -576,20 +587,35 @@ struct PairEnergyFdi
     double m[5], p[5];
 };
 
+// Spectral energies y = nu / T below this take the reference's rational Fermi
+// integrals throughout.  Psi differences them over 15 y^2 z^2: at y = 0.01 (1
+// MeV at T = 100 MeV) an ulp moved kappa by up to 2e-7, at y = 0.025 by 2e-8, and
+// the noise falls as y^-2.  The grey integrals' low nodes carry weights that
+// make it invisible (1e-13).
+constexpr double kPairLowEnergy = 0.03125;
+
 // Psi_0(y, z) and Psi_0(z, y) of kernel_pair.hpp:16-120 from the per-energy
 // Fermi integrals: fam[k-1] = F_k(eta - y), fap = F_k(eta + y), fbm / fbp the
 // same for z; f3e / f4e are F_3(eta), F_4(eta).  Zero when eta - y - z > 200.
 BNSN_DI void pair_psi(double eta, double y, double z, const double* fam, const double* fap,
                       const double* fbm, const double* fbp, double f3e, double f4e,
-                      double* psi0, double* psi1)
+                      double* psi0, double* psi1, bool rational = false)
 {
     *psi0 = 0.;
     *psi1 = 0.;
     if (eta - y - z > 200.)
         return;
     double fmyz[3], fpyz[3];
-    fdi_orders<3, 5>(eta - y - z, fmyz);
-    fdi_orders<3, 5>(eta + y + z, fpyz);
+    if (rational)
+    {
+        fdi_rational<3, 5>(eta - y - z, fmyz);
+        fdi_rational<3, 5>(eta + y + z, fpyz);
+    }
+    else
+    {
+        fdi_orders<3, 5>(eta - y - z, fmyz);
+        fdi_orders<3, 5>(eta + y + z, fpyz);
+    }
     const double c0  = 20. * fam[3];
     const double c1  = 20. * fbp[3];
     const double c2  = 120. * fam[1] - 120. * fbp[1];
@@ -627,10 +653,10 @@ BNSN_DI void pair_psi(double eta, double y, double z, const double* fam, const d
 BNSN_DI void pair_kernel(double T, double eta, double omega, double omega_p,
                          double y, double z, const double* fam, const double* fap,
                          const double* fbm, const double* fbp, double f3e,
-                         double f4e, double* em, double* ab)
+                         double f4e, double* em, double* ab, bool rational = false)
 {
     double psi0, psi1;
-    pair_psi(eta, y, z, fam, fap, fbm, fbp, f3e, f4e, &psi0, &psi1);
+    pair_psi(eta, y, z, fam, fap, fbm, fbp, f3e, f4e, &psi0, &psi1, rational);
     const double aux = k::PairPhi * (T * T) / (1. - safe_exp(y + z));
     const double phi0 = ((k::PairA1e * k::PairA1e) * psi0 + (k::PairA2e * k::PairA2e) * psi1) * aux;
     const double phi1 = ((k::PairA1e * k::PairA1e) * psi1 + (k::PairA2e * k::PairA2e) * psi0) * aux;
@@ -681,12 +707,12 @@ BNSN_DI double hr98_g(double y, double eta_star)
     const double a1den = 25. * y2 + 1.;
     const double a1    = (0.5 + inv) / (1. + inv) * (1. / a1den) +
                       (0.5 + eta_star / 15.6) * 25. * y2 / a1den;
-    const double a2  = (0.63 + 0.04 * pow(eta_star, 1.45)) / (1. + 0.02 * pow(eta_star, 2.5));
-    const double p15 = pow(eta_star, 1.5);
+    const double a2  = (0.63 + 0.04 * fx::pow(eta_star, 1.45)) / (1. + 0.02 * fx::pow(eta_star, 2.5));
+    const double p15 = fx::pow(eta_star, 1.5);
     const double a3  = 1.2 * safe_exp(0.6 * eta_star - 0.4 * p15);
     const double p1  = (1.8 + 0.45 * eta_star) / (1. + 0.15 * p15);
     const double p2  = 2.3 - 0.05 * eta_star / (1. + 0.025 * eta_star);
-    return (a1 + a2 * pow(y, p1)) / (1. + a3 * pow(y, p2) + a2 * pow(y, p1 + 2.) / 13.75);
+    return (a1 + a2 * fx::pow(y, p1)) / (1. + a3 * fx::pow(y, p2) + a2 * fx::pow(y, p1 + 2.) / 13.75);
 }
 
 // Channel constants (kernel_brem_HR98.hpp:239-289 for everything but x);
@@ -714,8 +740,8 @@ BNSN_DI Hr98Channel hr98_channel(double nb, double yn, double yp, double T, int 
         c.weight = (28. / 3.) * n_nuc;
     }
     const double T10  = T * 0.1;
-    const double etas = pow(3. * k::PiSq * n_nuc, 2. / 3.) * k::BremAux1 / (2. * m_nuc * T);
-    c.gamma           = 1.63 * pow(etas, 1.5) * T10;
+    const double etas = fx::pow(3. * k::PiSq * n_nuc, 2. / 3.) * k::BremAux1 / (2. * m_nuc * T);
+    c.gamma           = 1.63 * fx::pow(etas, 1.5) * T10;
     const double y    = 1.94 / T10;
     const double gb   = hr98_g(y, etas);
     c.hgg             = 0.5 * c.gamma * gb;
@@ -728,11 +754,11 @@ BNSN_DI Hr98Channel hr98_channel(double nb, double yn, double yp, double T, int 
     double f_u        = (1. - 5. * u * atan(2. / u) / 6. + u2 / (3. * (u2 + 4.)) +
                   atan(1. / uarg) * uarg / 3.);
     c.f_u    = (fabs(f_u) < 1.e-14) ? 1.e-14 : f_u;
-    c.K1     = 3. * k::PiHalf52 * pow(e, -2.5);
+    c.K1     = 3. * k::PiHalf52 * fx::pow(e, -2.5);
     c.eta2p1 = 1. + e * e;
     c.sqe    = sqrt(e);
     c.ep2    = e + 0.2;
-    c.h      = 0.1 * e / (2.39 + 0.1 * pow(e, 1.1));
+    c.h      = 0.1 * e / (2.39 + 0.1 * fx::pow(e, 1.1));
     return c;
 }
 
@@ -747,8 +773,8 @@ BNSN_DI void hr98_point_common(double nb, double T, bool medium, Hr98Point* P)
     P->ey12       = safe_exp(-yc / 12.);
     P->poly_y     = 5. * (yc * yc) / 3.;
     P->y4p1       = 1. + yc * yc * yc * yc;
-    P->Dy         = 0.8 + 0.06 * pow(yc, 1.05);
-    const double p = 0.67 + 0.18 * pow(yc, 0.4);
+    P->Dy         = 0.8 + 0.06 * fx::pow(yc, 1.05);
+    const double p = 0.67 + 0.18 * fx::pow(yc, 0.4);
     P->mp         = -p;
     P->minv       = -1. / p;
     if (medium)
@@ -771,20 +797,20 @@ BNSN_DI void hr98_kernel(const Hr98Point& P, double omega, double omega_p,
     const double xs = (x > k::BremXmin) ? x : k::BremXmin;
     const double y  = P.y;
     // s_nd, Eq.(45)
-    const double snd_num = 2. * k::SqrtPi * pow(xs + 2. - P.ey12, 1.5) *
+    const double snd_num = 2. * k::SqrtPi * fx::pow(xs + 2. - P.ey12, 1.5) *
                            ((xs * xs) + 2. * xs * y + P.poly_y + 1.);
     const double q       = k::Pi18 + xs + y;
     const double s_nd    = snd_num / (k::SqrtPi + q * q * q * q);
     const double X2      = (xs * xs) + k::FourPiSq;
     const double den_sd  = k::FourPiSq * (1. - safe_exp(-xs));
-    const double px11    = pow(xs, 1.1);
-    const double xterm   = 3. + (xs - 1.2) * (xs - 1.2) + pow(xs, -4.);
+    const double px11    = fx::pow(xs, 1.1);
+    const double xterm   = 3. + (xs - 1.2) * (xs - 1.2) + fx::pow(xs, -4.);
     const double gpart   = 0.0044 * px11 * y / P.Dy;
     const double cnum    = 1.1 * px11;
-    const double px093   = pow(xs, 0.93);
-    const double px12    = 0.0001 * pow(xs, 1.2);
-    const double cden2   = 30. + 0.005 * pow(xs, 2.8);
-    const double snd_p   = pow(s_nd, P.mp);
+    const double px093   = fx::pow(xs, 0.93);
+    const double px12    = 0.0001 * fx::pow(xs, 1.2);
+    const double cden2   = 30. + 0.005 * fx::pow(xs, 2.8);
+    const double snd_p   = fx::pow(s_nd, P.mp);
     const double x2      = x * x;
     double tot           = 0.;
 #pragma unroll
@@ -795,7 +821,7 @@ BNSN_DI void hr98_kernel(const Hr98Point& P, double omega, double omega_p,
         const double f_brem  = 1. + 1. / (xterm * C.eta2p1 * P.y4p1);
         const double g_brem  = 1. - gpart * C.sqe / C.ep2;
         const double c_brem  = cnum * C.h / (2.3 + C.h * px093 + px12) * 30. / cden2;
-        const double s = pow(snd_p + pow(s_d, P.mp), P.minv) * f_brem * (1. + c_brem * g_brem);
+        const double s = fx::pow(snd_p + fx::pow(s_d, P.mp), P.minv) * f_brem * (1. + c_brem * g_brem);
         const double chan = C.gamma / (x2 + C.hgg * C.hgg) * s / P.T;
         tot += C.weight * chan;
     }
@@ -816,7 +842,7 @@ BNSN_DI double brt06_point(double nb, double T, double yn, double yp)
     const double rho = nb * k::Mb;
     const double q   = 2.0778e+02 * 0.5 * k::MeV *
                      ((yn * yn) + (yp * yp) + (28. / 3.) * yn * yp) * (rho * rho) *
-                     pow(T, 5.5);
+                     fx::pow(T, 5.5);
     const double T7 = T * T * T * T * T * T * T;
     return k::HC6FourPi2 * k::BremC4BRT06 * (q / T7);
 }
@@ -1091,7 +1117,7 @@ BNSN_DI void gp19_cell(const Gp19Point& P, double v0, double v1, double w, doubl
         k2 = (k2 < eps) ? eps : k2;
         k4 = (k4 < eps) ? eps : k4;
         const double m = log(k4 / k2) * 1.4426950408889634;
-        s = k2 * pow(P.T * 0.5, m);
+        s = k2 * fx::pow(P.T * 0.5, m);
         s = (s < eps) ? eps : s;
         break;
     }
@@ -1099,7 +1125,7 @@ BNSN_DI void gp19_cell(const Gp19Point& P, double v0, double v1, double w, doubl
     {
         const double k2 = P.C * v0, k4 = P.C * v1;
         const double m  = log(k4 / k2) * 1.4426950408889634;
-        s = k2 * pow(P.T * 0.5, m);
+        s = k2 * fx::pow(P.T * 0.5, m);
         break;
     }
     default: // 3, 5
@@ -1144,7 +1170,7 @@ BNSN_DI void gp19_kernel(const Gp19Table& G, double nb_nm, double ye_in, double 
             k2 = (k2 < eps) ? eps : k2;
             k4 = (k4 < eps) ? eps : k4;
             const double m = log(k4 / k2) * 1.4426950408889634;
-            s = k2 * pow(T * 0.5, m);
+            s = k2 * fx::pow(T * 0.5, m);
             s = (s < eps) ? eps : s;
         }
         else if (T > Tmax)
@@ -1162,7 +1188,7 @@ BNSN_DI void gp19_kernel(const Gp19Table& G, double nb_nm, double ye_in, double 
         const double k2 = gp19_in_range(G, nb, ye, 2.0, w);
         const double k4 = gp19_in_range(G, nb, ye, 4.0, w);
         const double m  = log(k4 / k2) * 1.4426950408889634;
-        s = k2 * pow(T * 0.5, m);
+        s = k2 * fx::pow(T * 0.5, m);
     }
     else if (T > Tmax)
     {

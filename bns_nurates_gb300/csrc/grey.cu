@@ -114,7 +114,7 @@ __device__ __forceinline__ double warp_sum(double v)
 __device__ __forceinline__ double total_nu_f1(double omega, const Distr& d, int s)
 {
     const double ft = fermi_distr(omega, d.temp_t[s], d.temp_t[s] * d.eta_t[s]);
-    const double fn = d.beta_f[s] * pow(omega, d.c_f[s]) * exp(-omega / d.temp_f[s]);
+    const double fn = d.beta_f[s] * fx::pow(omega, d.c_f[s]) * fx::exp(-omega / d.temp_f[s]);
     return d.w_t[s] * ft + d.w_f[s] * fn;
 }
 
@@ -915,8 +915,8 @@ __global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
                 const dfm::df yd = dfm::from_double(y);
                 X.yh[a] = yd.hi;
                 X.yl[a] = yd.lo;
-                X.eh[a] = exp(y - 0.5 * fabs(eta));
-                X.dn[a] = exp(-y);
+                X.eh[a] = fx::exp(y - 0.5 * fabs(eta));
+                X.dn[a] = fx::exp(-y);
             }
         }
         if (!MIXED && redo_only)

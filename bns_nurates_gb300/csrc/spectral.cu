@@ -309,12 +309,24 @@ __global__ void __launch_bounds__(kWarps * 32)
         const double yp = L.eos[3][p], yn = L.eos[4][p], mu_e = L.eos[7][p];
         const double eta_e = mu_e / T;
         EnergyRec* R       = rec + q * ne;
+        // energies so low that the pair kernel needs the reference's own Fermi
+        // integrals (kPairLowEnergy): the point's node tables then too
+        bool low = false;
+        if (L.use_pair && !MIX)
+        {
+            for (int c = lane; c < ne; c += 32)
+                low = low || (((emask >> c) & 1ull) && L.energies[c] < kPairLowEnergy * T);
+            low = __any_sync(0xffffffffu, low);
+        }
         __syncwarp();
         load_distr(dsc, q, &W.d, lane);
         if (lane == 28 && L.use_pair)
         {
             double f[2];
-            fdi_orders<3, 4>(eta_e, f);
+            if (low)
+                fdi_rational<3, 4>(eta_e, f);
+            else
+                fdi_orders<3, 4>(eta_e, f);
             W.fe3 = f[0];
             W.fe4 = f[1];
         }
@@ -373,8 +385,8 @@ __global__ void __launch_bounds__(kWarps * 32)
                 X.ybl[a] = yd.lo;
                 if (L.use_pair)
                 {
-                    X.ehz[a] = exp(W.zb[a] - 0.5 * fabs(eta_e));
-                    X.dnz[a] = exp(-W.zb[a]);
+                    X.ehz[a] = fx::exp(W.zb[a] - 0.5 * fabs(eta_e));
+                    X.dnz[a] = fx::exp(-W.zb[a]);
                 }
 #pragma unroll
                 for (int s = 0; s < 4; ++s)
@@ -392,7 +404,9 @@ __global__ void __launch_bounds__(kWarps * 32)
                 const int a    = t >> 1;
                 const int i    = a < n ? a : a - n;
                 const double z = (a < n ? ts * S.x[i] : ts / S.x[i]) / T;
-                if (t & 1)
+                if (low)
+                    fdi_rational<1, 5>(t & 1 ? eta_e + z : eta_e - z, t & 1 ? W.fpz[a] : W.fmz[a]);
+                else if (t & 1)
                     fdi_orders<1, 5>(eta_e + z, W.fpz[a]);
                 else
                     fdi_orders<1, 5>(eta_e - z, W.fmz[a]);
@@ -434,8 +448,16 @@ __global__ void __launch_bounds__(kWarps * 32)
                 const double y = L.energies[e0 + c] / T;
                 if (L.use_pair && !skip && !MIX)
                 {
-                    fdi_orders<1, 5>(eta_e - y, W.fmy[c]);
-                    fdi_orders<1, 5>(eta_e + y, W.fpy[c]);
+                    if (low && L.energies[e0 + c] < kPairLowEnergy * T)
+                    {
+                        fdi_rational<1, 5>(eta_e - y, W.fmy[c]);
+                        fdi_rational<1, 5>(eta_e + y, W.fpy[c]);
+                    }
+                    else
+                    {
+                        fdi_orders<1, 5>(eta_e - y, W.fmy[c]);
+                        fdi_orders<1, 5>(eta_e + y, W.fpy[c]);
+                    }
                 }
                 if (MIX)
                 {
@@ -444,8 +466,8 @@ __global__ void __launch_bounds__(kWarps * 32)
                     X.yel[c] = yd.lo;
                     if (L.use_pair)
                     {
-                        X.ehy[c] = exp(y - 0.5 * fabs(eta_e));
-                        X.dny[c] = exp(-y);
+                        X.ehy[c] = fx::exp(y - 0.5 * fabs(eta_e));
+                        X.dny[c] = fx::exp(-y);
                     }
                 }
             }
@@ -470,7 +492,7 @@ __global__ void __launch_bounds__(kWarps * 32)
                     gl[kk] = 0.f;
                     gp[kk] = 0.;
                 }
-                const double sbe = sb * exp(-w); // brem emission carries e^{-nu/T}
+                const double sbe = sb * fx::exp(-w); // brem emission carries e^{-nu/T}
                 const double inu2 = MIX ? 1. / (nu * nu) : 0.;
                 if (act && !skip)
                 {
@@ -483,7 +505,8 @@ __global__ void __launch_bounds__(kWarps * 32)
                         double be = 0., ba = 0.;
                         if (L.use_pair && !MIX)
                             pair_kernel(T, eta_e, nu, nub, w, W.zb[a], W.fmy[c], W.fpy[c],
-                                        W.fmz[a], W.fpz[a], W.fe3, W.fe4, pe, pa);
+                                        W.fmz[a], W.fpz[a], W.fe3, W.fe4, pe, pa,
+                                        low && nu < kPairLowEnergy * T);
                         if (L.use_brem && !b32)
                         {
                             if (L.brem_impl == 0)
@@ -815,8 +838,8 @@ __global__ void __launch_bounds__(kWarps * 32, MODE == kSpecMixed ? 4 : 1)
                     }
                     sig[0] = isfinite(sig[0]) ? sig[0] : 0.f;
                     sig[1] = isfinite(sig[1]) ? sig[1] : 0.f;
-                    sne    = sn * exp((double)sig[0]);
-                    sna    = sn * exp((double)sig[1]);
+                    sne    = sn * fx::exp((double)sig[0]);
+                    sna    = sn * fx::exp((double)sig[1]);
                 }
                 const dfm::df Wd = dfm::from_double(w);
                 if (run)
