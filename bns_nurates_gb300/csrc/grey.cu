@@ -1403,59 +1403,6 @@ __device__ __forceinline__ void neps_energies(int r, double xi, double xj, doubl
     }
 }
 
-// The FP64 item sums of one point (the plain path, and the mixed path's
-// fallback for points outside the FP32 range envelope).
-__device__ __forceinline__ void neps_items_fp64(const NepsPoint& NP, const Distr& d, bool same_cf,
-                                                int n2, double tn, bool stim, bool nbb,
-                                                const double* s_x2, const double* s_w2,
-                                                const double* s_wx, const double* s_wx3,
-                                                int t0, int stride, double* acc)
-{
-    const int nn2 = n2 * n2;
-    for (int it = t0; it < 2 * nn2; it += stride)
-    {
-        const int r   = it >= nn2;
-        const int rem = it - r * nn2;
-        const int i = rem / n2, j = rem - (rem / n2) * n2;
-        double nu, nub;
-        neps_energies(r, s_x2[i], s_x2[j], tn, &nu, &nub);
-        const double w4 = (nu * nu) * (nub * nub);
-        double g[4], gb[4];
-        total_nu_f4(nu, d, same_cf, g);
-        total_nu_f4(nub, d, same_cf, gb);
-        double em1[4], ab1[4], em2[4], ab2[4];
-        neps_pair(NP, nu, nub, em1, ab1, em2, ab2);
-        const double Wr = (r ? s_wx3[i] : s_wx[i]) * s_w2[j];
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-        {
-            const double e1 = em1[s] * gb[s];
-            const double a1 = ab1[s] * (nbb ? 1. : 1. - gb[s]);
-            const double e2 = em2[s] * g[s];
-            const double a2 = ab2[s] * (nbb ? 1. : 1. - g[s]);
-            double EM1, AB1, EM2, AB2;
-            if (stim)
-            {
-                AB1 = w4 * g[s] * (e1 + a1);
-                EM1 = w4 * e1;
-                AB2 = w4 * gb[s] * (e2 + a2);
-                EM2 = w4 * e2;
-            }
-            else
-            {
-                AB1 = w4 * g[s] * a1;
-                EM1 = w4 * (1. - g[s]) * e1;
-                AB2 = w4 * gb[s] * a2;
-                EM2 = w4 * (1. - gb[s]) * e2;
-            }
-            acc[s] += Wr * (EM1 + EM2);
-            acc[4 + s] += Wr * (AB1 + AB2);
-            acc[8 + s] += Wr * (nu * EM1 + nub * EM2);
-            acc[12 + s] += Wr * (nu * AB1 + nub * AB2);
-        }
-    }
-}
-
 // TotalNuF and 1 - TotalNuF in df (the accurate pass of the mixed path).
 __device__ __forceinline__ void total_nu_df(double omega, double lw, const NepsMixed& Q,
                                             const double* wt, const double* wf, dfm::df* g,
@@ -1576,34 +1523,23 @@ __device__ __forceinline__ void neps_item_df(const NepsPoint& P, const NepsMixed
     }
 }
 
-// NES launch modes.  The plain path runs kNesFp64All.  The mixed path runs
-// three launches per chunk, each over all points but working only on its own:
+// The mixed path's NES runs three launches per chunk, each over all points but
+// working only on its own:
 //   grey_nes_fast_kernel  FP32 kernel integrals (bnsn_nes32.cuh); flags a
 //                 point 1 when its sums cancel (terms of both signs, or
 //                 negative pair + brem sums) and 2 when it leaves the FP32
 //                 range envelope;
-//   kNesAccurate  flag 1: every product in df (cancellation up to ~1e5);
-//                 beyond that the point is flagged 2;
-//   kNesFp64Flag  flag 2: FP64 items.
-enum NesMode
-{
-    kNesFp64All = 0,
-    kNesAccurate = 2,
-    kNesFp64Flag
-};
+//   grey_neps_kernel      flag 1: every product in df (cancellation up to
+//                 ~1e5); beyond that the point is flagged 2;
+//   grey_nes64_kernel     flag 2: FP64 items (the plain path runs it over
+//                 every point).
+// The passes over the few flagged points run a point per CTA, its items over
+// all the CTA's threads (one warp alone would leave the pass as long as a
+// point's whole item loop).
+constexpr int kNesAccWarps = 8;
 
-// Warps per CTA of the NES kernels: the plain path runs a point per warp; the
-// mixed path's passes over the few points flagged by the fast pass run a
-// point per CTA, its items over all the CTA's threads (one warp alone would
-// leave the pass as long as a point's whole item loop).
-template <int MODE>
-__host__ __device__ constexpr int nes_warps()
-{
-    return MODE == kNesFp64All ? kWarps : 8;
-}
-
-template <int MODE, bool MULTI = false>
-__global__ void __launch_bounds__(nes_warps<MODE>() * 32, MODE == kNesAccurate ? 2 : 1)
+template <bool MULTI = false>
+__global__ void __launch_bounds__(kNesAccWarps * 32, 2)
     grey_neps_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
                      int64_t np, double* __restrict__ scratch)
 {
@@ -1617,15 +1553,12 @@ __global__ void __launch_bounds__(nes_warps<MODE>() * 32, MODE == kNesAccurate ?
     }
     if (MULTI && !L.use_inel)
         return;
-    constexpr bool MIX  = MODE == kNesAccurate;
-    constexpr bool WIDE = MODE != kNesFp64All;  // a point per CTA
-    constexpr int NW    = nes_warps<MODE>();
-    constexpr int NT    = WIDE ? 1 : NW;        // point tables in flight per CTA
+    constexpr int NW = kNesAccWarps;
     __shared__ double s_x2[kMaxQ], s_w2[kMaxQ], s_wx[kMaxQ], s_wx3[kMaxQ];
-    __shared__ NepsTab s_nt[NT];
-    __shared__ NepsMixed s_nm[MIX ? NT : 1];
+    __shared__ NepsTab N;
+    __shared__ NepsMixed Q;
     __shared__ dfm::FdiTab s_ftab;
-    __shared__ double s_red[WIDE ? NW : 1][32];
+    __shared__ double s_red[NW][32];
     for (int k = threadIdx.x; k < kMaxQ; k += blockDim.x)
     {
         s_x2[k]  = L.x2[k];
@@ -1633,45 +1566,32 @@ __global__ void __launch_bounds__(nes_warps<MODE>() * 32, MODE == kNesAccurate ?
         s_wx[k]  = L.wx[k];
         s_wx3[k] = L.wx3[k];
     }
-    if (MIX)
-        for (int k = threadIdx.x; k < (int)(sizeof(dfm::FdiTab) / sizeof(float)); k += blockDim.x)
-            ((float*)&s_ftab)[k] = ((const float*)&dfm::kFdiTab)[k];
+    for (int k = threadIdx.x; k < (int)(sizeof(dfm::FdiTab) / sizeof(float)); k += blockDim.x)
+        ((float*)&s_ftab)[k] = ((const float*)&dfm::kFdiTab)[k];
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int wid  = threadIdx.x >> 5;
-    NepsTab& N     = s_nt[WIDE ? 0 : wid];
     const int n2   = L.n2;
     const bool nbb = L.neglect_blocking != 0;
     // items of a point: thread t0, t0 + stride, ...
-    const int t0     = WIDE ? (int)threadIdx.x : lane;
-    const int stride = WIDE ? NW * 32 : 32;
-    const int64_t q0    = WIDE ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * NW + wid;
-    const int64_t qstep = WIDE ? (int64_t)gridDim.x : (int64_t)gridDim.x * NW;
+    const int t0     = (int)threadIdx.x;
+    const int stride = NW * 32;
 
-    for (int64_t q = q0; q < np; q += qstep)
+    for (int64_t q = blockIdx.x; q < np; q += gridDim.x)
     {
         const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
         PointTab* P     = (PointTab*)(scratch + q * kTabWords);
-        if (MODE == kNesAccurate && P->neps_fp64 != 1.)
-            continue;
-        if (MODE == kNesFp64Flag && P->neps_fp64 != 2.)
+        if (P->neps_fp64 != 1.)
             continue;
         const double T = L.eos[1][p], mu_e = L.eos[7][p];
-        if (WIDE)
-            __syncthreads(); // the previous point's readers are done
-        else
-            __syncwarp();
-        if (!WIDE || wid == 0)
+        __syncthreads(); // the previous point's readers are done
+        if (wid == 0)
         {
             warp_copy((double*)&N.d, (const double*)&P->d, 28 + 12 + 2, lane);
             if (lane == 0)
                 N.same_cf = P->same_cf;
         }
-        if (WIDE)
-            __syncthreads();
-        else
-            __syncwarp();
-        const bool same_cf = N.same_cf != 0.;
+        __syncthreads();
         NepsPoint NP;
         NP.T    = T;
         NP.pre  = k::NepsConst * (T * T);
@@ -1686,22 +1606,15 @@ __global__ void __launch_bounds__(nes_warps<MODE>() * 32, MODE == kNesAccurate ?
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk)
             acc[kk] = 0.;
-        if (!MIX)
-        {
-            neps_items_fp64(NP, N.d, same_cf, n2, tn, L.stim != 0, nbb, s_x2, s_w2, s_wx, s_wx3,
-                            t0, stride, acc);
-        }
-        else
         {
             int flag = 0;
             {
-                NepsMixed& Q = s_nm[WIDE ? 0 : wid];
-                if ((!WIDE || wid == 0) && lane < 2)
+                if (wid == 0 && lane < 2)
                 {
                     Q.eta[lane] = dfm::from_double(lane ? NP.eta1 : NP.eta0);
                     dfm::fdi_raw15(Q.eta[lane], Q.reta[lane], 1, &s_ftab);
                 }
-                else if ((!WIDE || wid == 0) && lane >= 8 && lane < 12)
+                else if (wid == 0 && lane >= 8 && lane < 12)
                 {
                     const int s    = lane - 8;
                     const Distr& d = N.d;
@@ -1711,10 +1624,7 @@ __global__ void __launch_bounds__(nes_warps<MODE>() * 32, MODE == kNesAccurate ?
                     Q.invTf[s] = 1. / d.temp_f[s];
                     Q.cf[s]    = d.c_f[s];
                 }
-                if (WIDE)
-                    __syncthreads();
-                else
-                    __syncwarp();
+                __syncthreads();
                 const double invT = 1. / T;
                 const double lhtn = log(0.5 * tn);
                 dfm::df dacc[16];
@@ -1812,20 +1722,8 @@ __global__ void __launch_bounds__(nes_warps<MODE>() * 32, MODE == kNesAccurate ?
 #pragma unroll
                 for (int kk = 0; kk < 16; ++kk)
                     macc[kk] = (double)mag[kk];
-                if (WIDE)
-                {
-                    block_sum<NW>(acc, s_red, 0);
-                    block_sum<NW>(macc, s_red, 16);
-                }
-                else
-                {
-#pragma unroll
-                    for (int kk = 0; kk < 16; ++kk)
-                    {
-                        acc[kk]  = warp_sum(acc[kk]);
-                        macc[kk] = warp_sum(macc[kk]);
-                    }
-                }
+                block_sum<NW>(acc, s_red, 0);
+                block_sum<NW>(macc, s_red, 16);
                 const double amp =
                     cancel_factor_tot(acc, macc, NP.pre * T4, NP.pre * T4 * T, other);
                 if (amp > kMaxCancelDf)
@@ -1836,7 +1734,7 @@ __global__ void __launch_bounds__(nes_warps<MODE>() * 32, MODE == kNesAccurate ?
             }
             if (flag != 0)
             {
-                if (WIDE ? threadIdx.x == 0 : lane == 0)
+                if (threadIdx.x == 0)
                 {
                     P->neps_fp64 = (double)flag;
                     atomicAdd(&g_grey_mixed[2], 1ull);
@@ -1844,22 +1742,312 @@ __global__ void __launch_bounds__(nes_warps<MODE>() * 32, MODE == kNesAccurate ?
                 continue; // a later launch writes this point's sums
             }
         }
-        if (!MIX) // (the mixed pass has summed over the point's threads already)
-        {
-            if (WIDE)
-                block_sum<NW>(acc, s_red, 0);
-            else
-            {
-#pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                    acc[kk] = warp_sum(acc[kk]);
-            }
-        }
-        if (WIDE ? threadIdx.x == 0 : lane == 0)
+        if (threadIdx.x == 0)
         {
 #pragma unroll
             for (int kk = 0; kk < 16; ++kk)
                 P->snes[kk] = acc[kk];
+        }
+    }
+}
+
+
+// ---------------------------------------------------------------------------
+// NES/NPS in FP64 (kernel_nes.hpp:50-359; the item sums of
+// m1_opacities.hpp:864-1057 and integration.hpp:687-768).
+//
+// MezzacappaIntOut is antisymmetric, linear in its couplings, and an item's
+// energies in units of T do not depend on the point.  With phi_k = F_k / k!,
+// D_k = phi_k(eta - w') - phi_k(eta - w), E_k = phi_k(eta) - phi_k(eta - d),
+// d = w' - w > 0, S = w + w', P = w w':
+//   R(w, w') = -R(w', w) = -(24 / P^2) pre (b1 A + b2 B),
+//   A = (E5 + D5) + w' (E4 + w' E3 / 2) + S (D4 + S D3 / 2 + P D2 / 2) + P^2 D1 / 4,
+//   B = (E5 + D5) + w (w E3 / 2 - E4),
+// and the weight (nu nubar)^2 of the item cancels 1 / P^2.  So a lepton
+// takes three sets of Fermi integrals and 17 FP64 operations, where the
+// four species and two directions separately took 16 evaluations of the
+// bracket with a division each (~560 instructions); both leptons' A and B
+// combine into the four species' kernels afterwards, R(w', w) costs nothing,
+// and the NEPSExpFunc factors, weights and w^0.6 sit in the CTA's item table.
+// Bound by the FP64 pipe (~180 operations an item) beside the integer work of
+// its exponentials and Fermi integrals; 8,192 points at n = 20: 5.4 ms (the
+// separate brackets with the same Fermi integrals ~14.5 ms).  The items follow the
+// host's order of ascending w', which keeps a warp's lanes in the same
+// regime of the Fermi integrals.
+//
+// A point per warp of 16-warp CTAs (the 51 KB item table is shared by 16
+// points), or (WIDE) a point per 8-warp CTA: the mixed path's few flagged
+// points, and launches of fewer points than the chip has warps to fill.
+// ---------------------------------------------------------------------------
+
+// One species' occupation constants for x = omega / T: g = wt / (1 + e^{x rt -
+// eta}) + kf x^cf e^{-x rf}.
+struct Occ64
+{
+    double rt, eta, rf, wt, kf, cf;
+};
+
+__device__ __forceinline__ void occ64_from(const Distr& d, int s, double T, Occ64* o)
+{
+    o->rt  = T / d.temp_t[s];
+    o->eta = d.eta_t[s];
+    o->rf  = T / d.temp_f[s];
+    o->wt  = d.w_t[s];
+    o->cf  = d.c_f[s];
+    o->kf  = d.w_f[s] * (d.beta_f[s] * fx::pow(T, d.c_f[s]));
+}
+
+// TotalNuF (distribution.hpp:298-315) of four species at x; xc = x^0.6,
+// common: every cf is 0.6 (the reconstruction's value).
+__device__ __forceinline__ void occ64_eval(const Occ64* o, double x, double xc, bool common,
+                                           double* g)
+{
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+    {
+        const double ft = fx::rcp(safe_exp(fma(x, o[s].rt, -o[s].eta)) + 1.);
+        const double p  = common ? xc : fx::pow(x, o[s].cf);
+        g[s] = fma(o[s].wt, ft, o[s].kf * (p * fx::exp(-x * o[s].rf)));
+    }
+}
+
+// Sums the 16 values of the warp's lanes: lane l returns the total of value
+// sum_index(l).  Each round halves the values a lane carries, 16 additions in
+// all instead of 80 for 16 butterfly sums.
+__device__ __forceinline__ double warp_sum16(double* v, int lane)
+{
+#pragma unroll
+    for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1)
+    {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < n; ++k)
+        {
+            const double mine = up ? v[k + n] : v[k], theirs = up ? v[k] : v[k + n];
+            v[k] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+__device__ __forceinline__ int sum_index(int lane)
+{
+    return ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+}
+
+template <int NW>
+struct Nes64Smem
+{
+    double w[kMaxQ * kMaxQ * 2], wp[kMaxQ * kMaxQ * 2];   // w, w'
+    double ka[kMaxQ * kMaxQ * 2], m[kMaxQ * kMaxQ * 2];   // 24 weight e / (1 - e), 24 weight
+    double wc[kMaxQ * kMaxQ * 2], wpc[kMaxQ * kMaxQ * 2]; // w^0.6, w'^0.6
+    Occ64 occ[NW][4];
+    double fe[NW][2][6], fd0[NW][2];
+    double red[NW][16];
+};
+
+template <bool WIDE>
+__host__ __device__ constexpr int nes64_warps()
+{
+    return WIDE ? 8 : 16;
+}
+
+template <bool WIDE, bool MULTI = false>
+__global__ void __launch_bounds__(nes64_warps<WIDE>() * 32, WIDE ? 2 : 1)
+    grey_nes64_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
+                      int64_t np, double* __restrict__ scratch, int flagged)
+{
+    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
+    if (MULTI)
+    {
+        const GroupChunk& gcz = GA.gc[blockIdx.z];
+        p0      = gcz.p0;
+        np      = gcz.np;
+        scratch = gcz.ws;
+    }
+    if (MULTI && !L.use_inel)
+        return;
+    constexpr int NW = nes64_warps<WIDE>();
+    extern __shared__ __align__(16) unsigned char nes_smem_raw[];
+    Nes64Smem<NW>& S = *reinterpret_cast<Nes64Smem<NW>*>(nes_smem_raw);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int n2 = L.n2, nn2 = n2 * n2, nit = 2 * nn2;
+    const bool nbb = L.neglect_blocking != 0, stim = L.stim != 0;
+    const int t0        = WIDE ? (int)threadIdx.x : lane;
+    const int stride    = WIDE ? NW * 32 : 32;
+    const int64_t q0    = WIDE ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * NW + wid;
+    const int64_t qstep = WIDE ? (int64_t)gridDim.x : (int64_t)gridDim.x * NW;
+    const int own       = WIDE ? 0 : wid;
+    const auto make_table = [&]() {
+        // w = c x_i (1 -+ x_j) for r = 0 and c (1 -+ x_j) / x_i for r = 1
+        // (m1_opacities.hpp:880-905), c = 2 x 2.182
+        constexpr double c = 2. * k::TempMultiple;
+        for (int k = threadIdx.x; k < nit; k += blockDim.x)
+        {
+            const int it  = L.nes_order[k];
+            const int r   = it >= nn2;
+            const int rem = it - r * nn2;
+            const int i = rem / n2, j = rem - (rem / n2) * n2;
+            const double xi = L.x2[i], xj = L.x2[j];
+            const double w  = r ? c * (1. - xj) / xi : c * xi * (1. - xj);
+            const double wp = r ? c * (1. + xj) / xi : c * xi * (1. + xj);
+            const double e1 = -expm1(-(wp - w)); // 1 - e
+            const double m  = 24. * ((r ? L.wx3[i] : L.wx[i]) * L.w2[j]);
+            S.w[k]   = w;
+            S.wp[k]  = wp;
+            S.m[k]   = m;
+            S.ka[k]  = m * ((1. - e1) / e1);
+            S.wc[k]  = fx::pow(w, k::CF);
+            S.wpc[k] = fx::pow(wp, k::CF);
+        }
+    };
+    bool table = !WIDE;
+    if (!WIDE)
+    {
+        make_table();
+        __syncthreads();
+    }
+    for (int64_t q = q0; q < np; q += qstep)
+    {
+        const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
+        PointTab* P     = (PointTab*)(scratch + q * kTabWords);
+        if (WIDE && flagged && P->neps_fp64 != 2.)
+            continue; // uniform: a point per CTA
+        if (!table)
+        {
+            make_table(); // before the point's first barrier below
+            table = true;
+        }
+        const double T = L.eos[1][p], mu_e = L.eos[7][p];
+        if (WIDE)
+            __syncthreads(); // the previous point's readers are done
+        else
+            __syncwarp();
+        if (!WIDE || wid == 0)
+        {
+            if (lane < 4)
+                occ64_from(P->d, lane, T, &S.occ[own][lane]);
+            else if (lane >= 16 && lane < 28)
+                (&S.fe[own][0][0])[lane - 16] = (&P->fe[0][0])[lane - 16];
+            else if (lane >= 28 && lane < 30)
+                S.fd0[own][lane - 28] = P->fd0[lane - 28];
+        }
+        if (WIDE)
+            __syncthreads();
+        else
+            __syncwarp();
+        const Occ64* occ  = S.occ[own];
+        const bool common = occ[0].cf == k::CF && occ[1].cf == k::CF && occ[2].cf == k::CF &&
+                            occ[3].cf == k::CF;
+        NepsPoint NP;
+        NP.T    = T;
+        NP.pre  = k::NepsConst * (T * T);
+        NP.eta0 = mu_e / T;
+        NP.eta1 = -mu_e / T;
+        NP.fd00 = S.fd0[own][0];
+        NP.fd01 = S.fd0[own][1];
+        NP.fe0  = S.fe[own][0];
+        NP.fe1  = S.fe[own][1];
+        double acc[16];
+#pragma unroll
+        for (int kk = 0; kk < 16; ++kk)
+            acc[kk] = 0.;
+#pragma unroll 1
+        for (int it = t0; it < nit; it += stride)
+        {
+            const double w = S.w[it], wp = S.wp[it];
+            const double dl = wp - w, sm = w + wp, pr = w * wp;
+            const double hs = 0.5 * sm, hp = 0.5 * pr, qp = hp * hp; // qp = P^2 / 4
+            const double hx = 0.5 * wp, hy = 0.5 * w;
+            double U = 0., V = 0.; // A of e- + B of e+, B of e- + A of e+
+            double ct[4] = {0., 0., 0., 0.};
+#pragma unroll 1
+            for (int e = 0; e < 2; ++e)
+            {
+                const double eta = e ? NP.eta1 : NP.eta0;
+                const double* fe = S.fe[own][e];
+                if (w > eta * 1e-3)
+                {
+                    double a[5], b[5], f[3];
+                    fx::fd_orders<1, 5, true>(eta - wp, a);
+                    fx::fd_orders<1, 5, true>(eta - w, b);
+                    fx::fd_orders<3, 5, true>(eta - dl, f);
+                    const double E3 = fma(fe[3], 1. / 6., -f[0]);
+                    const double E4 = fma(fe[4], 1. / 24., -f[1]);
+                    const double ED = fma(fe[5], 1. / 120., -f[2]) + (a[4] - b[4]);
+                    double A = fma(wp, fma(hx, E3, E4), ED);
+                    A        = fma(sm, fma(hp, a[1] - b[1], fma(hs, a[2] - b[2], a[3] - b[3])), A);
+                    A        = fma(qp, a[0] - b[0], A);
+                    const double B = fma(w, fma(hy, E3, -E4), ED);
+                    U += e ? B : A;
+                    V += e ? A : B;
+                }
+                else
+                {
+                    // the reference's Taylor branches (kernel_nes.hpp:82-132)
+                    double r1[4], r2[4];
+                    neps_taylor(NP, e, w, wp, wp, w, -1, 1, r1, r2);
+#pragma unroll
+                    for (int s = 0; s < 4; ++s)
+                        ct[s] = fma(r1[s], qp * (-1. / 6.), ct[s]);
+                }
+            }
+            constexpr double bp = k::NepsBPlus, bm = k::NepsBMinus, bz = k::NepsBZero;
+            const double c[4] = {fma(bp, U, fma(bz, V, ct[0])), fma(bp, V, fma(bz, U, ct[1])),
+                                 fma(bm, U, fma(bz, V, ct[2])), fma(bm, V, fma(bz, U, ct[3]))};
+            double g[4], gb[4];
+            occ64_eval(occ, w, S.wc[it], common, g);
+            occ64_eval(occ, wp, S.wpc[it], common, gb);
+            const double ka = S.ka[it], kb = ka + S.m[it];
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+            {
+                // emission and absorption kernels nu -> nubar; nubar -> nu swaps them
+                const double ke = kb * c[s], kk = ka * c[s];
+                const double e1 = ke * gb[s], e2 = kk * g[s];
+                const double a1 = nbb ? kk : kk * (1. - gb[s]);
+                const double a2 = nbb ? ke : ke * (1. - g[s]);
+                double EM1, AB1, EM2, AB2;
+                if (stim)
+                {
+                    AB1 = g[s] * (e1 + a1);
+                    EM1 = e1;
+                    AB2 = gb[s] * (e2 + a2);
+                    EM2 = e2;
+                }
+                else
+                {
+                    AB1 = g[s] * a1;
+                    EM1 = (1. - g[s]) * e1;
+                    AB2 = gb[s] * a2;
+                    EM2 = (1. - gb[s]) * e2;
+                }
+                acc[s] += EM1 + EM2;
+                acc[4 + s] += AB1 + AB2;
+                acc[8 + s]  = fma(w, EM1, fma(wp, EM2, acc[8 + s]));
+                acc[12 + s] = fma(w, AB1, fma(wp, AB2, acc[12 + s]));
+            }
+        }
+        const double T4   = (T * T) * (T * T);
+        double tot        = warp_sum16(acc, lane);
+        const int idx     = sum_index(lane);
+        const double unit = NP.pre * T4 * (idx >= 8 ? T : 1.);
+        if (!WIDE)
+        {
+            if (!(lane & 1))
+                P->snes[idx] = tot * unit;
+        }
+        else
+        {
+            if (!(lane & 1))
+                S.red[wid][idx] = tot;
+            __syncthreads();
+            if (wid == 0 && !(lane & 1))
+            {
+                double t = 0.;
+                for (int v = 0; v < NW; ++v)
+                    t += S.red[v][idx];
+                P->snes[idx] = t * unit;
+            }
         }
     }
 }
@@ -2426,6 +2614,33 @@ cudaError_t launch_nes_fast(const Step& S, cudaStream_t st, int sms)
     return cudaGetLastError();
 }
 
+// Launches of fewer points run a point per CTA where the kernel has that form.
+constexpr int64_t kWidePoints = 1024;
+
+template <bool WIDE, bool MULTI>
+cudaError_t launch_nes64(const Step& S, cudaStream_t st, int sms, int flagged)
+{
+    constexpr int NW      = nes64_warps<WIDE>();
+    constexpr int smem    = (int)sizeof(Nes64Smem<NW>);
+    const auto kernel     = grey_nes64_kernel<WIDE, MULTI>;
+    const cudaError_t e   = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 smem);
+    if (e != cudaSuccess)
+        return e;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NW * 32, smem) !=
+            cudaSuccess ||
+        per_sm < 1)
+        per_sm = 1;
+    const int64_t work = WIDE ? S.np : (S.np + NW - 1) / NW;
+    int64_t cap        = (int64_t)((double)sms * per_sm * g_grid_scale);
+    cap                = cap < 1 ? 1 : cap;
+    const int grid     = (int)(work < cap ? (work > 0 ? work : 1) : cap);
+    kernel<<<dim3(grid, 1, MULTI ? S.G : 1), NW * 32, smem, st>>>(*S.L, S.GA, S.p0, S.np, S.ws,
+                                                                  flagged);
+    return cudaGetLastError();
+}
+
 template <bool MIXED, int IMPL, bool WIDE, bool MULTI>
 void launch_brem_impl(const Step& S, cudaStream_t st, int sms, int add, int redo_only)
 {
@@ -2524,25 +2739,23 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
                 return err;
             phase_mark(kPhNeps, 1, st);
             phase_mark(kPhNepsAccurate, 0, st);
-            constexpr int wa = nes_warps<kNesAccurate>() * 32;
-            grey_neps_kernel<kNesAccurate, MULTI>
-                <<<dim3(grid_for(grey_neps_kernel<kNesAccurate, MULTI>, wa, np, sms), 1, gz), wa,
-                   0, st>>>(L, S.GA, S.p0, np, S.ws);
+            constexpr int wa = kNesAccWarps * 32;
+            grey_neps_kernel<MULTI>
+                <<<dim3(grid_for(grey_neps_kernel<MULTI>, wa, np, sms), 1, gz), wa, 0, st>>>(
+                    L, S.GA, S.p0, np, S.ws);
             phase_mark(kPhNepsAccurate, 1, st);
             phase_mark(kPhNepsFp64, 0, st);
-            constexpr int wf = nes_warps<kNesFp64Flag>() * 32;
-            grey_neps_kernel<kNesFp64Flag, MULTI>
-                <<<dim3(grid_for(grey_neps_kernel<kNesFp64Flag, MULTI>, wf, np, sms), 1, gz), wf,
-                   0, st>>>(L, S.GA, S.p0, np, S.ws);
+            if ((err = launch_nes64<true, MULTI>(S, st, sms, 1)) != cudaSuccess)
+                return err;
             phase_mark(kPhNepsFp64, 1, st);
         }
         else
         {
             phase_mark(kPhNeps, 0, st);
-            grey_neps_kernel<kNesFp64All, MULTI>
-                <<<dim3(grid_for(grey_neps_kernel<kNesFp64All, MULTI>, kWarps * 32, wb, sms), 1,
-                        gz),
-                   kWarps * 32, 0, st>>>(L, S.GA, S.p0, np, S.ws);
+            err = np < kWidePoints ? launch_nes64<true, MULTI>(S, st, sms, 0)
+                                   : launch_nes64<false, MULTI>(S, st, sms, 0);
+            if (err != cudaSuccess)
+                return err;
             phase_mark(kPhNeps, 1, st);
         }
     }
