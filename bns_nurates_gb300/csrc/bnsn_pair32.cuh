@@ -317,6 +317,28 @@ __device__ __forceinline__ bool make_cell(double y, double z, double eta, Cell& 
     return true;
 }
 
+// The absorption kernels of one cell before the species' couplings, times
+// (nu nubar)^2: k0 = sc Psi_0(y, z) e^s / (1 - e^s) 15 y^2 z^2 and k1 the same
+// with y and z exchanged, from the FP32 integral.  eh = e^{y - |eta| / 2} of
+// each side (e^{Lref} = eh_y eh_z where Lref != 0); sc = (Phi T^2 / 2) T^4 / 15,
+// the point's factor.
+__device__ __forceinline__ void absorption_q(dfm::df Y, dfm::df Z, double ehy, double ehz,
+                                             dfm::df ETA, double sc, double* k0, double* k1)
+{
+    Cell c;
+    int lcase;
+    if (!make_cell(Y, Z, ETA, c, lcase))
+    {
+        *k0 = *k1 = 0.;
+        return;
+    }
+    double Q0, Q1;
+    cell_integrals(c, Q0, Q1);
+    const double f = lcase == kLrefZero ? sc : sc * (ehy * ehz);
+    *k0 = f * Q0;
+    *k1 = f * Q1;
+}
+
 // The pair kernel of one cell for the four species: em and ab of
 // kernel_pair.hpp:135-198 times (nu nubar)^2, from the FP32 integral:
 // ab = (Phi T^2 / 2) alpha . (Psi / (1 - e^s)) e^{s}, em = ab / SafeExp(s).

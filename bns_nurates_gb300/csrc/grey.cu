@@ -111,6 +111,29 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
+// Sums the 16 values of the warp's lanes: lane l returns the total of value
+// sum_index(l).  Each round halves the values a lane carries, 16 additions in
+// all instead of 80 for 16 butterfly sums.
+__device__ __forceinline__ double warp_sum16(double* v, int lane)
+{
+#pragma unroll
+    for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1)
+    {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < n; ++k)
+        {
+            const double mine = up ? v[k + n] : v[k], theirs = up ? v[k] : v[k + n];
+            v[k] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+__device__ __forceinline__ int sum_index(int lane)
+{
+    return ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+}
+
 __device__ __forceinline__ double total_nu_f1(double omega, const Distr& d, int s)
 {
     const double ft = fermi_distr(omega, d.temp_t[s], d.temp_t[s] * d.eta_t[s]);
@@ -785,72 +808,230 @@ __device__ __forceinline__ void fill_tab32(CellTab32& D, const CellTab& C, int M
     }
 }
 
-// Weight algebra of add_cell for the mixed pair cells, with w4 = 1 (the
-// caller folds (nu nubar)^2 into the kernel) and the emission terms'
-// magnitudes: the pair kernels are non-negative and so are the absorption
-// terms (em + am = em (1 + g (e^s - 1)) >= 0), so only the emission terms,
-// through 1 - g < 0, can carry the opposite sign.
-template <bool STIM>
-__device__ __forceinline__ void add_cell_pair(double* acc, double* magem, const double* Kem,
-                                              const double* Kab, const double* ga,
-                                              const double* gb, bool nb_block, double W1,
-                                              double W2)
+// ---------------------------------------------------------------------------
+// Cell phases with row sums.  A symmetric pair of cells (a, b), (b, a) costs one
+// kernel evaluation; its weighting into the 16 moments of m1_opacities.hpp:577-758
+// took ~100 FP64 operations per pair, more than the kernel itself.  The moments
+// are bilinear in node vectors, so the phase first stores the absorption kernel
+// K(a, b) of all cells in shared memory and then sums rows:
+//   F_a = dn_a sum_b K(a, b) dn_b q_b (1 - g_b)   (emission: K e^{-(y_a + y_b)}),
+//   G_a = sum_b K(a, b) q_b g_b,
+// per partner species, after which a row adds q_a F_a, q_a g_a (F_a + G_a) and
+// the same with the energy weight: 8 operations per directed cell (16 where
+// K(b, a) != K(a, b)) and ~45 per row.  Two warps share a point (64 threads: 13
+// and 4 rounds of cells at n = 20 and 10, 12 to 25 KB of shared memory per
+// point).
+// ---------------------------------------------------------------------------
+constexpr int kCellThreads = 64;
+
+struct CellNodes
 {
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
+    double K[kMaxM][kMaxM + 1];        // absorption kernel of (row, column)
+    double vE[kMaxM][4], vA[kMaxM][4]; // q dn (1 - g), q g
+    double g[kMaxM][4];
+    double q[kMaxM], qe[kMaxM]; // number and energy weights of a node
+    double dn[kMaxM];           // e^{-y}
+    double nu[kMaxM], y[kMaxM];
+    double red[2][2][16];
+    double A1[kMaxM], A2[kMaxM];
+    uint16_t cells[kMaxCells]; // a | b << 8
+    int splits;                // column ranges a row is cut into
+};
+
+// Launch constants of the CTA, and the column split: rows x splits tasks of
+// (M / splits) columns over the CTA's threads, chosen for the fewest rounds x
+// (columns x products + the row's epilogue).
+template <bool SYM>
+__device__ __forceinline__ void cell_constants(CellNodes& C, const OpacityLaunch& L)
+{
+    const int M = 2 * L.n2;
+    for (int k = threadIdx.x; k < kMaxM; k += kCellThreads)
     {
-        const int ps    = s ^ 1;
-        const double bf = nb_block ? 1. : 1. - gb[ps];
-        const double em = Kem[s] * bf;
-        const double am = Kab[s] * gb[ps];
-        double EM, AB, EMA;
-        if (STIM)
+        C.A1[k] = L.A1[k];
+        C.A2[k] = L.A2[k];
+    }
+    for (int k = threadIdx.x; k < L.ncell; k += kCellThreads)
+    {
+        const uint32_t ab = L.cells[k];
+        C.cells[k]        = (uint16_t)((ab & 0xffu) | ((ab >> 16) << 8));
+    }
+    if (threadIdx.x == 0)
+    {
+        int best = 1, cost = 1 << 30;
+        for (int h = 1; h <= 8 && h <= M; ++h)
         {
-            AB  = ga[s] * (em + am);
-            EM  = em;
-            EMA = Kem[s] * fabs(bf);
+            const int c = ((M * h + kCellThreads - 1) / kCellThreads) *
+                          (((M + h - 1) / h) * (SYM ? 8 : 16) + 45);
+            if (c < cost)
+            {
+                cost = c;
+                best = h;
+            }
         }
-        else
-        {
-            AB  = am * ga[s];
-            EM  = em * (1. - ga[s]);
-            EMA = Kem[s] * fabs(bf) * fabs(1. - ga[s]);
-        }
-        acc[s] += EM * W1;
-        acc[4 + s] += AB * W1;
-        acc[8 + s] += EM * W2;
-        acc[12 + s] += AB * W2;
-        magem[s] += EMA * W1;
-        magem[4 + s] += EMA * W2;
+        C.splits = best;
     }
 }
 
-// Per-warp node tables of the mixed pair phase: y = nu/T as double-float,
-// e^{y - |eta|/2} (e^{Lref} = its product over the two nodes when |eta| >= s)
-// and e^{-y} (e^{-s} = the product when s <= 700).
+// Node data of a point; nu2: the weights carry nu^2 (kernels without it).
+__device__ __forceinline__ bool cell_nodes(CellNodes& C, const PointTab* __restrict__ P, int M,
+                                           bool nbb, bool nu2)
+{
+    bool above = false; // an occupation above 1
+    const int a = threadIdx.x;
+    if (a < M)
+    {
+        const double nu = P->nu[a], y = P->y[a];
+        const double w  = nu2 ? nu * nu : 1.;
+        const double q  = C.A1[a] * w;
+        const double dn = fx::exp(-y);
+        C.nu[a] = nu;
+        C.y[a]  = y;
+        C.q[a]  = q;
+        C.qe[a] = C.A2[a] * w;
+        C.dn[a] = dn;
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+        {
+            const double g = P->g[a][s];
+            above          = above || g > 1.;
+            C.g[a][s]      = g;
+            C.vA[a][s]     = q * g;
+            C.vE[a][s]     = q * dn * (nbb ? 1. : 1. - g);
+        }
+    }
+    return above;
+}
+
+// Adds the rows' contributions of this thread to the 16 moments.  The kernel of
+// species 0 (2) at (a, b) is e0 K(a, b) + e1 K(b, a) (x0, x1); species 1 and 3
+// exchange K(a, b) and K(b, a) (kernel_pair.hpp:200-216).  SYM: one symmetric
+// kernel for all species.  ABS: sums of |term| of the emission moments alone.
+template <bool SYM, bool ABS>
+__device__ __forceinline__ void cell_row_sums(const CellNodes& C, int M, bool stim, double e0,
+                                              double e1, double x0, double x1, double* acc)
+{
+    const int h = C.splits;
+    for (int t = threadIdx.x; t < M * h; t += kCellThreads)
+    {
+        const int part = t / M, a = t - part * M;
+        const int b0 = part * M / h, b1 = (part + 1) * M / h;
+        double F[2][4], G[2][4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            F[0][s] = F[1][s] = G[0][s] = G[1][s] = 0.;
+        for (int b = b0; b < b1; ++b)
+        {
+            const double k = C.K[a][b];
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+            {
+                const double v = ABS ? fabs(C.vE[b][s]) : C.vE[b][s];
+                F[0][s]        = fma(k, v, F[0][s]);
+                if (!ABS)
+                    G[0][s] = fma(k, C.vA[b][s], G[0][s]);
+            }
+            if (!SYM)
+            {
+                const double kt = C.K[b][a];
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                {
+                    const double v = ABS ? fabs(C.vE[b][s]) : C.vE[b][s];
+                    F[1][s]        = fma(kt, v, F[1][s]);
+                    if (!ABS)
+                        G[1][s] = fma(kt, C.vA[b][s], G[1][s]);
+                }
+            }
+        }
+        const double q = C.q[a], qe = C.qe[a], dn = C.dn[a];
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+        {
+            const int ps    = s ^ 1, o = s & 1;
+            const double c0 = s < 2 ? e0 : x0, c1 = s < 2 ? e1 : x1;
+            const double Fs = dn * (SYM ? F[0][ps] : fma(c0, F[o][ps], c1 * F[1 - o][ps]));
+            const double g  = C.g[a][s];
+            if (ABS)
+            {
+                const double m = stim ? Fs : fabs(1. - g) * Fs;
+                acc[s]     = fma(q, m, acc[s]);
+                acc[8 + s] = fma(qe, m, acc[8 + s]);
+                continue;
+            }
+            const double Gs = SYM ? G[0][ps] : fma(c0, G[o][ps], c1 * G[1 - o][ps]);
+            const double em = stim ? Fs : (1. - g) * Fs;
+            const double ab = g * (stim ? Fs + Gs : Gs);
+            acc[s]      = fma(q, em, acc[s]);
+            acc[4 + s]  = fma(q, ab, acc[4 + s]);
+            acc[8 + s]  = fma(qe, em, acc[8 + s]);
+            acc[12 + s] = fma(qe, ab, acc[12 + s]);
+        }
+    }
+}
+
+// Totals of the CTA's two warps: lane l of warp 0 holds that of moment
+// sum_index(l).
+__device__ __forceinline__ double cell_total(CellNodes& C, double* acc, int slot)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const double v = warp_sum16(acc, lane);
+    if (!(lane & 1))
+        C.red[slot][wid][sum_index(lane)] = v;
+    __syncthreads();
+    return C.red[slot][0][sum_index(lane)] + C.red[slot][1][sum_index(lane)];
+}
+
+// Node tables of the mixed pair phase: y = nu/T as double-float and
+// e^{y - |eta|/2} (e^{Lref} = its product over the two nodes when |eta| >= s).
 struct PairTab32
 {
     float yh[kMaxM], yl[kMaxM];
-    double eh[kMaxM], dn[kMaxM];
+    double eh[kMaxM];
 };
 
-// Pair cell (a, b) of the mixed path from the per-warp node tables
-// (pair32::kernel_q).
-__device__ __forceinline__ void pair_kernel_q(const PairTab32& X, int a, int b, dfm::df ETA,
-                                              double sc, double* em, double* ab)
+// Fermi integrals of the FP64 pair kernel at the nodes, scaled as Psi needs
+// them: 120 F_1, 120 F_2, 40 F_3, 20 F_4, 4 F_5 at eta -+ y; 1 / y^2.
+struct PairTab64
 {
-    pair32::kernel_q(dfm::df{X.yh[a], X.yl[a]}, dfm::df{X.yh[b], X.yl[b]}, X.eh[a], X.eh[b],
-                     X.dn[a], X.dn[b], ETA, sc, em, ab);
+    double m[kMaxM][5], p[kMaxM][5], iy2[kMaxM];
+};
+
+// 15 y^2 z^2 Psi_0(y, z) and Psi_0(z, y) (kernel_pair.hpp:16-120) of nodes a, b, the
+// sums in the reference's order: they cancel, and another order of c10 alone moves
+// ill-conditioned outputs by more than the reference's own rounding does.
+__device__ __forceinline__ void pair_psi_nodes(const PairTab64& W, int a, int b, double eta,
+                                               double y, double z, double f40, double f20,
+                                               double* p0, double* p1)
+{
+    double fm[3], fp[3];
+    fdi_orders<3, 5>(eta - y - z, fm);
+    fdi_orders<3, 5>(eta + y + z, fp);
+    const double *am = W.m[a], *ap = W.p[a], *bm = W.m[b], *bp = W.p[b];
+    const double c5 = fma(40., fm[0], -f40), c7 = fma(20., fm[1], -f20);
+    const double c8 = fma(-40., fp[0], f40), c9 = fma(20., fp[1], -f20);
+    const double c10 = fma(-4., fp[2], fma(4., fm[2], -am[4]) - bm[4] + ap[4]) + bp[4];
+    const double d01 = bp[3] - am[3], c2 = am[1] - bp[1], c3 = bp[2] - am[2];
+    const double d11 = bm[3] - ap[3], c14 = bm[1] - ap[1], c13 = ap[2] - bm[2];
+    const double u0 = fma(z, fma(z, bp[0] - am[0], c2), c3 + c5);
+    const double v0 = fma(z, fma(-c2, z, -2. * c3), fma(y, u0, d01 + c7));
+    *p0 = fma(z, fma(z, c3 + c8, c9 - d01), fma(y, v0, c10));
+    const double u1 = fma(y, fma(y, ap[0] - bm[0], c14), c13 + c5);
+    const double v1 = fma(z, u1, fma(y, fma(-c14, y, -2. * c13), c7 - d11));
+    *p1 = fma(z, v1, fma(y, fma(y, c13 + c8, d11 + c9), c10));
 }
 
-// MIXED: pair cells from the FP32 integral; the sums, their magnitudes and
-// s2d are written to the record (PairMixed).  !MIXED: the FP64 pair kernel
-// (kernel_pair.hpp), with redo_only the mixed path's second pass over the
-// points the final kernel marked (predo), whose pair part of s2d it replaces;
-// that pass computes its Fermi-integral tables itself.  WIDE (that pass):
-// a point per CTA, its cells over all threads (the marked points are few).
-template <bool MIXED, bool WIDE = false, bool MULTI = false>
-__global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
+// e+e- pair phase.  MIXED: cells from the FP32 integral (bnsn_pair32.cuh); the
+// sums and the magnitudes of their terms are written to the record (PairMixed).
+// The pair kernels are non-negative and so are the absorption terms (em + am =
+// em (1 + g (e^s - 1)) >= 0), so only the emission terms, through 1 - g < 0, can
+// carry the opposite sign.  !MIXED: the FP64 kernel (kernel_pair.hpp); with
+// redo_only the mixed path's second pass over the points the final kernel
+// marked (predo), whose pair part of s2d it replaces; that pass computes its
+// Fermi-integral tables itself.
+// 8,192 points, n = 20: FP64 2.95 -> 1.35 ms, mixed with its redo pass 2.46 ->
+// 1.52 ms; one point, n = 10: 74 -> 29 us.
+template <bool MIXED, bool MULTI = false>
+__global__ void __launch_bounds__(kCellThreads)
     grey_pair_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
                      int64_t np, double* __restrict__ scratch, int redo_only)
 {
@@ -864,178 +1045,132 @@ __global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
     }
     if (MULTI && !L.use_pair)
         return; // a group without pair (uniform over the CTA)
-    constexpr int NW = WIDE ? 8 : kWarps;
-    __shared__ double s_A1[kMaxM], s_A2[kMaxM];
-    __shared__ uint32_t s_cells[kMaxCells];
-    __shared__ CellTab s_ct[WIDE ? 1 : kWarps];
-    __shared__ PairTab32 s_pt[MIXED ? kWarps : 1];
-    __shared__ double s_red[WIDE ? NW : 1][32];
-    for (int k = threadIdx.x; k < kMaxM; k += blockDim.x)
-    {
-        s_A1[k]  = L.A1[k];
-        s_A2[k]  = L.A2[k];
-    }
-    for (int k = threadIdx.x; k < L.ncell; k += blockDim.x)
-        s_cells[k] = L.cells[k];
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int wid  = threadIdx.x >> 5;
-    CellTab& C     = s_ct[WIDE ? 0 : wid];
-    PairTab32& X   = s_pt[MIXED ? wid : 0];
-    const int M    = 2 * L.n2;
-    const bool nbb = L.neglect_blocking != 0;
-    // cells of a point: thread t0, t0 + stride, ...
-    const int t0        = WIDE ? (int)threadIdx.x : lane;
-    const int stride    = WIDE ? NW * 32 : 32;
-    const int64_t q0    = WIDE ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * NW + wid;
-    const int64_t qstep = WIDE ? (int64_t)gridDim.x : (int64_t)gridDim.x * NW;
+    __shared__ CellNodes C;
+    __shared__ PairTab32 X;
+    __shared__ PairTab64 W;
+    const int M     = 2 * L.n2;
+    const int ncell = L.ncell;
+    const bool nbb = L.neglect_blocking != 0, stim = L.stim != 0;
+    bool ready = false; // launch constants staged
 
-    for (int64_t q = q0; q < np; q += qstep)
+    for (int64_t q = blockIdx.x; q < np; q += gridDim.x)
     {
-        const int64_t p  = L.pidx ? L.pidx[p0 + q] : p0 + q;
-        PointTab* P      = (PointTab*)(scratch + q * kTabWords);
+        const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
+        PointTab* P     = (PointTab*)(scratch + q * kTabWords);
         if (!MIXED && redo_only && pair_mixed(P)->predo != 1.)
-            continue;
+            continue; // uniform: a point per CTA
+        if (!ready)
+        {
+            cell_constants<false>(C, L);
+            ready = true;
+        }
         const double T   = L.eos[1][p];
         const double eta = L.eos[7][p] / T;
-        if (WIDE)
-            __syncthreads(); // the previous point's readers are done
-        else
-            __syncwarp();
-        if (!WIDE || wid == 0)
-            load_cell_tab(C, P, M, !MIXED && !redo_only, lane);
-        if (WIDE)
-            __syncthreads();
-        if (MIXED)
+        __syncthreads(); // the previous point's readers are done
+        const bool above = __syncthreads_or(cell_nodes(C, P, M, nbb, !MIXED));
+        const int a0 = threadIdx.x;
+        if (a0 < M)
         {
-            __syncwarp();
-            for (int a = lane; a < M; a += 32)
+            const double y = C.y[a0];
+            if (MIXED)
             {
-                const double y = C.y[a];
                 const dfm::df yd = dfm::from_double(y);
-                X.yh[a] = yd.hi;
-                X.yl[a] = yd.lo;
-                X.eh[a] = fx::exp(y - 0.5 * fabs(eta));
-                X.dn[a] = fx::exp(-y);
+                X.yh[a0] = yd.hi;
+                X.yl[a0] = yd.lo;
+                X.eh[a0] = fx::exp(y - 0.5 * fabs(eta));
             }
+            else
+                W.iy2[a0] = 1. / (y * y);
         }
-        if (!MIXED && redo_only)
+        if (!MIXED)
         {
-            // the F_1..F_5 tables the mixed prelude left out
-            for (int qq = t0; qq < 2 * M; qq += stride)
+            for (int qq = threadIdx.x; qq < 2 * M; qq += kCellThreads)
             {
                 const int a = qq >> 1;
-                if (qq & 1)
-                    fdi_orders<1, 5>(eta + C.y[a], C.fp[a]);
+                double f[5];
+                if (redo_only) // the tables the mixed prelude left out
+                    fdi_orders<1, 5>(qq & 1 ? eta + C.y[a] : eta - C.y[a], f);
                 else
-                    fdi_orders<1, 5>(eta - C.y[a], C.fm[a]);
+                {
+#pragma unroll
+                    for (int k = 0; k < 5; ++k)
+                        f[k] = qq & 1 ? P->fp[a][k] : P->fm[a][k];
+                }
+                double* o = qq & 1 ? W.p[a] : W.m[a];
+                o[0] = 120. * f[0];
+                o[1] = 120. * f[1];
+                o[2] = 40. * f[2];
+                o[3] = 20. * f[3];
+                o[4] = 4. * f[4];
             }
         }
-        if (WIDE)
-            __syncthreads();
-        else
-            __syncwarp();
-        double acc[16], magem[MIXED ? 8 : 1];
+        __syncthreads();
+        const dfm::df ETA = dfm::from_double(eta);
+        const double T2   = T * T;
+        const double f40 = 40. * P->fe[0][3], f20 = 20. * P->fe[0][4];
+        // em = Phi T^2 / 2 (alpha1^2 Psi(y, z) + alpha2^2 Psi(z, y)) / (1 - e^s), ab = e^s em
+        const double sc = MIXED ? 0.5 * k::PairPhi * T2 * (T2 * T2) / 15.
+                                : -0.5 * k::PairPhi * T2 / 15.;
+        for (int c = threadIdx.x; c < ncell; c += kCellThreads)
+        {
+            const uint32_t ab = C.cells[c];
+            const int a = ab & 0xffu, b = ab >> 8;
+            double k0 = 0., k1 = 0.;
+            if (MIXED)
+                pair32::absorption_q(dfm::df{X.yh[a], X.yl[a]}, dfm::df{X.yh[b], X.yl[b]},
+                                     X.eh[a], X.eh[b], ETA, sc, &k0, &k1);
+            else
+            {
+                const double y = C.y[a], z = C.y[b];
+                if (!(eta - y - z > 200.))
+                {
+                    pair_psi_nodes(W, a, b, eta, y, z, f40, f20, &k0, &k1);
+                    const double f =
+                        sc * (W.iy2[a] * W.iy2[b]) * fx::rcp(1. - C.dn[a] * C.dn[b]);
+                    k0 *= f;
+                    k1 *= f;
+                }
+            }
+            C.K[a][b] = k0;
+            if (a != b)
+                C.K[b][a] = k1;
+        }
+        __syncthreads();
+        constexpr double e0 = k::PairA1e * k::PairA1e, e1 = k::PairA2e * k::PairA2e;
+        constexpr double x0 = k::PairA1x * k::PairA1x, x1 = k::PairA2x * k::PairA2x;
+        double acc[16];
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk)
             acc[kk] = 0.;
-#pragma unroll
-        for (int kk = 0; kk < (MIXED ? 8 : 1); ++kk)
-            magem[kk] = 0.;
-        const dfm::df ETA = dfm::from_double(eta);
-        const double T2 = T * T;
-        const double scq = 0.5 * k::PairPhi * T2 * (T2 * T2) / 15.;
-        for (int c = t0; c < L.ncell; c += stride)
-        {
-            const uint32_t ab = s_cells[c];
-            const int a = ab & 0xffffu, b = ab >> 16;
-            const double nua = C.nu[a], nub = C.nu[b];
-            double pe[4], pa[4];
-            if (MIXED)
-                pair_kernel_q(X, a, b, ETA, scq, pe, pa);
-            else
-                pair_kernel(T, eta, nua, nub, C.y[a], C.y[b], C.fm[a], C.fp[a], C.fm[b],
-                            C.fp[b], C.f3e, C.f4e, pe, pa);
-            const double w4 = (nua * nua) * (nub * nub);
-            const double W1 = s_A1[a] * s_A1[b];
-            // (b, a): the inverse kernel swaps partner species (kernel_pair.hpp:200-216)
-            const double qe[4] = {pe[1], pe[0], pe[3], pe[2]};
-            const double qa[4] = {pa[1], pa[0], pa[3], pa[2]};
-            if (MIXED)
-            {
-                if (L.stim)
-                    add_cell_pair<true>(acc, magem, pe, pa, C.g[a], C.g[b], nbb, W1,
-                                        s_A2[a] * s_A1[b]);
-                else
-                    add_cell_pair<false>(acc, magem, pe, pa, C.g[a], C.g[b], nbb, W1,
-                                         s_A2[a] * s_A1[b]);
-                if (a != b)
-                {
-                    if (L.stim)
-                        add_cell_pair<true>(acc, magem, qe, qa, C.g[b], C.g[a], nbb, W1,
-                                            s_A2[b] * s_A1[a]);
-                    else
-                        add_cell_pair<false>(acc, magem, qe, qa, C.g[b], C.g[a], nbb, W1,
-                                             s_A2[b] * s_A1[a]);
-                }
-            }
-            else
-            {
-                if (L.stim)
-                    add_cell<true>(acc, pe, pa, C.g[a], C.g[b], nbb, w4, W1, s_A2[a] * s_A1[b]);
-                else
-                    add_cell<false>(acc, pe, pa, C.g[a], C.g[b], nbb, w4, W1, s_A2[a] * s_A1[b]);
-                if (a != b)
-                {
-                    if (L.stim)
-                        add_cell<true>(acc, qe, qa, C.g[b], C.g[a], nbb, w4, W1,
-                                       s_A2[b] * s_A1[a]);
-                    else
-                        add_cell<false>(acc, qe, qa, C.g[b], C.g[a], nbb, w4, W1,
-                                        s_A2[b] * s_A1[a]);
-                }
-            }
-        }
-        double magd[16];
-        if (WIDE)
-            block_sum<NW>(acc, s_red, 0);
-        else
+        cell_row_sums<false, false>(C, M, stim, e0, e1, x0, x1, acc);
+        const double tot = cell_total(C, acc, 0);
+        double mag       = fabs(tot);
+        if (MIXED && above)
         {
 #pragma unroll
             for (int kk = 0; kk < 16; ++kk)
-                acc[kk] = warp_sum(acc[kk]);
+                acc[kk] = 0.;
+            cell_row_sums<false, true>(C, M, stim, e0, e1, x0, x1, acc);
+            const double m = cell_total(C, acc, 1);
+            if (!(sum_index(threadIdx.x & 31) & 4))
+                mag = m;
         }
-        if (MIXED)
+        if (threadIdx.x < 32 && !(threadIdx.x & 1))
         {
-            // emission moments: sum of |term|; absorption terms are non-negative
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                magd[s]      = warp_sum(magem[s]);
-                magd[8 + s]  = warp_sum(magem[4 + s]);
-                magd[4 + s]  = fabs(acc[4 + s]);
-                magd[12 + s] = fabs(acc[12 + s]);
-            }
-        }
-        if (WIDE ? threadIdx.x == 0 : lane == 0)
-        {
-            PairMixed* X = pair_mixed(P);
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
-            {
-                if (MIXED)
-                {
-                    P->s2d[kk]   = acc[kk];
-                    X->spair[kk] = acc[kk];
-                    X->pmag[kk]  = magd[kk];
-                }
-                else if (redo_only)
-                    P->s2d[kk] = P->s2d[kk] - X->spair[kk] + acc[kk];
-                else
-                    P->s2d[kk] = acc[kk];
-            }
+            PairMixed* Y  = pair_mixed(P);
+            const int idx = sum_index(threadIdx.x);
             if (MIXED)
-                X->predo = 0.;
+            {
+                P->s2d[idx]   = tot;
+                Y->spair[idx] = tot;
+                Y->pmag[idx]  = mag;
+            }
+            else if (redo_only)
+                P->s2d[idx] = P->s2d[idx] - Y->spair[idx] + tot;
+            else
+                P->s2d[idx] = tot;
+            if (MIXED && threadIdx.x == 0)
+                Y->predo = 0.;
         }
     }
 }
@@ -1809,29 +1944,6 @@ __device__ __forceinline__ void occ64_eval(const Occ64* o, double x, double xc, 
         const double p  = common ? xc : fx::pow(x, o[s].cf);
         g[s] = fma(o[s].wt, ft, o[s].kf * (p * fx::exp(-x * o[s].rf)));
     }
-}
-
-// Sums the 16 values of the warp's lanes: lane l returns the total of value
-// sum_index(l).  Each round halves the values a lane carries, 16 additions in
-// all instead of 80 for 16 butterfly sums.
-__device__ __forceinline__ double warp_sum16(double* v, int lane)
-{
-#pragma unroll
-    for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1)
-    {
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int k = 0; k < n; ++k)
-        {
-            const double mine = up ? v[k + n] : v[k], theirs = up ? v[k] : v[k + n];
-            v[k] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
-        }
-    }
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-__device__ __forceinline__ int sum_index(int lane)
-{
-    return ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
 }
 
 template <int NW>
@@ -2641,6 +2753,14 @@ cudaError_t launch_nes64(const Step& S, cudaStream_t st, int sms, int flagged)
     return cudaGetLastError();
 }
 
+template <bool MIXED, bool MULTI>
+void launch_pair(const Step& S, cudaStream_t st, int sms, int redo_only)
+{
+    const auto kernel = grey_pair_kernel<MIXED, MULTI>;
+    kernel<<<dim3(grid_for(kernel, kCellThreads, S.np, sms), 1, MULTI ? S.G : 1), kCellThreads, 0,
+             st>>>(*S.L, S.GA, S.p0, S.np, S.ws, redo_only);
+}
+
 template <bool MIXED, int IMPL, bool WIDE, bool MULTI>
 void launch_brem_impl(const Step& S, cudaStream_t st, int sms, int add, int redo_only)
 {
@@ -2712,15 +2832,9 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
     {
         phase_mark(kPhPair, 0, st);
         if (L.mixed)
-            grey_pair_kernel<true, false, MULTI>
-                <<<dim3(grid_for(grey_pair_kernel<true, false, MULTI>, kWarps * 32, wb, sms), 1,
-                        gz),
-                   kWarps * 32, 0, st>>>(L, S.GA, S.p0, np, S.ws, 0);
+            launch_pair<true, MULTI>(S, st, sms, 0);
         else
-            grey_pair_kernel<false, false, MULTI>
-                <<<dim3(grid_for(grey_pair_kernel<false, false, MULTI>, kWarps * 32, wb, sms), 1,
-                        gz),
-                   kWarps * 32, 0, st>>>(L, S.GA, S.p0, np, S.ws, 0);
+            launch_pair<false, MULTI>(S, st, sms, 0);
         phase_mark(kPhPair, 1, st);
     }
     if (L.use_brem)
@@ -2770,9 +2884,7 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
         if (L.use_pair)
         {
             phase_mark(kPhPair, 0, st);
-            grey_pair_kernel<false, true, MULTI>
-                <<<dim3(grid_for(grey_pair_kernel<false, true, MULTI>, 8 * 32, np, sms), 1, gz),
-                   8 * 32, 0, st>>>(L, S.GA, S.p0, np, S.ws, 1);
+            launch_pair<false, MULTI>(S, st, sms, 1);
             phase_mark(kPhPair, 1, st);
         }
         if (L.use_brem && (err = launch_brem<false, MULTI>(S, st, sms, L.use_pair, 1)) !=
