@@ -2007,7 +2007,7 @@ __global__ void __launch_bounds__(nes64_warps<WIDE>() * 32, WIDE ? 2 : 1)
             S.w[k]   = w;
             S.wp[k]  = wp;
             S.m[k]   = m;
-            S.ka[k]  = m * ((1. - e1) / e1);
+            S.ka[k]  = m * (fx::exp(w - wp) / e1);
             S.wc[k]  = fx::pow(w, k::CF);
             S.wpc[k] = fx::pow(wp, k::CF);
         }
