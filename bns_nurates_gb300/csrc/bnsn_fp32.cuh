@@ -33,8 +33,21 @@ struct Hr98Mixed
     double outer;
 };
 
-BNSN_DI void hr98_mixed_from(const fp64::Hr98Point& P, Hr98Mixed* M)
+// ch = 0..2: the constants of a channel; ch = 3: the rest (four lanes of a warp).
+BNSN_DI void hr98_mixed_part(const fp64::Hr98Point& P, int ch, Hr98Mixed* M)
 {
+    if (ch < 3)
+    {
+        const fp64::Hr98Channel& C = P.ch[ch];
+        M->K1fu[ch]   = (float)(C.K1 * C.f_u / k::FourPiSq);
+        M->eta2p1[ch] = (float)C.eta2p1;
+        M->sqe[ch]    = (float)C.sqe;
+        M->ep2[ch]    = (float)C.ep2;
+        M->h[ch]      = (float)C.h;
+        M->hgg2[ch]   = (float)(C.hgg * C.hgg);
+        M->pre[ch]    = (float)(C.weight * C.gamma / P.T);
+        return;
+    }
     M->y      = (float)P.y;
     M->poly_y = (float)P.poly_y;
     M->y4p1   = (float)P.y4p1;
@@ -45,19 +58,13 @@ BNSN_DI void hr98_mixed_from(const fp64::Hr98Point& P, Hr98Mixed* M)
     M->cq     = dfm::from_double(k::Pi18 + P.y);
     M->cp     = dfm::from_double(P.poly_y + 1.);
     M->y2     = dfm::from_double(2. * P.y);
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-    {
-        const fp64::Hr98Channel& C = P.ch[c];
-        M->K1fu[c]   = (float)(C.K1 * C.f_u / k::FourPiSq);
-        M->eta2p1[c] = (float)C.eta2p1;
-        M->sqe[c]    = (float)C.sqe;
-        M->ep2[c]    = (float)C.ep2;
-        M->h[c]      = (float)C.h;
-        M->hgg2[c]   = (float)(C.hgg * C.hgg);
-        M->pre[c]    = (float)(C.weight * C.gamma / P.T);
-    }
-    M->outer = 3. * k::BremConst / P.mcorr;
+    M->outer  = 3. * k::BremConst / P.mcorr;
+}
+
+BNSN_DI void hr98_mixed_from(const fp64::Hr98Point& P, Hr98Mixed* M)
+{
+    for (int ch = 0; ch < 4; ++ch)
+        hr98_mixed_part(P, ch, M);
 }
 
 // x^p for x > 0 to about 1 ulp: log2 x = k + log2 m with the binary exponent

@@ -83,7 +83,7 @@ BNSN_DI double bessk1(double x)
     if (x <= 2.)
     {
         y   = x * x / 4.;
-        ans = (log(x / 2.) * bessi1(x)) +
+        ans = (fx::log(x / 2.) * bessi1(x)) +
               (1.0 / x) * (1.0 + y * (0.15443144 + y * (-0.67278579 + y * (-0.18156897 +
               y * (-0.1919402e-1 + y * (-0.110404e-2 + y * (-0.4686e-4)))))));
     }
@@ -788,8 +788,107 @@ BNSN_DI void hr98_point_common(double nb, double T, bool medium, Hr98Point* P)
     }
 }
 
-// l = 0 HR98 kernel (kernel_brem_HR98.hpp:342-393) at x = (w + w')/T:
-// absorption and emission (detailed balance) kernels.
+// Constants of the absorption kernel in the form hr98_absorption takes: every
+// power of the fit is an exp2 of a multiple of a fixed-point log2 (bnsn_fx.cuh),
+// logarithms in units of 2^-56.
+struct Hr98Cell
+{
+    double y2, cX, cp, cq;       // 2 y, 2 - e^{-y/12}, 5 y^2 / 3 + 1, pi^(1/8) + y
+    double pre[3];               // 3 C_brem / medium x weight gamma / T per channel
+    double hgg2[3], A0[3], h[3]; // (0.5 gamma g)^2, (1 + eta*^2)(1 + y^4), h(eta*)
+    double cg[3];                // 0.0044 y sqrt(eta*) / (D(y) (eta* + 0.2))
+    int64_t lK[3];               // log2(K1 f_u / 4 pi^2)
+    int64_t mp, minv;            // -p and -1/p in 2^-58
+    int fast;                    // all of these in range (else hr98_kernel)
+};
+
+// Channel ch (0..2) of the constants; ch = 3: the rest.
+BNSN_DI void hr98_cell_from(const Hr98Point& P, int ch, Hr98Cell* M)
+{
+    if (ch < 3)
+    {
+        const Hr98Channel& C = P.ch[ch];
+        const double kf      = C.K1 * C.f_u / k::FourPiSq;
+        M->pre[ch]  = 3. * k::BremConst / P.mcorr * (C.weight * C.gamma / P.T);
+        M->hgg2[ch] = C.hgg * C.hgg;
+        M->A0[ch]   = C.eta2p1 * P.y4p1;
+        M->h[ch]    = C.h;
+        M->cg[ch]   = 0.0044 * P.y * C.sqe / (P.Dy * C.ep2);
+        M->lK[ch]   = fx::log2_range(kf) ? fx::log2_q56(kf) : 0;
+    }
+    else
+    {
+        M->y2   = 2. * P.y;
+        M->cX   = 2. - P.ey12;
+        M->cp   = P.poly_y + 1.;
+        M->cq   = k::Pi18 + P.y;
+        M->mp   = fx::pow_exponent(P.mp);
+        M->minv = fx::pow_exponent(P.minv);
+        bool ok = P.mp < -0.05 && P.mp > -30. && P.minv > -30. && P.y4p1 < 1e60;
+        for (int c = 0; c < 3; ++c)
+        {
+            const double kf = P.ch[c].K1 * P.ch[c].f_u; // logarithms stay below 2^7
+            ok = ok && kf > 1e-11 && kf < 1e13 && P.ch[c].eta2p1 < 1e60 && P.ch[c].hgg < 1e60;
+        }
+        M->fast = ok;
+    }
+}
+
+// l = 0 HR98 absorption kernel (kernel_brem_HR98.hpp:342-393) at x = (w + w')/T in
+// [1e-6, 1e5], ex = e^{-x}.  s = (s_nd^-p + s_d^-p)^(-1/p) is min(s_nd, s_d) (1 +
+// r^p)^(-1/p) with r = min / max, so the powers act on numbers in [0, 2]; the
+// three quotients of a channel share one reciprocal.  13 pow took 1300 FP64
+// operations a cell; here 60, beside ~20 fixed-point exponentials and logs.
+BNSN_DI double hr98_absorption(const Hr98Cell& M, double x, double ex)
+{
+    constexpr int64_t kP11 = (int64_t)(1.1 * 288230376151711744.);
+    constexpr int64_t kP093 = (int64_t)(0.93 * 288230376151711744.);
+    constexpr int64_t kP12 = (int64_t)(1.2 * 288230376151711744.);
+    constexpr int64_t kP28 = (int64_t)(2.8 * 288230376151711744.);
+    const int64_t L  = fx::log2_q56(x);
+    const double x2  = x * x;
+    // s_nd = 2 sqrt(pi) X^1.5 (x^2 + 2 x y + 5 y^2 / 3 + 1) / (sqrt(pi) + q^4)
+    const double q   = x + M.cq, q2 = q * q;
+    const int64_t LX = fx::log2_q56(x + M.cX);
+    constexpr int64_t kL2SqrtPi = (int64_t)(1.8257480647361594 * 72057594037927936.);
+    const int64_t Ln = LX + (LX >> 1) + kL2SqrtPi + fx::log2_q56(fma(x, x + M.y2, M.cp)) -
+                       fx::log2_q56(fma(q2, q2, k::SqrtPi));
+    // s_d = K1 f_u x (x^2 + 4 pi^2) / (4 pi^2 (1 - e^-x))
+    const int64_t Lc = fx::log2_q56(x * (x2 + k::FourPiSq)) - fx::log2_q56(1. - ex);
+    const double px11  = fx::pow_q(L, kP11);
+    const double px093 = fx::pow_q(L, kP093);
+    const double px12  = fx::pow_q(L, kP12);
+    const double px28  = fx::pow_q(L, kP28);
+    const double ix4   = fx::rcp(x2 * x2);
+    const double d12   = x - 1.2;
+    const double xterm = 3. + d12 * d12 + ix4;
+    const double cb    = 33. * px11 * fx::rcp(fma(0.005, px28, 30.));
+    const double cd    = fma(0.0001, px12, 2.3);
+    double tot         = 0.;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+    {
+        const int64_t Ld = Lc + M.lK[c];
+        const int64_t lo = Ln < Ld ? Ln : Ld, dl = Ln < Ld ? Ld - Ln : Ln - Ld;
+        const double t   = fx::pow_q(dl, M.mp); // (min / max)^p
+        fx::Exp2 E       = fx::scale_log(fx::log2_q56(1. + t), M.minv);
+        // + lo
+        const uint64_t F = E.F + ((uint64_t)lo << 8);
+        E.I += (int)(lo >> 56) + (F < E.F ? 1 : 0);
+        E.F = F;
+        const double sb = fx::exp2(E);
+        // (1 + 1/A) (1 + cb h g / den) / B
+        const double A   = xterm * M.A0[c];
+        const double den = fma(M.h[c], px093, cd);
+        const double g   = fma(-M.cg[c], px11, 1.);
+        const double num = sb * ((A + 1.) * fma(cb * M.h[c], g, den));
+        const double iv  = fx::rcp(A * ((x2 + M.hgg2[c]) * den));
+        tot = fma(M.pre[c], num * iv, tot);
+    }
+    return tot;
+}
+
+// The same at any argument, with the library's powers.
 BNSN_DI void hr98_kernel(const Hr98Point& P, double omega, double omega_p,
                          double* em, double* ab)
 {
@@ -847,13 +946,25 @@ BNSN_DI double brt06_point(double nb, double T, double yn, double yp)
     return k::HC6FourPi2 * k::BremC4BRT06 * (q / T7);
 }
 
+// K_1(x) e^{x} / x, with the reference's clamp of e^{x} at x = 700 (its exp(-x)
+// keeps falling): the polynomial fits of bessi1 / bessk1.
+BNSN_DI double brt06_shape(double x)
+{
+    if (x <= 2.)
+        return bessk1(x) * fx::exp(x) / x;
+    const double ix = fx::rcp(x), y = 2. * ix;
+    const double p  = 1.25331414 + y * (0.23498619 + y * (-0.3655620e-1 + y * (0.1504268e-1 +
+                      y * (-0.780353e-2 + y * (0.325614e-2 + y * (-0.68245e-3))))));
+    const double r = p * ix * sqrt(ix);
+    return x > k::ExpUpp ? r * fx::exp(k::ExpUpp - x) : r;
+}
+
 BNSN_DI void brt06_kernel(double pre, double T, double omega, double omega_p,
                           double* em, double* ab)
 {
-    const double x   = 0.5 * (omega + omega_p) / T;
-    const double tmp = pre * bessk1(x) / x;
-    *em              = tmp * safe_exp(-x);
-    *ab              = tmp * safe_exp(x);
+    const double x = 0.5 * (omega + omega_p) / T;
+    *ab            = pre * brt06_shape(x);
+    *em            = *ab * safe_exp(-2. * x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1101,9 +1212,8 @@ BNSN_DI double gp19_high_t_from(double R48, double R50, double nbnm, double T, d
 }
 
 // One cell from the profiles: v0, v1 are the profile values interpolated at
-// the clipped w; w0 = omega + omega' unclipped.
-BNSN_DI void gp19_cell(const Gp19Point& P, double v0, double v1, double w, double w0,
-                       double* em, double* ab)
+// the clipped w.
+BNSN_DI double gp19_absorption(const Gp19Point& P, double v0, double v1, double w)
 {
     double s;
     switch (P.regime)
@@ -1116,7 +1226,7 @@ BNSN_DI void gp19_cell(const Gp19Point& P, double v0, double v1, double w, doubl
         double k2 = P.C * v0, k4 = P.C * v1;
         k2 = (k2 < eps) ? eps : k2;
         k4 = (k4 < eps) ? eps : k4;
-        const double m = log(k4 / k2) * 1.4426950408889634;
+        const double m = fx::log2(k4 / k2);
         s = k2 * fx::pow(P.T * 0.5, m);
         s = (s < eps) ? eps : s;
         break;
@@ -1124,7 +1234,7 @@ BNSN_DI void gp19_cell(const Gp19Point& P, double v0, double v1, double w, doubl
     case 4:
     {
         const double k2 = P.C * v0, k4 = P.C * v1;
-        const double m  = log(k4 / k2) * 1.4426950408889634;
+        const double m  = fx::log2(k4 / k2);
         s = k2 * fx::pow(P.T * 0.5, m);
         break;
     }
@@ -1132,9 +1242,15 @@ BNSN_DI void gp19_cell(const Gp19Point& P, double v0, double v1, double w, doubl
         s = gp19_high_t_from(P.C * v0, P.C * v1, P.nbnm, P.T, w) * P.r2;
         break;
     }
-    s   = fabs(3. * s);
-    *ab = s;
-    *em = s * safe_exp(-w0 / P.T);
+    return fabs(3. * s);
+}
+
+// The same with the emission kernel; w0 = omega + omega' unclipped.
+BNSN_DI void gp19_cell(const Gp19Point& P, double v0, double v1, double w, double w0,
+                       double* em, double* ab)
+{
+    *ab = gp19_absorption(P, v0, v1, w);
+    *em = *ab * safe_exp(-w0 / P.T);
 }
 
 // kernel_brem_GP19.hpp:357-481

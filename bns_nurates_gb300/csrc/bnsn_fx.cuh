@@ -197,19 +197,20 @@ BNSN_FX_HD int64_t log2_q56(double x)
     const int64_t Zn  = Z * 128;                                      // z 2^70
     const uint64_t az = (uint64_t)(Zn < 0 ? -Zn : Zn);
     const uint64_t S  = mulhi3(az, az); // z^2 2^76
-    // ln(1 + z) = z - z^2 (1/2 + w), w = -z/3 + z^2/4 - z^3/5 + z^4/6; W = w 2^40
+    // ln(1 + z) = z - z^2 (1/2 + w), w = -z/3 + v, v = z^2 (1/4 - z/5 + z^2/6)
     const int32_t z32 = (int32_t)(Zn >> 32); // z 2^38
-    int32_t t         = -209715 + smulhi(2731, z32);
-    t                 = 33554432 + 2 * smulhi(t, z32);
-    t                 = -1431655765 + 2 * smulhi(t, z32);
-    const int32_t W   = smulhi(t, z32) - z32;
-    const int64_t C   = (int64_t)(S >> 1) + (((int64_t)(int32_t)(S >> 32) * W) >> 8); // 2^76
+    int32_t t         = 2 * smulhi(43691, z32) - 6710886;
+    t                 = 1073741824 + 2 * smulhi(t, z32);
+    const int64_t V   = (int64_t)(int32_t)(S >> 32) * t;                        // v 2^76
+    const int64_t w   = (V >> 6) - mulhi3s(Zn, 0x5555555555555556ull);          // w 2^70
+    const int64_t C   = (int64_t)(S >> 1) + (mulhi3s(w, S) >> 6);               // 2^76
     const int64_t N   = Z - (C >> 13);                                    // ln(1 + z) 2^63
     const int64_t N2  = N + mulhi3s(N, 0x71547652B82FE177ull);            // x log2(e)
     return ((int64_t)e << 56) + (((int64_t)row.l + N2 + 64) >> 7);
 }
 
 BNSN_FX_OUT double pow_special(double x, double p) { return ::pow(x, p); }
+BNSN_FX_OUT double log_special(double x) { return ::log(x); }
 
 // The exponent p as p 2^58 (|p| < 31.9).
 BNSN_FX_HD int64_t pow_exponent(double p) { return (int64_t)(p * 288230376151711744.); }
@@ -237,6 +238,17 @@ BNSN_FX_HD double pow_q(int64_t L, int64_t P) { return exp2(scale_log(L, P)); }
 BNSN_FX_HD bool log2_range(double x)
 {
     return ((uint32_t)(bits_of(x) >> 52) - (1023u - 120u)) < 240u;
+}
+
+// log2(x) and log(x) for any x (absolute error 2^-57 near x = 1).
+BNSN_FX_HD double log2(double x)
+{
+    return log2_range(x) ? (double)log2_q56(x) * 1.3877787807814457e-17
+                         : log_special(x) * 1.4426950408889634;
+}
+BNSN_FX_HD double log(double x)
+{
+    return log2_range(x) ? (double)log2_q56(x) * (0.693147180559945309 * 1.3877787807814457e-17) : log_special(x);
 }
 
 // x^p for any x and p.

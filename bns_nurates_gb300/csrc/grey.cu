@@ -97,6 +97,20 @@ __device__ __forceinline__ PairMixed* pair_mixed(PointTab* P)
     return reinterpret_cast<PairMixed*>(&P->fm[0][0]);
 }
 
+// GP19 brem: the point's extrapolation regime and the corners of its profiles
+// take the words of the HR98 constants.
+struct Gp19Record
+{
+    Gp19Point pt;
+    Gp19Corners cor[2];
+};
+static_assert(sizeof(Gp19Record) <= sizeof(Hr98Point), "Gp19Record overlay");
+
+__device__ __forceinline__ Gp19Record* gp19_record(PointTab* P)
+{
+    return reinterpret_cast<Gp19Record*>(&P->hr);
+}
+
 size_t grey_point_scratch_bytes() { return sizeof(PointTab); }
 
 namespace {
@@ -178,6 +192,7 @@ __device__ __forceinline__ void beta_scales(double T, double eta_e, const double
 //   0..3  distribution parameters of species 0..3 (or a copy of the given ones)
 //   4, 5  F_0..F_5 and FermiDistr(0, 1, .) at +eta_e, -eta_e
 //   6..8  HR98 channel constants; 9: HR98 point constants; 10: BRT06 prefactor
+//   6, 7  GP19: the point's regime and the corners of its two profiles
 //   11    eta_NN of protons and neutrons (iso scattering)
 // written straight into the point's scratch record, whose header the prelude
 // then loads.  Inside the one-warp-per-point prelude these tasks ran on one to
@@ -199,7 +214,8 @@ __global__ void __launch_bounds__(128)
         scratch = gcz.ws;
     }
     const int task = blockIdx.y;
-    if ((task >= 6 && task <= 9 && !(L.use_brem && L.brem_impl == 0)) ||
+    const bool gp19 = L.use_brem && L.brem_impl == 2 && L.gp19.d3 <= kGp19MaxW;
+    if ((task >= 6 && task <= 9 && !(L.use_brem && L.brem_impl == 0) && !(gp19 && task < 8)) ||
         (task == 10 && !(L.use_brem && L.brem_impl == 1)) || (task == 11 && !L.use_iso))
         return;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < np;
@@ -233,6 +249,19 @@ __global__ void __launch_bounds__(128)
             for (int kk = 0; kk < 6; ++kk)
                 P->fe[e][kk] = f[kk];
             P->fd0[e] = fermi_distr(0., 1., et);
+        }
+        else if (task < 9 && gp19)
+        {
+            const Gp19Table G = {L.gp19.d0, L.gp19.d1, L.gp19.d2, L.gp19.d3,
+                                 L.gp19.nb, L.gp19.ye, L.gp19.t,  L.gp19.w,
+                                 L.gp19.lognb, L.gp19.logw, L.gp19.data};
+            Gp19Point pt;
+            gp19_point(G, nb, L.eos[2][p], T, &pt);
+            Gp19Record* R = gp19_record(P);
+            if (task == 6)
+                R->pt = pt;
+            if (task == 6 || pt.regime >= 2)
+                gp19_profile_corners(G, pt.nbp, pt.yep, pt.pT[task - 6], &R->cor[task - 6]);
         }
         else if (task < 9)
             P->hr.ch[task - 6] = hr98_channel(nb, L.eos[4][p], L.eos[3][p], T, task - 6);
@@ -540,73 +569,24 @@ __global__ void __launch_bounds__(kWarps * 32)
     }
 }
 
-// ---------------------------------------------------------------------------
-// weight algebra of m1_opacities.hpp:577-758 for one directed cell (a, b):
-// em_s = K_em[s] bf_b[partner(s)], ab_s = K_ab[s] g_b[partner(s)], then
-// stimulated absorption and the nu^2 nubar^2 weight, summed with the number
-// (W1) and energy (W2) quadrature weights.  The moments are linear in the
-// kernel, so pair and brem contributions are summed in separate phases.
-// ---------------------------------------------------------------------------
-template <bool STIM>
-__device__ __forceinline__ void add_cell(double* acc, const double* Kem, const double* Kab,
-                                         const double* ga, const double* gb, bool nb_block,
-                                         double w4, double W1, double W2)
-{
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-    {
-        const int ps    = s ^ 1;
-        const double em = Kem[s] * (nb_block ? 1. : 1. - gb[ps]);
-        const double am = Kab[s] * gb[ps];
-        double EM, AB;
-        if (STIM)
-        {
-            AB = w4 * ga[s] * (em + am);
-            EM = em * w4;
-        }
-        else
-        {
-            AB = am * (w4 * ga[s]);
-            EM = em * (w4 * (1. - ga[s]));
-        }
-        acc[s] += EM * W1;
-        acc[4 + s] += AB * W1;
-        acc[8 + s] += EM * W2;
-        acc[12 + s] += AB * W2;
-    }
-}
-
-// Shared-memory copy of the energy tables a cell loop needs.
+// Shared-memory copy of the energy tables the FP32 brem cells need.
 struct CellTab
 {
     double nu[kMaxM];
     double y[kMaxM];
     double g[kMaxM][4];
-    double fm[kMaxM][5];
-    double fp[kMaxM][5];
-    double f3e, f4e;
     double brt06_pre;
-    Hr98Point hr;
     fp32::Hr98Mixed hm;
 };
 
 __device__ __forceinline__ void load_cell_tab(CellTab& C, const PointTab* __restrict__ P,
-                                              int M, bool pair_tables, int lane)
+                                              int M, int lane)
 {
     warp_copy(C.nu, P->nu, M, lane);
     warp_copy(C.y, P->y, M, lane);
     warp_copy(&C.g[0][0], &P->g[0][0], 4 * M, lane);
-    if (pair_tables)
-    {
-        warp_copy(&C.fm[0][0], &P->fm[0][0], 5 * M, lane);
-        warp_copy(&C.fp[0][0], &P->fp[0][0], 5 * M, lane);
-    }
     if (lane == 0)
-    {
-        C.f3e       = P->fe[0][3];
-        C.f4e       = P->fe[0][4];
         C.brt06_pre = P->brt06_pre;
-    }
 }
 
 // Mixed-path cell tables (FP32): g and 1 - g per species (1 - g formed in
@@ -734,6 +714,22 @@ __device__ __forceinline__ void beta_in_sum_units(const PointTab* P, double T, d
     }
 }
 
+// Element idx of the same (each lane of a warp takes its own).
+__device__ __forceinline__ double beta_in_sum_unit(const PointTab* P, double T, double eta_e,
+                                                   bool use_abs_em, bool to_nes, int idx)
+{
+    const int s = idx & 3, m = idx >> 2; // species; number em, ab, energy em, ab
+    if (!use_abs_em || s >= 2)
+        return 0.;
+    const bool big = (eta_e > 30.) == (s == 0);
+    const double sb = (eta_e > -30. && eta_e < 30.) ? T * P->fe[s][5] / P->fe[s][4]
+                                                    : (big ? T * eta_e * 0.8333333333333333 : T * 5.);
+    const double t2d = k::TempMultiple * T, t2 = t2d * t2d;
+    const double un  = k::FourPiHc3 * (to_nes ? 8. * t2 : t2);
+    const double u   = (m >= 2 && !to_nes) ? un * t2d : un;
+    return P->sbeta[(m & 1) * 4 + (m >> 1) * 2 + s] * sb / u;
+}
+
 // Mixed sums whose terms cancel by more than this are recomputed in FP64: the
 // FP32 rounding of each term (a few 1e-7) must stay below 1e-6 in the result.
 constexpr double kMaxCancel = 2.0;
@@ -824,6 +820,7 @@ __device__ __forceinline__ void fill_tab32(CellTab32& D, const CellTab& C, int M
 // ---------------------------------------------------------------------------
 constexpr int kCellThreads = 64;
 
+template <int NT>
 struct CellNodes
 {
     double K[kMaxM][kMaxM + 1];        // absorption kernel of (row, column)
@@ -832,7 +829,7 @@ struct CellNodes
     double q[kMaxM], qe[kMaxM]; // number and energy weights of a node
     double dn[kMaxM];           // e^{-y}
     double nu[kMaxM], y[kMaxM];
-    double red[2][2][16];
+    double red[2][NT / 32][16];
     double A1[kMaxM], A2[kMaxM];
     uint16_t cells[kMaxCells]; // a | b << 8
     int splits;                // column ranges a row is cut into
@@ -841,16 +838,16 @@ struct CellNodes
 // Launch constants of the CTA, and the column split: rows x splits tasks of
 // (M / splits) columns over the CTA's threads, chosen for the fewest rounds x
 // (columns x products + the row's epilogue).
-template <bool SYM>
-__device__ __forceinline__ void cell_constants(CellNodes& C, const OpacityLaunch& L)
+template <bool SYM, int NT>
+__device__ __forceinline__ void cell_constants(CellNodes<NT>& C, const OpacityLaunch& L)
 {
     const int M = 2 * L.n2;
-    for (int k = threadIdx.x; k < kMaxM; k += kCellThreads)
+    for (int k = threadIdx.x; k < kMaxM; k += NT)
     {
         C.A1[k] = L.A1[k];
         C.A2[k] = L.A2[k];
     }
-    for (int k = threadIdx.x; k < L.ncell; k += kCellThreads)
+    for (int k = threadIdx.x; k < L.ncell; k += NT)
     {
         const uint32_t ab = L.cells[k];
         C.cells[k]        = (uint16_t)((ab & 0xffu) | ((ab >> 16) << 8));
@@ -860,7 +857,7 @@ __device__ __forceinline__ void cell_constants(CellNodes& C, const OpacityLaunch
         int best = 1, cost = 1 << 30;
         for (int h = 1; h <= 8 && h <= M; ++h)
         {
-            const int c = ((M * h + kCellThreads - 1) / kCellThreads) *
+            const int c = ((M * h + NT - 1) / NT) *
                           (((M + h - 1) / h) * (SYM ? 8 : 16) + 45);
             if (c < cost)
             {
@@ -873,7 +870,8 @@ __device__ __forceinline__ void cell_constants(CellNodes& C, const OpacityLaunch
 }
 
 // Node data of a point; nu2: the weights carry nu^2 (kernels without it).
-__device__ __forceinline__ bool cell_nodes(CellNodes& C, const PointTab* __restrict__ P, int M,
+template <int NT>
+__device__ __forceinline__ bool cell_nodes(CellNodes<NT>& C, const PointTab* __restrict__ P, int M,
                                            bool nbb, bool nu2)
 {
     bool above = false; // an occupation above 1
@@ -906,12 +904,12 @@ __device__ __forceinline__ bool cell_nodes(CellNodes& C, const PointTab* __restr
 // species 0 (2) at (a, b) is e0 K(a, b) + e1 K(b, a) (x0, x1); species 1 and 3
 // exchange K(a, b) and K(b, a) (kernel_pair.hpp:200-216).  SYM: one symmetric
 // kernel for all species.  ABS: sums of |term| of the emission moments alone.
-template <bool SYM, bool ABS>
-__device__ __forceinline__ void cell_row_sums(const CellNodes& C, int M, bool stim, double e0,
+template <bool SYM, bool ABS, int NT>
+__device__ __forceinline__ void cell_row_sums(const CellNodes<NT>& C, int M, bool stim, double e0,
                                               double e1, double x0, double x1, double* acc)
 {
     const int h = C.splits;
-    for (int t = threadIdx.x; t < M * h; t += kCellThreads)
+    for (int t = threadIdx.x; t < M * h; t += NT)
     {
         const int part = t / M, a = t - part * M;
         const int b0 = part * M / h, b1 = (part + 1) * M / h;
@@ -969,16 +967,20 @@ __device__ __forceinline__ void cell_row_sums(const CellNodes& C, int M, bool st
     }
 }
 
-// Totals of the CTA's two warps: lane l of warp 0 holds that of moment
-// sum_index(l).
-__device__ __forceinline__ double cell_total(CellNodes& C, double* acc, int slot)
+// Totals over the CTA: lane l of a warp holds that of moment sum_index(l).
+template <int NT>
+__device__ __forceinline__ double cell_total(CellNodes<NT>& C, double* acc, int slot)
 {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double v = warp_sum16(acc, lane);
     if (!(lane & 1))
         C.red[slot][wid][sum_index(lane)] = v;
     __syncthreads();
-    return C.red[slot][0][sum_index(lane)] + C.red[slot][1][sum_index(lane)];
+    double t = C.red[slot][0][sum_index(lane)];
+#pragma unroll
+    for (int w = 1; w < NT / 32; ++w)
+        t += C.red[slot][w][sum_index(lane)];
+    return t;
 }
 
 // Node tables of the mixed pair phase: y = nu/T as double-float and
@@ -1045,7 +1047,7 @@ __global__ void __launch_bounds__(kCellThreads)
     }
     if (MULTI && !L.use_pair)
         return; // a group without pair (uniform over the CTA)
-    __shared__ CellNodes C;
+    __shared__ CellNodes<kCellThreads> C;
     __shared__ PairTab32 X;
     __shared__ PairTab64 W;
     const int M     = 2 * L.n2;
@@ -1175,22 +1177,241 @@ __global__ void __launch_bounds__(kCellThreads)
     }
 }
 
-// Per-warp GP19 state of the brem kernel.
+// ---------------------------------------------------------------------------
+// Bremsstrahlung in FP64 (kernel_brem_HR98.hpp, _BRT06.hpp, _GP19.hpp): the cells'
+// absorption kernels (emission is K e^{-(w + w')/T}) and the row sums of the cell
+// phases.  IMPL: 0 HR98, 1 BRT06, 2 GP19.
+// ---------------------------------------------------------------------------
+
+// Order-preserving integer image of a double (comparisons off the FP64 pipe).
+__device__ __forceinline__ int64_t order_key(double v)
+{
+    const int64_t b = __double_as_longlong(v);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+
+template <int IMPL>
+struct Brem64Extra
+{
+};
+template <>
+struct Brem64Extra<0>
+{
+    Hr98Cell hc;
+    Hr98Point hr;
+};
+template <>
+struct Brem64Extra<2>
+{
+    Gp19Record r;
+    double p[2][kGp19MaxW];
+    double lw[kGp19MaxW], idl[kGp19MaxW]; // log w axis, 1 / its intervals
+    int64_t key[kGp19MaxW];
+};
+
+template <int IMPL, int NT>
+struct Brem64Smem
+{
+    CellNodes<NT> C;
+    Brem64Extra<IMPL> X;
+};
+
+__device__ __forceinline__ Gp19Table gp19_table(const OpacityLaunch& L)
+{
+    return {L.gp19.d0, L.gp19.d1, L.gp19.d2,    L.gp19.d3,   L.gp19.nb,  L.gp19.ye,
+            L.gp19.t,  L.gp19.w,  L.gp19.lognb, L.gp19.logw, L.gp19.data};
+}
+
+// Launch constants (once per CTA; brem64_point's first barrier orders them).
+template <int IMPL, int NT>
+__device__ __forceinline__ void brem64_constants(Brem64Smem<IMPL, NT>& S, const OpacityLaunch& L)
+{
+    cell_constants<true>(S.C, L);
+    if constexpr (IMPL == 2)
+    {
+        if (L.gp19.d3 <= kGp19MaxW)
+            for (int k = threadIdx.x; k < L.gp19.d3; k += NT)
+            {
+                const double* lw = L.gp19.logw;
+                S.X.lw[k]  = lw[k];
+                S.X.key[k] = order_key(lw[k]);
+                S.X.idl[k] = k + 1 < L.gp19.d3 ? 1. / (lw[k + 1] - lw[k]) : 0.;
+            }
+    }
+}
+
+// The brem sums of a point, by all NT threads: lane l of each warp returns the
+// total of moment sum_index(l).
+template <int IMPL, int NT>
+__device__ __forceinline__ double brem64_point(Brem64Smem<IMPL, NT>& S, const OpacityLaunch& L,
+                                               PointTab* P, int64_t p)
+{
+    CellNodes<NT>& C = S.C;
+    const int M      = 2 * L.n2;
+    const double T   = L.eos[1][p];
+    __syncthreads(); // the previous point's readers are done
+    cell_nodes(C, P, M, L.neglect_blocking != 0, true);
+    bool fast = true; // HR98: every cell within hr98_absorption's range
+    if constexpr (IMPL == 0)
+    {
+        for (int k = threadIdx.x; k < (int)(sizeof(Hr98Point) / sizeof(double)); k += NT)
+            ((double*)&S.X.hr)[k] = ((const double*)&P->hr)[k];
+        __syncthreads();
+        if (threadIdx.x < 4)
+            hr98_cell_from(S.X.hr, threadIdx.x, &S.X.hc);
+        const bool out = threadIdx.x < M &&
+                         !(C.y[threadIdx.x] > 1e-6 && C.y[threadIdx.x] < 4e4);
+        fast = !__syncthreads_or(out);
+        fast = fast && S.X.hc.fast;
+    }
+    bool prof = false;
+    if constexpr (IMPL == 2)
+    {
+        prof = L.gp19.d3 <= kGp19MaxW;
+        if (prof)
+        {
+            for (int k = threadIdx.x; k < (int)(sizeof(Gp19Record) / sizeof(double)); k += NT)
+                ((double*)&S.X.r)[k] = ((const double*)gp19_record(P))[k];
+            __syncthreads();
+            const Gp19Table G = gp19_table(L);
+            const int np19    = S.X.r.pt.regime >= 2 ? 2 : 1;
+            for (int e = threadIdx.x; e < np19 * G.d3; e += NT)
+            {
+                const int pr = e / G.d3, l = e - pr * G.d3;
+                S.X.p[pr][l] = gp19_profile_eval(G, S.X.r.cor[pr], l);
+            }
+        }
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < L.ncell; c += NT)
+    {
+        const uint32_t ab = C.cells[c];
+        const int a = ab & 0xffu, b = ab >> 8;
+        double K, em;
+        if constexpr (IMPL == 0)
+        {
+            if (fast)
+                K = hr98_absorption(S.X.hc, C.y[a] + C.y[b], C.dn[a] * C.dn[b]);
+            else
+                hr98_kernel(S.X.hr, C.nu[a], C.nu[b], &em, &K);
+        }
+        else if constexpr (IMPL == 1)
+            K = P->brt06_pre * brt06_shape(0.5 * (C.y[a] + C.y[b]));
+        else
+        {
+            const Gp19Table G = gp19_table(L);
+            if (prof)
+            {
+                const double w  = fmax(fmin(C.nu[a] + C.nu[b], G.w[G.d3 - 1]), G.w[0]);
+                const double lw = fx::log(w);
+                const int64_t k = order_key(lw);
+                // smallest l in [0, d3 - 2] with lw <= axis[l + 1]
+                int lo = 0, hi = G.d3 - 2;
+                while (lo < hi)
+                {
+                    const int mid = (lo + hi) >> 1;
+                    if (k <= S.X.key[mid + 1])
+                        hi = mid;
+                    else
+                        lo = mid + 1;
+                }
+                const double tw = (lw - S.X.lw[lo]) * S.X.idl[lo], t0 = 1. - tw;
+                const double v0 = fma(S.X.p[0][lo + 1], tw, S.X.p[0][lo] * t0);
+                const double v1 = S.X.r.pt.regime >= 2
+                                      ? fma(S.X.p[1][lo + 1], tw, S.X.p[1][lo] * t0)
+                                      : 0.;
+                K = gp19_absorption(S.X.r.pt, v0, v1, w);
+            }
+            else
+                gp19_kernel(G, L.eos[0][p], L.eos[2][p], T, C.nu[a], C.nu[b], &em, &K);
+        }
+        C.K[a][b] = K;
+        C.K[b][a] = K;
+    }
+    __syncthreads();
+    double acc[16];
+#pragma unroll
+    for (int kk = 0; kk < 16; ++kk)
+        acc[kk] = 0.;
+    cell_row_sums<true, false>(C, M, L.stim != 0, 1., 0., 1., 0., acc);
+    return cell_total(C, acc, 0);
+}
+
+// Every point (the plain path), or with redo_only the points the mixed path's
+// final kernel marked (bredo = 1), whose brem part of s2d it replaces.
+// 8,192 points: HR98 n = 10 1.40 -> 0.44 ms, GP19 n = 20 2.66 -> 0.84 ms, BRT06 n = 10
+// 0.65 -> 0.26 ms.
+template <int IMPL, bool MULTI = false>
+__global__ void __launch_bounds__(kCellThreads)
+    grey_brem_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
+                     int64_t np, double* __restrict__ scratch, int add, int redo_only)
+{
+    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
+    if (MULTI)
+    {
+        const GroupChunk& gcz = GA.gc[blockIdx.z];
+        p0      = gcz.p0;
+        np      = gcz.np;
+        scratch = gcz.ws;
+        if (!L.use_brem || L.brem_impl != IMPL)
+            return; // another brem variant's launch serves this group
+        add = L.use_pair;
+    }
+    __shared__ Brem64Smem<IMPL, kCellThreads> S;
+    bool ready = false;
+    for (int64_t q = blockIdx.x; q < np; q += gridDim.x)
+    {
+        const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
+        PointTab* P     = (PointTab*)(scratch + q * kTabWords);
+        if (redo_only && P->bredo != 1.)
+            continue; // uniform: a point per CTA
+        if (!ready)
+        {
+            brem64_constants(S, L);
+            ready = true;
+        }
+        const double tot = brem64_point(S, L, P, p);
+        if (threadIdx.x < 32 && !(threadIdx.x & 1))
+        {
+            const int idx     = sum_index(threadIdx.x);
+            const double base = add ? (redo_only ? P->s2d[idx] - P->sbrem[idx] : P->s2d[idx]) : 0.;
+            P->s2d[idx]   = base + tot;
+            P->sbrem[idx] = tot;
+            P->bmag[idx]  = 0.;
+        }
+    }
+}
+
+// Per-warp GP19 state of the FP32 brem kernel.
 struct Gp19Warp
 {
-    Gp19Point pt;
-    Gp19Corners cor[2];
+    Gp19Record r;
     double p[2][kGp19MaxW];
     float pf[2][kGp19MaxW];
 };
 
-// IMPL: 0 HR98, 1 BRT06, 2 GP19.  ADD: accumulate onto the pair sums.
-// WIDE (the mixed path's FP64 pass over the few marked points): a point per
-// CTA, its cells over all threads.
-template <bool MIXED, int IMPL, bool WIDE = false, bool MULTI = false>
-__global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
-    grey_brem_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
-                     int64_t np, double* __restrict__ scratch, int add, int redo_only)
+// Shared memory of the FP32 brem kernel (later the FP64 one's).
+template <int IMPL>
+struct Brem32Smem
+{
+    static constexpr int kWF = IMPL == 2 ? kGp19MaxW : 1;
+    dfm::df A1d[kMaxM], A2d[kMaxM];
+    uint32_t cells[kMaxCells];
+    CellTab ct[kWarps];
+    CellTab32 c32[kWarps];
+    Gp19Warp gw[IMPL == 2 ? kWarps : 1];
+    double lw[kWF], wax[kWF], iw[kWF];
+    float lwf[kWF], idl[kWF];
+};
+
+// Bremsstrahlung of the mixed path: FP32 cells (bnsn_fp32.cuh), a point per warp.
+// Points with the GP19 high-T extrapolation (which differences two table values),
+// with tables too long for profiles, or whose cells the other reactions cancel
+// are marked (bredo = 2) and evaluated in FP64 by the whole CTA at the end.
+template <int IMPL, bool MULTI = false>
+__global__ void __launch_bounds__(kWarps * 32, 3)
+    grey_brem32_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
+                     int64_t np, double* __restrict__ scratch, int add)
 {
     const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
     if (MULTI)
@@ -1206,127 +1427,79 @@ __global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
             return; // another brem variant's launch serves this group
         add = L.use_pair;
     }
-    constexpr int NW = WIDE ? 8 : kWarps;
-    constexpr int NT = WIDE ? 1 : kWarps; // point tables in flight per CTA
-    __shared__ double s_A1[kMaxM], s_A2[kMaxM];
-    __shared__ dfm::df s_A1d[MIXED ? kMaxM : 1], s_A2d[MIXED ? kMaxM : 1];
-    __shared__ uint32_t s_cells[kMaxCells];
-    __shared__ CellTab s_ct[NT];
-    __shared__ CellTab32 s_c32[MIXED ? kWarps : 1];
-    __shared__ Gp19Warp s_gw[IMPL == 2 ? NT : 1];
-    __shared__ double s_red[WIDE ? NW : 1][32];
-    __shared__ double s_lw[IMPL == 2 ? kGp19MaxW : 1];
-    __shared__ float s_lwf[IMPL == 2 ? kGp19MaxW : 1];
-    constexpr int kWF = (IMPL == 2 && MIXED) ? kGp19MaxW : 1;
-    __shared__ double s_wax[kWF], s_iw[kWF];
-    __shared__ float s_idl[kWF];
-    const Gp19Table G19 = {L.gp19.d0, L.gp19.d1, L.gp19.d2,    L.gp19.d3,   L.gp19.nb,  L.gp19.ye,
-                           L.gp19.t,  L.gp19.w,  L.gp19.lognb, L.gp19.logw, L.gp19.data};
+    constexpr size_t kBytes = sizeof(Brem32Smem<IMPL>) > sizeof(Brem64Smem<IMPL, kWarps * 32>)
+                                  ? sizeof(Brem32Smem<IMPL>)
+                                  : sizeof(Brem64Smem<IMPL, kWarps * 32>);
+    __shared__ __align__(16) unsigned char s_raw[kBytes];
+    Brem32Smem<IMPL>& S = *reinterpret_cast<Brem32Smem<IMPL>*>(s_raw);
+    const Gp19Table G19 = gp19_table(L);
     const bool prof = IMPL == 2 && G19.d3 <= kGp19MaxW;
     for (int k = threadIdx.x; k < kMaxM; k += blockDim.x)
     {
-        s_A1[k] = L.A1[k];
-        s_A2[k] = L.A2[k];
-        if (MIXED)
-        {
-            s_A1d[k] = dfm::from_double(L.A1[k]);
-            s_A2d[k] = dfm::from_double(L.A2[k]);
-        }
+        S.A1d[k] = dfm::from_double(L.A1[k]);
+        S.A2d[k] = dfm::from_double(L.A2[k]);
     }
     for (int k = threadIdx.x; k < L.ncell; k += blockDim.x)
-        s_cells[k] = L.cells[k];
+        S.cells[k] = L.cells[k];
     if (IMPL == 2 && prof)
         for (int k = threadIdx.x; k < G19.d3; k += blockDim.x)
         {
-            s_lw[k]  = G19.logw[k];
-            s_lwf[k] = (float)G19.logw[k];
-            if (MIXED)
-            {
-                s_wax[k] = G19.w[k];
-                s_iw[k]  = 1. / G19.w[k];
-                s_idl[k] = k + 1 < G19.d3 ? (float)(1. / (G19.logw[k + 1] - G19.logw[k])) : 0.f;
-            }
+            S.lw[k]  = G19.logw[k];
+            S.lwf[k] = (float)G19.logw[k];
+            S.wax[k] = G19.w[k];
+            S.iw[k]  = 1. / G19.w[k];
+            S.idl[k] = k + 1 < G19.d3 ? (float)(1. / (G19.logw[k + 1] - G19.logw[k])) : 0.f;
         }
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int wid  = threadIdx.x >> 5;
-    CellTab& C     = s_ct[WIDE ? 0 : wid];
+    CellTab& C     = S.ct[wid];
     const int M    = 2 * L.n2;
     const bool nbb = L.neglect_blocking != 0;
-    // cells of a point: thread t0, t0 + stride, ...
-    const int t0        = WIDE ? (int)threadIdx.x : lane;
-    const int stride    = WIDE ? NW * 32 : 32;
-    const int64_t q0    = WIDE ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * NW + wid;
-    const int64_t qstep = WIDE ? (int64_t)gridDim.x : (int64_t)gridDim.x * NW;
+    const int64_t qstep = (int64_t)gridDim.x * kWarps;
     const double wmin = IMPL == 2 ? G19.w[0] : 0., wmax = IMPL == 2 ? G19.w[G19.d3 - 1] : 0.;
 
-    for (int64_t q = q0; q < np; q += qstep)
+    for (int64_t q = (int64_t)blockIdx.x * kWarps + wid; q < np; q += qstep)
     {
         const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
         PointTab* P     = (PointTab*)(scratch + q * kTabWords);
-        if (redo_only && P->bredo != 1.)
-            continue; // uniform: one point per warp (per CTA when WIDE)
         const double T  = L.eos[1][p];
-        if (WIDE)
-            __syncthreads(); // the previous point's readers are done
-        else
-            __syncwarp();
-        if (!WIDE || wid == 0)
+        Gp19Warp& GW    = S.gw[IMPL == 2 ? wid : 0];
+        __syncwarp();
+        if (IMPL == 2)
         {
-            load_cell_tab(C, P, M, false, lane);
-            if (IMPL == 0)
-                warp_copy((double*)&C.hr, (const double*)&P->hr,
-                          sizeof(Hr98Point) / sizeof(double), lane);
+            if (prof)
+                warp_copy((double*)&GW.r, (const double*)gp19_record(P),
+                          sizeof(Gp19Record) / sizeof(double), lane);
+            __syncwarp();
+            if (!prof || GW.r.pt.regime == 3 || GW.r.pt.regime == 5)
+            {
+                if (lane == 0)
+                    P->bredo = 2.;
+                continue; // uniform: one point per warp
+            }
         }
-        if (WIDE)
-            __syncthreads();
-        else
-            __syncwarp();
-        if (IMPL == 0 && MIXED && lane == 0)
-            fp32::hr98_mixed_from(C.hr, &C.hm);
-        const double nbp = L.eos[0][p], yep = L.eos[2][p];
-        Gp19Warp& GW     = s_gw[IMPL == 2 && !WIDE ? wid : 0];
-        if (IMPL == 2 && prof)
+        load_cell_tab(C, P, M, lane);
+        if (IMPL == 0 && lane < 4)
+            fp32::hr98_mixed_part(P->hr, lane, &C.hm);
+        if (IMPL == 2)
         {
-            if (WIDE ? threadIdx.x == 0 : lane == 0)
-                gp19_point(G19, nbp, yep, T, &GW.pt);
-            if (WIDE)
-                __syncthreads();
-            else
-                __syncwarp();
-            const int np19 = (GW.pt.regime >= 2) ? 2 : 1;
-            if (t0 < np19)
-                gp19_profile_corners(G19, GW.pt.nbp, GW.pt.yep, GW.pt.pT[t0], &GW.cor[t0]);
-            if (WIDE)
-                __syncthreads();
-            else
-                __syncwarp();
-            for (int e = t0; e < np19 * G19.d3; e += stride)
+            const int np19 = (GW.r.pt.regime >= 2) ? 2 : 1;
+            for (int e = lane; e < np19 * G19.d3; e += 32)
             {
                 const int pr = e / G19.d3, l = e - pr * G19.d3;
-                const double v = gp19_profile_eval(G19, GW.cor[pr], l);
+                const double v = gp19_profile_eval(G19, GW.r.cor[pr], l);
                 GW.p[pr][l]  = v;
                 GW.pf[pr][l] = (float)v;
             }
-            if (WIDE)
-                __syncthreads();
-            else
-                __syncwarp();
         }
-        // Mixed cells in FP32 except the GP19 high-T extrapolation (which
-        // differences two table values); points whose cells the other
-        // reactions cancel go to FP64 below (the guard).
-        const bool fp32_cells =
-            MIXED && (IMPL == 0 || IMPL == 1 ||
-                      (IMPL == 2 && prof && GW.pt.regime != 3 && GW.pt.regime != 5));
-        double acc[16], bm[16];
+        __syncwarp();
+        double acc[16];
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk)
-            acc[kk] = bm[kk] = 0.;
-        bool redo = false;
-        if (fp32_cells)
+            acc[kk] = 0.;
         {
-            CellTab32& D = s_c32[MIXED ? wid : 0];
+            CellTab32& D = S.c32[wid];
             fill_tab32(D, C, M, lane);
             __syncwarp();
             double scale = (T * T) * (T * T);
@@ -1337,9 +1510,9 @@ __global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
                 scale *= C.brt06_pre;
             else
             {
-                scale *= 3. * GW.pt.C;
-                thr = (float)(1e-30 / GW.pt.C);
-                lt2 = (float)log2(T * 0.5);
+                scale *= 3. * GW.r.pt.C;
+                thr = (float)(1e-30 / GW.r.pt.C);
+                lt2 = (float)fx::log2(T * 0.5);
             }
             Acc32 A;
             A.clear();
@@ -1349,7 +1522,7 @@ __global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
             int pending = 0;
             for (int c = lane; c < L.ncell; c += 32)
             {
-                const uint32_t ab = s_cells[c];
+                const uint32_t ab = S.cells[c];
                 const int a = ab & 0xffffu, b = ab >> 16;
                 // x = (nu_a + nu_b) / T as hi + lo (accurate exponent)
                 const dfm::df xs = dfm::add(dfm::df{D.yh[a], D.yl[a]}, dfm::df{D.yh[b], D.yl[b]});
@@ -1370,16 +1543,16 @@ __global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
                     double wv = C.nu[a] + C.nu[b];
                     wv        = wv > wmax ? wmax : (wv < wmin ? wmin : wv);
                     float tw;
-                    const int l = gp19_bracket32(wv, s_lwf, s_wax, s_iw, s_idl, G19.d3, &tw);
+                    const int l = gp19_bracket32(wv, S.lwf, S.wax, S.iw, S.idl, G19.d3, &tw);
                     const float v0 = GW.pf[0][l] + tw * (GW.pf[0][l + 1] - GW.pf[0][l]);
-                    if (GW.pt.regime <= 1)
+                    if (GW.r.pt.regime <= 1)
                         Kab = v0;
                     else
                     {
                         const float v1 = GW.pf[1][l] + tw * (GW.pf[1][l + 1] - GW.pf[1][l]);
                         Kab = v0 * exp2f(log2f(v1 / v0) * lt2);
                         // regime 2 clips k2, k4 and s at 1e-30 (rare: exact FP64 cell)
-                        slow = GW.pt.regime == 2 && (v0 < thr || v1 < thr || Kab < thr);
+                        slow = GW.r.pt.regime == 2 && (v0 < thr || v1 < thr || Kab < thr);
                     }
                     Kab = fabsf(Kab);
                 }
@@ -1390,25 +1563,25 @@ __global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
                     double w = nua + nub;
                     w        = w > wmax ? wmax : (w < wmin ? wmin : w);
                     double tw;
-                    const int l = bracket_sorted<double>(log(w), s_lw, G19.d3, &tw);
+                    const int l = bracket_sorted<double>(log(w), S.lw, G19.d3, &tw);
                     const double v0 = GW.p[0][l] * (1. - tw) + GW.p[0][l + 1] * tw;
                     const double v1 = GW.p[1][l] * (1. - tw) + GW.p[1][l + 1] * tw;
                     double em, abv;
-                    gp19_cell(GW.pt, v0, v1, w, nua + nub, &em, &abv);
-                    Kab = (float)(abv / (3. * GW.pt.C));
-                    Kem = (float)(em / (3. * GW.pt.C));
+                    gp19_cell(GW.r.pt, v0, v1, w, nua + nub, &em, &abv);
+                    Kab = (float)(abv / (3. * GW.r.pt.C));
+                    Kem = (float)(em / (3. * GW.r.pt.C));
                 }
                 const dfm::df yab = dfm::mul(dfm::df{D.yh[a], D.yl[a]}, dfm::df{D.yh[b], D.yl[b]});
                 const dfm::df w4  = dfm::mul(yab, yab); // (y_a y_b)^2
-                const float P1    = cell_weight(w4, s_A1d[a], s_A1d[b]);
-                const float P2    = cell_weight(w4, s_A2d[a], s_A1d[b]);
+                const float P1    = cell_weight(w4, S.A1d[a], S.A1d[b]);
+                const float P2    = cell_weight(w4, S.A2d[a], S.A1d[b]);
                 if (L.stim)
                     add_cell32<true>(A, Kem, Kab, D.g[a], D.gm[a], D.g[b], D.gm[b], nbb, P1, P2);
                 else
                     add_cell32<false>(A, Kem, Kab, D.g[a], D.gm[a], D.g[b], D.gm[b], nbb, P1, P2);
                 if (a != b)
                 {
-                    const float P2r = cell_weight(w4, s_A2d[b], s_A1d[a]);
+                    const float P2r = cell_weight(w4, S.A2d[b], S.A1d[a]);
                     if (L.stim)
                         add_cell32<true>(A, Kem, Kab, D.g[b], D.gm[b], D.g[a], D.gm[a], nbb, P1,
                                          P2r);
@@ -1429,86 +1602,54 @@ __global__ void __launch_bounds__((WIDE ? 8 : kWarps) * 32)
             for (int kk = 0; kk < 16; ++kk)
                 acc[kk] = acc[kk] + (double)A.v[kk];
             // cells of both signs (occupation above 1 makes 1 - g negative), or
-            // a brem sum cancelling the pair sum or the beta rates: recompute
-            // this point in FP64
-            double other[16];
-            beta_in_sum_units(P, T, L.eos[7][p] / T, L.use_abs_em, false, other);
+            // a brem sum cancelling the pair sum or the beta rates: this point
+            // goes to FP64.  Each lane checks the moment whose total it holds.
+            double mg[16];
 #pragma unroll
             for (int kk = 0; kk < 16; ++kk)
-                other[kk] += add ? P->s2d[kk] : 0.;
-            redo = cancel_factor(acc, A.mag, scale, scale, other) > kMaxCancelBrem;
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
+                mg[kk] = (double)A.mag[kk];
+            const int idx      = sum_index(lane);
+            const double tot   = warp_sum16(acc, lane) * scale;
+            const double mag   = warp_sum16(mg, lane) * scale;
+            const double base  = add ? P->s2d[idx] : 0.;
+            const double other =
+                beta_in_sum_unit(P, T, L.eos[7][p] / T, L.use_abs_em, false, idx) + base;
+            const bool redo = __any_sync(0xffffffffu,
+                                         mag > 0. && mag > kMaxCancelBrem * fabs(tot + other));
+            if (lane == 0)
+                P->bredo = redo ? 2. : 0.;
+            if (!redo && !(lane & 1))
             {
-                acc[kk] = redo ? 0. : acc[kk] * scale;
-                bm[kk]  = redo ? 0. : warp_sum((double)A.mag[kk]) * scale;
-            }
-        }
-        if (!fp32_cells || redo)
-        {
-            for (int c = t0; c < L.ncell; c += stride)
-            {
-                const uint32_t ab = s_cells[c];
-                const int a = ab & 0xffffu, b = ab >> 16;
-                const double nua = C.nu[a], nub = C.nu[b];
-                double be, ba;
-                if (IMPL == 0)
-                    hr98_kernel(C.hr, nua, nub, &be, &ba);
-                else if (IMPL == 1)
-                    brt06_kernel(C.brt06_pre, T, nua, nub, &be, &ba);
-                else if (prof)
-                {
-                    double w = nua + nub;
-                    w        = w > wmax ? wmax : (w < wmin ? wmin : w);
-                    double tw;
-                    const int l = bracket_sorted<double>(log(w), s_lw, G19.d3, &tw);
-                    const double v0 = GW.p[0][l] * (1. - tw) + GW.p[0][l + 1] * tw;
-                    const double v1 =
-                        GW.pt.regime >= 2 ? GW.p[1][l] * (1. - tw) + GW.p[1][l + 1] * tw : 0.;
-                    gp19_cell(GW.pt, v0, v1, w, nua + nub, &be, &ba);
-                }
-                else
-                    gp19_kernel(G19, nbp, yep, T, nua, nub, &be, &ba);
-                const double Kem[4] = {be, be, be, be};
-                const double Kab[4] = {ba, ba, ba, ba};
-                const double w4 = (nua * nua) * (nub * nub);
-                const double W1 = s_A1[a] * s_A1[b];
-                if (L.stim)
-                    add_cell<true>(acc, Kem, Kab, C.g[a], C.g[b], nbb, w4, W1, s_A2[a] * s_A1[b]);
-                else
-                    add_cell<false>(acc, Kem, Kab, C.g[a], C.g[b], nbb, w4, W1, s_A2[a] * s_A1[b]);
-                if (a != b)
-                {
-                    if (L.stim)
-                        add_cell<true>(acc, Kem, Kab, C.g[b], C.g[a], nbb, w4, W1,
-                                       s_A2[b] * s_A1[a]);
-                    else
-                        add_cell<false>(acc, Kem, Kab, C.g[b], C.g[a], nbb, w4, W1,
-                                        s_A2[b] * s_A1[a]);
-                }
-            }
-        }
-        if (WIDE)
-            block_sum<NW>(acc, s_red, 0);
-        else
-        {
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
-                acc[kk] = warp_sum(acc[kk]);
-        }
-        if (WIDE ? threadIdx.x == 0 : lane == 0)
-        {
-            // a redo replaces the FP32 brem part of s2d by the FP64 one
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
-            {
-                const double base = add ? (redo_only ? P->s2d[kk] - P->sbrem[kk] : P->s2d[kk]) : 0.;
-                P->s2d[kk]   = base + acc[kk];
-                P->sbrem[kk] = acc[kk];
-                P->bmag[kk]  = bm[kk];
+                P->s2d[idx]   = base + tot;
+                P->sbrem[idx] = tot;
+                P->bmag[idx]  = mag;
             }
         }
     }
+    // the marked points of this CTA
+    Brem64Smem<IMPL, kWarps * 32>& S64 = *reinterpret_cast<Brem64Smem<IMPL, kWarps * 32>*>(s_raw);
+    __syncthreads(); // the FP32 tables' readers are done
+    bool ready = false;
+    for (int64_t qb = (int64_t)blockIdx.x * kWarps; qb < np; qb += qstep)
+        for (int64_t q = qb; q < qb + kWarps && q < np; ++q)
+        {
+            PointTab* P = (PointTab*)(scratch + q * kTabWords);
+            if (P->bredo != 2.)
+                continue; // uniform
+            if (!ready)
+            {
+                brem64_constants(S64, L);
+                ready = true;
+            }
+            const double tot = brem64_point(S64, L, P, L.pidx ? L.pidx[p0 + q] : p0 + q);
+            if (threadIdx.x < 32 && !(threadIdx.x & 1))
+            {
+                const int idx = sum_index(threadIdx.x);
+                P->s2d[idx]   = (add ? P->s2d[idx] : 0.) + tot;
+                P->sbrem[idx] = tot;
+                P->bmag[idx]  = 0.;
+            }
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -2761,46 +2902,42 @@ void launch_pair(const Step& S, cudaStream_t st, int sms, int redo_only)
              st>>>(*S.L, S.GA, S.p0, S.np, S.ws, redo_only);
 }
 
-template <bool MIXED, int IMPL, bool WIDE, bool MULTI>
-void launch_brem_impl(const Step& S, cudaStream_t st, int sms, int add, int redo_only)
+// Brem variant IMPL; redo is the FP64 pass over the points the mixed path's
+// final kernel marked.
+template <int IMPL, bool MULTI>
+void launch_brem_impl(const Step& S, cudaStream_t st, int sms, bool mixed, int add, bool redo)
 {
-    constexpr int threads = (WIDE ? 8 : kWarps) * 32;
-    const int64_t work    = WIDE ? S.np : (S.np + kWarps - 1) / kWarps;
-    const int gx          = grid_for(grey_brem_kernel<MIXED, IMPL, WIDE, MULTI>, threads, work, sms);
+    const unsigned gz = MULTI ? S.G : 1;
     phase_mark(kPhBrem, 0, st);
-    grey_brem_kernel<MIXED, IMPL, WIDE, MULTI><<<dim3(gx, 1, MULTI ? S.G : 1), threads, 0, st>>>(
-        *S.L, S.GA, S.p0, S.np, S.ws, add, redo_only);
+    if (mixed && !redo)
+    {
+        const auto k32     = grey_brem32_kernel<IMPL, MULTI>;
+        const int64_t work = (S.np + kWarps - 1) / kWarps;
+        k32<<<dim3(grid_for(k32, kWarps * 32, work, sms), 1, gz), kWarps * 32, 0, st>>>(
+            *S.L, S.GA, S.p0, S.np, S.ws, add);
+    }
+    else
+    {
+        const auto k64 = grey_brem_kernel<IMPL, MULTI>;
+        k64<<<dim3(grid_for(k64, kCellThreads, S.np, sms), 1, gz), kCellThreads, 0, st>>>(
+            *S.L, S.GA, S.p0, S.np, S.ws, add, redo ? 1 : 0);
+    }
     phase_mark(kPhBrem, 1, st);
 }
 
-template <bool MIXED, bool WIDE, bool MULTI>
-void launch_brem_set(const Step& S, cudaStream_t st, int sms, int add, int redo_only)
+// Single launch: the launch's variant; multi-group: one launch per variant
+// present (each returns at once for the other variants' groups).
+template <bool MULTI>
+cudaError_t launch_brem(const Step& S, cudaStream_t st, int sms, bool mixed, int add,
+                        bool redo = false)
 {
-    // single launch: the launch's variant; multi-group: one launch per variant
-    // present (each returns at once for the other variants' groups)
     const unsigned set = MULTI ? S.brem_set : 1u << S.L->brem_impl;
     if (set & 1u)
-        launch_brem_impl<MIXED, 0, WIDE, MULTI>(S, st, sms, add, redo_only);
+        launch_brem_impl<0, MULTI>(S, st, sms, mixed, add, redo);
     if (set & 2u)
-        launch_brem_impl<MIXED, 1, WIDE, MULTI>(S, st, sms, add, redo_only);
+        launch_brem_impl<1, MULTI>(S, st, sms, mixed, add, redo);
     if (set & 4u)
-        launch_brem_impl<MIXED, 2, WIDE, MULTI>(S, st, sms, add, redo_only);
-}
-
-// redo_only (the FP64 pass over the points the final kernel marked) runs a
-// point per CTA.
-template <bool MIXED, bool MULTI>
-cudaError_t launch_brem(const Step& S, cudaStream_t st, int sms, int add, int redo_only = 0)
-{
-    if constexpr (!MIXED)
-    {
-        if (redo_only)
-            launch_brem_set<false, true, MULTI>(S, st, sms, add, redo_only);
-        else
-            launch_brem_set<false, false, MULTI>(S, st, sms, add, redo_only);
-    }
-    else
-        launch_brem_set<true, false, MULTI>(S, st, sms, add, redo_only);
+        launch_brem_impl<2, MULTI>(S, st, sms, mixed, add, redo);
     return cudaGetLastError();
 }
 
@@ -2839,8 +2976,7 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
     }
     if (L.use_brem)
     {
-        err = L.mixed ? launch_brem<true, MULTI>(S, st, sms, L.use_pair) :
-                        launch_brem<false, MULTI>(S, st, sms, L.use_pair);
+        err = launch_brem<MULTI>(S, st, sms, L.mixed != 0, L.use_pair);
         if (err != cudaSuccess)
             return err;
     }
@@ -2887,7 +3023,7 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
             launch_pair<false, MULTI>(S, st, sms, 1);
             phase_mark(kPhPair, 1, st);
         }
-        if (L.use_brem && (err = launch_brem<false, MULTI>(S, st, sms, L.use_pair, 1)) !=
+        if (L.use_brem && (err = launch_brem<MULTI>(S, st, sms, true, L.use_pair, true)) !=
                               cudaSuccess)
             return err;
         phase_mark(kPhFinal, 0, st);

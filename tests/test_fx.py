@@ -27,6 +27,8 @@ void t_exp(const double* x, const double*, double* o, long n) { for (long i = 0;
 void t_pow(const double* x, const double* p, double* o, long n) { for (long i = 0; i < n; ++i) o[i] = fx::pow(x[i], p[i]); }
 void t_fd(const double* x, const double*, double* o, long n) { for (long i = 0; i < n; ++i) fx::fd_orders<0, 5>(x[i], o + 6 * i); }
 void t_phi(const double* x, const double*, double* o, long n) { for (long i = 0; i < n; ++i) fx::fd_orders<0, 5, true>(x[i], o + 6 * i); }
+void t_log(const double* x, const double*, double* o, long n) { for (long i = 0; i < n; ++i) o[i] = fx::log(x[i]); }
+void t_log2(const double* x, const double*, double* o, long n) { for (long i = 0; i < n; ++i) o[i] = fx::log2(x[i]); }
 void t_quot(const double* x, const double* p, double* o, long n) { for (long i = 0; i < n; ++i) o[i] = fx::quot(x[i], p[i]); }
 }
 """
@@ -87,6 +89,17 @@ def test_pow(call, p):
     x = np.concatenate([np.exp(rng.uniform(-40., 40., 600)), rng.uniform(0.99, 1.01, 100), [1.]])
     want = [mp.mpf(float(v)) ** mp.mpf(p) for v in x]
     assert worst(call("t_pow", x, np.full_like(x, p)), want) <= 2. ** -52 + abs(p) * 2. ** -55
+
+
+@pytest.mark.parametrize("name,base", [("t_log", None), ("t_log2", 2)])
+def test_log(call, name, base):
+    """Absolute error 2^-56 (the fixed-point unit) plus the result's rounding."""
+    mp.dps = 40
+    x = np.concatenate([np.exp(np.random.default_rng(5).uniform(-80., 80., 500)),
+                        np.linspace(0.98, 1.02, 101), [1e-300, 1e300]])
+    for g, v in zip(call(name, x), x):
+        want = mp.log(mp.mpf(float(v))) / (mp.log(base) if base else 1)
+        assert abs(mp.mpf(float(g)) - want) <= 2. ** -56 + 3. * 2. ** -53 * abs(want)
 
 
 def test_pow_outside_the_fixed_point_range(call):
