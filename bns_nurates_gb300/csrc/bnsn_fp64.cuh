@@ -383,37 +383,39 @@ BNSN_DI void total_nu_f4(double omega, const Distr& d, bool same_cf, double* g)
 // ---------------------------------------------------------------------------
 
 // weak_magnetism.hpp:45-104; reac 1: protons, 2: neutrons, 3: charged current.
-// The four quotients by (1 + tau) share one reciprocal (FP64 division is a
-// multi-instruction sequence on the FP64 pipe; the results move by an ulp).
+// The four quotients by (1 + tau) share one reciprocal; reciprocals are
+// fx::rcp's (3 FP64 operations and an approximation against 5.4; the results
+// move by an ulp).
 BNSN_DI void nuc_form_factors(double E, int reac, double* cv, double* ca, double* F2)
 {
     const double lamp = 1.793, lamn = -1.913;
     const double ehor = E * k::WmEScale;
-    const double tau  = 0.5 * (ehor * ehor) / (1. + ehor);
-    const double eta  = 1. / (1. + 5.6 * tau);
+    const double tau  = 0.5 * (ehor * ehor) * fx::rcp(1. + ehor);
+    const double eta  = fx::rcp(1. + 5.6 * tau);
     const double gq   = 1. + 4.97 * tau;
-    const double Gt   = 1. / ((gq * gq) * (1. + tau)); // G / (1 + tau)
+    const double Gt   = fx::rcp((gq * gq) * (1. + tau)); // G / (1 + tau)
     const double Fp1  = (1. + tau * (1. + lamp)) * Gt;
     const double Fp2  = lamp * Gt;
     const double Fn1  = tau * lamn * (1. - eta) * Gt;
     const double Fn2  = lamn * (1. + tau * eta) * Gt;
     const double d3   = 1. + 3.53 * tau;
+    const double id3  = fx::rcp(d3 * d3);
     if (reac == 1)
     {
         *cv = (0.5 - 2. * k::SinThW2) * Fp1 - 0.5 * Fn1;
-        *ca = 0.5 * (k::Ga - k::Gs) / (d3 * d3);
+        *ca = 0.5 * (k::Ga - k::Gs) * id3;
         *F2 = (0.5 - 2. * k::SinThW2) * Fp2 - 0.5 * Fn2;
     }
     else if (reac == 2)
     {
         *cv = (0.5 - 2. * k::SinThW2) * Fn1 - 0.5 * Fp1;
-        *ca = -0.5 * (k::Ga + k::Gs) / (d3 * d3);
+        *ca = -0.5 * (k::Ga + k::Gs) * id3;
         *F2 = (0.5 - 2. * k::SinThW2) * Fn2 - 0.5 * Fp2;
     }
     else
     {
         *cv = Fp1 - Fn1;
-        *ca = k::Ga / (d3 * d3);
+        *ca = k::Ga * id3;
         *F2 = Fp2 - Fn2;
     }
 }
@@ -431,7 +433,7 @@ BNSN_DI void wm_abs_em(double omega, double* R, double* Rbar)
                         (8. / 3.) * cv * F2 * e2 +
                         (5. / 3.) * e2 * (1. + (2. / 5.) * e) * (F2 * F2);
     const double tmp2 = 4. * (cv + F2) * ca * e * (1. + (4. / 3.) * e);
-    const double itmp3 = 1. / (((k::Gv * k::Gv) + 3. * (k::Ga * k::Ga)) * (b * b * b));
+    const double itmp3 = fx::rcp(((k::Gv * k::Gv) + 3. * (k::Ga * k::Ga)) * (b * b * b));
     *R    = (tmp1 + tmp2) * itmp3;
     *Rbar = (tmp1 - tmp2) * itmp3;
 }
@@ -467,9 +469,17 @@ BNSN_DI double eta_nn_abs(double n_in, double n_out, double mu_hat, double T)
 // Per-point constants of AbsOpacitySingleLep for electrons.
 struct BetaPoint
 {
-    double T, Qprime, etanp, etapn, mu_e, mu_p, mu_n;
+    double T, iT, Qprime, etanp, etapn, mu_e;
+    double mu0, mu1; // mu_p + mu_e - mu_n and mu_n - mu_p - mu_e, each as the reference rounds it
     int use_WM_ab, use_decay;
 };
+
+// x / T from the stored reciprocal, with one correction of the quotient.
+BNSN_DI double over_T(const BetaPoint& b, double x)
+{
+    const double q = x * b.iT;
+    return fma(fma(-b.T, q, x), b.iT, q);
+}
 
 BNSN_DI BetaPoint beta_point(double nb, double T, double yp, double yn,
                              double mu_p, double mu_n, double mu_e, double dU_in,
@@ -487,50 +497,42 @@ BNSN_DI BetaPoint beta_point(double nb, double T, double yp, double yn,
     b.etanp     = eta_nn_abs(nn, np, mu_np, T);
     b.etapn     = eta_nn_abs(np, nn, -mu_np, T);
     b.T         = T;
+    b.iT        = 1. / T;
     b.mu_e      = mu_e;
-    b.mu_p      = mu_p;
-    b.mu_n      = mu_n;
+    b.mu0       = mu_p + mu_e - mu_n;
+    b.mu1       = mu_n - mu_p - mu_e;
     b.use_WM_ab = use_WM_ab;
     b.use_decay = use_decay;
     return b;
 }
 
 // formulas_beta_iso.hpp:138-279 for one species: anti = 0 gives
-// (absorption, emission) of nu_e, anti = 1 of anti-nu_e, [s^-1].
+// (absorption, emission) of nu_e, anti = 1 of anti-nu_e, [s^-1].  E is the
+// energy of the captured lepton; E^2 sqrt(1 - m^2 / E^2) is |E| sqrt((E - m)(E +
+// m)).  The decay term (E < -m: a strong mean-field shift) is rare and takes
+// the complement of the other lepton's occupation.
 BNSN_DI void beta_rates(const BetaPoint& b, double omega, int anti, double* ab,
                         double* em)
 {
-    const double m2 = k::Me * k::Me;
-    double R = 1., Rbar = 1.;
-    if (b.use_WM_ab)
-        wm_abs_em(omega, &R, &Rbar);
-    double cap = 0., dec = 0.;
-    if (!anti)
+    const double E  = anti ? omega - b.Qprime : omega + b.Qprime;
+    const double mu = anti ? -b.mu_e : b.mu_e;
+    double rate     = 0.;
+    if (E - k::Me >= 0.)
     {
-        const double Ee = omega + b.Qprime, Ep = -Ee;
-        const double Ee2 = Ee * Ee, Ep2 = Ep * Ep;
-        const double fe = fermi_distr(Ee, b.T, +b.mu_e);
-        const double fp = fermi_distr(Ep, b.T, -b.mu_e);
-        if (Ee - k::Me >= 0.)
-            cap = Ee2 * sqrt(1. - m2 / Ee2) * R;
-        if (b.use_decay && Ep - k::Me >= 0.)
-            dec = Ep2 * sqrt(1. - m2 / Ep2);
-        *em = k::BetaConst * b.etapn * (cap * fe + dec * (1. - fp));
-        *ab = *em * safe_exp((omega - (b.mu_p + b.mu_e - b.mu_n)) / b.T);
+        double R = 1.;
+        if (b.use_WM_ab)
+        {
+            double Rn, Rb;
+            wm_abs_em(omega, &Rn, &Rb);
+            R = anti ? Rb : Rn;
+        }
+        const double f = fx::rcp(safe_exp(over_T(b, E - mu)) + 1.);
+        rate = E * sqrt((E - k::Me) * (E + k::Me)) * R * f;
     }
-    else
-    {
-        const double Ep = omega - b.Qprime, Ee = -Ep;
-        const double Ee2 = Ee * Ee, Ep2 = Ep * Ep;
-        const double fe = fermi_distr(Ee, b.T, +b.mu_e);
-        const double fp = fermi_distr(Ep, b.T, -b.mu_e);
-        if (Ep - k::Me >= 0.)
-            cap = Ep2 * sqrt(1. - m2 / Ep2) * Rbar;
-        if (b.use_decay && Ee - k::Me >= 0.)
-            dec = Ee2 * sqrt(1. - m2 / Ee2);
-        *em = k::BetaConst * b.etanp * (cap * fp + dec * (1. - fe));
-        *ab = *em * safe_exp((omega - (b.mu_n - b.mu_p - b.mu_e)) / b.T);
-    }
+    else if (b.use_decay && -E - k::Me >= 0.)
+        rate = -E * sqrt((E - k::Me) * (E + k::Me)) * (1. - fermi_distr(-E, b.T, -mu));
+    *em = k::BetaConst * (anti ? b.etanp : b.etapn) * rate;
+    *ab = *em * safe_exp(over_T(b, omega - (anti ? b.mu1 : b.mu0)));
 }
 
 // ---------------------------------------------------------------------------
@@ -549,20 +551,27 @@ BNSN_DI double eta_nn_sc(double nb, double temp, double yN)
 }
 
 // formulas_beta_iso.hpp:411-507: IsoScattTotal with the two eta_NN factors
-// precomputed per point.
+// precomputed per point: eta_NN (C0 R0 - C1 R1 / 3) per nucleon, where C0 R0 =
+// IsoConst (cv^2 + 3 ca^2 + 1.5 (e F2)^2 + 2 e^2 cv F2) and C1 R1 alike
+// (weak_magnetism.hpp:165-210): the normalisations cancel.
 BNSN_DI double iso_scatt_total(double omega, double eta_pp, double eta_nn,
                                bool use_wm)
 {
-    double R0p = 1., R1p = 1., R0n = 1., R1n = 1.;
-    if (use_wm)
-    {
-        wm_scatt(omega, 1, &R0p, &R1p);
-        wm_scatt(omega, 2, &R0n, &R1n);
-    }
     constexpr double third = 1. / 3.;
-    const double pr = eta_pp * ((k::IsoC0p * R0p) - (k::IsoC1p * R1p) * third);
-    const double ne = eta_nn * ((k::IsoC0n * R0n) - (k::IsoC1n * R1n) * third);
-    return pr + ne;
+    if (!use_wm)
+        return eta_pp * (k::IsoC0p - k::IsoC1p * third) + eta_nn * (k::IsoC0n - k::IsoC1n * third);
+    double s[2];
+#pragma unroll
+    for (int r = 1; r <= 2; ++r)
+    {
+        double cv, ca, F2;
+        nuc_form_factors(omega, r, &cv, &ca, &F2);
+        const double e   = omega * k::WmEScale;
+        const double cv2 = cv * cv, ca2 = ca * ca, ef = e * F2, x = (e * e) * cv * F2;
+        const double ef2 = ef * ef;
+        s[r - 1] = (cv2 + 3. * ca2 + 1.5 * ef2 + 2. * x) - (cv2 - ca2 - 2. * ef2 - 4. * x) * third;
+    }
+    return k::IsoConst * (eta_pp * s[0] + eta_nn * s[1]);
 }
 
 // formulas_beta_iso.hpp:523-564 (l = 0)

@@ -35,8 +35,6 @@
 
 #include <cuda_runtime.h>
 
-#include <cstddef>
-
 #include "bnsn_df.cuh"
 #include "bnsn_fp32.cuh"
 #include "bnsn_mixed.cuh"
@@ -148,13 +146,6 @@ __device__ __forceinline__ int sum_index(int lane)
     return ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
 }
 
-__device__ __forceinline__ double total_nu_f1(double omega, const Distr& d, int s)
-{
-    const double ft = fermi_distr(omega, d.temp_t[s], d.temp_t[s] * d.eta_t[s]);
-    const double fn = d.beta_f[s] * fx::pow(omega, d.c_f[s]) * fx::exp(-omega / d.temp_f[s]);
-    return d.w_t[s] * ft + d.w_f[s] * fn;
-}
-
 // Cooperative copy of `words` doubles (lane-strided, coalesced).
 __device__ __forceinline__ void warp_copy(double* __restrict__ dst,
                                           const double* __restrict__ src, int words,
@@ -185,101 +176,46 @@ __device__ __forceinline__ void beta_scales(double T, double eta_e, const double
     }
 }
 
-// ---------------------------------------------------------------------------
-// point constants: the per-point quantities that do not depend on an energy
-// node, as 12 independent tasks, one thread per (point, task) with the task
-// in blockIdx.y (every warp runs one code path):
-//   0..3  distribution parameters of species 0..3 (or a copy of the given ones)
-//   4, 5  F_0..F_5 and FermiDistr(0, 1, .) at +eta_e, -eta_e
-//   6..8  HR98 channel constants; 9: HR98 point constants; 10: BRT06 prefactor
-//   6, 7  GP19: the point's regime and the corners of its two profiles
-//   11    eta_NN of protons and neutrons (iso scattering)
-// written straight into the point's scratch record, whose header the prelude
-// then loads.  Inside the one-warp-per-point prelude these tasks ran on one to
-// four lanes each, one after the other.
-// ---------------------------------------------------------------------------
-constexpr int kPointTasks = 12;
-
-template <bool MULTI = false>
-__global__ void __launch_bounds__(128)
-    grey_point_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
-                      int64_t np, double* __restrict__ scratch)
+// The scale of species s alone, from its F_4, F_5.
+__device__ __forceinline__ double beta_scale(double f4, double f5, double T, double eta_e, int s)
 {
-    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
-    if (MULTI)
-    {
-        const GroupChunk& gcz = GA.gc[blockIdx.z];
-        p0      = gcz.p0;
-        np      = gcz.np;
-        scratch = gcz.ws;
-    }
-    const int task = blockIdx.y;
-    const bool gp19 = L.use_brem && L.brem_impl == 2 && L.gp19.d3 <= kGp19MaxW;
-    if ((task >= 6 && task <= 9 && !(L.use_brem && L.brem_impl == 0) && !(gp19 && task < 8)) ||
-        (task == 10 && !(L.use_brem && L.brem_impl == 1)) || (task == 11 && !L.use_iso))
-        return;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < np;
-         q += (int64_t)gridDim.x * blockDim.x)
-    {
-        const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
-        PointTab* P     = (PointTab*)(scratch + q * kTabWords);
-        const double nb = L.eos[0][p], T = L.eos[1][p];
-        if (task < 4)
-        {
-            const int s = task;
-            Distr& d    = P->d;
-            if (L.has_distr)
-            {
-#pragma unroll
-                for (int f = 0; f < 7; ++f)
-                    (&d.w_t[0])[f * 4 + s] = L.distr[f * 4 + s][p];
-            }
-            else
-                distr_species(L.m1[s][p], L.m1[4 + s][p], L.m1[8 + s][p], L.gamma36, &d.w_t[s],
-                              &d.temp_t[s], &d.eta_t[s], &d.w_f[s], &d.temp_f[s], &d.c_f[s],
-                              &d.beta_f[s]);
-        }
-        else if (task < 6)
-        {
-            const int e     = task - 4;
-            const double et = e ? -L.eos[7][p] / T : L.eos[7][p] / T;
-            double f[6];
-            fdi_orders<0, 5>(et, f);
-#pragma unroll
-            for (int kk = 0; kk < 6; ++kk)
-                P->fe[e][kk] = f[kk];
-            P->fd0[e] = fermi_distr(0., 1., et);
-        }
-        else if (task < 9 && gp19)
-        {
-            const Gp19Table G = {L.gp19.d0, L.gp19.d1, L.gp19.d2, L.gp19.d3,
-                                 L.gp19.nb, L.gp19.ye, L.gp19.t,  L.gp19.w,
-                                 L.gp19.lognb, L.gp19.logw, L.gp19.data};
-            Gp19Point pt;
-            gp19_point(G, nb, L.eos[2][p], T, &pt);
-            Gp19Record* R = gp19_record(P);
-            if (task == 6)
-                R->pt = pt;
-            if (task == 6 || pt.regime >= 2)
-                gp19_profile_corners(G, pt.nbp, pt.yep, pt.pT[task - 6], &R->cor[task - 6]);
-        }
-        else if (task < 9)
-            P->hr.ch[task - 6] = hr98_channel(nb, L.eos[4][p], L.eos[3][p], T, task - 6);
-        else if (task == 9)
-            hr98_point_common(nb, T, L.use_medium != 0, &P->hr); // leaves hr.ch alone
-        else if (task == 10)
-            P->brt06_pre = brt06_point(nb, T, L.eos[4][p], L.eos[3][p]);
-        else
-        {
-            P->eta_pp = eta_nn_sc(nb, T, L.eos[3][p]);
-            P->eta_nn = eta_nn_sc(nb, T, L.eos[4][p]);
-        }
-    }
+    if (eta_e > -30. && eta_e < 30.)
+        return T * f5 / f4;
+    return (eta_e > 30.) == (s == 0) ? T * eta_e * 0.8333333333333333 : T * 5.;
 }
 
-// Words of the record header written by grey_point_kernel (everything
-// before the energy tables).
-constexpr int kHeadWords = (int)(offsetof(PointTab, nu) / sizeof(double));
+// One species' occupation constants (distribution.hpp:298-315) for x = omega / u:
+// g = wt / (1 + e^{x rt - eta}) + kf x^cf e^{-x rf}.
+struct Occ64
+{
+    double rt, eta, rf, wt, kf, cf;
+};
+
+__device__ __forceinline__ void occ64_from(const Distr& d, int s, double u, Occ64* o)
+{
+    o->rt  = u / d.temp_t[s];
+    o->eta = d.eta_t[s];
+    o->rf  = u / d.temp_f[s];
+    o->wt  = d.w_t[s];
+    o->cf  = d.c_f[s];
+    o->kf  = d.w_f[s] * (u == 1. ? d.beta_f[s] : d.beta_f[s] * fx::pow(u, d.c_f[s]));
+}
+
+// One species at x, p = x^cf.
+__device__ __forceinline__ double occ64_one(const Occ64& o, double x, double p)
+{
+    const double ft = fx::rcp(safe_exp(fma(x, o.rt, -o.eta)) + 1.);
+    return fma(o.wt, ft, o.kf * (p * fx::exp(-x * o.rf)));
+}
+
+// Four species at x; xc = x^c0, common: every cf is c0.
+__device__ __forceinline__ void occ64_eval(const Occ64* o, double x, double xc, bool common,
+                                           double* g)
+{
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+        g[s] = occ64_one(o[s], x, common ? xc : fx::pow(x, o[s].cf));
+}
 
 // TotalNuF of one species in FP32 with its exponent arguments in df form
 // (distribution.hpp:298-315): x rt - eta_t and P0 + c_f log x - x rf.  The
@@ -349,11 +285,163 @@ __device__ __forceinline__ void total_nu_q(dfm::df W, dfm::df LW, const NuSpecie
         total_nu_one(W, LW, sp[s], g[s], gm[s]);
 }
 
+// What the prelude needs beyond the record's header, written by the point kernel
+// into the words of the sums that later phases fill (s2d .. bmag).
+struct PreRecord
+{
+    double rt[4], rf[4], kf[4]; // Occ64 of omega in MeV
+    NuSpecies nu[4];            // mixed path
+    BetaPoint bp;
+    double t[6], lt[6];         // energy scales of beta (2) and iso (4), their logs (mixed)
+};
+static_assert(sizeof(PreRecord) <= 76 * sizeof(double), "PreRecord overlay (s2d .. bmag)");
+
+__device__ __forceinline__ PreRecord* pre_record(PointTab* P)
+{
+    return reinterpret_cast<PreRecord*>(&P->s2d[0]);
+}
+
 // ---------------------------------------------------------------------------
-// prelude
+// point constants: the per-point quantities that do not depend on an energy
+// node, as 13 independent tasks, one thread per (point, task) with the task
+// in blockIdx.y (every warp runs one code path):
+//   0..3  distribution parameters of species 0..3 (or a copy of the given ones),
+//         their occupation constants and the iso integral's energy scale
+//   4, 5  F_0..F_5 and FermiDistr(0, 1, .) at +eta_e, -eta_e, the beta scale
+//   6..8  HR98 channel constants; 9: HR98 point constants; 10: BRT06 prefactor
+//   6, 7  GP19: the point's regime and the corners of its two profiles
+//   11    eta_NN of protons and neutrons (iso scattering)
+//   12    beta-process constants
+// written straight into the point's scratch record, whose header the prelude
+// then loads.  Inside the one-warp-per-point prelude these tasks ran on one to
+// four lanes each, one after the other.
 // ---------------------------------------------------------------------------
+constexpr int kPointTasks = 13;
+
 template <bool MULTI = false>
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void __launch_bounds__(128)
+    grey_point_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
+                      int64_t np, double* __restrict__ scratch)
+{
+    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
+    if (MULTI)
+    {
+        const GroupChunk& gcz = GA.gc[blockIdx.z];
+        p0      = gcz.p0;
+        np      = gcz.np;
+        scratch = gcz.ws;
+    }
+    const int task = blockIdx.y;
+    const bool gp19 = L.use_brem && L.brem_impl == 2 && L.gp19.d3 <= kGp19MaxW;
+    if ((task >= 6 && task <= 9 && !(L.use_brem && L.brem_impl == 0) && !(gp19 && task < 8)) ||
+        (task == 10 && !(L.use_brem && L.brem_impl == 1)) || (task == 11 && !L.use_iso) ||
+        (task == 12 && !L.use_abs_em))
+        return;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < np;
+         q += (int64_t)gridDim.x * blockDim.x)
+    {
+        const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
+        PointTab* P     = (PointTab*)(scratch + q * kTabWords);
+        const double nb = L.eos[0][p], T = L.eos[1][p];
+        if (task < 4)
+        {
+            const int s = task;
+            Distr& d    = P->d;
+            if (L.has_distr)
+            {
+#pragma unroll
+                for (int f = 0; f < 7; ++f)
+                    (&d.w_t[0])[f * 4 + s] = L.distr[f * 4 + s][p];
+            }
+            else
+                distr_species(L.m1[s][p], L.m1[4 + s][p], L.m1[8 + s][p], L.gamma36, &d.w_t[s],
+                              &d.temp_t[s], &d.eta_t[s], &d.w_f[s], &d.temp_f[s], &d.c_f[s],
+                              &d.beta_f[s]);
+            PreRecord* R = pre_record(P);
+            Occ64 o;
+            occ64_from(d, s, 1., &o);
+            R->rt[s] = o.rt;
+            R->rf[s] = o.rf;
+            R->kf[s] = o.kf;
+            const double ns = L.m1[s][p];
+            const double t  = (ns > k::ThresholdN) ? (L.m1[4 + s][p] / ns) : 1.5 * T;
+            R->t[2 + s] = t;
+            if (L.mixed)
+            {
+                nu_species(d, s, 1., 0., &R->nu[s]);
+                R->lt[2 + s] = fx::log(t);
+            }
+        }
+        else if (task < 6)
+        {
+            const int e     = task - 4;
+            const double et = e ? -L.eos[7][p] / T : L.eos[7][p] / T;
+            double f[6];
+            fdi_orders<0, 5>(et, f);
+#pragma unroll
+            for (int kk = 0; kk < 6; ++kk)
+                P->fe[e][kk] = f[kk];
+            P->fd0[e]      = fermi_distr(0., 1., et);
+            const double t = beta_scale(f[4], f[5], T, e ? -et : et, e);
+            pre_record(P)->t[e] = t;
+            if (L.mixed)
+                pre_record(P)->lt[e] = fx::log(t);
+        }
+        else if (task < 9 && gp19)
+        {
+            const Gp19Table G = {L.gp19.d0, L.gp19.d1, L.gp19.d2, L.gp19.d3,
+                                 L.gp19.nb, L.gp19.ye, L.gp19.t,  L.gp19.w,
+                                 L.gp19.lognb, L.gp19.logw, L.gp19.data};
+            Gp19Point pt;
+            gp19_point(G, nb, L.eos[2][p], T, &pt);
+            Gp19Record* R = gp19_record(P);
+            if (task == 6)
+                R->pt = pt;
+            if (task == 6 || pt.regime >= 2)
+                gp19_profile_corners(G, pt.nbp, pt.yep, pt.pT[task - 6], &R->cor[task - 6]);
+        }
+        else if (task < 9)
+            P->hr.ch[task - 6] = hr98_channel(nb, L.eos[4][p], L.eos[3][p], T, task - 6);
+        else if (task == 9)
+            hr98_point_common(nb, T, L.use_medium != 0, &P->hr); // leaves hr.ch alone
+        else if (task == 10)
+            P->brt06_pre = brt06_point(nb, T, L.eos[4][p], L.eos[3][p]);
+        else if (task == 12)
+            pre_record(P)->bp = beta_point(nb, T, L.eos[3][p], L.eos[4][p], L.eos[5][p],
+                                           L.eos[6][p], L.eos[7][p], L.eos[9][p], L.eos[10][p],
+                                           L.use_dU, L.use_dm_eff, L.use_WM_ab, L.use_decay);
+        else
+        {
+            P->eta_pp = eta_nn_sc(nb, T, L.eos[3][p]);
+            P->eta_nn = eta_nn_sc(nb, T, L.eos[4][p]);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// prelude: the energy tables of the double integral (m1_opacities.hpp:783-787),
+// the beta integrals (m1_opacities.hpp:93-237, integration.hpp:805-844) and the
+// iso-energetic scattering integrals (m1_opacities.hpp:39-91, integration.hpp:
+// 770-802).  Four warps share a point; a warp takes every fourth of the point's
+// units of 32 nodes of one kind (2 units of occupations, 3 of Fermi integrals, 3
+// of beta and 5 of iso nodes at n = 20), so that warps do not diverge and a
+// single point's chain is four units long.  FP64 pipe bound.  8,192 points, n =
+// 20: 1.09 -> 0.68 ms, mixed 0.81 -> 0.44 ms; one point, n = 10: 94 -> 46 us
+// (with the point kernel).
+// ---------------------------------------------------------------------------
+constexpr int kPreWarps = 4;
+
+struct PreSmem
+{
+    double B1[kMaxM], x1[kMaxM];       // 1-D nodes x_i and 1 / x_i, their weights
+    double y2[kMaxM], lx1[kMaxM];      // 2-D nodes nu / T, log of the 1-D nodes
+    double red[kPreWarps][12];
+    Occ64 occ[4];
+    PreRecord R;
+};
+
+template <bool MULTI = false>
+__global__ void __launch_bounds__(kPreWarps * 32, 4)
     grey_prelude_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
                         int64_t np, double* __restrict__ scratch)
 {
@@ -365,207 +453,170 @@ __global__ void __launch_bounds__(kWarps * 32)
         np      = gcz.np;
         scratch = gcz.ws;
     }
-    __shared__ double s_B1[kMaxM], s_x1[kMaxQ], s_x2[kMaxQ], s_lx1[kMaxQ];
-    __shared__ PointTab s_tab[kWarps];
-    // mixed path: the occupation of the beta and iso items in FP32
-    // (total_nu_one), omega in MeV; the FP64 path keeps total_nu_f1
-    __shared__ NuSpecies s_nu[kWarps][4];
+    __shared__ PreSmem S;
+    const int n1 = L.n1, n2 = L.n2, M = 2 * n2, M1 = 2 * n1;
     for (int k = threadIdx.x; k < kMaxM; k += blockDim.x)
-        s_B1[k] = L.B1[k];
-    for (int k = threadIdx.x; k < kMaxQ; k += blockDim.x)
     {
-        s_x1[k]  = L.x1[k];
-        s_x2[k]  = L.x2[k];
-        s_lx1[k] = L.lx1[k];
+        S.B1[k] = L.B1[k];
+        if (k < M1)
+        {
+            const int i = k < n1 ? k : k - n1;
+            S.x1[k]     = k < n1 ? L.x1[i] : 1. / L.x1[i];
+            S.lx1[k]    = k < n1 ? L.lx1[i] : -L.lx1[i];
+        }
+        if (k < M)
+            S.y2[k] = k < n2 ? k::TempMultiple * L.x2[k] : k::TempMultiple / L.x2[k - n2];
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    PointTab& W    = s_tab[threadIdx.x >> 5];
-    NuSpecies* Snu = s_nu[threadIdx.x >> 5];
-    const int n1 = L.n1, n2 = L.n2, M = 2 * n2;
-    const int64_t nwarp = (int64_t)gridDim.x * kWarps;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const bool mixed = L.mixed != 0;
+    // units of each kind
+    const int u_node = (L.use_pair || L.use_brem) ? (M + 31) / 32 : 0;
+    const int u_fdi  = u_node + (L.use_pair && !mixed ? (2 * M + 31) / 32 : 0);
+    const int u_beta = u_fdi + (L.use_abs_em ? (2 * M1 + 31) / 32 : 0);
+    const int u_iso  = u_beta + (L.use_iso ? (4 * M1 + 31) / 32 : 0);
 
-    for (int64_t q = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5); q < np; q += nwarp)
+    for (int64_t q = blockIdx.x; q < np; q += gridDim.x)
     {
         const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
-        const double nb = L.eos[0][p], T = L.eos[1][p];
-        const double yp = L.eos[3][p], yn = L.eos[4][p];
-        const double mu_e = L.eos[7][p];
-        const double eta_e = mu_e / T;
-
-        // header of the record (distribution, F_k(+-eta_e), brem and iso
-        // constants) from grey_point_kernel
-        __syncwarp();
-        warp_copy((double*)&W, scratch + q * kTabWords, kHeadWords, lane);
-        __syncwarp();
-        if (lane == 0)
+        PointTab* P     = (PointTab*)(scratch + q * kTabWords);
+        const double T = L.eos[1][p], eta_e = L.eos[7][p] / T;
+        __syncthreads(); // the previous point's readers are done
+        for (int k = threadIdx.x; k < (int)(sizeof(PreRecord) / sizeof(double)); k += blockDim.x)
+            ((double*)&S.R)[k] = ((const double*)pre_record(P))[k];
+        if (threadIdx.x >= 96 && threadIdx.x < 100)
         {
-            const double c0 = W.d.c_f[0];
-            W.same_cf = ((W.d.c_f[1] == c0) && (W.d.c_f[2] == c0) && (W.d.c_f[3] == c0)) ? 1. : 0.;
+            const int s  = threadIdx.x - 96;
+            S.occ[s].eta = P->d.eta_t[s];
+            S.occ[s].wt  = P->d.w_t[s];
+            S.occ[s].cf  = P->d.c_f[s];
         }
-        else if (L.mixed && lane >= 8 && lane < 12)
-            nu_species(W.d, lane - 8, 1., 0., &Snu[lane - 8]);
-        __syncwarp();
-        const bool same_cf = W.same_cf != 0.;
-
-        // energy tables of the double integral (m1_opacities.hpp:783-787)
-        if (L.use_pair || L.use_brem)
+        __syncthreads();
+        if (threadIdx.x < 4)
         {
-            const double t2d = k::TempMultiple * T;
-            for (int a = lane; a < M; a += 32)
+            const int s = threadIdx.x;
+            S.occ[s].rt = S.R.rt[s];
+            S.occ[s].rf = S.R.rf[s];
+            S.occ[s].kf = S.R.kf[s];
+        }
+        __syncthreads();
+        const double c0    = S.occ[0].cf;
+        const bool same_cf = S.occ[1].cf == c0 && S.occ[2].cf == c0 && S.occ[3].cf == c0;
+        if (threadIdx.x == 0)
+            P->same_cf = same_cf ? 1. : 0.;
+        const double eta_pp = P->eta_pp, eta_nn = P->eta_nn;
+        // a lane's species is fixed: lane & 1 in the beta units, lane & 3 in the iso units
+        double bn_em = 0., bj_em = 0., bn_ab = 0., bj_ab = 0., iso_sum = 0.;
+#pragma unroll 1
+        for (int u = wid; u < u_iso; u += kPreWarps)
+        {
+            if (u < u_node)
             {
-                const int i     = a < n2 ? a : a - n2;
-                const double nu = a < n2 ? t2d * s_x2[i] : t2d / s_x2[i];
-                W.nu[a]         = nu;
-                W.y[a]          = nu / T;
-                total_nu_f4(nu, W.d, same_cf, W.g[a]);
-            }
-            if (L.use_pair && !L.mixed) // the mixed pair phase needs no F tables
-            {
-                for (int qq = lane; qq < 2 * M; qq += 32)
+                const int a = u * 32 + lane;
+                if (a < M)
                 {
-                    const int a     = qq >> 1;
-                    const int i     = a < n2 ? a : a - n2;
-                    const double nu = a < n2 ? t2d * s_x2[i] : t2d / s_x2[i];
-                    const double y  = nu / T;
-                    if (qq & 1)
-                        fdi_orders<1, 5>(eta_e + y, W.fp[a]);
+                    const double y = S.y2[a], nu = y * T;
+                    double g[4];
+                    occ64_eval(S.occ, nu, same_cf ? fx::pow(nu, c0) : 0., same_cf, g);
+                    P->nu[a] = nu;
+                    P->y[a]  = y;
+#pragma unroll
+                    for (int s = 0; s < 4; ++s)
+                        P->g[a][s] = g[s];
+                }
+            }
+            else if (u < u_fdi)
+            {
+                const int t = (u - u_node) * 32 + lane;
+                if (t < 2 * M)
+                {
+                    const double y = S.y2[t >> 1];
+                    double f[5];
+                    fdi_orders<1, 5>(t & 1 ? eta_e + y : eta_e - y, f);
+                    double* o = t & 1 ? P->fp[t >> 1] : P->fm[t >> 1];
+#pragma unroll
+                    for (int k = 0; k < 5; ++k)
+                        o[k] = f[k];
+                }
+            }
+            else
+            {
+                const bool beta = u < u_beta;
+                const int it    = (u - (beta ? u_fdi : u_beta)) * 32 + lane;
+                const int s     = it & (beta ? 1 : 3), a = it >> (beta ? 1 : 2);
+                if (a < M1)
+                {
+                    const int sc    = beta ? s : 2 + s;
+                    const double nu = S.R.t[sc] * S.x1[a];
+                    double g;
+                    if (mixed)
+                    {
+                        float gf, gmf;
+                        total_nu_one(dfm::from_double(nu), dfm::from_double(S.R.lt[sc] + S.lx1[a]),
+                                     S.R.nu[s], gf, gmf);
+                        g = gf;
+                    }
                     else
-                        fdi_orders<1, 5>(eta_e - y, W.fm[a]);
+                        g = occ64_one(S.occ[s], nu, fx::pow(nu, S.occ[s].cf));
+                    const double nu2 = nu * nu, w2 = S.B1[a] * nu2;
+                    if (beta)
+                    {
+                        double ab, em;
+                        beta_rates(S.R.bp, nu, s, &ab, &em);
+                        if (L.stim)
+                            ab = ab + em;
+                        const double ev = w2 * em, av = w2 * (g * ab);
+                        bn_em += ev;
+                        bn_ab += av;
+                        bj_em = fma(nu, ev, bj_em);
+                        bj_ab = fma(nu, av, bj_ab);
+                    }
+                    else
+                    {
+                        // mixed: the weak-magnetism factors in FP32 (positive terms; the
+                        // iso sum enters kappa_s alone, no other reaction cancels it)
+                        const double iso =
+                            (mixed && L.use_WM_sc)
+                                ? k::IsoConst *
+                                      (eta_pp * (double)fp32::iso_wm_factor((float)nu, 1) +
+                                       eta_nn * (double)fp32::iso_wm_factor((float)nu, 2))
+                                : iso_scatt_total(nu, eta_pp, eta_nn, L.use_WM_sc != 0);
+                        iso_sum = fma(4. * k::Pi * (nu2 * nu) * w2, g * iso, iso_sum);
+                    }
                 }
             }
         }
-
-        // beta processes (m1_opacities.hpp:93-237, integration.hpp:805-844)
-        if (L.use_abs_em)
+        // lanes of one species; then the four warps
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1)
+            iso_sum += __shfl_xor_sync(0xffffffffu, iso_sum, o);
         {
-            double sb[2];
-            beta_scales(T, eta_e, W.fe, sb);
-            const BetaPoint bp =
-                beta_point(nb, T, yp, yn, L.eos[5][p], L.eos[6][p], mu_e, L.eos[9][p],
-                           L.eos[10][p], L.use_dU, L.use_dm_eff, L.use_WM_ab, L.use_decay);
-            double acc[8];
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-                acc[kk] = 0.;
-            const int m1n = 2 * n1;
-            const double lsb0 = L.mixed ? log(sb[0]) : 0., lsb1 = L.mixed ? log(sb[1]) : 0.;
-            for (int it = lane; it < 2 * m1n; it += 32)
-            {
-                const int s = it >= m1n;
-                const int a = it - s * m1n;
-                const int i = a < n1 ? a : a - n1;
-                const double t  = sb[s];
-                const double nu = a < n1 ? t * s_x1[i] : t / s_x1[i];
-                double g;
-                if (L.mixed)
-                {
-                    float gf, gmf;
-                    const double lnu = (s ? lsb1 : lsb0) + (a < n1 ? s_lx1[i] : -s_lx1[i]);
-                    total_nu_one(dfm::from_double(nu), dfm::from_double(lnu), Snu[s], gf, gmf);
-                    g = gf;
-                }
-                else
-                    g = total_nu_f1(nu, W.d, s);
-                double ab, em;
-                beta_rates(bp, nu, s, &ab, &em);
-                if (L.stim)
-                    ab = ab + em;
-                const double nu2 = nu * nu;
-                const double ev  = nu2 * em;
-                const double av  = nu2 * g * ab;
-                const double wn  = s_B1[a];
-                const double wj  = wn * nu;
-                if (s == 0)
-                {
-                    acc[0] += wn * ev;
-                    acc[2] += wj * ev;
-                    acc[4] += wn * av;
-                    acc[6] += wj * av;
-                }
-                else
-                {
-                    acc[1] += wn * ev;
-                    acc[3] += wj * ev;
-                    acc[5] += wn * av;
-                    acc[7] += wj * av;
-                }
-            }
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-                acc[kk] = warp_sum(acc[kk]);
-            if (lane == 0)
-            {
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk)
-                    W.sbeta[kk] = acc[kk];
-            }
+            const bool hi = (lane & 16) != 0, hj = (lane & 8) != 0;
+            const double a0 = (hi ? bn_ab : bn_em) +
+                              __shfl_xor_sync(0xffffffffu, hi ? bn_em : bn_ab, 16);
+            const double a1 = (hi ? bj_ab : bj_em) +
+                              __shfl_xor_sync(0xffffffffu, hi ? bj_em : bj_ab, 16);
+            double b = (hj ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hj ? a0 : a1, 8);
+            b += __shfl_xor_sync(0xffffffffu, b, 4);
+            b += __shfl_xor_sync(0xffffffffu, b, 2);
+            // sbeta order: n_em, j_em, n_ab, j_ab of species 0, 1
+            if ((lane & 6) == 0)
+                S.red[wid][(hi ? 4 : 0) + (hj ? 2 : 0) + (lane & 1)] = b;
+            if (lane < 4)
+                S.red[wid][8 + lane] = iso_sum;
         }
-
-        // iso-energetic scattering (m1_opacities.hpp:39-91, integration.hpp:770-802)
-        if (L.use_iso)
+        __syncthreads();
+        if (threadIdx.x < 12)
         {
-            double s_iso[4];
+            const int k = threadIdx.x;
+            double t    = S.red[0][k];
 #pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                const double ns = L.m1[s][p];
-                s_iso[s] = (ns > k::ThresholdN) ? (L.m1[4 + s][p] / ns) : 1.5 * T;
-            }
-            double acc[4] = {0., 0., 0., 0.};
-            double lsi[4] = {0., 0., 0., 0.};
-            if (L.mixed)
-            {
-#pragma unroll
-                for (int s = 0; s < 4; ++s)
-                    lsi[s] = log(s_iso[s]);
-            }
-            const int m1n = 2 * n1;
-            for (int it = lane; it < 4 * m1n; it += 32)
-            {
-                const int s = it / m1n;
-                const int a = it - s * m1n;
-                const int i = a < n1 ? a : a - n1;
-                const double t   = s == 0 ? s_iso[0] : s == 1 ? s_iso[1] : s == 2 ? s_iso[2] : s_iso[3];
-                const double nu  = a < n1 ? t * s_x1[i] : t / s_x1[i];
-                double g;
-                if (L.mixed)
-                {
-                    float gf, gmf;
-                    const double ls  = s == 0 ? lsi[0] : s == 1 ? lsi[1] : s == 2 ? lsi[2] : lsi[3];
-                    const double lnu = ls + (a < n1 ? s_lx1[i] : -s_lx1[i]);
-                    total_nu_one(dfm::from_double(nu), dfm::from_double(lnu), Snu[s], gf, gmf);
-                    g = gf;
-                }
-                else
-                    g = total_nu_f1(nu, W.d, s);
-                // mixed: the weak-magnetism factors in FP32 (positive terms; the
-                // iso sum enters kappa_s alone, no other reaction cancels it)
-                const double iso =
-                    (L.mixed && L.use_WM_sc)
-                        ? k::IsoConst * (W.eta_pp * (double)fp32::iso_wm_factor((float)nu, 1) +
-                                         W.eta_nn * (double)fp32::iso_wm_factor((float)nu, 2))
-                        : iso_scatt_total(nu, W.eta_pp, W.eta_nn, L.use_WM_sc != 0);
-                const double aux = 4. * k::Pi * (nu * nu) * (nu * nu) * nu * iso;
-                const double v   = g * aux * s_B1[a];
-                if (s == 0) acc[0] += v;
-                else if (s == 1) acc[1] += v;
-                else if (s == 2) acc[2] += v;
-                else acc[3] += v;
-            }
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-                acc[kk] = warp_sum(acc[kk]);
-            if (lane == 0)
-            {
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    W.siso[kk] = acc[kk];
-            }
+            for (int w = 1; w < kPreWarps; ++w)
+                t += S.red[w][k];
+            if (k < 8)
+                P->sbeta[k] = t;
+            else
+                P->siso[k - 8] = t;
         }
-        __syncwarp();
-        warp_copy(scratch + q * kTabWords, (const double*)&W, kTabWords, lane);
-        __syncwarp();
     }
 }
 
@@ -721,9 +772,7 @@ __device__ __forceinline__ double beta_in_sum_unit(const PointTab* P, double T, 
     const int s = idx & 3, m = idx >> 2; // species; number em, ab, energy em, ab
     if (!use_abs_em || s >= 2)
         return 0.;
-    const bool big = (eta_e > 30.) == (s == 0);
-    const double sb = (eta_e > -30. && eta_e < 30.) ? T * P->fe[s][5] / P->fe[s][4]
-                                                    : (big ? T * eta_e * 0.8333333333333333 : T * 5.);
+    const double sb = beta_scale(P->fe[s][4], P->fe[s][5], T, eta_e, s);
     const double t2d = k::TempMultiple * T, t2 = t2d * t2d;
     const double un  = k::FourPiHc3 * (to_nes ? 8. * t2 : t2);
     const double u   = (m >= 2 && !to_nes) ? un * t2d : un;
@@ -2056,37 +2105,6 @@ __global__ void __launch_bounds__(kNesAccWarps * 32, 2)
 // points, and launches of fewer points than the chip has warps to fill.
 // ---------------------------------------------------------------------------
 
-// One species' occupation constants for x = omega / T: g = wt / (1 + e^{x rt -
-// eta}) + kf x^cf e^{-x rf}.
-struct Occ64
-{
-    double rt, eta, rf, wt, kf, cf;
-};
-
-__device__ __forceinline__ void occ64_from(const Distr& d, int s, double T, Occ64* o)
-{
-    o->rt  = T / d.temp_t[s];
-    o->eta = d.eta_t[s];
-    o->rf  = T / d.temp_f[s];
-    o->wt  = d.w_t[s];
-    o->cf  = d.c_f[s];
-    o->kf  = d.w_f[s] * (d.beta_f[s] * fx::pow(T, d.c_f[s]));
-}
-
-// TotalNuF (distribution.hpp:298-315) of four species at x; xc = x^0.6,
-// common: every cf is 0.6 (the reconstruction's value).
-__device__ __forceinline__ void occ64_eval(const Occ64* o, double x, double xc, bool common,
-                                           double* g)
-{
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-    {
-        const double ft = fx::rcp(safe_exp(fma(x, o[s].rt, -o[s].eta)) + 1.);
-        const double p  = common ? xc : fx::pow(x, o[s].cf);
-        g[s] = fma(o[s].wt, ft, o[s].kf * (p * fx::exp(-x * o[s].rf)));
-    }
-}
-
 template <int NW>
 struct Nes64Smem
 {
@@ -2949,7 +2967,6 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
 {
     const OpacityLaunch& L = *S.L;
     const int64_t np       = S.np;
-    const int64_t wb       = (np + kWarps - 1) / kWarps;
     const unsigned gz      = MULTI ? S.G : 1;
     cudaError_t err        = cudaSuccess;
     phase_mark(kPhPrelude, 0, st);
@@ -2962,8 +2979,8 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
     phase_mark(kPhPrelude, 1, st);
     phase_mark(kPhPrelude, 0, st);
     grey_prelude_kernel<MULTI>
-        <<<dim3(grid_for(grey_prelude_kernel<MULTI>, kWarps * 32, wb, sms), 1, gz), kWarps * 32,
-           0, st>>>(L, S.GA, S.p0, np, S.ws);
+        <<<dim3(grid_for(grey_prelude_kernel<MULTI>, kPreWarps * 32, np, sms), 1, gz),
+           kPreWarps * 32, 0, st>>>(L, S.GA, S.p0, np, S.ws);
     phase_mark(kPhPrelude, 1, st);
     if (L.use_pair)
     {
