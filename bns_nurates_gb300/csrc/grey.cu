@@ -2094,36 +2094,35 @@ __global__ void __launch_bounds__(kNesAccWarps * 32, 2)
 // bracket with a division each (~560 instructions); both leptons' A and B
 // combine into the four species' kernels afterwards, R(w', w) costs nothing,
 // and the NEPSExpFunc factors, weights and w^0.6 sit in the CTA's item table.
-// Bound by the FP64 pipe (~180 operations an item) beside the integer work of
-// its exponentials and Fermi integrals; 8,192 points at n = 20: 5.4 ms (the
-// separate brackets with the same Fermi integrals ~14.5 ms).  The items follow the
-// host's order of ascending w', which keeps a warp's lanes in the same
-// regime of the Fermi integrals.
+// The items follow the host's order of ascending w', which keeps a warp's lanes in
+// the same regime of the Fermi integrals.
 //
-// A point per warp of 16-warp CTAs (the 51 KB item table is shared by 16
-// points), or (WIDE) a point per 8-warp CTA: the mixed path's few flagged
-// points, and launches of fewer points than the chip has warps to fill.
+// Bound by the FP64 pipe (~200 operations an item) beside the integer work of
+// its exponentials and Fermi integrals.  Two warps share a point in 16-warp CTAs
+// (the 38 KB item table serves 8 points; one warp per point left the last of
+// 3.4 waves over 8,192 points 60% empty), or (WIDE) eight in 8-warp CTAs: the
+// mixed path's few flagged points, and launches with fewer points than the chip
+// has warps to fill.  8,192 points, n = 20: 5.55 -> 3.69 ms.
 // ---------------------------------------------------------------------------
 
-template <int NW>
+template <bool WIDE>
 struct Nes64Smem
 {
-    double w[kMaxQ * kMaxQ * 2], wp[kMaxQ * kMaxQ * 2];   // w, w'
-    double ka[kMaxQ * kMaxQ * 2], m[kMaxQ * kMaxQ * 2];   // 24 weight e / (1 - e), 24 weight
-    double wc[kMaxQ * kMaxQ * 2], wpc[kMaxQ * kMaxQ * 2]; // w^0.6, w'^0.6
-    Occ64 occ[NW][4];
-    double fe[NW][2][6], fd0[NW][2];
-    double red[NW][16];
+    static constexpr int kItems = kMaxQ * kMaxQ * 2;
+    static constexpr int kNW    = WIDE ? 8 : 16;  // warps of the CTA
+    static constexpr int kWPP   = WIDE ? 8 : 2;   // warps per point
+    static constexpr int kPts   = kNW / kWPP;
+    double w[kItems], wp[kItems];   // w, w'
+    double ka[kItems], m[kItems];   // 24 weight e / (1 - e), 24 weight
+    double wc[kItems], wpc[kItems]; // w^0.6, w'^0.6
+    Occ64 occ[kPts][4];
+    double fe[kPts][2][6], fd0[kPts][2];
+    double red[kPts][kWPP][16];
+    int twin[kPts];
 };
 
-template <bool WIDE>
-__host__ __device__ constexpr int nes64_warps()
-{
-    return WIDE ? 8 : 16;
-}
-
 template <bool WIDE, bool MULTI = false>
-__global__ void __launch_bounds__(nes64_warps<WIDE>() * 32, WIDE ? 2 : 1)
+__global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
     grey_nes64_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
                       int64_t np, double* __restrict__ scratch, int flagged)
 {
@@ -2137,17 +2136,21 @@ __global__ void __launch_bounds__(nes64_warps<WIDE>() * 32, WIDE ? 2 : 1)
     }
     if (MULTI && !L.use_inel)
         return;
-    constexpr int NW = nes64_warps<WIDE>();
+    using Smem = Nes64Smem<WIDE>;
+    constexpr int kStride = Smem::kWPP * 32;
     extern __shared__ __align__(16) unsigned char nes_smem_raw[];
-    Nes64Smem<NW>& S = *reinterpret_cast<Nes64Smem<NW>*>(nes_smem_raw);
+    Smem& S        = *reinterpret_cast<Smem*>(nes_smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int slot = wid / Smem::kWPP, wsub = wid - slot * Smem::kWPP;
     const int n2 = L.n2, nn2 = n2 * n2, nit = 2 * nn2;
     const bool nbb = L.neglect_blocking != 0, stim = L.stim != 0;
-    const int t0        = WIDE ? (int)threadIdx.x : lane;
-    const int stride    = WIDE ? NW * 32 : 32;
-    const int64_t q0    = WIDE ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * NW + wid;
-    const int64_t qstep = WIDE ? (int64_t)gridDim.x : (int64_t)gridDim.x * NW;
-    const int own       = WIDE ? 0 : wid;
+    // the warps of a point (every thread of them runs the same iterations)
+    const auto point_sync = [&]() {
+        if (WIDE)
+            __syncthreads();
+        else
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(kStride) : "memory");
+    };
     const auto make_table = [&]() {
         // w = c x_i (1 -+ x_j) for r = 0 and c (1 -+ x_j) / x_i for r = 1
         // (m1_opacities.hpp:880-905), c = 2 x 2.182
@@ -2177,7 +2180,8 @@ __global__ void __launch_bounds__(nes64_warps<WIDE>() * 32, WIDE ? 2 : 1)
         make_table();
         __syncthreads();
     }
-    for (int64_t q = q0; q < np; q += qstep)
+    for (int64_t q = (int64_t)blockIdx.x * Smem::kPts + slot; q < np;
+         q += (int64_t)gridDim.x * Smem::kPts)
     {
         const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
         PointTab* P     = (PointTab*)(scratch + q * kTabWords);
@@ -2189,108 +2193,130 @@ __global__ void __launch_bounds__(nes64_warps<WIDE>() * 32, WIDE ? 2 : 1)
             table = true;
         }
         const double T = L.eos[1][p], mu_e = L.eos[7][p];
-        if (WIDE)
-            __syncthreads(); // the previous point's readers are done
-        else
-            __syncwarp();
-        if (!WIDE || wid == 0)
+        point_sync(); // the previous point's readers are done
+        if (wsub == 0)
         {
+            const Distr& d = P->d;
             if (lane < 4)
-                occ64_from(P->d, lane, T, &S.occ[own][lane]);
+                occ64_from(d, lane, T, &S.occ[slot][lane]);
             else if (lane >= 16 && lane < 28)
-                (&S.fe[own][0][0])[lane - 16] = (&P->fe[0][0])[lane - 16];
+                (&S.fe[slot][0][0])[lane - 16] = (&P->fe[0][0])[lane - 16];
             else if (lane >= 28 && lane < 30)
-                S.fd0[own][lane - 28] = P->fd0[lane - 28];
+                S.fd0[slot][lane - 28] = P->fd0[lane - 28];
+            else if (lane == 30) // heavy-lepton neutrinos evolved as one species
+                S.twin[slot] = d.w_t[2] == d.w_t[3] && d.temp_t[2] == d.temp_t[3] &&
+                               d.eta_t[2] == d.eta_t[3] && d.w_f[2] == d.w_f[3] &&
+                               d.temp_f[2] == d.temp_f[3] && d.c_f[2] == d.c_f[3] &&
+                               d.beta_f[2] == d.beta_f[3];
         }
-        if (WIDE)
-            __syncthreads();
-        else
-            __syncwarp();
-        const Occ64* occ  = S.occ[own];
+        point_sync();
+        const Occ64* occ  = S.occ[slot];
         const bool common = occ[0].cf == k::CF && occ[1].cf == k::CF && occ[2].cf == k::CF &&
                             occ[3].cf == k::CF;
-        NepsPoint NP;
-        NP.T    = T;
-        NP.pre  = k::NepsConst * (T * T);
-        NP.eta0 = mu_e / T;
-        NP.eta1 = -mu_e / T;
-        NP.fd00 = S.fd0[own][0];
-        NP.fd01 = S.fd0[own][1];
-        NP.fe0  = S.fe[own][0];
-        NP.fe1  = S.fe[own][1];
+        const int nocc   = S.twin[slot] ? 3 : 4;
+        const double pre = k::NepsConst * (T * T), eta_e = mu_e / T;
         double acc[16];
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk)
             acc[kk] = 0.;
 #pragma unroll 1
-        for (int it = t0; it < nit; it += stride)
+        for (int it = wsub * 32 + lane; it < nit; it += kStride)
         {
             const double w = S.w[it], wp = S.wp[it];
-            const double dl = wp - w, sm = w + wp, pr = w * wp;
-            const double hs = 0.5 * sm, hp = 0.5 * pr, qp = hp * hp; // qp = P^2 / 4
-            const double hx = 0.5 * wp, hy = 0.5 * w;
+            const double dl = wp - w, sm = w + wp, hp = 0.5 * (w * wp), qp = hp * hp; // P^2 / 4
             double U = 0., V = 0.; // A of e- + B of e+, B of e- + A of e+
-            double ct[4] = {0., 0., 0., 0.};
 #pragma unroll 1
             for (int e = 0; e < 2; ++e)
             {
-                const double eta = e ? NP.eta1 : NP.eta0;
-                const double* fe = S.fe[own][e];
-                if (w > eta * 1e-3)
+                const double eta = e ? -eta_e : eta_e, thr = eta * 1e-3;
+                const double* fe = S.fe[slot][e];
+                double A, B;
+                if (w > thr)
                 {
                     double a[5], b[5], f[3];
                     fx::fd_orders<1, 5, true>(eta - wp, a);
                     fx::fd_orders<1, 5, true>(eta - w, b);
                     fx::fd_orders<3, 5, true>(eta - dl, f);
-                    const double E3 = fma(fe[3], 1. / 6., -f[0]);
+                    const double E3 = fma(fe[3], 0.5 / 6., -0.5 * f[0]); // E_3 / 2
                     const double E4 = fma(fe[4], 1. / 24., -f[1]);
                     const double ED = fma(fe[5], 1. / 120., -f[2]) + (a[4] - b[4]);
-                    double A = fma(wp, fma(hx, E3, E4), ED);
-                    A        = fma(sm, fma(hp, a[1] - b[1], fma(hs, a[2] - b[2], a[3] - b[3])), A);
-                    A        = fma(qp, a[0] - b[0], A);
-                    const double B = fma(w, fma(hy, E3, -E4), ED);
-                    U += e ? B : A;
-                    V += e ? A : B;
+                    A = fma(wp, fma(wp, E3, E4), ED);
+                    A = fma(sm, fma(hp, a[1] - b[1], fma(0.5 * sm, a[2] - b[2], a[3] - b[3])), A);
+                    A = fma(qp, a[0] - b[0], A);
+                    B = fma(w, fma(w, E3, -E4), ED);
                 }
                 else
                 {
-                    // the reference's Taylor branches (kernel_nes.hpp:82-132)
-                    double r1[4], r2[4];
-                    neps_taylor(NP, e, w, wp, wp, w, -1, 1, r1, r2);
-#pragma unroll
-                    for (int s = 0; s < 4; ++s)
-                        ct[s] = fma(r1[s], qp * (-1. / 6.), ct[s]);
+                    // the reference's Taylor branches (kernel_nes.hpp:82-132) in the
+                    // same units: R = -(24 / P^2) pre (b1 A + b2 B)
+                    const double fd0 = S.fd0[slot][e];
+                    const double x = wp, y = w, y2 = y * y, xy = x * y, x2 = x * x;
+                    const double c = qp * y * (-1. / 6.) * fx::rcp(x2);
+                    if (x > thr)
+                    {
+                        double f[3];
+                        fdi_orders<0, 2>(eta - x, f);
+                        const double f0 = f[2] - fe[2], f1 = f[1], f2 = fe[1];
+                        const double f3 = f[0] + y * fermi_distr(0., 1., eta - x) * (1. / 6.);
+                        const double f4 = fe[0] - y * fd0 * (1. / 6.);
+                        A = c * (2. * f0 + (y + 4. * x) * f1 + (3. * y - 4. * x) * f2 +
+                                 (0.2 * y2 + xy + 2. * x2) * f3 - (1.2 * y2 - 3. * xy + 2. * x2) * f4);
+                        B = c * (2. * f0 + 3. * y * f1 + y * f2 + 1.2 * y2 * f3 - 0.2 * y2 * f4);
+                    }
+                    else
+                    {
+                        const double u =
+                            4. * fe[1] + fd0 * (11. * y2 - 25. * xy + 20. * x2) * (1. / 30.);
+                        const double v = (2. * x - y) * fe[0];
+                        A = -dl * c * (u + v);
+                        B = -dl * c * (u - v);
+                    }
                 }
+                U += e ? B : A;
+                V += e ? A : B;
             }
             constexpr double bp = k::NepsBPlus, bm = k::NepsBMinus, bz = k::NepsBZero;
-            const double c[4] = {fma(bp, U, fma(bz, V, ct[0])), fma(bp, V, fma(bz, U, ct[1])),
-                                 fma(bm, U, fma(bz, V, ct[2])), fma(bm, V, fma(bz, U, ct[3]))};
+            const double zU = bz * U, zV = bz * V;
+            const double c[4] = {fma(bp, U, zV), fma(bp, V, zU), fma(bm, U, zV), fma(bm, V, zU)};
             double g[4], gb[4];
-            occ64_eval(occ, w, S.wc[it], common, g);
-            occ64_eval(occ, wp, S.wpc[it], common, gb);
-            const double ka = S.ka[it], kb = ka + S.m[it];
+            const double wc = S.wc[it], wpc = S.wpc[it];
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+            {
+                if (s < nocc)
+                {
+                    g[s]  = occ64_one(occ[s], w, common ? wc : fx::pow(w, occ[s].cf));
+                    gb[s] = occ64_one(occ[s], wp, common ? wpc : fx::pow(wp, occ[s].cf));
+                }
+                else
+                {
+                    g[s]  = g[2];
+                    gb[s] = gb[2];
+                }
+            }
+            const double m = S.m[it], ka = S.ka[it], kb = ka + m;
 #pragma unroll
             for (int s = 0; s < 4; ++s)
             {
                 // emission and absorption kernels nu -> nubar; nubar -> nu swaps them
                 const double ke = kb * c[s], kk = ka * c[s];
                 const double e1 = ke * gb[s], e2 = kk * g[s];
-                const double a1 = nbb ? kk : kk * (1. - gb[s]);
-                const double a2 = nbb ? ke : ke * (1. - g[s]);
                 double EM1, AB1, EM2, AB2;
                 if (stim)
                 {
-                    AB1 = g[s] * (e1 + a1);
+                    // e + a = e + k (1 - g), the difference of the kernels in one product
+                    const double mc = nbb ? 0. : m * c[s];
                     EM1 = e1;
-                    AB2 = gb[s] * (e2 + a2);
                     EM2 = e2;
+                    AB1 = g[s] * (nbb ? e1 + kk : fma(gb[s], mc, kk));
+                    AB2 = gb[s] * (nbb ? e2 + ke : fma(-g[s], mc, ke));
                 }
                 else
                 {
-                    AB1 = g[s] * a1;
                     EM1 = (1. - g[s]) * e1;
-                    AB2 = gb[s] * a2;
                     EM2 = (1. - gb[s]) * e2;
+                    AB1 = g[s] * (nbb ? kk : kk * (1. - gb[s]));
+                    AB2 = gb[s] * (nbb ? ke : ke * (1. - g[s]));
                 }
                 acc[s] += EM1 + EM2;
                 acc[4 + s] += AB1 + AB2;
@@ -2298,27 +2324,18 @@ __global__ void __launch_bounds__(nes64_warps<WIDE>() * 32, WIDE ? 2 : 1)
                 acc[12 + s] = fma(w, AB1, fma(wp, AB2, acc[12 + s]));
             }
         }
-        const double T4   = (T * T) * (T * T);
-        double tot        = warp_sum16(acc, lane);
-        const int idx     = sum_index(lane);
-        const double unit = NP.pre * T4 * (idx >= 8 ? T : 1.);
-        if (!WIDE)
+        const double tot = warp_sum16(acc, lane);
+        const int idx    = sum_index(lane);
+        if (!(lane & 1))
+            S.red[slot][wsub][idx] = tot;
+        point_sync();
+        if (wsub == 0 && !(lane & 1))
         {
-            if (!(lane & 1))
-                P->snes[idx] = tot * unit;
-        }
-        else
-        {
-            if (!(lane & 1))
-                S.red[wid][idx] = tot;
-            __syncthreads();
-            if (wid == 0 && !(lane & 1))
-            {
-                double t = 0.;
-                for (int v = 0; v < NW; ++v)
-                    t += S.red[v][idx];
-                P->snes[idx] = t * unit;
-            }
+            double t = S.red[slot][0][idx];
+#pragma unroll
+            for (int v = 1; v < Smem::kWPP; ++v)
+                t += S.red[slot][v][idx];
+            P->snes[idx] = t * (pre * ((T * T) * (T * T)) * (idx >= 8 ? T : 1.));
         }
     }
 }
@@ -2885,14 +2902,18 @@ cudaError_t launch_nes_fast(const Step& S, cudaStream_t st, int sms)
     return cudaGetLastError();
 }
 
-// Launches of fewer points run a point per CTA where the kernel has that form.
-constexpr int64_t kWidePoints = 1024;
+// Launches of fewer points than this many per SM run a point per CTA in the NES
+// kernels.  A chip-wide round of the two-warp form is 8 points per SM and takes
+// as long for one point as for 1,216; a point per CTA takes time in proportion.
+// FP64, n = 6, 10, 20: a round 81, 162, 555 us; a point per CTA 70, 113, 351 us at
+// 600 points, 101, 163, 518 us at 900.
+constexpr int64_t kWidePointsPerSm = 5;
 
 template <bool WIDE, bool MULTI>
 cudaError_t launch_nes64(const Step& S, cudaStream_t st, int sms, int flagged)
 {
-    constexpr int NW      = nes64_warps<WIDE>();
-    constexpr int smem    = (int)sizeof(Nes64Smem<NW>);
+    constexpr int NW      = Nes64Smem<WIDE>::kNW;
+    constexpr int smem    = (int)sizeof(Nes64Smem<WIDE>);
     const auto kernel     = grey_nes64_kernel<WIDE, MULTI>;
     const cudaError_t e   = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  smem);
@@ -2903,7 +2924,8 @@ cudaError_t launch_nes64(const Step& S, cudaStream_t st, int sms, int flagged)
             cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
-    const int64_t work = WIDE ? S.np : (S.np + NW - 1) / NW;
+    constexpr int kPts = Nes64Smem<WIDE>::kPts;
+    const int64_t work = (S.np + kPts - 1) / kPts;
     int64_t cap        = (int64_t)((double)sms * per_sm * g_grid_scale);
     cap                = cap < 1 ? 1 : cap;
     const int grid     = (int)(work < cap ? (work > 0 ? work : 1) : cap);
@@ -3019,7 +3041,7 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
         else
         {
             phase_mark(kPhNeps, 0, st);
-            err = np < kWidePoints ? launch_nes64<true, MULTI>(S, st, sms, 0)
+            err = np < kWidePointsPerSm * sms ? launch_nes64<true, MULTI>(S, st, sms, 0)
                                    : launch_nes64<false, MULTI>(S, st, sms, 0);
             if (err != cudaSuccess)
                 return err;
