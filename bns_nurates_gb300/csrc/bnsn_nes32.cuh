@@ -318,8 +318,8 @@ __device__ __forceinline__ Lepton make_lepton(double eta)
     const double lref = eta < 0. ? eta : 0.;
     Lp.eta = dfm::from_double(eta);
     Lp.vsh = dfm::from_double(eta - lref);
-    Lp.A   = (float)exp(lref);
-    Lp.iA  = (float)exp(-lref);
+    Lp.A   = (float)fx::exp(lref);
+    Lp.iA  = (float)fx::exp(-lref);
     Lp.z1  = Lp.eta.hi - kEdge;
     Lp.z2  = Lp.eta.hi + kEdge;
     Lp.thr = dfm::from_double(eta * 1e-3);

@@ -271,18 +271,36 @@ __device__ __forceinline__ void nu_species(const Distr& d, int s, double xscale_
     S->wf   = (float)d.w_f[s];
     S->etat = dfm::from_double(d.eta_t[s]);
     S->rt   = dfm::from_double(xscale_inv / d.temp_t[s]);
-    const double lbf = d.beta_f[s] > 0. ? log(d.beta_f[s]) : 0.;
+    const double lbf = d.beta_f[s] > 0. ? fx::log(d.beta_f[s]) : 0.;
     S->P0   = dfm::from_double(lbf - d.c_f[s] * lxs);
     S->cf   = dfm::from_double(d.c_f[s]);
     S->rf   = dfm::from_double(xscale_inv / d.temp_f[s]);
 }
 
-__device__ __forceinline__ void total_nu_q(dfm::df W, dfm::df LW, const NuSpecies* sp, float* g,
-                                           float* gm)
+// The four species; with nocc = 3 species 3 equals species 2.
+__device__ __forceinline__ void total_nu_q(dfm::df W, dfm::df LW, const NuSpecies* sp, int nocc,
+                                           float* g, float* gm)
 {
 #pragma unroll
     for (int s = 0; s < 4; ++s)
-        total_nu_one(W, LW, sp[s], g[s], gm[s]);
+    {
+        if (s < nocc)
+            total_nu_one(W, LW, sp[s], g[s], gm[s]);
+        else
+        {
+            g[s]  = g[2];
+            gm[s] = gm[2];
+        }
+    }
+}
+
+// Heavy-lepton neutrinos and antineutrinos evolved as one species: their
+// occupations are the same.
+__device__ __forceinline__ bool species_twins(const Distr& d)
+{
+    return d.w_t[2] == d.w_t[3] && d.temp_t[2] == d.temp_t[3] && d.eta_t[2] == d.eta_t[3] &&
+           d.w_f[2] == d.w_f[3] && d.temp_f[2] == d.temp_f[3] && d.c_f[2] == d.c_f[3] &&
+           d.beta_f[2] == d.beta_f[3];
 }
 
 // What the prelude needs beyond the record's header, written by the point kernel
@@ -683,22 +701,6 @@ __device__ __forceinline__ double cancel_factor_tot(const double* acc, const dou
         const double sc  = s < 8 ? scale : scale_e;
         const double m   = mag[s] * sc;
         const double tot = fabs(acc[s] * sc + other[s]);
-        amp = fmax(amp, m > 0. ? m / tot : 1.);
-    }
-    return amp;
-}
-
-// (element by element: the 16 warp sums are not held at once)
-__device__ __forceinline__ double cancel_factor(const double* acc, const float* mag, double scale,
-                                                double scale_e, const double* other)
-{
-    double amp = 1.;
-#pragma unroll
-    for (int s = 0; s < 16; ++s)
-    {
-        const double sc  = s < 8 ? scale : scale_e;
-        const double m   = warp_sum((double)mag[s]) * sc;
-        const double tot = fabs(warp_sum(acc[s]) * sc + other[s]);
         amp = fmax(amp, m > 0. ? m / tot : 1.);
     }
     return amp;
@@ -2117,8 +2119,9 @@ struct Nes64Smem
     double wc[kItems], wpc[kItems]; // w^0.6, w'^0.6
     Occ64 occ[kPts][4];
     double fe[kPts][2][6], fd0[kPts][2];
-    double red[kPts][kWPP][16];
+    double red[kPts][2][16];
     int twin[kPts];
+    double terms[WIDE ? 16 : 1][WIDE ? kNW * 32 : 1]; // EM1, AB1, EM2, AB2 of a round's items
 };
 
 template <bool WIDE, bool MULTI = false>
@@ -2204,10 +2207,7 @@ __global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
             else if (lane >= 28 && lane < 30)
                 S.fd0[slot][lane - 28] = P->fd0[lane - 28];
             else if (lane == 30) // heavy-lepton neutrinos evolved as one species
-                S.twin[slot] = d.w_t[2] == d.w_t[3] && d.temp_t[2] == d.temp_t[3] &&
-                               d.eta_t[2] == d.eta_t[3] && d.w_f[2] == d.w_f[3] &&
-                               d.temp_f[2] == d.temp_f[3] && d.c_f[2] == d.c_f[3] &&
-                               d.beta_f[2] == d.beta_f[3];
+                S.twin[slot] = species_twins(d);
         }
         point_sync();
         const Occ64* occ  = S.occ[slot];
@@ -2219,9 +2219,9 @@ __global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk)
             acc[kk] = 0.;
-#pragma unroll 1
-        for (int it = wsub * 32 + lane; it < nit; it += kStride)
-        {
+        // EM1[4], AB1[4], EM2[4], AB2[4] of item it; products are rounded here so
+        // that both forms of the kernel add the same numbers
+        const auto item_terms = [&](int it, double* o) {
             const double w = S.w[it], wp = S.wp[it];
             const double dl = wp - w, sm = w + wp, hp = 0.5 * (w * wp), qp = hp * hp; // P^2 / 4
             double U = 0., V = 0.; // A of e- + B of e+, B of e- + A of e+
@@ -2300,41 +2300,88 @@ __global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
             {
                 // emission and absorption kernels nu -> nubar; nubar -> nu swaps them
                 const double ke = kb * c[s], kk = ka * c[s];
-                const double e1 = ke * gb[s], e2 = kk * g[s];
-                double EM1, AB1, EM2, AB2;
+                const double e1 = __dmul_rn(ke, gb[s]), e2 = __dmul_rn(kk, g[s]);
                 if (stim)
                 {
                     // e + a = e + k (1 - g), the difference of the kernels in one product
-                    const double mc = nbb ? 0. : m * c[s];
-                    EM1 = e1;
-                    EM2 = e2;
-                    AB1 = g[s] * (nbb ? e1 + kk : fma(gb[s], mc, kk));
-                    AB2 = gb[s] * (nbb ? e2 + ke : fma(-g[s], mc, ke));
+                    const double mc = m * c[s];
+                    o[s]      = e1;
+                    o[8 + s]  = e2;
+                    o[4 + s]  = __dmul_rn(g[s], nbb ? e1 + kk : fma(gb[s], mc, kk));
+                    o[12 + s] = __dmul_rn(gb[s], nbb ? e2 + ke : fma(-g[s], mc, ke));
                 }
                 else
                 {
-                    EM1 = (1. - g[s]) * e1;
-                    EM2 = (1. - gb[s]) * e2;
-                    AB1 = g[s] * (nbb ? kk : kk * (1. - gb[s]));
-                    AB2 = gb[s] * (nbb ? ke : ke * (1. - g[s]));
+                    o[s]      = __dmul_rn(1. - g[s], e1);
+                    o[8 + s]  = __dmul_rn(1. - gb[s], e2);
+                    o[4 + s]  = __dmul_rn(g[s], nbb ? kk : kk * (1. - gb[s]));
+                    o[12 + s] = __dmul_rn(gb[s], nbb ? ke : ke * (1. - g[s]));
                 }
-                acc[s] += EM1 + EM2;
-                acc[4 + s] += AB1 + AB2;
-                acc[8 + s]  = fma(w, EM1, fma(wp, EM2, acc[8 + s]));
-                acc[12 + s] = fma(w, AB1, fma(wp, AB2, acc[12 + s]));
+            }
+        };
+        const auto add_terms = [&](int it, const double* o) {
+            const double w = S.w[it], wp = S.wp[it];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) // emission, absorption
+            {
+                acc[s]     = __dadd_rn(acc[s], __dadd_rn(o[s], o[8 + s]));
+                acc[8 + s] = fma(w, o[s], fma(wp, o[8 + s], acc[8 + s]));
+            }
+        };
+        if (!WIDE)
+        {
+#pragma unroll 1
+            for (int it = wsub * 32 + lane; it < nit; it += 64)
+            {
+                double o[16];
+                item_terms(it, o);
+                add_terms(it, o);
             }
         }
-        const double tot = warp_sum16(acc, lane);
-        const int idx    = sum_index(lane);
-        if (!(lane & 1))
-            S.red[slot][wsub][idx] = tot;
+        else
+        {
+            // rounds of 256 items; the first two warps add them as the two-warp
+            // form does (64 partial sums), so that a point's sums do not depend on
+            // the form
+#pragma unroll 1
+            for (int base = 0; base < nit; base += kStride)
+            {
+                const int it = base + (int)threadIdx.x;
+                if (it < nit)
+                {
+                    double o[16];
+                    item_terms(it, o);
+#pragma unroll
+                    for (int kk = 0; kk < 16; ++kk)
+                        S.terms[kk][threadIdx.x] = o[kk];
+                }
+                __syncthreads();
+                if (wid < 2)
+                {
+#pragma unroll 1
+                    for (int v = threadIdx.x; v < kStride && base + v < nit; v += 64)
+                    {
+                        double o[16];
+#pragma unroll
+                        for (int kk = 0; kk < 16; ++kk)
+                            o[kk] = S.terms[kk][v];
+                        add_terms(base + v, o);
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        if (wsub < 2)
+        {
+            const double v = warp_sum16(acc, lane);
+            if (!(lane & 1))
+                S.red[slot][wsub][sum_index(lane)] = v;
+        }
         point_sync();
         if (wsub == 0 && !(lane & 1))
         {
-            double t = S.red[slot][0][idx];
-#pragma unroll
-            for (int v = 1; v < Smem::kWPP; ++v)
-                t += S.red[slot][v][idx];
+            const int idx  = sum_index(lane);
+            const double t = S.red[slot][0][idx] + S.red[slot][1][idx];
             P->snes[idx] = t * (pre * ((T * T) * (T * T)) * (idx >= 8 ? T : 1.));
         }
     }
@@ -2362,33 +2409,38 @@ struct NesItem
     float pad;
 };
 
-// Per-warp data of the point in work.
-struct NesWarp
+// Data of the point in work.
+struct NesPointData
 {
-    NepsTab N; // distribution and F_k(eta) for the FP64 Taylor branches
+    NepsTab N; // F_k(eta) for the FP64 Taylor branches
     nes32::Lepton lep[2];
     NuSpecies sp[4];
+    int twin; // species 2 and 3 share one distribution
 };
 
+template <bool WIDE>
 struct NesSmem
 {
+    static constexpr int kWPP = WIDE ? kNesWarps : 2; // warps per point
+    static constexpr int kPts = kNesWarps / kWPP;
     NesItem items[kNesItems];
-    NesWarp w[kNesWarps];
-    uint16_t q[kNesWarps][kNesItems]; // items (| lepton mask << 14) for the Taylor branches
-    float2 dacc[16][kNesWarps * 32];  // per-lane df sums of the 16 moments
-    float4 mag[4][kNesWarps * 32];    // per-lane sums of |term|
+    NesPointData pt[kPts];
+    static constexpr int kSum = kPts * 64; // partial sums: 64 lanes per point
+    uint16_t q[kPts * 2][kNesItems / 2 + 32]; // items (| lepton mask << 14) for the Taylor branches
+    float2 dacc[16][kSum]; // per-lane df sums of the 16 moments
+    float4 mag[4][kSum];   // per-lane sums of |term|
+    double red[kPts][2][2][16];
+    float tm[WIDE ? 16 : 1][WIDE ? kNesWarps * 32 : 1]; // terms of a round's items
+    uint8_t tmk[WIDE ? kNesWarps * 32 : 1];             // their Taylor mask, bit 2: has terms
 };
 
-// Adds one item's terms to the lane's sums: em1..ab2 are R(nu, nubar) and
-// R(nubar, nu) with NEPSExpFunc applied, times (w w')^2 (m1_opacities.hpp:880-905).
-__device__ __forceinline__ void nes_accumulate(NesSmem& S, int t, bool stim, bool nbb, float Wf,
-                                               float fw, float fwp, const float* g,
-                                               const float* gm, const float* gb,
-                                               const float* gbm, const float* em1,
-                                               const float* ab1, const float* em2,
-                                               const float* ab2)
+// One item's terms of the 16 moments: em1..ab2 are R(nu, nubar) and R(nubar, nu)
+// with NEPSExpFunc applied, times (w w')^2 (m1_opacities.hpp:880-905).
+__device__ __forceinline__ void nes_terms(bool stim, bool nbb, float Wf, float fw, float fwp,
+                                          const float* g, const float* gm, const float* gb,
+                                          const float* gbm, const float* em1, const float* ab1,
+                                          const float* em2, const float* ab2, float* tm)
 {
-    float tm[16];
 #pragma unroll
     for (int s = 0; s < 4; ++s)
     {
@@ -2416,6 +2468,12 @@ __device__ __forceinline__ void nes_accumulate(NesSmem& S, int t, bool stim, boo
         tm[8 + s]  = Wf * (fw * EM1 + fwp * EM2);
         tm[12 + s] = Wf * (fw * AB1 + fwp * AB2);
     }
+}
+
+// Adds them to the sums of (virtual) lane t.
+template <class Smem>
+__device__ __forceinline__ void nes_accumulate(Smem& S, int t, const float* tm)
+{
 #pragma unroll
     for (int kk = 0; kk < 16; ++kk)
     {
@@ -2435,7 +2493,13 @@ __device__ __forceinline__ void nes_accumulate(NesSmem& S, int t, bool stim, boo
     }
 }
 
-template <bool MULTI = false>
+// Two warps share a point, rows of 32 items alternating between them (with a warp
+// per point the last of 3.4 waves over 8,192 points ran 60% empty), or (WIDE, for
+// launches with fewer points than the chip has warps to fill) all eight.  The 16
+// moments' totals and magnitudes are summed so that a lane holds one moment,
+// whose cancellation it checks.  8,192 points, n = 20: 2.78 -> 2.45 ms; one point, n =
+// 10: 148 -> 58 us.
+template <bool WIDE, bool MULTI = false>
 __global__ void __launch_bounds__(kNesWarps * 32, 2)
     grey_nes_fast_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA,
                          int64_t p0, int64_t np, double* __restrict__ scratch)
@@ -2451,7 +2515,8 @@ __global__ void __launch_bounds__(kNesWarps * 32, 2)
     if (MULTI && !L.use_inel)
         return;
     extern __shared__ __align__(16) unsigned char nes_smem_raw[];
-    NesSmem& S   = *reinterpret_cast<NesSmem*>(nes_smem_raw);
+    using Smem   = NesSmem<WIDE>;
+    Smem& S      = *reinterpret_cast<Smem*>(nes_smem_raw);
     const int n2 = L.n2, nn2 = n2 * n2, nit = 2 * nn2;
     {
         // w = c x_i (1 -+ x_j) for r = 0 and c (1 -+ x_j) / x_i for r = 1, c = 2 x 2.182
@@ -2491,69 +2556,89 @@ __global__ void __launch_bounds__(kNesWarps * 32, 2)
     const int lane = threadIdx.x & 31;
     const int wid  = threadIdx.x >> 5;
     const int t    = threadIdx.x;
-    NesWarp& Wd    = S.w[wid];
-    uint16_t* qw   = S.q[wid];
+    const int slot = wid / Smem::kWPP, wsub = wid - slot * Smem::kWPP;
+    NesPointData& Wd = S.pt[slot];
+    uint16_t* qw     = S.q[WIDE ? (wid & 1) : wid];
+    // the warps of a point (every thread of them runs the same iterations)
+    const auto point_sync = [&]() {
+        if (WIDE)
+            __syncthreads();
+        else
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(Smem::kWPP * 32) : "memory");
+    };
     const bool nbb  = L.neglect_blocking != 0;
     const bool stim = L.stim != 0;
-    const int64_t nwarp = (int64_t)gridDim.x * kNesWarps;
     constexpr float kBp = (float)k::NepsBPlus, kBm = (float)k::NepsBMinus,
                     kBz = (float)k::NepsBZero;
 
-    for (int64_t qp = (int64_t)blockIdx.x * kNesWarps + wid; qp < np; qp += nwarp)
+    for (int64_t qp = (int64_t)blockIdx.x * Smem::kPts + slot; qp < np;
+         qp += (int64_t)gridDim.x * Smem::kPts)
     {
         const int64_t p = L.pidx ? L.pidx[p0 + qp] : p0 + qp;
         PointTab* P     = (PointTab*)(scratch + qp * kTabWords);
         const double T = L.eos[1][p], mu_e = L.eos[7][p];
-        __syncwarp();
-        warp_copy((double*)&Wd.N.d, (const double*)&P->d, 28 + 12 + 2, lane);
-        if (lane == 0)
-            Wd.N.same_cf = P->same_cf;
-        __syncwarp();
         NepsPoint NP;
         NP.T    = T;
         NP.pre  = k::NepsConst * (T * T);
         NP.eta0 = mu_e / T;
         NP.eta1 = -mu_e / T;
-        NP.fd00 = Wd.N.fd0[0];
-        NP.fd01 = Wd.N.fd0[1];
-        NP.fe0  = Wd.N.fe[0];
-        NP.fe1  = Wd.N.fe[1];
         // range envelope: the occupation of every species far above the FP32
         // normal range at its peak; e^{-Lref} of the e+ integrals finite
         bool ok = isfinite(NP.eta0) && NP.eta0 > -80.;
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
+        if (lane < 4)
         {
-            const Distr& d = Wd.N.d;
-            ok = ok && (d.w_t[s] == 0. || d.eta_t[s] > -60.) &&
-                 (d.w_f[s] == 0. || d.beta_f[s] > 1e-30) && (d.temp_t[s] > 0.) &&
-                 (d.temp_f[s] > 0.) && isfinite(d.eta_t[s]) && isfinite(d.beta_f[s]);
+            const Distr& d = P->d;
+            ok = ok && (d.w_t[lane] == 0. || d.eta_t[lane] > -60.) &&
+                 (d.w_f[lane] == 0. || d.beta_f[lane] > 1e-30) && (d.temp_t[lane] > 0.) &&
+                 (d.temp_f[lane] > 0.) && isfinite(d.eta_t[lane]) && isfinite(d.beta_f[lane]);
         }
-        int flag = ok ? 0 : 2;
-        double acc[16];
+        int flag = __all_sync(0xffffffffu, ok) ? 0 : 2;
         if (flag == 0)
         {
-            if (lane < 2)
-                Wd.lep[lane] = nes32::make_lepton(lane ? NP.eta1 : NP.eta0);
-            else if (lane >= 8 && lane < 12)
+            point_sync(); // the previous point's readers are done
+            if (wsub == 0)
             {
-                // x = w = omega / T
-                nu_species(Wd.N.d, lane - 8, T, -log(T), &Wd.sp[lane - 8]);
+                if (lane < 2)
+                    Wd.lep[lane] = nes32::make_lepton(lane ? NP.eta1 : NP.eta0);
+                else if (lane >= 4 && lane < 16)
+                    (&Wd.N.fe[0][0])[lane - 4] = (&P->fe[0][0])[lane - 4];
+                else if (lane >= 16 && lane < 18)
+                    Wd.N.fd0[lane - 16] = P->fd0[lane - 16];
+                else if (lane == 18)
+                    Wd.twin = species_twins(P->d);
+                else if (lane >= 24 && lane < 28) // x = w = omega / T
+                    nu_species(P->d, lane - 24, T, -fx::log(T), &Wd.sp[lane - 24]);
             }
+            if (wsub < 2)
+            {
 #pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
-                S.dacc[kk][t] = make_float2(0.f, 0.f);
+                for (int kk = 0; kk < 16; ++kk)
+                    S.dacc[kk][t] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4)
-                S.mag[k4][t] = make_float4(0.f, 0.f, 0.f, 0.f);
-            __syncwarp();
+                for (int k4 = 0; k4 < 4; ++k4)
+                    S.mag[k4][t] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            point_sync();
+            NP.fd00 = Wd.N.fd0[0];
+            NP.fd01 = Wd.N.fd0[1];
+            NP.fe0  = Wd.N.fe[0];
+            NP.fe1  = Wd.N.fe[1];
+            const int nocc = Wd.twin ? 3 : 4;
             // e+ terms scale as e^{-eta_e}: below 1e-13 of the e- terms for eta_e > 30
             const int nlep = NP.eta0 > 30. ? 1 : 2;
             int nq = 0;
-            for (int base = 0; base < nit; base += 32)
+            const auto queue_items = [&](int k, unsigned tmk) {
+                const unsigned tb = __ballot_sync(0xffffffffu, tmk != 0);
+                if (tmk)
+                    qw[nq + __popc(tb & ((1u << lane) - 1u))] = (uint16_t)(k | (tmk << 14));
+                nq += __popc(tb);
+            };
+            for (int base = 0; base < nit; base += Smem::kWPP * 32)
             {
-                const int k  = base + lane;
+                const int k  = base + wsub * 32 + lane;
                 unsigned tmk = 0;
+                bool any     = false;
+                float tm[16];
                 if (k < nit)
                 {
                     const NesItem I    = S.items[k];
@@ -2562,7 +2647,6 @@ __global__ void __launch_bounds__(kNesWarps * 32, 2)
                     // A e^{-Lref}-scaled kernel sum b1 I_1 + b2 I_2 per species
                     // over the leptons: R(nu, nubar) (w w')^2 = sign x c
                     float c[4] = {0.f, 0.f, 0.f, 0.f};
-                    bool any   = false;
 #pragma unroll 1
                     for (int e = 0; e < nlep; ++e)
                     {
@@ -2595,16 +2679,43 @@ __global__ void __launch_bounds__(kNesWarps * 32, 2)
                             ab1[s] = em2[s] = c[s] * I.sefa;
                         }
                         float g[4], gm[4], gb[4], gbm[4];
-                        total_nu_q(W, dfm::df{I.lwh, I.lwl}, Wd.sp, g, gm);
-                        total_nu_q(WP, dfm::df{I.lwph, I.lwpl}, Wd.sp, gb, gbm);
-                        nes_accumulate(S, t, stim, nbb, I.wf, I.wh, I.wph, g, gm, gb, gbm, em1,
-                                       ab1, em2, ab2);
+                        total_nu_q(W, dfm::df{I.lwh, I.lwl}, Wd.sp, nocc, g, gm);
+                        total_nu_q(WP, dfm::df{I.lwph, I.lwpl}, Wd.sp, nocc, gb, gbm);
+                        nes_terms(stim, nbb, I.wf, I.wh, I.wph, g, gm, gb, gbm, em1, ab1, em2,
+                                  ab2, tm);
                     }
                 }
-                const unsigned tb = __ballot_sync(0xffffffffu, tmk != 0);
-                if (tmk)
-                    qw[nq + __popc(tb & ((1u << lane) - 1u))] = (uint16_t)(k | (tmk << 14));
-                nq += __popc(tb);
+                if (!WIDE)
+                {
+                    if (any)
+                        nes_accumulate(S, t, tm);
+                    queue_items(k, tmk);
+                }
+                else
+                {
+                    // the first two warps add the round's four rows of 64 items in
+                    // order, as the two-warp form does
+                    S.tmk[t] = (uint8_t)(tmk | (any ? 4u : 0u));
+#pragma unroll
+                    for (int kk = 0; kk < 16; ++kk)
+                        S.tm[kk][t] = tm[kk];
+                    __syncthreads();
+                    if (wid < 2)
+                        for (int v = t; v < Smem::kWPP * 32; v += 64)
+                        {
+                            const unsigned f = S.tmk[v];
+                            if (f & 4u)
+                            {
+                                float o[16];
+#pragma unroll
+                                for (int kk = 0; kk < 16; ++kk)
+                                    o[kk] = S.tm[kk][v];
+                                nes_accumulate(S, t, o);
+                            }
+                            queue_items(base + v, f & 3u);
+                        }
+                    __syncthreads();
+                }
             }
             __syncwarp();
             // items in the reference's Taylor branches (w or w' below 1e-3 eta,
@@ -2647,63 +2758,64 @@ __global__ void __launch_bounds__(kNesWarps * 32, 2)
                     }
                 }
                 float g[4], gm[4], gb[4], gbm[4];
-                total_nu_q(dfm::df{I.wh, I.wl}, dfm::df{I.lwh, I.lwl}, Wd.sp, g, gm);
-                total_nu_q(dfm::df{I.wph, I.wpl}, dfm::df{I.lwph, I.lwpl}, Wd.sp, gb, gbm);
-                nes_accumulate(S, t, stim, nbb, I.wf, I.wh, I.wph, g, gm, gb, gbm, em1, ab1, em2,
-                               ab2);
+                total_nu_q(dfm::df{I.wh, I.wl}, dfm::df{I.lwh, I.lwl}, Wd.sp, nocc, g, gm);
+                total_nu_q(dfm::df{I.wph, I.wpl}, dfm::df{I.lwph, I.lwpl}, Wd.sp, nocc, gb, gbm);
+                float tm[16];
+                nes_terms(stim, nbb, I.wf, I.wh, I.wph, g, gm, gb, gbm, em1, ab1, em2, ab2, tm);
+                nes_accumulate(S, t, tm);
             }
-            float mag[16];
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
+            if (wsub < 2)
             {
-                const float2 a = S.dacc[kk][t];
-                acc[kk]        = (double)a.x + (double)a.y;
-            }
+                double acc[16], mag[16];
 #pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4)
-            {
-                const float4 m = S.mag[k4][t];
-                mag[4 * k4]     = m.x;
-                mag[4 * k4 + 1] = m.y;
-                mag[4 * k4 + 2] = m.z;
-                mag[4 * k4 + 3] = m.w;
+                for (int kk = 0; kk < 16; ++kk)
+                {
+                    const float2 a = S.dacc[kk][t];
+                    acc[kk]        = (double)a.x + (double)a.y;
+                }
+#pragma unroll
+                for (int k4 = 0; k4 < 4; ++k4)
+                {
+                    const float4 m  = S.mag[k4][t];
+                    mag[4 * k4]     = m.x;
+                    mag[4 * k4 + 1] = m.y;
+                    mag[4 * k4 + 2] = m.z;
+                    mag[4 * k4 + 3] = m.w;
+                }
+                const double ta = warp_sum16(acc, lane), tg = warp_sum16(mag, lane);
+                if (!(lane & 1))
+                {
+                    S.red[slot][wsub][0][sum_index(lane)] = ta;
+                    S.red[slot][wsub][1][sum_index(lane)] = tg;
+                }
             }
+            point_sync();
+            if (wsub != 0)
+                continue;
+            const int idx = sum_index(lane);
+            double tot    = S.red[slot][0][0][idx] + S.red[slot][1][0][idx];
+            double mtot   = S.red[slot][0][1][idx] + S.red[slot][1][1][idx];
             // terms of both signs (occupation above 1), or NES sums cancelling
             // the pair + brem sums of the same output (those enter the assembly
             // with t2d^2 = hn / 8, times t2d for energy moments) or the beta
             // rates: the point goes to the accurate pass
-            const double T4 = (T * T) * (T * T);
-            double other[16];
-            beta_in_sum_units(P, T, NP.eta0, L.use_abs_em, true, other);
+            const double unit = NP.pre * ((T * T) * (T * T)) * (idx >= 8 ? T : 1.);
+            tot *= unit;
+            mtot *= unit;
             const double t2d = k::TempMultiple * T;
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
-                other[kk] += (L.use_pair || L.use_brem)
-                                 ? 0.125 * P->s2d[kk] * (kk >= 8 ? t2d : 1.)
-                                 : 0.;
-            const double amp = cancel_factor(acc, mag, NP.pre * T4, NP.pre * T4 * T, other);
-            if (amp > kMaxCancel)
+            const double other =
+                beta_in_sum_unit(P, T, NP.eta0, L.use_abs_em, true, idx) +
+                ((L.use_pair || L.use_brem) ? 0.125 * P->s2d[idx] * (idx >= 8 ? t2d : 1.) : 0.);
+            if (__any_sync(0xffffffffu, mtot > 0. && mtot > kMaxCancel * fabs(tot + other)))
                 flag = 1;
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
-                acc[kk] *= NP.pre * T4 * (kk >= 8 ? T : 1.);
+            if (flag == 0 && !(lane & 1)) // else a later launch writes this point's sums
+                P->snes[idx] = tot;
         }
-        if (lane == 0)
+        if (wsub == 0 && lane == 0)
         {
             P->neps_fp64 = (double)flag;
             if (flag != 0)
                 atomicAdd(&g_grey_mixed[flag], 1ull);
-        }
-        if (flag != 0)
-            continue; // a later launch writes this point's sums
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk)
-            acc[kk] = warp_sum(acc[kk]);
-        if (lane == 0)
-        {
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
-                P->snes[kk] = acc[kk];
         }
     }
 }
@@ -2878,36 +2990,39 @@ struct Step
     double* ws;
 };
 
+// Chunks of fewer points than this many per SM run a point per CTA in the NES
+// kernels (both forms add a point's terms in the same order, so its results do
+// not depend on the form).  A chip-wide round of the two-warp form is 8 points per
+// SM and takes as long for one point as for 1,216; a point per CTA takes time in
+// proportion.  FP64, n = 6, 10, 20: a round 80, 162, 553 us; a point per CTA 67, 110,
+// 357 us at 600 points, 100, 160, 518 us at 900.  Mixed: a round 95, 135, 346 us; a
+// point per CTA 69, 82, 175 us at 300 points (one wave), 115, 144, 314 us at 500.
+constexpr int64_t kWide64PerSm = 5, kWideFastPerSm = 2;
+
 // The fast NES pass: 8-warp CTAs with the item table and the per-lane sums in
 // dynamic shared memory (two CTAs per SM).
-template <bool MULTI>
+template <bool WIDE, bool MULTI>
 cudaError_t launch_nes_fast(const Step& S, cudaStream_t st, int sms)
 {
-    const int smem    = (int)sizeof(NesSmem);
-    cudaError_t e     = cudaFuncSetAttribute(grey_nes_fast_kernel<MULTI>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr int smem = (int)sizeof(NesSmem<WIDE>), kPts = NesSmem<WIDE>::kPts;
+    const auto kernel  = grey_nes_fast_kernel<WIDE, MULTI>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               smem);
     if (e != cudaSuccess)
         return e;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grey_nes_fast_kernel<MULTI>,
-                                                      kNesWarps * 32, smem) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kNesWarps * 32, smem) !=
+            cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
-    const int64_t work = (S.np + kNesWarps - 1) / kNesWarps;
+    const int64_t work = (S.np + kPts - 1) / kPts;
     int64_t cap        = (int64_t)((double)sms * per_sm * g_grid_scale);
     cap                = cap < 1 ? 1 : cap;
     const int grid     = (int)(work < cap ? (work > 0 ? work : 1) : cap);
-    grey_nes_fast_kernel<MULTI><<<dim3(grid, 1, MULTI ? S.G : 1), kNesWarps * 32, smem, st>>>(
-        *S.L, S.GA, S.p0, S.np, S.ws);
+    kernel<<<dim3(grid, 1, MULTI ? S.G : 1), kNesWarps * 32, smem, st>>>(*S.L, S.GA, S.p0, S.np,
+                                                                         S.ws);
     return cudaGetLastError();
 }
-
-// Launches of fewer points than this many per SM run a point per CTA in the NES
-// kernels.  A chip-wide round of the two-warp form is 8 points per SM and takes
-// as long for one point as for 1,216; a point per CTA takes time in proportion.
-// FP64, n = 6, 10, 20: a round 81, 162, 555 us; a point per CTA 70, 113, 351 us at
-// 600 points, 101, 163, 518 us at 900.
-constexpr int64_t kWidePointsPerSm = 5;
 
 template <bool WIDE, bool MULTI>
 cudaError_t launch_nes64(const Step& S, cudaStream_t st, int sms, int flagged)
@@ -2990,6 +3105,8 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
     const OpacityLaunch& L = *S.L;
     const int64_t np       = S.np;
     const unsigned gz      = MULTI ? S.G : 1;
+    const bool wide64 = !MULTI && np < kWide64PerSm * sms;
+    const bool wide32 = !MULTI && np <= kWideFastPerSm * sms;
     cudaError_t err        = cudaSuccess;
     phase_mark(kPhPrelude, 0, st);
     {
@@ -3024,7 +3141,9 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
         if (L.mixed)
         {
             phase_mark(kPhNeps, 0, st);
-            if ((err = launch_nes_fast<MULTI>(S, st, sms)) != cudaSuccess)
+            err = wide32 ? launch_nes_fast<true, MULTI>(S, st, sms)
+                         : launch_nes_fast<false, MULTI>(S, st, sms);
+            if (err != cudaSuccess)
                 return err;
             phase_mark(kPhNeps, 1, st);
             phase_mark(kPhNepsAccurate, 0, st);
@@ -3041,8 +3160,8 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
         else
         {
             phase_mark(kPhNeps, 0, st);
-            err = np < kWidePointsPerSm * sms ? launch_nes64<true, MULTI>(S, st, sms, 0)
-                                   : launch_nes64<false, MULTI>(S, st, sms, 0);
+            err = wide64 ? launch_nes64<true, MULTI>(S, st, sms, 0)
+                         : launch_nes64<false, MULTI>(S, st, sms, 0);
             if (err != cudaSuccess)
                 return err;
             phase_mark(kPhNeps, 1, st);

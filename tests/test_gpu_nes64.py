@@ -36,3 +36,19 @@ def test_nes64_forms(cuda, port, port_fma, batch, nq, stim, nbb, cf):
     want = oracle_grey(port, sub[0], *args, stim=stim, distr=sub[2])
     pr = grey_probes(port, port_fma, sub[0], *args, stim=stim, distr=sub[2])
     assert_close(got, want, pr, what=f"batch {batch} nq {nq}")
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nq,stim", [(1, 1), (5, 0), (12, 1), (20, 1)])
+def test_nes_forms_agree_bitwise(cuda, precision, nq, stim):
+    """A point's NES sums do not depend on how many warps share it: the same
+    points in a call small enough for a point per CTA and in a large one."""
+    torch = cuda
+    eos, m1 = bn.synthetic_points(78, 1600)
+    e, m = torch.from_numpy(eos).cuda(), torch.from_numpy(m1).cuda()
+    q = bn.gauss_legendre(nq)
+    args = (bn.opacity_flags(*NES), bn.opacity_params(), q)
+    large = bn.m1_opacities(e, m, *args, stim_abs=stim, precision=precision)
+    small = bn.m1_opacities(e[:, :100].contiguous(), m[:, :100].contiguous(), *args,
+                            stim_abs=stim, precision=precision)
+    assert torch.equal(large[:, :100], small)
