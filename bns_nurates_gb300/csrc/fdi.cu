@@ -4,22 +4,24 @@
 // continued below j = -1 by dF_{j+1}/dx = (j + 1) F_j) and k2 = 0 .. 21
 // (FDI_0, FDI_p12, FDI_p1, ..., FDI_p10, FDI_p212).
 //
-// Integer orders 0..5 run the restatement of the reference's rational
-// approximations (fdi_orders).  Every other order reads the tables of
-// bnsn_fdi_tab.h (made by fdi_tables.py from mpmath): an alternating series
-// in e^x below x = -4, one Chebyshev expansion per interval of [-4, 100) and
-// the Sommerfeld expansion above.  The tables agree with the reference's
-// approximations to a few 1e-16 (relative, away from the zeros of the
-// negative orders).
+// Integer orders 0..5 run the fixed-point Taylor tables of bnsn_fx.cuh.  Every
+// other order is a factor times one polynomial of degree 15 in the tables of
+// bnsn_fdi_tab.h (made by fdi_tables.py from mpmath): the alternating series in
+// e^x below x = -4, one of 70 intervals of [-4, 100), the Sommerfeld expansion
+// above.  The tables agree with the reference's approximations to a few 1e-16
+// (relative, away from the zeros of the negative orders).
 //
 // Non-finite arguments follow the reference: NaN gives NaN for the
 // half-integer orders and 0 for the integer ones; -inf gives 0; +inf gives
 // +inf for j > -1 and -0 or +0 (the sign of x^(j+1) / (j+1)) below.
 //
-// One thread per argument, grid-stride, the order's coefficients staged in
-// shared memory per CTA; FP64-pipe bound (about 60 FP64 operations per
-// argument against 16 bytes of traffic).
-
+// One thread per argument, grid-stride, the order's table (9 KB) in shared memory
+// per CTA.  Arguments come in any order, so a warp usually meets all three regimes:
+// they share the polynomial, and the factors (e^x, x^(j+1)) run on the integer
+// pipes (bnsn_fx.cuh).  FP64-pipe bound, ~30 operations per argument against 16 bytes of
+// traffic.  A loop per regime instead (16 + 25 Clenshaw + 12 terms, exp, sqrt and two
+// divisions) cost a mixed warp the sum of them: ~150.  4,000,037 arguments uniform in
+// [-50, 150), order 1/2: 978 -> 265 us.
 #include <cuda_runtime.h>
 
 #include "bnsn_fdi_tab.h"
@@ -40,20 +42,17 @@ constexpr int slot_of(int k2)
     return -1;
 }
 
-// One order's coefficients staged in shared memory; the Chebyshev table is
-// transposed to [term][interval] so that the lanes of a warp, which read the
-// same term of different intervals, hit consecutive words.
+// One order's coefficients in shared memory, [term][row]: the lanes of a warp read the
+// same term of different rows.
 struct FdiShared
 {
-    double series[fdit::kSeriesTerms];
-    double cheb[fdit::kChebTerms][fdit::kPieces];
-    double asym[fdit::kAsymTerms];
+    double c[fdit::kDegree + 1][fdit::kRows];
 };
 
-// x^(h/2) for x >= 100 (or +inf) and |h| <= 23: an integer power by repeated
-// squaring, times sqrt(x) for odd h, inverted for negative h (far cheaper
-// than pow, within a few ulp).
-__device__ __forceinline__ double pow_half(double x, int h)
+// x^(h/2) for x >= 100 (or +inf) and |h| <= 23 outside the fixed-point range (x >
+// 2^120 or a result that leaves the exponent range): an integer power by repeated
+// squaring, times sqrt(x) for odd h, inverted for negative h.
+__device__ __noinline__ double pow_half(double x, int h)
 {
     const int a = h < 0 ? -h : h;
     int q       = a >> 1;
@@ -71,63 +70,51 @@ __device__ __forceinline__ double pow_half(double x, int h)
     return h < 0 ? 1. / v : v;
 }
 
-__device__ __forceinline__ double fdi_table(const FdiShared& S, int h, bool integer, double x)
+// P = j + 1 in 2^-58 units, ij1 = 1 / (j + 1).
+__device__ __forceinline__ double fdi_table(const FdiShared& S, int h, int64_t P, double ij1,
+                                            bool integer, double x)
 {
-    const double j1 = 0.5 * h; // j + 1
     using namespace fdit;
+    double v, f = 1.;
+    int row;
     if (x < kXlo)
     {
-        // sum_n (-1)^(n+1) c_n e^(n x) = e^x sum_m c_(m+1) (-e^x)^m
-        const double e = exp(x);
-        const double z = -e;
-        double p       = S.series[kSeriesTerms - 1];
-#pragma unroll
-        for (int n = kSeriesTerms - 2; n >= 0; --n)
-            p = fma(p, z, S.series[n]);
-        return e * p;
+        f   = fx::exp(x);
+        v   = -f;
+        row = 0;
     }
-    if (x < kXhi)
+    else if (x < kXhi)
     {
-        int i;
-        double cen, sc;
-        if (x < kXmid)
+        const bool narrow = x < kXmid;
+        const double lo   = narrow ? kXlo : kXmid;
+        int i = (int)((x - lo) * (narrow ? 1. / kWidth : 1. / kWide));
+        const int last = narrow ? kNarrow - 1 : kPieces - kNarrow - 1;
+        i   = i > last ? last : i;
+        v   = (x - (lo + (narrow ? kWidth : kWide) * ((double)i + 0.5))) *
+              (narrow ? 2. / kWidth : 2. / kWide);
+        row = 1 + i + (narrow ? 0 : kNarrow);
+    }
+    else
+    {
+        if (x != x) // NaN fails both regime tests above
+            return integer ? 0. : x;
+        row = kPieces + 1;
+        if (x < 0x1p80)
         {
-            i   = (int)floor((x - kXlo) * (1. / kWidth));
-            i   = i < 0 ? 0 : (i > kNarrow - 1 ? kNarrow - 1 : i);
-            cen = kXlo + kWidth * i + 0.5 * kWidth;
-            sc  = 2. / kWidth;
+            v = fx::rcp(x * x);
+            f = fx::pow_q(fx::log2_q56(x), P) * ij1;
         }
         else
         {
-            int k = (int)floor((x - kXmid) * (1. / kWide));
-            k     = k < 0 ? 0 : (k > kPieces - kNarrow - 1 ? kPieces - kNarrow - 1 : k);
-            i     = kNarrow + k;
-            cen   = kXmid + kWide * k + 0.5 * kWide;
-            sc    = 2. / kWide;
+            v = 1. / (x * x);
+            f = pow_half(x, h) * ij1;
         }
-        const double t  = (x - cen) * sc;
-        const double t2 = 2. * t;
-        // Clenshaw recurrence for sum_m c_m T_m(t) (c_0 stored halved)
-        double b1 = 0., b2 = 0.;
-#pragma unroll
-        for (int m = kChebTerms - 1; m >= 1; --m)
-        {
-            const double b0 = fma(t2, b1, S.cheb[m][i] - b2);
-            b2              = b1;
-            b1              = b0;
-        }
-        return fma(t, b1, S.cheb[0][i] - b2);
     }
-    if (x != x) // NaN fails both regime tests above
-        return integer ? 0. : x;
-    // x^(j+1) / (j+1) (1 + sum_k a_k x^(-2k))
-    const double u = 1. / (x * x);
-    double s       = S.asym[kAsymTerms - 1];
+    double p = S.c[kDegree][row];
 #pragma unroll
-    for (int k = kAsymTerms - 2; k >= 0; --k)
-        s = fma(s, u, S.asym[k]);
-    s = fma(s, u, 1.);
-    return pow_half(x, h) / j1 * s;
+    for (int m = kDegree - 1; m >= 0; --m)
+        p = fma(p, v, S.c[m][row]);
+    return f * p;
 }
 
 template <int K>
@@ -143,19 +130,17 @@ __global__ void fdi_table_kernel(int slot, int h, int integer, const double* __r
 {
     using namespace fdit;
     __shared__ FdiShared S;
-    for (int k = threadIdx.x; k < kSeriesTerms; k += blockDim.x)
-        S.series[k] = kSeries[slot][k];
-    for (int k = threadIdx.x; k < kPieces * kChebTerms; k += blockDim.x)
+    for (int k = threadIdx.x; k < kRows * (kDegree + 1); k += blockDim.x)
     {
-        const int i = k / kChebTerms, m = k - i * kChebTerms;
-        S.cheb[m][i] = kCheb[slot][i][m];
+        const int row = k / (kDegree + 1), m = k - row * (kDegree + 1);
+        S.c[m][row] = kPoly[slot][row][m];
     }
-    for (int k = threadIdx.x; k < kAsymTerms; k += blockDim.x)
-        S.asym[k] = kAsym[slot][k];
+    const int64_t P  = fx::pow_exponent(0.5 * h);
+    const double ij1 = 2. / h;
     __syncthreads();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = fdi_table(S, h, integer != 0, x[i]);
+        out[i] = fdi_table(S, h, P, ij1, integer != 0, x[i]);
 }
 
 } // namespace

@@ -5,24 +5,25 @@ F_j(x) = integral_0^inf t^j / (exp(t - x) + 1) dt for j > -1, without the
 continued to j < -1 by dF_{j+1}/dx = (j + 1) F_j; for every j,
 F_j(x) = -Gamma(j + 1) Li_{j+1}(-e^x).
 
-The integer orders 0..5 are evaluated by the library's restatement of the
-reference's rational approximations (bnsn_fp64.cuh).  Every other member of
-the family the reference defines (FDI_m92 .. FDI_m12, FDI_p12 .. FDI_p212 and
-FDI_p6 .. FDI_p10) is evaluated in three regimes with tables made here:
+The integer orders 0..5 are evaluated by the library's fixed-point Taylor
+tables (fx_tables.py).  Every other member of the family the reference defines
+(FDI_m92 .. FDI_m12, FDI_p12 .. FDI_p212 and FDI_p6 .. FDI_p10) is a factor
+times one polynomial of degree 15, f * sum_m c_m v^m, whose row of coefficients
+depends on the interval of x:
 
-  x < -4        : the alternating series
-                  sum_{n=1}^{16} (-1)^{n+1} Gamma(j+1) n^{-(j+1)} e^{n x},
-                  in Horner form in -e^x
-  -4 <= x < 100 : 28 Chebyshev expansions of degree 24, one per interval:
-                  [-4 + 2i, -2 + 2i] below 40, [40 + 10i, 50 + 10i] above (the
-                  only singularities of F_j are at x = +-i pi, +-3i pi, ..., so
-                  on the narrow intervals the coefficients fall by >= 6.7 per
-                  degree and on the wide ones by >= 18)
-  x >= 100      : the Sommerfeld expansion
-                  x^{j+1} / (j+1) (1 + sum_k 2 eta(2k) (j+1)(j)...(j+2-2k) x^{-2k}),
-                  12 terms; the truncation and the exponentially small
-                  remainder are below 1e-20 of the leading term; x^{j+1}
-                  by repeated squaring times sqrt(x) for half-integer j
+  x < -4        : f = e^x, v = -e^x, c_m = Gamma(j+1) (m+1)^{-(j+1)} (the
+                  alternating series in e^x)
+  -4 <= x < 100 : f = 1, v in [-1, 1] the position in one of 70 intervals,
+                  of width 11/16 below 40 and 10 above
+                  (the only singularities of F_j are at x = +-i pi, +-3i pi, ...,
+                  so a Chebyshev expansion falls by >= 18 per degree)
+  x >= 100      : f = x^{j+1} / (j+1), v = x^{-2} (the Sommerfeld expansion),
+                  c_0 = 1, c_k = 2 eta(2k) (j+1) j ... (j+2-2k); the truncation and
+                  the exponentially small remainder are below 1e-20 of the
+                  leading term
+
+One degree for every interval keeps the threads of a warp, whose arguments lie
+in any of them, in one instruction stream.
 
 ``generate()`` computes the coefficients with mpmath at 34 digits and writes
 csrc/bnsn_fdi_tab.h (checked in; mpmath is only needed to regenerate it).
@@ -46,14 +47,13 @@ ORDERS2 = (-9, -7, -5, -3, -1, 1, 3, 5, 7, 9, 11, 12, 13, 14, 15, 16, 17, 18, 19
 # Every twice-order of the family (functions.hpp:442-4375).
 FAMILY2 = (-9, -7, -5, -3, -1) + tuple(range(0, 22))
 
-SERIES_TERMS = 16
+DEGREE = 15
 X_LO, X_MID, X_HI = -4.0, 40.0, 100.0
-WIDTH, WIDE = 2.0, 10.0
+WIDTH, WIDE = 0.6875, 10.0  # no interval ends within 0.1 of a zero of F_j
 NARROW = int((X_MID - X_LO) / WIDTH)
 PIECES = NARROW + int((X_HI - X_MID) / WIDE)
-CHEB_TERMS = 25
-CHEB_NODES = 40
-ASYM_TERMS = 12
+ROWS = PIECES + 2  # the series, the intervals, the Sommerfeld expansion
+CHEB_NODES = 32
 DPS = 34
 
 
@@ -96,35 +96,42 @@ def f_mp(j, x):
 def _series(j):
     mp = _mp()
     g = mp.gamma(mp.mpf(j) + 1)
-    return [float(g * mp.power(n, -(mp.mpf(j) + 1))) for n in range(1, SERIES_TERMS + 1)]
+    return [float(g * mp.power(n, -(mp.mpf(j) + 1))) for n in range(1, DEGREE + 2)]
 
 
-def _cheb_piece(args):
+def _piece_row(args):
+    """Monomial coefficients in v of the Chebyshev expansion of degree DEGREE."""
     j, i = args
     mp = _mp()
     centre, half = (mp.mpf(c) for c in piece(i))
     th = [mp.pi * (k + mp.mpf(0.5)) / CHEB_NODES for k in range(CHEB_NODES)]
     fv = [f_mp(j, centre + half * mp.cos(t)) for t in th]
-    out = []
-    for m in range(CHEB_TERMS):
+    out = [mp.mpf(0)] * (DEGREE + 1)
+    t0, t1 = [mp.mpf(1)], [mp.mpf(0), mp.mpf(1)]  # T_0, T_1 in powers of v
+    for m in range(DEGREE + 1):
         c = 2 * mp.fsum(fv[k] * mp.cos(m * th[k]) for k in range(CHEB_NODES)) / CHEB_NODES
-        out.append(float(c / 2 if m == 0 else c))
-    return j, i, out
+        for k, a in enumerate(t0):
+            out[k] += a * (c / 2 if m == 0 else c)
+        t2 = [mp.mpf(0)] + [2 * a for a in t1]
+        for k, a in enumerate(t0):
+            t2[k] -= a
+        t0, t1 = t1, t2
+    return j, i, [float(c) for c in out]
 
 
 def piece(i):
-    """Centre and half-width of Chebyshev interval i."""
+    """Centre and half-width of interval i."""
     if i < NARROW:
         return X_LO + WIDTH * i + WIDTH / 2, WIDTH / 2
     return X_MID + WIDE * (i - NARROW) + WIDE / 2, WIDE / 2
 
 
 def _asym(j):
-    """2 eta(2k) (j+1) j ... (j+2-2k), k = 1..ASYM_TERMS (eta: Dirichlet eta)."""
+    """1 and 2 eta(2k) (j+1) j ... (j+2-2k), k = 1..DEGREE (eta: Dirichlet eta)."""
     mp = _mp()
     j1 = mp.mpf(j) + 1
-    out, fall = [], mp.mpf(1)
-    for k in range(1, ASYM_TERMS + 1):
+    out, fall = [1.0], mp.mpf(1)
+    for k in range(1, DEGREE + 1):
         fall *= (j1 - (2 * k - 2)) * (j1 - (2 * k - 1))
         out.append(float(2 * mp.altzeta(2 * k) * fall))
     return out
@@ -141,48 +148,40 @@ def generate(path=HEADER, workers=None):
     jobs = [(k2 / 2, i) for k2 in ORDERS2 for i in range(PIECES)]
     ctx = mproc.get_context("spawn")
     with ctx.Pool(workers or os.cpu_count()) as pool:
-        res = pool.map(_cheb_piece, jobs, chunksize=4)
-    cheb = {(j, i): c for j, i, c in res}
+        res = pool.map(_piece_row, jobs, chunksize=4)
+    rows = {(j, i): c for j, i, c in res}
     lines = [
         "// Generated by bns_nurates_gb300/fdi_tables.py (mpmath %s, %d digits); do not edit."
         % (mp.__version__, DPS),
-        "// Tables of the Fermi-Dirac integral family evaluated by fdi.cu:",
-        "// alternating-series coefficients (x < -4), Chebyshev coefficients of",
-        "// the intervals of [-4, 100) and Sommerfeld coefficients (x >= 100).",
+        "// Tables of the Fermi-Dirac integral family evaluated by fdi.cu: polynomials",
+        "// of the alternating series (x < -4), of the intervals of [-4, 100) and of",
+        "// the Sommerfeld expansion (x >= 100).",
         "#pragma once",
         "",
         "namespace bnsn {",
         "namespace fdit {",
         "",
         "constexpr int kNumOrders   = %d;" % len(ORDERS2),
-        "constexpr int kSeriesTerms = %d;" % SERIES_TERMS,
+        "constexpr int kDegree      = %d;" % DEGREE,
         "constexpr int kPieces      = %d;" % PIECES,
-        "constexpr int kChebTerms   = %d;" % CHEB_TERMS,
-        "constexpr int kAsymTerms   = %d;" % ASYM_TERMS,
         "constexpr int kNarrow      = %d;" % NARROW,
+        "constexpr int kRows        = kPieces + 2;",
         "constexpr double kXlo = %r, kXmid = %r, kXhi = %r;" % (X_LO, X_MID, X_HI),
         "constexpr double kWidth = %r, kWide = %r;" % (WIDTH, WIDE),
         "",
         "// twice the order of each slot",
         "constexpr int kTwice[kNumOrders] = {%s};" % ", ".join(str(k) for k in ORDERS2),
         "",
-        "// Gamma(j + 1) n^-(j + 1), n = 1..kSeriesTerms",
-        "__device__ const double kSeries[kNumOrders][kSeriesTerms] = {",
-        "    " + _hex_rows([_series(k2 / 2) for k2 in ORDERS2], "    ") + "};",
-        "",
-        "// Chebyshev coefficients c_0 .. c_24 of F_j on interval i, c_0 halved:",
-        "// [-4 + 2i, -2 + 2i] for i < kNarrow, else [40 + 10k, 50 + 10k], k = i - kNarrow",
-        "__device__ const double kCheb[kNumOrders][kPieces][kChebTerms] = {",
+        "// c_0 .. c_15 of the series (row 0), the intervals (rows 1 .. kPieces) and",
+        "// the Sommerfeld expansion (row kPieces + 1)",
+        "__device__ const double kPoly[kNumOrders][kRows][kDegree + 1] = {",
     ]
     for n, k2 in enumerate(ORDERS2):
-        rows = [cheb[(k2 / 2, i)] for i in range(PIECES)]
-        lines.append("    {" + _hex_rows(rows, "     ") + "}" + ("," if n + 1 < len(ORDERS2) else ""))
+        j = k2 / 2
+        r = [_series(j)] + [rows[(j, i)] for i in range(PIECES)] + [_asym(j)]
+        lines.append("    {" + _hex_rows(r, "     ") + "}" + ("," if n + 1 < len(ORDERS2) else ""))
     lines += [
         "};",
-        "",
-        "// 2 eta(2k) (j+1) j ... (j+2-2k), k = 1..kAsymTerms",
-        "__device__ const double kAsym[kNumOrders][kAsymTerms] = {",
-        "    " + _hex_rows([_asym(k2 / 2) for k2 in ORDERS2], "    ") + "};",
         "",
         "} // namespace fdit",
         "} // namespace bnsn",
@@ -193,7 +192,7 @@ def generate(path=HEADER, workers=None):
 
 
 def load_header(path=HEADER):
-    """The tables of csrc/bnsn_fdi_tab.h as numpy arrays (exact, hex literals)."""
+    """The table of csrc/bnsn_fdi_tab.h as a numpy array (exact, hex literals)."""
     with open(path) as f:
         text = f.read()
 
@@ -203,16 +202,12 @@ def load_header(path=HEADER):
         return np.array([float.fromhex(v) for v in vals])
 
     n = len(ORDERS2)
-    return {
-        "series": block("kSeries").reshape(n, SERIES_TERMS),
-        "cheb": block("kCheb").reshape(n, PIECES, CHEB_TERMS),
-        "asym": block("kAsym").reshape(n, ASYM_TERMS),
-    }
+    return block("kPoly").reshape(n, ROWS, DEGREE + 1)
 
 
 def pow_half(x, h):
-    """x^(h/2) as the kernel forms it: an integer power by repeated squaring,
-    times sqrt(x) for odd h, inverted for negative h."""
+    """x^(h/2): an integer power by repeated squaring, times sqrt(x) for odd h,
+    inverted for negative h."""
     a = abs(h)
     q = a >> 1
     v = np.ones_like(x)
@@ -232,19 +227,18 @@ def evaluate(k2, x, tabs):
     """F_{k2/2}(x) for a table order, in FP64 with the kernel's operation order."""
     slot = ORDERS2.index(k2)
     x = np.asarray(x, dtype=np.float64)
-    out = np.empty_like(x)
     j1 = 0.5 * k2 + 1.0
+    nan = np.isnan(x)
     lo = x < X_LO
     hi = x >= X_HI
-    mid = ~(lo | hi | np.isnan(x))
+    row = np.where(lo, 0, PIECES + 1)
+    v = np.zeros_like(x)
+    f = np.ones_like(x)
     with np.errstate(over="ignore", invalid="ignore", divide="ignore", under="ignore"):
         e = np.exp(x[lo])
-        z = -e
-        c = tabs["series"][slot]
-        p = np.full_like(z, c[-1])
-        for n in range(SERIES_TERMS - 2, -1, -1):
-            p = p * z + c[n]
-        out[lo] = e * p
+        v[lo], f[lo] = -e, e
+        v[hi], f[hi] = 1.0 / (x[hi] * x[hi]), pow_half(x[hi], k2 + 2) / j1
+        mid = ~(lo | hi | nan)
         xm = x[mid]
         i = np.where(xm < X_MID, np.floor((xm - X_LO) * (1.0 / WIDTH)),
                      NARROW + np.floor((xm - X_MID) * (1.0 / WIDE)))
@@ -252,24 +246,13 @@ def evaluate(k2, x, tabs):
         narrow = i < NARROW
         cen = np.where(narrow, X_LO + WIDTH * i + WIDTH / 2,
                        X_MID + WIDE * (i - NARROW) + WIDE / 2)
-        t = (xm - cen) * np.where(narrow, 2.0 / WIDTH, 2.0 / WIDE)
-        cc = tabs["cheb"][slot][i]
-        b1 = np.zeros_like(t)
-        b2 = np.zeros_like(t)
-        t2 = 2.0 * t
-        for m in range(CHEB_TERMS - 1, 0, -1):
-            b0 = t2 * b1 + (cc[:, m] - b2)
-            b2, b1 = b1, b0
-        out[mid] = t * b1 + (cc[:, 0] - b2)
-        xh = x[hi]
-        u = 1.0 / (xh * xh)
-        a = tabs["asym"][slot]
-        s = np.full_like(u, a[-1])
-        for k in range(ASYM_TERMS - 2, -1, -1):
-            s = s * u + a[k]
-        s = s * u + 1.0
-        out[hi] = pow_half(xh, k2 + 2) / j1 * s
-    nan = np.isnan(x)
+        v[mid] = (xm - cen) * np.where(narrow, 2.0 / WIDTH, 2.0 / WIDE)
+        row[mid] = i + 1
+        c = tabs[slot][row]
+        p = c[..., DEGREE]
+        for m in range(DEGREE - 1, -1, -1):
+            p = p * v + c[..., m]
+        out = f * p
     out[nan] = 0.0 if k2 % 2 == 0 else np.nan
     return out
 
