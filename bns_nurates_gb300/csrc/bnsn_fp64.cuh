@@ -307,8 +307,8 @@ BNSN_DI void distr_species(double n_in, double J_in, double chi, double gamma36,
     const double n = (n_in > 1e-100) ? n_in : 1e-100;
     const double J = (J_in > 1e-100) ? J_in : 1e-100;
     *w_t           = 1.5 * (1. - chi);
-    const double q = n / J;
-    const double y = n * (q * q * q) / k::FourPiHc3;
+    const double q = fx::div(n, J);
+    const double y = n * (q * q * q) * (1. / k::FourPiHc3);
     double eta;
     if (y < 0.005)
     {
@@ -319,7 +319,7 @@ BNSN_DI void distr_species(double n_in, double J_in, double chi, double gamma36,
         const double den =
             y * (y * (y * (y * (y * (y + 1.0) + 38840.0743174942) - 99.9009680656931) -
                       171.874844843596) + 75.7101579899442) + 83.0160130941424;
-        eta = log(num / den);
+        eta = fx::log(fx::div(num, den));
     }
     else if (y <= 0.7)
     {
@@ -331,7 +331,7 @@ BNSN_DI void distr_species(double n_in, double J_in, double chi, double gamma36,
             y * (y * (y * (y * (y * (y + 1.8888797407042) - 5.35488690539183) +
                            1.94673781342617) + 0.483128792035557) +
                  0.0113386564109086) + 2.64160073447322e-5;
-        eta = num / den - 30.;
+        eta = fx::div(num, den) - 30.;
     }
     else if (y > 0.7 && y < 0.7901234567745267)
     {
@@ -353,13 +353,13 @@ BNSN_DI void distr_species(double n_in, double J_in, double chi, double gamma36,
     double f23[2];
     fdi_orders<2, 3>(eta, f23);
     *eta_t  = eta;
-    *temp_t = f23[0] * J / (f23[1] * n);
+    *temp_t = fx::div(f23[0] * J, f23[1] * n);
 
     *w_f             = 0.5 * (3. * chi - 1.);
     *c_f             = k::CF;
-    const double Tnu = J / (n * (k::CF + 3.));
+    const double Tnu = fx::div(J, n * (k::CF + 3.));
     *temp_f          = Tnu;
-    *beta_f          = n / (k::FourPiHc3 * gamma36 * fx::pow(Tnu, k::CF + 3.));
+    *beta_f          = fx::div(n, k::FourPiHc3 * gamma36 * fx::pow(Tnu, k::CF + 3.));
 }
 
 // distribution.hpp:298-315 (TotalNuF) for the 4 species at one energy;

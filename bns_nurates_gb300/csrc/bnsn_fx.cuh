@@ -116,6 +116,20 @@ BNSN_FX_HD double quot(double a, double b)
     return fma(fma(-b, q, a), r, q);
 }
 
+// x in [2^-400, 2^400)
+BNSN_FX_HD bool mid_range(double x)
+{
+    return (((uint32_t)(bits_of(x) >> 52) & 0x7ffu) - (1023u - 400u)) < 800u;
+}
+
+BNSN_FX_OUT double div_special(double a, double b) { return a / b; }
+
+// a/b for any a and b.
+BNSN_FX_HD double div(double a, double b)
+{
+    return mid_range(a) && mid_range(b) ? quot(a, b) : div_special(a, b);
+}
+
 // An exponent of two, I + F / 2^64.
 struct Exp2
 {

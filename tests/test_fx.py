@@ -30,6 +30,7 @@ void t_phi(const double* x, const double*, double* o, long n) { for (long i = 0;
 void t_log(const double* x, const double*, double* o, long n) { for (long i = 0; i < n; ++i) o[i] = fx::log(x[i]); }
 void t_log2(const double* x, const double*, double* o, long n) { for (long i = 0; i < n; ++i) o[i] = fx::log2(x[i]); }
 void t_quot(const double* x, const double* p, double* o, long n) { for (long i = 0; i < n; ++i) o[i] = fx::quot(x[i], p[i]); }
+void t_div(const double* x, const double* p, double* o, long n) { for (long i = 0; i < n; ++i) o[i] = fx::div(x[i], p[i]); }
 }
 """
 
@@ -132,3 +133,14 @@ def test_quotient(call):
     rng = np.random.default_rng(4)
     a, b = np.exp(rng.uniform(-50., 50., (2, 2000)))
     assert np.abs(call("t_quot", a, b) / (a / b) - 1.).max() <= 2. ** -51
+
+
+def test_division_outside_the_quotient_range(call):
+    v = np.array([0., 1., 3e-320, 1e-130, 1e130, 1e-300, 1e300, np.inf, np.nan, -7.])
+    a, b = (w.ravel() for w in np.meshgrid(v, v))
+    with np.errstate(all="ignore"):
+        want = a / b
+    got = call("t_div", a, b)
+    near = np.isfinite(want) & (np.abs(want) > 1e-290)
+    assert np.abs(got[near] / want[near] - 1.).max() <= 2. ** -51
+    np.testing.assert_array_equal(got[~near], want[~near])
