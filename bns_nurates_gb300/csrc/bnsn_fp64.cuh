@@ -43,18 +43,6 @@ BNSN_DI double fermi_distr(double e, double temp, double mu)
     return arg > 0. ? t * r : r;
 }
 
-// functions.hpp:4401-4413 for d1 = w' - w and d2 = w - w' at once (both
-// share e^{-|d|}); d2 is passed explicitly so that w == w' gives +0 for both,
-// as in the reference.
-BNSN_DI void neps_exp_pair(double d1, double d2, double* f1, double* f2)
-{
-    const double e = safe_exp(-fabs(d1));
-    const int n1   = signbit(d1) != 0;
-    const int n2   = signbit(d2) != 0;
-    *f1            = (n1 - (!n1) * e) / (1. - e + (d1 == 0.));
-    *f2            = (n2 - (!n2) * e) / (1. - e + (d2 == 0.));
-}
-
 // functions.hpp:99-137, 140-180: modified Bessel I1 / K1 polynomial fits
 BNSN_DI double bessi1(double x)
 {
@@ -603,28 +591,21 @@ struct PairEnergyFdi
 // make it invisible (1e-13).
 constexpr double kPairLowEnergy = 0.03125;
 
-// Psi_0(y, z) and Psi_0(z, y) of kernel_pair.hpp:16-120 from the per-energy
-// Fermi integrals: fam[k-1] = F_k(eta - y), fap = F_k(eta + y), fbm / fbp the
-// same for z; f3e / f4e are F_3(eta), F_4(eta).  Zero when eta - y - z > 200.
-BNSN_DI void pair_psi(double eta, double y, double z, const double* fam, const double* fap,
-                      const double* fbm, const double* fbp, double f3e, double f4e,
-                      double* psi0, double* psi1, bool rational = false)
+// Psi_0(y, z) and Psi_0(z, y) of kernel_pair.hpp:16-120 in the reference's order
+// and with its Fermi integrals (energies below kPairLowEnergy): fam[k-1] = F_k(eta -
+// y), fap = F_k(eta + y), fbm / fbp the same for z; f3e / f4e are F_3(eta), F_4(eta).
+// Zero when eta - y - z > 200.
+BNSN_DI void pair_psi_low(double eta, double y, double z, const double* fam, const double* fap,
+                          const double* fbm, const double* fbp, double f3e, double f4e,
+                          double* psi0, double* psi1)
 {
     *psi0 = 0.;
     *psi1 = 0.;
     if (eta - y - z > 200.)
         return;
     double fmyz[3], fpyz[3];
-    if (rational)
-    {
-        fdi_rational<3, 5>(eta - y - z, fmyz);
-        fdi_rational<3, 5>(eta + y + z, fpyz);
-    }
-    else
-    {
-        fdi_orders<3, 5>(eta - y - z, fmyz);
-        fdi_orders<3, 5>(eta + y + z, fpyz);
-    }
+    fdi_rational<3, 5>(eta - y - z, fmyz);
+    fdi_rational<3, 5>(eta + y + z, fpyz);
     const double c0  = 20. * fam[3];
     const double c1  = 20. * fbp[3];
     const double c2  = 120. * fam[1] - 120. * fbp[1];
@@ -655,30 +636,6 @@ BNSN_DI void pair_psi(double eta, double y, double z, const double* fam, const d
              z * (c13 + c5 + y * (c14 + y * (-120. * fbm[0] + 120. * fap[0]))));
     *psi0 = p0 / den;
     *psi1 = p1 / den;
-}
-
-// Pair kernel at (omega = y T, omega' = z T), kernel_pair.hpp:135-198:
-// em[4] = Phi/2 per species, ab[4] = e^{(w + w')/T} em.
-BNSN_DI void pair_kernel(double T, double eta, double omega, double omega_p,
-                         double y, double z, const double* fam, const double* fap,
-                         const double* fbm, const double* fbp, double f3e,
-                         double f4e, double* em, double* ab, bool rational = false)
-{
-    double psi0, psi1;
-    pair_psi(eta, y, z, fam, fap, fbm, fbp, f3e, f4e, &psi0, &psi1, rational);
-    const double aux = k::PairPhi * (T * T) / (1. - safe_exp(y + z));
-    const double phi0 = ((k::PairA1e * k::PairA1e) * psi0 + (k::PairA2e * k::PairA2e) * psi1) * aux;
-    const double phi1 = ((k::PairA1e * k::PairA1e) * psi1 + (k::PairA2e * k::PairA2e) * psi0) * aux;
-    const double phi2 = ((k::PairA1x * k::PairA1x) * psi0 + (k::PairA2x * k::PairA2x) * psi1) * aux;
-    const double phi3 = ((k::PairA1x * k::PairA1x) * psi1 + (k::PairA2x * k::PairA2x) * psi0) * aux;
-    em[0] = 0.5 * phi0;
-    em[1] = 0.5 * phi1;
-    em[2] = 0.5 * phi2;
-    em[3] = 0.5 * phi3;
-    const double ex = safe_exp((omega + omega_p) / T);
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-        ab[s] = ex * em[s];
 }
 
 // ---------------------------------------------------------------------------
@@ -1340,17 +1297,6 @@ struct NepsPoint
     const double* fe1;
 };
 
-// kernel_nes.hpp:50-78
-BNSN_DI double mb_int_out(double w, double wp, double x, double y, int sign,
-                          double b1, double b2, const double* dw, const double* dabs)
-{
-    return (((b1 + b2) * (sign * dabs[2] - dw[4]) * 0.2 -
-             b1 * (w + wp) * (dw[3] + 2. * ((w + wp) * dw[2] + 3. * w * wp * dw[1])) +
-             sign * ((b1 * x - b2 * y) * dabs[1] + 2. * (b1 * x * x + b2 * y * y) * dabs[0])) /
-                (w * w * wp * wp) -
-            6. * b1 * dw[0]);
-}
-
 // kernel_nes.hpp:82-107
 BNSN_DI double mb_int_one(double x, double y, int sign, double b1, double b2, const double* f)
 {
@@ -1380,184 +1326,6 @@ BNSN_DI void neps_couplings(int e, int s, double* b1, double* b2)
     const bool first = ((s & 1) == 0) != (e == 1);
     *b1 = first ? bo : k::NepsBZero;
     *b2 = first ? k::NepsBZero : bo;
-}
-
-// NES + NPS kernels (kernel_nes.hpp:139-359) for both directions of one
-// energy pair: k1 = R(nu, nub), k2 = R(nub, nu); em/ab[4] each.  The Fermi
-// integrals at eta - w, eta - w', eta - |w - w'| are evaluated once and
-// shared by the two directions and the four species.
-BNSN_DI void neps_pair(const NepsPoint& P, double nu, double nub, double* em1,
-                       double* ab1, double* em2, double* ab2)
-{
-    const double T  = P.T;
-    const double w  = nu / T;
-    const double wp = nub / T;
-    const double x  = (w > wp) ? w : wp;
-    const double y  = (w < wp) ? w : wp;
-    double efa, efb; // NEPSExpFunc(wp - w), NEPSExpFunc(w - wp)
-    neps_exp_pair(wp - w, w - wp, &efa, &efb);
-    const int sign1 = 2 * (signbit(wp - w) != 0) - 1;
-    const int sign2 = 2 * (signbit(w - wp) != 0) - 1;
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-    {
-        em1[s] = ab1[s] = em2[s] = ab2[s] = 0.;
-    }
-#pragma unroll 1
-    for (int e = 0; e < 2; ++e)
-    {
-        const double eta  = e ? P.eta1 : P.eta0;
-        const double* f0e = e ? P.fe1 : P.fe0;
-        const double fd0  = e ? P.fd01 : P.fd00;
-        double r1[4], r2[4];
-        if (y > eta * 1e-3)
-        {
-            double fw[5], fwp[5], fa[3];
-            fdi_orders<1, 5>(eta - w, fw);
-            fdi_orders<1, 5>(eta - wp, fwp);
-            fdi_orders<3, 5>(eta - fabs(w - wp), fa);
-            double dw1[5], dw2[5], dabs[3];
-#pragma unroll
-            for (int kk = 0; kk < 5; ++kk)
-            {
-                dw1[kk] = fwp[kk] - fw[kk];
-                dw2[kk] = fw[kk] - fwp[kk];
-            }
-#pragma unroll
-            for (int kk = 0; kk < 3; ++kk)
-                dabs[kk] = f0e[3 + kk] - fa[kk];
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                double b1, b2;
-                neps_couplings(e, s, &b1, &b2);
-                r1[s] = P.pre * mb_int_out(w, wp, x, y, sign1, b1, b2, dw1, dabs);
-                r2[s] = P.pre * mb_int_out(wp, w, x, y, sign2, b1, b2, dw2, dabs);
-            }
-        }
-        else if (x > eta * 1e-3)
-        {
-            double fx[3];
-            fdi_orders<0, 2>(eta - x, fx);
-            const double f[5] = {fx[2] - f0e[2], fx[1], f0e[1],
-                                 fx[0] + y * fermi_distr(0., 1., eta - x) / 6.,
-                                 f0e[0] - y * fd0 / 6.};
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                double b1, b2;
-                neps_couplings(e, s, &b1, &b2);
-                r1[s] = P.pre * mb_int_one(x, y, sign1, b1, b2, f);
-                r2[s] = P.pre * mb_int_one(x, y, sign2, b1, b2, f);
-            }
-        }
-        else
-        {
-            const double f[3] = {fd0, f0e[0], f0e[1]};
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                double b1, b2;
-                neps_couplings(e, s, &b1, &b2);
-                r1[s] = P.pre * mb_int_two(w, wp, x, y, b1, b2, f);
-                r2[s] = P.pre * mb_int_two(wp, w, x, y, b1, b2, f);
-            }
-        }
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-        {
-            em1[s] += -r1[s] * efb;
-            ab1[s] += r1[s] * efa;
-            em2[s] += -r2[s] * efa;
-            ab2[s] += r2[s] * efb;
-        }
-    }
-}
-
-// NES + NPS kernel R(nu, nub) in one direction (kernel_nes.hpp:139-359) for
-// the spectral integrals; fw0 / fw1 hold F_0..F_5 at eta - nu/T for electrons
-// and positrons (per energy, shared by all nodes).
-BNSN_DI void neps_one(const NepsPoint& P, double nu, double nub, const double* fw0,
-                      const double* fw1, double* em, double* ab)
-{
-    const double T  = P.T;
-    const double w  = nu / T;
-    const double wp = nub / T;
-    const double x  = (w > wp) ? w : wp;
-    const double y  = (w < wp) ? w : wp;
-    double efa, efb;
-    neps_exp_pair(wp - w, w - wp, &efa, &efb);
-    const int sign = 2 * (signbit(wp - w) != 0) - 1;
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-        em[s] = ab[s] = 0.;
-#pragma unroll 1
-    for (int e = 0; e < 2; ++e)
-    {
-        const double eta  = e ? P.eta1 : P.eta0;
-        const double* f0e = e ? P.fe1 : P.fe0;
-        const double fd0  = e ? P.fd01 : P.fd00;
-        const double* fw  = e ? fw1 : fw0;
-        double r[4];
-        if (y > eta * 1e-3)
-        {
-            double fwp[5], fa[3], dw[5], dabs[3];
-            fdi_orders<1, 5>(eta - wp, fwp);
-            fdi_orders<3, 5>(eta - fabs(w - wp), fa);
-#pragma unroll
-            for (int kk = 0; kk < 5; ++kk)
-                dw[kk] = fwp[kk] - fw[1 + kk];
-#pragma unroll
-            for (int kk = 0; kk < 3; ++kk)
-                dabs[kk] = f0e[3 + kk] - fa[kk];
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                double b1, b2;
-                neps_couplings(e, s, &b1, &b2);
-                r[s] = P.pre * mb_int_out(w, wp, x, y, sign, b1, b2, dw, dabs);
-            }
-        }
-        else if (x > eta * 1e-3)
-        {
-            double fx[3];
-            if (x == w)
-            {
-                fx[0] = fw[0];
-                fx[1] = fw[1];
-                fx[2] = fw[2];
-            }
-            else
-                fdi_orders<0, 2>(eta - x, fx);
-            const double f[5] = {fx[2] - f0e[2], fx[1], f0e[1],
-                                 fx[0] + y * fermi_distr(0., 1., eta - x) / 6.,
-                                 f0e[0] - y * fd0 / 6.};
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                double b1, b2;
-                neps_couplings(e, s, &b1, &b2);
-                r[s] = P.pre * mb_int_one(x, y, sign, b1, b2, f);
-            }
-        }
-        else
-        {
-            const double f[3] = {fd0, f0e[0], f0e[1]};
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                double b1, b2;
-                neps_couplings(e, s, &b1, &b2);
-                r[s] = P.pre * mb_int_two(w, wp, x, y, b1, b2, f);
-            }
-        }
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-        {
-            em[s] += -r[s] * efb;
-            ab[s] += r[s] * efa;
-        }
-    }
 }
 
 #undef BNSN_DI

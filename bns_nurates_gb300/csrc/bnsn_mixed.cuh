@@ -3,6 +3,7 @@
 
 #include "bnsn_df.cuh"
 #include "bnsn_fp64.cuh"
+#include "bnsn_internal.h"
 
 namespace bnsn {
 namespace {
@@ -24,6 +25,186 @@ __device__ __forceinline__ int bracket_sorted(R lw, const R* ax, int d3, R* t)
     }
     *t = (lw - ax[lo]) / (ax[lo + 1] - ax[lo]);
     return lo;
+}
+
+// Order-preserving integer image of a double (comparisons off the FP64 pipe).
+__device__ __forceinline__ int64_t order_key(double v)
+{
+    const int64_t b = __double_as_longlong(v);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+
+__device__ __forceinline__ Gp19Table gp19_table(const OpacityLaunch& L)
+{
+    return {L.gp19.d0, L.gp19.d1, L.gp19.d2,    L.gp19.d3,   L.gp19.nb,  L.gp19.ye,
+            L.gp19.t,  L.gp19.w,  L.gp19.lognb, L.gp19.logw, L.gp19.data};
+}
+
+// The GP19 log w axis in shared memory: values, their order_key and the inverse
+// intervals.
+struct Gp19Axis
+{
+    double lw[kGp19MaxW], idl[kGp19MaxW];
+    int64_t key[kGp19MaxW];
+};
+
+__device__ __forceinline__ void gp19_axis_entry(Gp19Axis& A, const double* logw, int d3, int k)
+{
+    A.lw[k]  = logw[k];
+    A.key[k] = order_key(logw[k]);
+    A.idl[k] = k + 1 < d3 ? 1. / (logw[k + 1] - logw[k]) : 0.;
+}
+
+// GP19 absorption kernel at w (clipped to the axis) from a point's profiles.
+__device__ __forceinline__ double gp19_profile_absorption(const Gp19Point& pt,
+                                                          const double (*p)[kGp19MaxW],
+                                                          const Gp19Axis& A, int d3, double w)
+{
+    const double lw = fx::log(w);
+    const int64_t k = order_key(lw);
+    // smallest l in [0, d3 - 2] with lw <= axis[l + 1]
+    int lo = 0, hi = d3 - 2;
+    while (lo < hi)
+    {
+        const int mid = (lo + hi) >> 1;
+        if (k <= A.key[mid + 1])
+            hi = mid;
+        else
+            lo = mid + 1;
+    }
+    const double tw = (lw - A.lw[lo]) * A.idl[lo], t0 = 1. - tw;
+    const double v0 = fma(p[0][lo + 1], tw, p[0][lo] * t0);
+    const double v1 = pt.regime >= 2 ? fma(p[1][lo + 1], tw, p[1][lo] * t0) : 0.;
+    return gp19_absorption(pt, v0, v1, w);
+}
+
+// One species' occupation constants (distribution.hpp:298-315) for x = omega / u:
+// g = wt / (1 + e^{x rt - eta}) + kf x^cf e^{-x rf}.
+struct Occ64
+{
+    double rt, eta, rf, wt, kf, cf;
+};
+
+__device__ __forceinline__ void occ64_from(const Distr& d, int s, double u, Occ64* o)
+{
+    o->rt  = u / d.temp_t[s];
+    o->eta = d.eta_t[s];
+    o->rf  = u / d.temp_f[s];
+    o->wt  = d.w_t[s];
+    o->cf  = d.c_f[s];
+    o->kf  = d.w_f[s] * (u == 1. ? d.beta_f[s] : d.beta_f[s] * fx::pow(u, d.c_f[s]));
+}
+
+// One species at x, p = x^cf.
+__device__ __forceinline__ double occ64_one(const Occ64& o, double x, double p)
+{
+    const double ft = fx::rcp(safe_exp(fma(x, o.rt, -o.eta)) + 1.);
+    return fma(o.wt, ft, o.kf * (p * fx::exp(-x * o.rf)));
+}
+
+// Four species at x; xc = x^c0, common: every cf is c0.
+__device__ __forceinline__ void occ64_eval(const Occ64* o, double x, double xc, bool common,
+                                           double* g)
+{
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+        g[s] = occ64_one(o[s], x, common ? xc : fx::pow(x, o[s].cf));
+}
+
+// Heavy-lepton neutrinos and antineutrinos evolved as one species: their
+// occupations are the same.
+__device__ __forceinline__ bool species_twins(const Distr& d)
+{
+    return d.w_t[2] == d.w_t[3] && d.temp_t[2] == d.temp_t[3] && d.eta_t[2] == d.eta_t[3] &&
+           d.w_f[2] == d.w_f[3] && d.temp_f[2] == d.temp_f[3] && d.c_f[2] == d.c_f[3] &&
+           d.beta_f[2] == d.beta_f[3];
+}
+
+// 15 y^2 z^2 Psi_0(y, z) and Psi_0(z, y) (kernel_pair.hpp:16-120) from Fermi
+// integrals scaled as Psi needs them (pair_scale): am, ap at eta -+ y, bm, bp at
+// eta -+ z; f40, f20 = 40 F_3(eta), 20 F_4(eta).  The sums are in the reference's
+// order: they cancel, and another order of c10 alone moves ill-conditioned
+// outputs by more than the reference's own rounding does.
+__device__ __forceinline__ void pair_psi_scaled(const double* am, const double* ap,
+                                                const double* bm, const double* bp, double eta,
+                                                double y, double z, double f40, double f20,
+                                                double* p0, double* p1)
+{
+    double fm[3], fp[3];
+    fdi_orders<3, 5>(eta - y - z, fm);
+    fdi_orders<3, 5>(eta + y + z, fp);
+    const double c5 = fma(40., fm[0], -f40), c7 = fma(20., fm[1], -f20);
+    const double c8 = fma(-40., fp[0], f40), c9 = fma(20., fp[1], -f20);
+    const double c10 = fma(-4., fp[2], fma(4., fm[2], -am[4]) - bm[4] + ap[4]) + bp[4];
+    const double d01 = bp[3] - am[3], c2 = am[1] - bp[1], c3 = bp[2] - am[2];
+    const double d11 = bm[3] - ap[3], c14 = bm[1] - ap[1], c13 = ap[2] - bm[2];
+    const double u0 = fma(z, fma(z, bp[0] - am[0], c2), c3 + c5);
+    const double v0 = fma(z, fma(-c2, z, -2. * c3), fma(y, u0, d01 + c7));
+    *p0 = fma(z, fma(z, c3 + c8, c9 - d01), fma(y, v0, c10));
+    const double u1 = fma(y, fma(y, ap[0] - bm[0], c14), c13 + c5);
+    const double v1 = fma(z, u1, fma(y, fma(-c14, y, -2. * c13), c7 - d11));
+    *p1 = fma(z, v1, fma(y, fma(y, c13 + c8, d11 + c9), c10));
+}
+
+// F_1..F_5 scaled for it: 120 F_1, 120 F_2, 40 F_3, 20 F_4, 4 F_5.
+__device__ __forceinline__ void pair_scale(const double* f, double* o)
+{
+    o[0] = 120. * f[0];
+    o[1] = 120. * f[1];
+    o[2] = 40. * f[2];
+    o[3] = 20. * f[3];
+    o[4] = 4. * f[4];
+}
+
+// The NES/NPS bracket of one lepton at energies x > y (in units of T, dl = x - y):
+// MezzacappaIntOut = +-(24 / P^2) (b1 A + b2 B) with P = x y, + for w = x (scattering
+// down).  With phi_k = F_k / k!, D_k = phi_k(eta - x) - phi_k(eta - y), E_k =
+// phi_k(eta) - phi_k(eta - dl), S = x + y:
+//   A = (E5 + D5) + x (E4 + x E3 / 2) + S (D4 + S D3 / 2 + P D2 / 2) + P^2 D1 / 4,
+//   B = (E5 + D5) + y (y E3 / 2 - E4).
+// fx, fy: phi_1..phi_5 at eta - x, eta - y; fe: F_0..F_5 at eta.
+__device__ __forceinline__ void nes_bracket(double eta, double x, double y, double dl,
+                                            const double* fx5, const double* fy5,
+                                            const double* fe, double* A, double* B)
+{
+    double f[3];
+    fx::fd_orders<3, 5, true>(eta - dl, f);
+    const double sm = x + y, hp = 0.5 * (x * y), qp = hp * hp; // P^2 / 4
+    const double E3 = fma(fe[3], 0.5 / 6., -0.5 * f[0]);       // E_3 / 2
+    const double E4 = fma(fe[4], 1. / 24., -f[1]);
+    const double ED = fma(fe[5], 1. / 120., -f[2]) + (fx5[4] - fy5[4]);
+    double a = fma(x, fma(x, E3, E4), ED);
+    a = fma(sm, fma(hp, fx5[1] - fy5[1], fma(0.5 * sm, fx5[2] - fy5[2], fx5[3] - fy5[3])), a);
+    *A = fma(qp, fx5[0] - fy5[0], a);
+    *B = fma(y, fma(y, E3, -E4), ED);
+}
+
+// The reference's Taylor branches (kernel_nes.hpp:82-132, y <= 10^-3 eta) in the
+// same units; fd0 = FermiDistr(0, 1, eta).
+__device__ __forceinline__ void nes_bracket_taylor(double eta, double x, double y, double dl,
+                                                   const double* fe, double fd0, double* A,
+                                                   double* B)
+{
+    const double hp = 0.5 * (x * y), y2 = y * y, xy = x * y, x2 = x * x;
+    const double c  = hp * hp * y * (-1. / 6.) * fx::rcp(x2);
+    if (x > eta * 1e-3)
+    {
+        double f[3];
+        fdi_orders<0, 2>(eta - x, f);
+        const double f0 = f[2] - fe[2], f1 = f[1], f2 = fe[1];
+        const double f3 = f[0] + y * fermi_distr(0., 1., eta - x) * (1. / 6.);
+        const double f4 = fe[0] - y * fd0 * (1. / 6.);
+        *A = c * (2. * f0 + (y + 4. * x) * f1 + (3. * y - 4. * x) * f2 +
+                  (0.2 * y2 + xy + 2. * x2) * f3 - (1.2 * y2 - 3. * xy + 2. * x2) * f4);
+        *B = c * (2. * f0 + 3. * y * f1 + y * f2 + 1.2 * y2 * f3 - 0.2 * y2 * f4);
+    }
+    else
+    {
+        const double u = 4. * fe[1] + fd0 * (11. * y2 - 25. * xy + 20. * x2) * (1. / 30.);
+        const double v = (2. * x - y) * fe[0];
+        *A = -dl * c * (u + v);
+        *B = -dl * c * (u - v);
+    }
 }
 
 // Interval of w on the GP19 w axis and its interpolation weight in FP32, for
@@ -112,18 +293,60 @@ __device__ __noinline__ void neps_taylor(const NepsPoint& P, int e, double w, do
 namespace bnsn {
 namespace {
 
-// Spectral NES/NPS kernel of neps_one (one direction) before the detailed-
-// balance factors: R[s] = sum over e-, e+ of R(w, w') for species s, with the
-// Fermi integrals and brackets in df, dimensionless (the caller applies the
-// NEPS prefactor, NEPSExpFunc and the occupations).  rw[e] are the
-// unreflected F_1..F_5 at aw[e] = eta_e - nu/T, staged per energy.  DF: R in
-// df (the accurate pass), else rounded to FP32 per lepton.
-// W, WP are w, wp in df.
-template <bool DF>
-__device__ __forceinline__ void neps_r_core(const NepsPoint& P, const NepsMixed& Q,
-                                            const dfm::FdiTab* ftab, double w, double wp,
-                                            dfm::df W, dfm::df WP, const dfm::df (*rw)[5],
-                                            const dfm::df* aw, dfm::df* Rd, float* Rf)
+// Spectral NES/NPS kernel of one direction before the detailed-balance factors:
+// R[s] = sum over e-, e+ of R(w, w') for species s, dimensionless (the caller
+// applies the NEPS prefactor, NEPSExpFunc and the occupations), the FP64 bracket
+// of each lepton rounded to FP32.  fw[e]: phi_1..phi_5 at eta_e - w.
+__device__ __forceinline__ void neps_r_mixed(const NepsPoint& P, double w, double wp,
+                                             const double (*fw)[5], float* R)
+{
+    const bool down  = w > wp;
+    const double x   = down ? w : wp, y = down ? wp : w, dl = x - y;
+    const double xy  = w * wp;
+    const double sc  = (down ? 24. : -24.) * fx::rcp(xy * xy);
+    const int nlep   = P.eta0 > 30. ? 1 : 2; // e+ terms below 1e-13 of e- for eta_e > 30
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+        R[s] = 0.f;
+#pragma unroll 1
+    for (int e = 0; e < nlep; ++e)
+    {
+        const double eta = e ? P.eta1 : P.eta0;
+        const double* fe = e ? P.fe1 : P.fe0;
+        double A, B;
+        if (y > eta * 1e-3)
+        {
+            double fp[5];
+            fx::fd_orders<1, 5, true>(eta - wp, fp);
+            nes_bracket(eta, x, y, dl, down ? fw[e] : fp, down ? fp : fw[e], fe, &A, &B);
+        }
+        else
+            nes_bracket_taylor(eta, x, y, dl, fe, e ? P.fd01 : P.fd00, &A, &B);
+        A *= sc;
+        B *= sc;
+        constexpr double bp = k::NepsBPlus, bm = k::NepsBMinus, bz = k::NepsBZero;
+        const double U = e ? B : A, V = e ? A : B;
+        R[0] += (float)fma(bp, U, bz * V);
+        R[1] += (float)fma(bp, V, bz * U);
+        R[2] += (float)fma(bm, U, bz * V);
+        R[3] += (float)fma(bm, V, bz * U);
+    }
+}
+
+// What neps_r_df needs of a point: eta and the unreflected F_1..F_5 of e- and e+.
+struct NesDf
+{
+    dfm::df reta[2][5], eta[2];
+};
+
+// The same with the Fermi integrals and brackets in double-float, for energies nu/T
+// below kSpecNesDfW: the brackets difference their integrals over (w w')^2, so there
+// the low bits of the integrals show in R (1e-7 at nu/T = 0.05, 4e-9 at 0.2), and
+// these are the ones such outputs have always had.  rw[e]: the unreflected F_1..F_5
+// at eta_e - w; W, WP are w, wp in df.
+__device__ __forceinline__ void neps_r_df(const NepsPoint& P, const NesDf& Q,
+                                       const dfm::FdiTab* ftab, double w, double wp, dfm::df W,
+                                       dfm::df WP, const dfm::df (*rw)[5], float* R)
 {
     using namespace dfm;
     const double x = (w > wp) ? w : wp;
@@ -132,12 +355,7 @@ __device__ __forceinline__ void neps_r_core(const NepsPoint& P, const NepsMixed&
     const float sign1 = n1 ? 1.f : -1.f;
 #pragma unroll
     for (int s = 0; s < 4; ++s)
-    {
-        if (DF)
-            Rd[s] = mk(0.f);
-        else
-            Rf[s] = 0.f;
-    }
+        R[s] = 0.f;
     const df S = add(W, WP), Pp = mul(W, WP), Dn = mul(Pp, Pp);
     const df X = n1 ? W : WP, Y = n1 ? WP : W;
     // bracket arguments from FP64 differences (eta up to ~1e3 needs 53 bits)
@@ -151,14 +369,14 @@ __device__ __forceinline__ void neps_r_core(const NepsPoint& P, const NepsMixed&
         const double eta = e ? P.eta1 : P.eta0;
         if (y > eta * 1e-3)
         {
-            const df awp = from_double(eta - wp);
+            const df aw = from_double(eta - w), awp = from_double(eta - wp);
             const df aab = from_double(eta - ad);
             df rwp[5], rab[5];
             fdi_raw15(awp, rwp, 1, ftab);
             fdi_raw15(aab, rab, 3, ftab);
             rab[0] = rab[1] = Q.reta[e][0];
             df dw[5], d5[5];
-            fdi_diff15(rw[e], rwp, aw[e], awp, dlt, dw);
+            fdi_diff15(rw[e], rwp, aw, awp, dlt, dw);
             fdi_diff15(rab, Q.reta[e], aab, Q.eta[e], adw, d5);
             const df dabs[3] = {d5[2], d5[3], d5[4]};
             const df T1 = add(dw[3], mul(add(mul(S, dw[2]), mul(mul(Pp, 3.f), dw[1])), 2.f));
@@ -176,10 +394,7 @@ __device__ __forceinline__ void neps_r_core(const NepsPoint& P, const NepsMixed&
                 const bool first = ((s & 1) == 0) != (e == 1);
                 const df r = first ? add(mul(A1, bo), mul(B1, mk(kBz)))
                                    : add(mul(A1, mk(kBz)), mul(B1, bo));
-                if (DF)
-                    Rd[s] = add(Rd[s], r);
-                else
-                    Rf[s] += r.hi;
+                R[s] += r.hi;
             }
         }
         else
@@ -188,22 +403,9 @@ __device__ __forceinline__ void neps_r_core(const NepsPoint& P, const NepsMixed&
             neps_taylor(P, e, w, wp, x, y, (int)sign1, n1 ? -1 : 1, t1, t2);
 #pragma unroll
             for (int s = 0; s < 4; ++s)
-            {
-                if (DF)
-                    Rd[s] = add(Rd[s], from_double(t1[s]));
-                else
-                    Rf[s] += (float)t1[s];
-            }
+                R[s] += (float)t1[s];
         }
     }
-}
-
-__device__ __forceinline__ void neps_r_mixed(const NepsPoint& P, const NepsMixed& Q,
-                                             const dfm::FdiTab* ftab, double w, double wp,
-                                             dfm::df W, dfm::df WP, const dfm::df (*rw)[5],
-                                             const dfm::df* aw, float* R)
-{
-    neps_r_core<false>(P, Q, ftab, w, wp, W, WP, rw, aw, nullptr, R);
 }
 
 } // namespace
@@ -313,18 +515,21 @@ __device__ __forceinline__ float exp_of(dfm::df x) { return expf(x.hi) * (1.f + 
 // functions.hpp:4401-4413).  de[s], da[s] bound the dropped components of
 // te[s], ta[s].
 // Node arguments in df: W = nu/T, WP = nubar/T, NB = nubar, LB = log nubar
-// (w, wp the same in FP64 for the branch tests of the kernel).
-__device__ __forceinline__ void nes_spec_node(const NepsPoint& P, const NepsMixed& Q,
-                                              const NesSpec& Z, const dfm::FdiTab* ftab,
-                                              double w, double wp, dfm::df W, dfm::df WP,
-                                              dfm::df NB, dfm::df LB, float wa, float sig_e,
-                                              float sig_a, bool nbb, const dfm::df (*rw)[5],
-                                              const dfm::df* aw, float* te, float* ta, float* de,
-                                              float* da)
+// (w, wp the same in FP64 for the kernel).  fw: the Fermi integrals at eta_e - w,
+// phi_1..phi_5, or with Q (double-float kernel) the unreflected F_1..F_5 in df.
+__device__ __forceinline__ void nes_spec_node(const NepsPoint& P, const NesSpec& Z, double w,
+                                              double wp, dfm::df W, dfm::df WP, dfm::df NB,
+                                              dfm::df LB, float wa, float sig_e, float sig_a,
+                                              bool nbb, const double (*fw)[5], const NesDf* Q,
+                                              const dfm::FdiTab* ftab, float* te, float* ta,
+                                              float* de, float* da)
 {
     using namespace dfm;
     float R[4];
-    neps_r_mixed(P, Q, ftab, w, wp, W, WP, rw, aw, R);
+    if (Q) // known at compile time
+        neps_r_df(P, *Q, ftab, w, wp, W, WP, (const dfm::df (*)[5])fw, R);
+    else
+        neps_r_mixed(P, w, wp, fw, R);
     const bool first = wp < w;
     const df D       = first ? sub(W, WP) : sub(WP, W); // |w - wp|
     const float ea   = expf(-D.hi);
@@ -391,90 +596,6 @@ __device__ __forceinline__ void nes_spec_node(const NepsPoint& P, const NepsMixe
         ta[s] = k * gm;
         de[s] = fabsf(k) * le;
         da[s] = fabsf(k) * la;
-    }
-}
-
-// nes_spec_node with every product after the Fermi integrals in df (the
-// accurate pass over energies whose FP32 terms cancel): te, ta in the same
-// scaled units, rounded to FP64.
-__device__ __forceinline__ void nes_spec_node_df(const NepsPoint& P, const NepsMixed& Q,
-                                                 const NesSpec& Z, const dfm::FdiTab* ftab,
-                                                 double w, double wp, dfm::df W, dfm::df WP,
-                                                 dfm::df NB, dfm::df LB, double wa, float sig_e,
-                                                 float sig_a, bool nbb, const dfm::df (*rw)[5],
-                                                 const dfm::df* aw, double* te, double* ta,
-                                                 float* de, float* da)
-{
-    using namespace dfm;
-    df R[4];
-    neps_r_core<true>(P, Q, ftab, w, wp, W, WP, rw, aw, R, nullptr);
-    const bool first = wp < w;
-    const df D       = first ? sub(W, WP) : sub(WP, W);
-    const df dn      = add(neg(exp_df(neg(D))), 1.f); // 1 - e^{-D}, D > 0
-    const df Se = first ? add(D, sig_e) : mk(sig_e);
-    const df Sa = first ? mk(sig_a) : add(D, sig_a);
-    const df c  = div(mul(from_double(first ? wa : -wa), mul(WP, WP)), dn);
-    df gnb = mk(0.f);
-    float unb = 0.f;
-    if (nbb)
-    {
-        const df x = neg(Sa);
-        if (x.hi < kNesDropArg)
-            unb = kNesDrop;
-        else
-            gnb = exp_df(x);
-    }
-#pragma unroll 1
-    for (int s = 0; s < 4; ++s)
-    {
-        const bool ht = (Z.has_t >> s) & 1, hfe = (Z.has_fe >> s) & 1;
-        const bool hfa = (Z.has_fa >> s) & 1;
-        df ge = mk(0.f), gm = nbb ? gnb : mk(0.f);
-        float le = 0.f, la = nbb ? unb : 0.f;
-        if (ht)
-        {
-            const df A     = sub(mul(NB, Z.invTt[s]), Z.etat[s]);
-            const bool pos = A.hi > 0.f;
-            const df t     = exp_df(pos ? neg(A) : A); // e^{-|A|}
-            const df inv   = div(mk(1.f), add(t, 1.f));
-            const df x1    = sub(pos ? sub(Z.lwt[s], A) : Z.lwt[s], Se);
-            if (x1.hi < kNesDropArg)
-                le += kNesDrop;
-            else
-                ge = add(ge, mul(exp_df(x1), inv));
-            if (!nbb)
-            {
-                const df x3 = sub(pos ? Z.lwt[s] : add(Z.lwt[s], A), Sa);
-                if (x3.hi < kNesDropArg)
-                    la += kNesDrop;
-                else
-                    gm = add(gm, mul(exp_df(x3), inv));
-            }
-        }
-        df Fn = mk(0.f);
-        if (hfe)
-        {
-            Fn          = add(Z.lbf[s], sub(mul(Z.cf[s], LB), mul(NB, Z.invTf[s])));
-            const df x2 = add(Fn, sub(Z.lwf[s], Se));
-            if (x2.hi < kNesDropArg)
-                le += kNesDrop;
-            else
-                ge = add(ge, exp_df(x2));
-        }
-        if (hfa && !nbb)
-        {
-            const df x4  = sub(Z.lwf[s], Sa);
-            const df omf = hfe ? add(neg(exp_df(Fn)), 1.f) : mk(1.f);
-            if (x4.hi < kNesDropArg)
-                la += kNesDrop;
-            else
-                gm = add(gm, mul(exp_df(x4), omf));
-        }
-        const df k = mul(c, R[s]);
-        te[s]      = to_double(mul(k, ge));
-        ta[s]      = to_double(mul(k, gm));
-        de[s]      = fabsf(k.hi) * le;
-        da[s]      = fabsf(k.hi) * la;
     }
 }
 

@@ -184,39 +184,6 @@ __device__ __forceinline__ double beta_scale(double f4, double f5, double T, dou
     return (eta_e > 30.) == (s == 0) ? T * eta_e * 0.8333333333333333 : T * 5.;
 }
 
-// One species' occupation constants (distribution.hpp:298-315) for x = omega / u:
-// g = wt / (1 + e^{x rt - eta}) + kf x^cf e^{-x rf}.
-struct Occ64
-{
-    double rt, eta, rf, wt, kf, cf;
-};
-
-__device__ __forceinline__ void occ64_from(const Distr& d, int s, double u, Occ64* o)
-{
-    o->rt  = u / d.temp_t[s];
-    o->eta = d.eta_t[s];
-    o->rf  = u / d.temp_f[s];
-    o->wt  = d.w_t[s];
-    o->cf  = d.c_f[s];
-    o->kf  = d.w_f[s] * (u == 1. ? d.beta_f[s] : d.beta_f[s] * fx::pow(u, d.c_f[s]));
-}
-
-// One species at x, p = x^cf.
-__device__ __forceinline__ double occ64_one(const Occ64& o, double x, double p)
-{
-    const double ft = fx::rcp(safe_exp(fma(x, o.rt, -o.eta)) + 1.);
-    return fma(o.wt, ft, o.kf * (p * fx::exp(-x * o.rf)));
-}
-
-// Four species at x; xc = x^c0, common: every cf is c0.
-__device__ __forceinline__ void occ64_eval(const Occ64* o, double x, double xc, bool common,
-                                           double* g)
-{
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-        g[s] = occ64_one(o[s], x, common ? xc : fx::pow(x, o[s].cf));
-}
-
 // TotalNuF of one species in FP32 with its exponent arguments in df form
 // (distribution.hpp:298-315): x rt - eta_t and P0 + c_f log x - x rf.  The
 // NES items take x = w = omega / T (rt = T / T_t, rf = T / T_f,
@@ -292,15 +259,6 @@ __device__ __forceinline__ void total_nu_q(dfm::df W, dfm::df LW, const NuSpecie
             gm[s] = gm[2];
         }
     }
-}
-
-// Heavy-lepton neutrinos and antineutrinos evolved as one species: their
-// occupations are the same.
-__device__ __forceinline__ bool species_twins(const Distr& d)
-{
-    return d.w_t[2] == d.w_t[3] && d.temp_t[2] == d.temp_t[3] && d.eta_t[2] == d.eta_t[3] &&
-           d.w_f[2] == d.w_f[3] && d.temp_f[2] == d.temp_f[3] && d.c_f[2] == d.c_f[3] &&
-           d.beta_f[2] == d.beta_f[3];
 }
 
 // What the prelude needs beyond the record's header, written by the point kernel
@@ -1049,30 +1007,6 @@ struct PairTab64
     double m[kMaxM][5], p[kMaxM][5], iy2[kMaxM];
 };
 
-// 15 y^2 z^2 Psi_0(y, z) and Psi_0(z, y) (kernel_pair.hpp:16-120) of nodes a, b, the
-// sums in the reference's order: they cancel, and another order of c10 alone moves
-// ill-conditioned outputs by more than the reference's own rounding does.
-__device__ __forceinline__ void pair_psi_nodes(const PairTab64& W, int a, int b, double eta,
-                                               double y, double z, double f40, double f20,
-                                               double* p0, double* p1)
-{
-    double fm[3], fp[3];
-    fdi_orders<3, 5>(eta - y - z, fm);
-    fdi_orders<3, 5>(eta + y + z, fp);
-    const double *am = W.m[a], *ap = W.p[a], *bm = W.m[b], *bp = W.p[b];
-    const double c5 = fma(40., fm[0], -f40), c7 = fma(20., fm[1], -f20);
-    const double c8 = fma(-40., fp[0], f40), c9 = fma(20., fp[1], -f20);
-    const double c10 = fma(-4., fp[2], fma(4., fm[2], -am[4]) - bm[4] + ap[4]) + bp[4];
-    const double d01 = bp[3] - am[3], c2 = am[1] - bp[1], c3 = bp[2] - am[2];
-    const double d11 = bm[3] - ap[3], c14 = bm[1] - ap[1], c13 = ap[2] - bm[2];
-    const double u0 = fma(z, fma(z, bp[0] - am[0], c2), c3 + c5);
-    const double v0 = fma(z, fma(-c2, z, -2. * c3), fma(y, u0, d01 + c7));
-    *p0 = fma(z, fma(z, c3 + c8, c9 - d01), fma(y, v0, c10));
-    const double u1 = fma(y, fma(y, ap[0] - bm[0], c14), c13 + c5);
-    const double v1 = fma(z, u1, fma(y, fma(-c14, y, -2. * c13), c7 - d11));
-    *p1 = fma(z, v1, fma(y, fma(y, c13 + c8, d11 + c9), c10));
-}
-
 // e+e- pair phase.  MIXED: cells from the FP32 integral (bnsn_pair32.cuh); the
 // sums and the magnitudes of their terms are written to the record (PairMixed).
 // The pair kernels are non-negative and so are the absorption terms (em + am =
@@ -1149,12 +1083,7 @@ __global__ void __launch_bounds__(kCellThreads)
                     for (int k = 0; k < 5; ++k)
                         f[k] = qq & 1 ? P->fp[a][k] : P->fm[a][k];
                 }
-                double* o = qq & 1 ? W.p[a] : W.m[a];
-                o[0] = 120. * f[0];
-                o[1] = 120. * f[1];
-                o[2] = 40. * f[2];
-                o[3] = 20. * f[3];
-                o[4] = 4. * f[4];
+                pair_scale(f, qq & 1 ? W.p[a] : W.m[a]);
             }
         }
         __syncthreads();
@@ -1177,7 +1106,8 @@ __global__ void __launch_bounds__(kCellThreads)
                 const double y = C.y[a], z = C.y[b];
                 if (!(eta - y - z > 200.))
                 {
-                    pair_psi_nodes(W, a, b, eta, y, z, f40, f20, &k0, &k1);
+                    pair_psi_scaled(W.m[a], W.p[a], W.m[b], W.p[b], eta, y, z, f40, f20, &k0,
+                                    &k1);
                     const double f =
                         sc * (W.iy2[a] * W.iy2[b]) * fx::rcp(1. - C.dn[a] * C.dn[b]);
                     k0 *= f;
@@ -1234,13 +1164,6 @@ __global__ void __launch_bounds__(kCellThreads)
 // phases.  IMPL: 0 HR98, 1 BRT06, 2 GP19.
 // ---------------------------------------------------------------------------
 
-// Order-preserving integer image of a double (comparisons off the FP64 pipe).
-__device__ __forceinline__ int64_t order_key(double v)
-{
-    const int64_t b = __double_as_longlong(v);
-    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
-}
-
 template <int IMPL>
 struct Brem64Extra
 {
@@ -1256,8 +1179,7 @@ struct Brem64Extra<2>
 {
     Gp19Record r;
     double p[2][kGp19MaxW];
-    double lw[kGp19MaxW], idl[kGp19MaxW]; // log w axis, 1 / its intervals
-    int64_t key[kGp19MaxW];
+    Gp19Axis axis;
 };
 
 template <int IMPL, int NT>
@@ -1266,12 +1188,6 @@ struct Brem64Smem
     CellNodes<NT> C;
     Brem64Extra<IMPL> X;
 };
-
-__device__ __forceinline__ Gp19Table gp19_table(const OpacityLaunch& L)
-{
-    return {L.gp19.d0, L.gp19.d1, L.gp19.d2,    L.gp19.d3,   L.gp19.nb,  L.gp19.ye,
-            L.gp19.t,  L.gp19.w,  L.gp19.lognb, L.gp19.logw, L.gp19.data};
-}
 
 // Launch constants (once per CTA; brem64_point's first barrier orders them).
 template <int IMPL, int NT>
@@ -1282,12 +1198,7 @@ __device__ __forceinline__ void brem64_constants(Brem64Smem<IMPL, NT>& S, const 
     {
         if (L.gp19.d3 <= kGp19MaxW)
             for (int k = threadIdx.x; k < L.gp19.d3; k += NT)
-            {
-                const double* lw = L.gp19.logw;
-                S.X.lw[k]  = lw[k];
-                S.X.key[k] = order_key(lw[k]);
-                S.X.idl[k] = k + 1 < L.gp19.d3 ? 1. / (lw[k + 1] - lw[k]) : 0.;
-            }
+                gp19_axis_entry(S.X.axis, L.gp19.logw, L.gp19.d3, k);
     }
 }
 
@@ -1353,25 +1264,8 @@ __device__ __forceinline__ double brem64_point(Brem64Smem<IMPL, NT>& S, const Op
             const Gp19Table G = gp19_table(L);
             if (prof)
             {
-                const double w  = fmax(fmin(C.nu[a] + C.nu[b], G.w[G.d3 - 1]), G.w[0]);
-                const double lw = fx::log(w);
-                const int64_t k = order_key(lw);
-                // smallest l in [0, d3 - 2] with lw <= axis[l + 1]
-                int lo = 0, hi = G.d3 - 2;
-                while (lo < hi)
-                {
-                    const int mid = (lo + hi) >> 1;
-                    if (k <= S.X.key[mid + 1])
-                        hi = mid;
-                    else
-                        lo = mid + 1;
-                }
-                const double tw = (lw - S.X.lw[lo]) * S.X.idl[lo], t0 = 1. - tw;
-                const double v0 = fma(S.X.p[0][lo + 1], tw, S.X.p[0][lo] * t0);
-                const double v1 = S.X.r.pt.regime >= 2
-                                      ? fma(S.X.p[1][lo + 1], tw, S.X.p[1][lo] * t0)
-                                      : 0.;
-                K = gp19_absorption(S.X.r.pt, v0, v1, w);
+                const double w = fmax(fmin(C.nu[a] + C.nu[b], G.w[G.d3 - 1]), G.w[0]);
+                K = gp19_profile_absorption(S.X.r.pt, S.X.p, S.X.axis, G.d3, w);
             }
             else
                 gp19_kernel(G, L.eos[0][p], L.eos[2][p], T, C.nu[a], C.nu[b], &em, &K);
@@ -2083,19 +1977,14 @@ __global__ void __launch_bounds__(kNesAccWarps * 32, 2)
 // NES/NPS in FP64 (kernel_nes.hpp:50-359; the item sums of
 // m1_opacities.hpp:864-1057 and integration.hpp:687-768).
 //
-// MezzacappaIntOut is antisymmetric, linear in its couplings, and an item's
-// energies in units of T do not depend on the point.  With phi_k = F_k / k!,
-// D_k = phi_k(eta - w') - phi_k(eta - w), E_k = phi_k(eta) - phi_k(eta - d),
-// d = w' - w > 0, S = w + w', P = w w':
-//   R(w, w') = -R(w', w) = -(24 / P^2) pre (b1 A + b2 B),
-//   A = (E5 + D5) + w' (E4 + w' E3 / 2) + S (D4 + S D3 / 2 + P D2 / 2) + P^2 D1 / 4,
-//   B = (E5 + D5) + w (w E3 / 2 - E4),
-// and the weight (nu nubar)^2 of the item cancels 1 / P^2.  So a lepton
-// takes three sets of Fermi integrals and 17 FP64 operations, where the
-// four species and two directions separately took 16 evaluations of the
-// bracket with a division each (~560 instructions); both leptons' A and B
-// combine into the four species' kernels afterwards, R(w', w) costs nothing,
-// and the NEPSExpFunc factors, weights and w^0.6 sit in the CTA's item table.
+// MezzacappaIntOut is antisymmetric, linear in its couplings (nes_bracket), and an
+// item's energies in units of T do not depend on the point; the weight (nu
+// nubar)^2 of the item cancels the bracket's 1 / P^2.  So a lepton takes three sets
+// of Fermi integrals and 17 FP64 operations, where the four species and two
+// directions separately took 16 evaluations of the bracket with a division each
+// (~560 instructions); both leptons' A and B combine into the four species'
+// kernels afterwards, R(w', w) = -R(w, w') costs nothing, and the NEPSExpFunc
+// factors, weights and w^0.6 sit in the CTA's item table.
 // The items follow the host's order of ascending w', which keeps a warp's lanes in
 // the same regime of the Fermi integrals.
 //
@@ -2223,7 +2112,7 @@ __global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
         // that both forms of the kernel add the same numbers
         const auto item_terms = [&](int it, double* o) {
             const double w = S.w[it], wp = S.wp[it];
-            const double dl = wp - w, sm = w + wp, hp = 0.5 * (w * wp), qp = hp * hp; // P^2 / 4
+            const double dl = wp - w;
             double U = 0., V = 0.; // A of e- + B of e+, B of e- + A of e+
 #pragma unroll 1
             for (int e = 0; e < 2; ++e)
@@ -2233,45 +2122,13 @@ __global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
                 double A, B;
                 if (w > thr)
                 {
-                    double a[5], b[5], f[3];
+                    double a[5], b[5];
                     fx::fd_orders<1, 5, true>(eta - wp, a);
                     fx::fd_orders<1, 5, true>(eta - w, b);
-                    fx::fd_orders<3, 5, true>(eta - dl, f);
-                    const double E3 = fma(fe[3], 0.5 / 6., -0.5 * f[0]); // E_3 / 2
-                    const double E4 = fma(fe[4], 1. / 24., -f[1]);
-                    const double ED = fma(fe[5], 1. / 120., -f[2]) + (a[4] - b[4]);
-                    A = fma(wp, fma(wp, E3, E4), ED);
-                    A = fma(sm, fma(hp, a[1] - b[1], fma(0.5 * sm, a[2] - b[2], a[3] - b[3])), A);
-                    A = fma(qp, a[0] - b[0], A);
-                    B = fma(w, fma(w, E3, -E4), ED);
+                    nes_bracket(eta, wp, w, dl, a, b, fe, &A, &B);
                 }
                 else
-                {
-                    // the reference's Taylor branches (kernel_nes.hpp:82-132) in the
-                    // same units: R = -(24 / P^2) pre (b1 A + b2 B)
-                    const double fd0 = S.fd0[slot][e];
-                    const double x = wp, y = w, y2 = y * y, xy = x * y, x2 = x * x;
-                    const double c = qp * y * (-1. / 6.) * fx::rcp(x2);
-                    if (x > thr)
-                    {
-                        double f[3];
-                        fdi_orders<0, 2>(eta - x, f);
-                        const double f0 = f[2] - fe[2], f1 = f[1], f2 = fe[1];
-                        const double f3 = f[0] + y * fermi_distr(0., 1., eta - x) * (1. / 6.);
-                        const double f4 = fe[0] - y * fd0 * (1. / 6.);
-                        A = c * (2. * f0 + (y + 4. * x) * f1 + (3. * y - 4. * x) * f2 +
-                                 (0.2 * y2 + xy + 2. * x2) * f3 - (1.2 * y2 - 3. * xy + 2. * x2) * f4);
-                        B = c * (2. * f0 + 3. * y * f1 + y * f2 + 1.2 * y2 * f3 - 0.2 * y2 * f4);
-                    }
-                    else
-                    {
-                        const double u =
-                            4. * fe[1] + fd0 * (11. * y2 - 25. * xy + 20. * x2) * (1. / 30.);
-                        const double v = (2. * x - y) * fe[0];
-                        A = -dl * c * (u + v);
-                        B = -dl * c * (u - v);
-                    }
-                }
+                    nes_bracket_taylor(eta, wp, w, dl, fe, S.fd0[slot][e], &A, &B);
                 U += e ? B : A;
                 V += e ? A : B;
             }

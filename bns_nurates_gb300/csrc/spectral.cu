@@ -3,20 +3,18 @@
 // Restates ComputeSpectralOpacities{NotStimulatedAbs,StimulatedAbs} and
 // SpectralIntegrand (m1_opacities.hpp:1317-1660).
 //
-// Phases per chunk of points, each a persistent launch with one warp per
-// point (the phase split keeps every kernel's code small enough for the
-// instruction cache; a single fused kernel spent most cycles waiting on
+// Phases per chunk of points (the phase split keeps every kernel's code small enough
+// for the instruction cache; a single fused kernel spent most cycles waiting on
 // instruction fetch):
 //   prelude   NuDistributionParams of each point -> chunk scratch;
 //   pb        pair + brem sums of every (point, energy) -> records;
 //   nes       NES/NPS sums -> records;
 //   assemble  beta, iso, the outer factors and the stimulated-absorption
 //             correction -> the caller's outputs.
-// In pb and nes the antineutrino grid of the integral (t x_i, t / x_i with
-// t = 2.182 T for pair/brem, nu x_i, nu / x_i for NES) is staged per point
-// and per energy in shared memory; lanes take (energy, node group) tasks with
-// groups of G consecutive lanes per energy (G a power of two) and combine the
-// group sums with an xor-shuffle inside each segment.  Each integrand is
+// In FP64 a CTA takes a point in pb and nes (spec_pb64_kernel, spec_nes64_kernel), in
+// the mixed path a warp (spec_pb_kernel, spec_nes_kernel).  The antineutrino grid of
+// the integral (t x_i, t / x_i with t = 2.182 T for pair/brem, nu x_i, nu / x_i for
+// NES) is staged per point or per energy in shared memory.  Each integrand is
 // evaluated once per node; the reference evaluates the full integrand once
 // per (output, node) (integration.hpp:524-543), which only repeats identical
 // values.
@@ -24,23 +22,24 @@
 // MIXED: pb evaluates the pair kernel as the cancellation-free FP32 integral
 // of the grey path (bnsn_pair32.cuh) and the brem kernel in FP32 (HR98
 // shape, GP19 profiles) with the factor e^{-nu/T} of the emissivity applied
-// in FP64 (BRT06 and the GP19 high-T extrapolation stay FP64), and nes uses
-// double-float Fermi integrals and brackets with FP32 occupation factors
-// formed as exponentials of double-float arguments minus a per-energy scale
-// (nes_spec_node), so that e^{-(w - w')} g(w') stays in range at any nu/T;
-// per-point data stay FP64 and every term is summed in FP64.  Both record an
-// error bound per output: the FP32 rounding bound (sum|t| over 1.25 for
-// brem, over 2.5 for the pair integrals, over 2 for NES) plus 1e9 x the
-// components dropped below 2^-120.
+// in FP64 (BRT06 and the GP19 high-T extrapolation stay FP64), and nes rounds its
+// FP64 brackets (double-float ones below nu/T = 0.2, in a second launch over those
+// energies) to FP32 and multiplies them by FP32 occupation factors formed as
+// exponentials of double-float arguments minus a per-energy scale (nes_spec_node), so
+// that e^{-(w - w')} g(w') stays in range at any nu/T; per-point data stay FP64 and
+// every term is summed in FP64.  Both record an error bound per output: the FP32
+// rounding bound (sum|t| over 1.25 for brem, over 2.5 for the pair integrals, over 2
+// for NES) plus 1e9 x the components dropped below 2^-120.
 // assemble compares the bounds with each output's total.  Where their sum
 // exceeds it (terms that cancel), or where a part could not run in FP32
-// (bound = inf: occupations outside the FP32 range, NES at nu/T < 0.05 where
-// the brackets lose double-float accuracy), it flags the part whose bound
-// exceeds half the total.  Flagged pair + brem parts are recomputed in FP64,
-// flagged NES parts with every product in double-float (sum|t| up to 1e5
-// |total|); assemble checks again with the remaining bounds and flags what
-// is left, and an FP64 round finishes those.  The FP64 passes pack each
-// point's flagged energies into full rounds.
+// (bound = inf: occupations outside the FP32 range, NES at nu/T < 0.05), it flags the
+// part whose bound exceeds half the total.  Flagged parts are recomputed by the FP64
+// kernels over the flagged energies of a point; assemble checks again with the
+// remaining bounds, and a last round finishes what is left.  (A double-float pass over
+// the flagged NES parts before the FP64 one took 2.2 ms of 10.8 per 4,096 points at
+// 5% occupancy, and the FP64 kernels are as fast per energy.)
+// 4,096 points x 24 energies: FP64 n = 10 HR98 without NES 9.1 -> 1.7 ms, n = 20 GP19
+// with NES 17.0 -> 4.1 ms; mixed n = 20 GP19 with NES 12.8 -> 5.8 ms.
 
 #include <cuda_runtime.h>
 
@@ -65,8 +64,8 @@ constexpr double kSpecCancelBrem = 1.25;    // sum|t| / |total| of the FP32 brem
 // a bound on the error of their sum, the scale of the other bounds
 constexpr double kSpecCancelPair = 2.5;
 constexpr double kSpecCancelNes  = 2.0;     // same for the NES/NPS terms
-constexpr double kSpecCancelDf   = 1e5;     // same for the double-float NES pass
 constexpr double kSpecNesMinW    = 0.05;    // NES in FP64 below nu/T = 0.05
+constexpr double kSpecNesDfW     = 0.2;    // NES brackets in double-float below nu/T = 0.2
 constexpr double kSpecFloor      = 7.2e-34; // 1e9 x the denormal floor of a sum
 
 // Per (point, energy) record of the chunk scratch.
@@ -84,8 +83,7 @@ enum SpecMode
     kSpecFp64 = 0, // plain path: every energy in FP64
     kSpecMixed,    // mixed path, first pass over every energy
     kSpecRedo,     // FP64 over the flagged energies; assemble re-checks and flags again
-    kSpecFinal,    // assemble only: the energies flagged twice, no guard
-    kSpecAcc       // nes only: double-float products over the flagged energies
+    kSpecFinal     // assemble only: the energies flagged twice, no guard
 };
 
 // Mixed-path statistics: [0] (point, energy) pairs evaluated, [1] of those
@@ -96,15 +94,15 @@ __device__ unsigned long long g_spec_counts[4];
 // (point, energy) pairs whose outputs hold a NaN or Inf.
 __device__ unsigned long long g_spec_nonfinite;
 
-// Lane group size for ne energy tasks of M nodes each (power of two <= 32)
-// minimising rounds x nodes per task.
-__host__ __device__ inline int pick_groups(int ne, int M)
+// Lane group size for ne energy tasks of M nodes each (power of two <= 32) on a
+// number of lanes, minimising rounds x nodes per task.
+__host__ __device__ inline int pick_groups(int ne, int M, int lanes)
 {
     int best       = 1;
     long best_cost = -1;
     for (int G = 1; G <= 32 && G <= M; G <<= 1)
     {
-        const int per_round = 32 / G;
+        const int per_round = lanes / G;
         const long rounds   = (ne + per_round - 1) / per_round;
         const long cost     = rounds * ((M + G - 1) / G);
         if (best_cost < 0 || cost < best_cost)
@@ -168,11 +166,10 @@ __device__ __forceinline__ uint64_t all_energies(int ne)
     return ne >= 64 ? ~0ull : ((1ull << ne) - 1ull);
 }
 
-// Energies of point q that a pb/nes pass works on (bit e: energy e of the launch).
-__device__ __forceinline__ uint64_t energy_mask(int mode, const uint64_t* flags, int64_t q, int ne)
+// Energies of point q that an FP64 pass works on (bit e: energy e of the launch).
+__device__ __forceinline__ uint64_t energy_mask(const uint64_t* flags, int64_t q, int ne)
 {
-    return (mode == kSpecRedo || mode == kSpecAcc) ? flags[q] & all_energies(ne)
-                                                   : all_energies(ne);
+    return flags ? flags[q] & all_energies(ne) : all_energies(ne);
 }
 
 // ---------------------------------------------------------------------------
@@ -205,14 +202,11 @@ __global__ void __launch_bounds__(128)
 struct PbWarp
 {
     Distr d;
-    double fe3, fe4; // F_3, F_4 at eta_e
     Hr98Point hr;
     double brt06_pre;
     int same_cf;
     double nb[kMaxM], zb[kMaxM]; // nubar and nubar / T
     double gb[kMaxM][4];
-    double fmz[kMaxM][5], fpz[kMaxM][5];
-    double fmy[kEChunk][5], fpy[kEChunk][5];
     Gp19Point gp;
     Gp19Corners gc[2];
     double gpp[2][kGp19MaxW];
@@ -229,7 +223,6 @@ struct PbWarpMixed
     float gp32[2][kGp19MaxW];
 };
 
-template <int MODE>
 struct PbShared
 {
     double x[kMaxQ], B1[kMaxM];
@@ -237,7 +230,7 @@ struct PbShared
     double lw[kGp19MaxW], wax[kGp19MaxW], iw[kGp19MaxW];
     float lwf[kGp19MaxW], idl[kGp19MaxW];
     PbWarp w[kWarps];
-    PbWarpMixed m[MODE == kSpecMixed ? kWarps : 1];
+    PbWarpMixed m[kWarps];
 };
 
 // GP19 kernel of one node from the per-point profiles in FP64.
@@ -256,18 +249,323 @@ __device__ __forceinline__ void gp19_profile_node(const Gp19Point& gp,
     gp19_cell(gp, v0, v1, w, nu + nub, be, ba);
 }
 
-template <int MODE>
+// Pair + brem in FP64: every energy, or (flags) the ones the mixed path's checks
+// flagged.  A CTA takes a point: the node and energy tables (Fermi integrals,
+// occupations times weights) over its threads, then the (energy, node) cells'
+// absorption kernels (pair, both orders of Psi, and brem; emission is e^{-(nu +
+// nubar)/T} of it) into shared memory, then a thread per (energy, output) sums its
+// row.  Bound by the FP64 pipe and the integer work of the fixed-point exponentials.
+// With a warp per point whose lanes split the nodes of an energy and carried eight
+// sums each, the node tables were 4x as much shared memory a resident warp, a third
+// of the lanes idled at n = 10, and a flagged energy held a whole warp of a nearly
+// empty grid.  Energies below kPairLowEnergy T take a second pass of their own
+// (rational Fermi integrals, the reference's order of sums).
+constexpr int kPbCells = 32 * 21; // cells of a pass: 32 energies at M = 20, 16 at M = 40
+template <int IMPL>
+struct Pb64Brem
+{
+};
+template <>
+struct Pb64Brem<0>
+{
+    Hr98Point hr;
+    Hr98Cell hc;
+};
+template <>
+struct Pb64Brem<1>
+{
+    double pre;
+};
+template <>
+struct Pb64Brem<2>
+{
+    Gp19Point pt;
+    Gp19Corners gc[2];
+    double p[2][kGp19MaxW];
+    Gp19Axis axis;
+};
+
+template <int IMPL>
+struct Pb64Smem
+{
+    double x[kMaxQ];
+    Occ64 occ[4];
+    double fe[2];                              // F_3, F_4 at eta_e
+    double nb[kMaxM], z[kMaxM], iz2[kMaxM], dnz[kMaxM]; // nubar, z = nubar / T, 1 / z^2, e^{-z}
+    double vE[4][kMaxM], vA[4][kMaxM];         // w nubar^2 (1 - g) e^{-z}, w nubar^2 g
+    double fm[kMaxM][5], fp[kMaxM][5];         // node tables at eta -+ z
+    int eid[kEChunk];
+    double nu[kEChunk], y[kEChunk], iy2[kEChunk], dny[kEChunk];
+    int far[kEChunk];                          // a node with (nu + nubar) / T > 700
+    double em[kEChunk][5], ep[kEChunk][5];     // energy tables at eta -+ y
+    double K[3][kPbCells];                     // pair Psi(y, z), Psi(z, y), brem
+    Pb64Brem<IMPL> X;
+};
+
+// A cell with x = (nu + nubar) / T > 700 from the pair kernel's sum of Psi and the brem
+// absorption kernel.  There the reference clamps e^x at e^700, its emission kernel
+// rounds in the denormal range and the pair absorption kernel is e^700 times that,
+// so both are formed in its order.
+__device__ __noinline__ double pb64_far(double psi, double Kbrem, double T, double x, int ab)
+{
+    const double ex = safe_exp(x);
+    const double em = 0.5 * (psi * (k::PairPhi * (T * T) / (1. - ex)));
+    return ab ? ex * em + Kbrem : em + Kbrem * safe_exp(-x);
+}
+
+template <int IMPL>
+__global__ void __launch_bounds__(kWarps * 32, 4)
+    spec_pb64_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0,
+                     const double* __restrict__ dsc, EnergyRec* __restrict__ rec,
+                     const uint64_t* __restrict__ flags)
+{
+    constexpr int NT = kWarps * 32;
+    const int64_t q  = blockIdx.x;
+    const int n = L.n1, M = 2 * n, ne = L.n_energies, tid = threadIdx.x;
+    const uint64_t emask = energy_mask(flags, q, ne);
+    if (emask == 0ull)
+        return;
+    __shared__ Pb64Smem<IMPL> S;
+    const int64_t p   = p0 + q;
+    const double nbar = L.eos[0][p], T = L.eos[1][p], ye = L.eos[2][p];
+    const double yp = L.eos[3][p], yn = L.eos[4][p];
+    const double eta = L.eos[7][p] / T;
+    const bool pair = L.use_pair != 0, brem = L.use_brem != 0;
+    const bool nbb  = L.neglect_blocking != 0;
+    const Gp19Table G19 = gp19_table(L);
+    const bool prof     = IMPL == 2 && brem && G19.d3 <= kGp19MaxW;
+    if (tid < n)
+        S.x[tid] = L.x1[tid];
+    if (tid >= 32 && tid < 36)
+        occ64_from(*(const Distr*)(dsc + q * 28), tid - 32, 1., &S.occ[tid - 32]);
+    if constexpr (IMPL == 0)
+    {
+        if (brem && tid >= 64 && tid < 67)
+            S.X.hr.ch[tid - 64] = hr98_channel(nbar, yn, yp, T, tid - 64);
+        if (brem && tid == 96)
+            hr98_point_common(nbar, T, L.use_medium != 0, &S.X.hr);
+    }
+    if constexpr (IMPL == 1)
+        if (brem && tid == 64)
+            S.X.pre = brt06_point(nbar, T, yn, yp);
+    if constexpr (IMPL == 2)
+        if (prof)
+        {
+            if (tid == 64)
+                gp19_point(G19, nbar, ye, T, &S.X.pt);
+            if (tid >= 96)
+                for (int k = tid - 96; k < G19.d3; k += 32)
+                    gp19_axis_entry(S.X.axis, G19.logw, G19.d3, k);
+        }
+    __syncthreads();
+    // antineutrino grid (m1_opacities.hpp:1542)
+    const double ts   = k::TempMultiple * T;
+    const bool common = S.occ[0].cf == k::CF && S.occ[1].cf == k::CF && S.occ[2].cf == k::CF &&
+                        S.occ[3].cf == k::CF;
+    for (int t = tid; t < 4 * M; t += NT)
+    {
+        const int a = t >> 2, s = t & 3;
+        const double nub = a < n ? ts * S.x[a] : ts / S.x[a - n];
+        const double g   = occ64_one(S.occ[s], nub, fx::pow(nub, common ? k::CF : S.occ[s].cf));
+        const double z = nub / T, dz = safe_exp(-z), wn = L.B1[a] * (nub * nub);
+        // species s ^ 1 is the partner of s
+        S.vE[s ^ 1][a] = (nbb ? wn : wn * (1. - g)) * dz;
+        S.vA[s ^ 1][a] = wn * g;
+        if (s == 0)
+        {
+            S.nb[a]  = nub;
+            S.z[a]   = z;
+            S.iz2[a] = 1. / (z * z);
+            S.dnz[a] = dz;
+        }
+    }
+    bool fast = false;
+    if constexpr (IMPL == 0)
+    {
+        if (brem && tid >= 64 && tid < 68)
+            hr98_cell_from(S.X.hr, tid - 64, &S.X.hc);
+    }
+    if constexpr (IMPL == 2)
+    {
+        if (prof)
+        {
+            const int np19 = S.X.pt.regime >= 2 ? 2 : 1;
+            if (tid < np19)
+                gp19_profile_corners(G19, S.X.pt.nbp, S.X.pt.yep, S.X.pt.pT[tid], &S.X.gc[tid]);
+            __syncthreads();
+            for (int e = tid; e < np19 * G19.d3; e += NT)
+            {
+                const int pr = e / G19.d3, l = e - pr * G19.d3;
+                S.X.p[pr][l] = gp19_profile_eval(G19, S.X.gc[pr], l);
+            }
+        }
+    }
+    uint64_t low = 0ull;
+    if (pair)
+        for (int e = 0; e < ne; ++e)
+            low |= (uint64_t)(L.energies[e] < kPairLowEnergy * T) << e;
+    const int Ms = M + 1, nc_max = kPbCells / Ms < kEChunk ? kPbCells / Ms : kEChunk;
+    const double scp = -0.5 * k::PairPhi * (T * T);
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass)
+    {
+        const uint64_t mask = emask & (pass ? low : ~low);
+        const int nt        = __popcll(mask);
+        if (nt == 0)
+            continue;
+        const int chunks = (nt + nc_max - 1) / nc_max, per = (nt + chunks - 1) / chunks;
+        __syncthreads(); // the node tables' readers are done
+        if (pair)
+            for (int t = tid; t < 2 * M + 1; t += NT)
+            {
+                if (t == 2 * M)
+                {
+                    if (pass)
+                        fdi_rational<3, 4>(eta, S.fe);
+                    else
+                        fdi_orders<3, 4>(eta, S.fe);
+                    continue;
+                }
+                const int a = t >> 1;
+                const double arg = t & 1 ? eta + S.z[a] : eta - S.z[a];
+                double* o        = t & 1 ? S.fp[a] : S.fm[a];
+                if (pass)
+                    fdi_rational<1, 5>(arg, o);
+                else
+                {
+                    double f[5];
+                    fdi_orders<1, 5>(arg, f);
+                    pair_scale(f, o);
+                }
+            }
+#pragma unroll 1
+        for (int k0 = 0; k0 < nt; k0 += per)
+        {
+            const int nc = nt - k0 < per ? nt - k0 : per;
+            __syncthreads(); // the last chunk's readers are done
+            for (int t = tid; t < 2 * nc; t += NT)
+            {
+                const int c = t >> 1, e = nth_bit(mask, k0 + c);
+                const double nu = L.energies[e], y = nu / T;
+                if ((t & 1) == 0)
+                {
+                    S.eid[c] = e;
+                    S.nu[c]  = nu;
+                    S.y[c]   = y;
+                    S.iy2[c] = 1. / (y * y);
+                    S.dny[c] = safe_exp(-y);
+                    S.far[c] = 0;
+                }
+                if (pair)
+                {
+                    const double arg = t & 1 ? eta + y : eta - y;
+                    double* o        = t & 1 ? S.ep[c] : S.em[c];
+                    if (pass)
+                        fdi_rational<1, 5>(arg, o);
+                    else
+                    {
+                        double f[5];
+                        fdi_orders<1, 5>(arg, f);
+                        pair_scale(f, o);
+                    }
+                }
+            }
+            __syncthreads();
+            if constexpr (IMPL == 0)
+                fast = S.X.hc.fast;
+            const double f40 = 40. * S.fe[0], f20 = 20. * S.fe[1];
+            for (int t = tid; t < nc * M; t += NT)
+            {
+                const int c = t / M, a = t - c * M;
+                const double y = S.y[c], z = S.z[a], ex = S.dny[c] * S.dnz[a];
+                const bool far = y + z > k::ExpUpp;
+                if (far)
+                    S.far[c] = 1;
+                double q0 = 0., q1 = 0., Kb = 0.;
+                if (pair)
+                {
+                    double f = far ? 1. : scp * fx::rcp(1. - ex); // far: Psi itself
+                    if (pass)
+                        pair_psi_low(eta, y, z, S.em[c], S.ep[c], S.fm[a], S.fp[a], S.fe[0],
+                                     S.fe[1], &q0, &q1);
+                    else if (!(eta - y - z > 200.))
+                    {
+                        pair_psi_scaled(S.em[c], S.ep[c], S.fm[a], S.fp[a], eta, y, z, f40, f20,
+                                        &q0, &q1);
+                        f *= (S.iy2[c] * S.iz2[a]) * (1. / 15.);
+                    }
+                    q0 *= f;
+                    q1 *= f;
+                }
+                if (brem)
+                {
+                    if constexpr (IMPL == 0)
+                    {
+                        double b;
+                        if (fast && y > 1e-6 && y < 4e4)
+                            Kb = hr98_absorption(S.X.hc, y + z, ex);
+                        else
+                            hr98_kernel(S.X.hr, S.nu[c], S.nb[a], &b, &Kb);
+                    }
+                    else if constexpr (IMPL == 1)
+                        Kb = S.X.pre * brt06_shape(0.5 * (y + z));
+                    else
+                    {
+                        double b;
+                        if (prof)
+                            Kb = gp19_profile_absorption(
+                                S.X.pt, S.X.p, S.X.axis, G19.d3,
+                                fmax(fmin(S.nu[c] + S.nb[a], G19.w[G19.d3 - 1]), G19.w[0]));
+                        else
+                            gp19_kernel(G19, nbar, ye, T, S.nu[c], S.nb[a], &b, &Kb);
+                    }
+                }
+                const int o = c * Ms + a;
+                S.K[0][o] = q0;
+                S.K[1][o] = q1;
+                S.K[2][o] = Kb;
+            }
+            __syncthreads();
+            for (int t = tid; t < 8 * nc; t += NT)
+            {
+                const int c = t >> 3, s = t & 3, ab = (t >> 2) & 1;
+                constexpr double e0 = k::PairA1e * k::PairA1e, e1 = k::PairA2e * k::PairA2e;
+                constexpr double x0 = k::PairA1x * k::PairA1x, x1 = k::PairA2x * k::PairA2x;
+                const double c0 = s < 2 ? e0 : x0, c1 = s < 2 ? e1 : x1;
+                const double* K0 = S.K[s & 1] + c * Ms;
+                const double* K1 = S.K[1 - (s & 1)] + c * Ms;
+                const double* Kb = S.K[2] + c * Ms;
+                const double* v  = ab ? S.vA[s] : S.vE[s];
+                double acc       = 0.;
+                if (S.far[c])
+                    for (int a = 0; a < M; ++a)
+                    {
+                        const double x = S.y[c] + S.z[a], Kp = fma(c0, K0[a], c1 * K1[a]);
+                        const double wn = L.B1[a], nb2 = S.nb[a] * S.nb[a];
+                        const double g = ab ? v[a] / (wn * nb2) : nbb ? 1. : v[a] / (S.dnz[a] * (wn * nb2));
+                        const double K = x > k::ExpUpp ? pb64_far(Kp, Kb[a], T, x, ab)
+                                                       : (Kp + Kb[a]) * (ab ? 1. : safe_exp(-x));
+                        acc += wn * (nb2 * (K * g));
+                    }
+                else
+                    for (int a = 0; a < M; ++a)
+                        acc = fma(fma(c0, K0[a], fma(c1, K1[a], Kb[a])), v[a], acc);
+                EnergyRec& E       = rec[q * ne + S.eid[c]];
+                E.pb[4 * ab + s]  = ab || S.far[c] ? acc : acc * S.dny[c];
+                E.bpb[4 * ab + s] = 0.;
+            }
+        }
+    }
+}
+
+// Pair + brem of the mixed path.
 __global__ void __launch_bounds__(kWarps * 32)
     spec_pb_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
-                   const double* __restrict__ dsc, EnergyRec* __restrict__ rec,
-                   const uint64_t* __restrict__ flags, int G)
+                   const double* __restrict__ dsc, EnergyRec* __restrict__ rec, int G)
 {
-    constexpr bool MIX = MODE == kSpecMixed;
     extern __shared__ __align__(16) unsigned char s_raw[];
-    PbShared<MODE>& S   = *reinterpret_cast<PbShared<MODE>*>(s_raw);
-    const Gp19Table G19 = {L.gp19.d0, L.gp19.d1, L.gp19.d2, L.gp19.d3, L.gp19.nb,
-                           L.gp19.ye, L.gp19.t,  L.gp19.w,  L.gp19.lognb,
-                           L.gp19.logw, L.gp19.data};
+    PbShared& S         = *reinterpret_cast<PbShared*>(s_raw);
+    const Gp19Table G19 = gp19_table(L);
     const bool prof   = L.use_brem && L.brem_impl == 2 && G19.d3 <= kGp19MaxW;
     const double wmin = prof ? G19.w[0] : 0., wmax = prof ? G19.w[G19.d3 - 1] : 0.;
     for (int k = threadIdx.x; k < kMaxQ; k += blockDim.x)
@@ -290,46 +588,21 @@ __global__ void __launch_bounds__(kWarps * 32)
 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     PbWarp& W      = S.w[wid];
-    PbWarpMixed& X = S.m[MIX ? wid : 0];
+    PbWarpMixed& X = S.m[wid];
     const int n = L.n1, M = 2 * n, ne = L.n_energies;
     const bool nbb      = L.neglect_blocking != 0;
     const int64_t nwarp = (int64_t)gridDim.x * kWarps;
+    const int grp = lane % G, per_round = 32 / G;
 
     for (int64_t q = (int64_t)blockIdx.x * kWarps + wid; q < np; q += nwarp)
     {
-        const uint64_t emask = energy_mask(MODE, flags, q, ne);
-        if (emask == 0ull)
-            continue;
-        // the redo passes pack this point's flagged energies into full rounds
-        const int Gq        = MODE == kSpecRedo ? pick_groups(__popcll(emask), M) : G;
-        const int grp       = lane % Gq;
-        const int per_round = 32 / Gq;
         const int64_t p     = p0 + q;
         const double nbar = L.eos[0][p], T = L.eos[1][p], ye = L.eos[2][p];
         const double yp = L.eos[3][p], yn = L.eos[4][p], mu_e = L.eos[7][p];
         const double eta_e = mu_e / T;
         EnergyRec* R       = rec + q * ne;
-        // energies so low that the pair kernel needs the reference's own Fermi
-        // integrals (kPairLowEnergy): the point's node tables then too
-        bool low = false;
-        if (L.use_pair && !MIX)
-        {
-            for (int c = lane; c < ne; c += 32)
-                low = low || (((emask >> c) & 1ull) && L.energies[c] < kPairLowEnergy * T);
-            low = __any_sync(0xffffffffu, low);
-        }
         __syncwarp();
         load_distr(dsc, q, &W.d, lane);
-        if (lane == 28 && L.use_pair)
-        {
-            double f[2];
-            if (low)
-                fdi_rational<3, 4>(eta_e, f);
-            else
-                fdi_orders<3, 4>(eta_e, f);
-            W.fe3 = f[0];
-            W.fe4 = f[1];
-        }
         if (L.use_brem && L.brem_impl == 0)
         {
             if (lane >= 6 && lane < 9)
@@ -345,7 +618,7 @@ __global__ void __launch_bounds__(kWarps * 32)
         if (lane == 0)
         {
             W.same_cf = same_cf_of(W.d);
-            if (MIX && L.use_brem && L.brem_impl == 0)
+            if (L.use_brem && L.brem_impl == 0)
                 fp32::hr98_mixed_from(W.hr, &X.hm);
         }
         if (prof)
@@ -359,8 +632,7 @@ __global__ void __launch_bounds__(kWarps * 32)
                 const int pr = e / G19.d3, l = e - pr * G19.d3;
                 const double v = gp19_profile_eval(G19, W.gc[pr], l);
                 W.gpp[pr][l] = v;
-                if (MIX)
-                    X.gp32[pr][l] = (float)v;
+                X.gp32[pr][l] = (float)v;
             }
         }
         __syncwarp();
@@ -378,45 +650,27 @@ __global__ void __launch_bounds__(kWarps * 32)
             W.nb[a]         = nu;
             W.zb[a]         = nu / T;
             total_nu_f4(nu, W.d, same_cf, W.gb[a]);
-            if (MIX)
+            const dfm::df yd = dfm::from_double(nu / T);
+            X.ybh[a] = yd.hi;
+            X.ybl[a] = yd.lo;
+            if (L.use_pair)
             {
-                const dfm::df yd = dfm::from_double(nu / T);
-                X.ybh[a] = yd.hi;
-                X.ybl[a] = yd.lo;
-                if (L.use_pair)
-                {
-                    X.ehz[a] = fx::exp(W.zb[a] - 0.5 * fabs(eta_e));
-                    X.dnz[a] = fx::exp(-W.zb[a]);
-                }
+                X.ehz[a] = fx::exp(W.zb[a] - 0.5 * fabs(eta_e));
+                X.dnz[a] = fx::exp(-W.zb[a]);
+            }
 #pragma unroll
-                for (int s = 0; s < 4; ++s)
-                {
-                    X.gb32[a][s]  = (float)W.gb[a][s];
-                    X.gbm32[a][s] = (float)(1. - W.gb[a][s]);
-                }
+            for (int s = 0; s < 4; ++s)
+            {
+                X.gb32[a][s]  = (float)W.gb[a][s];
+                X.gbm32[a][s] = (float)(1. - W.gb[a][s]);
             }
         }
-        // the FP64 pair kernel's Fermi integrals (the mixed pass uses the
-        // FP32 integral, bnsn_pair32.cuh)
-        if (L.use_pair && !MIX)
-            for (int t = lane; t < 2 * M; t += 32)
-            {
-                const int a    = t >> 1;
-                const int i    = a < n ? a : a - n;
-                const double z = (a < n ? ts * S.x[i] : ts / S.x[i]) / T;
-                if (low)
-                    fdi_rational<1, 5>(t & 1 ? eta_e + z : eta_e - z, t & 1 ? W.fpz[a] : W.fmz[a]);
-                else if (t & 1)
-                    fdi_orders<1, 5>(eta_e + z, W.fpz[a]);
-                else
-                    fdi_orders<1, 5>(eta_e - z, W.fmz[a]);
-            }
-        // mixed: FP32 brem for HR98 and the GP19 profiles (not the high-T
+        // FP32 brem for HR98 and the GP19 profiles (not the high-T
         // extrapolation) inside the FP32 range envelope
         bool b32  = false;
         double sb = 0.;
         float thr = 0.f, lt2 = 0.f;
-        if (MIX && L.use_brem)
+        if (L.use_brem)
         {
             b32 = (L.brem_impl == 0 || (prof && W.gp.regime != 3 && W.gp.regime != 5)) &&
                   fp32_envelope(W.d, eta_e);
@@ -431,61 +685,37 @@ __global__ void __launch_bounds__(kWarps * 32)
         }
         // brem in FP64 here when FP32 does not apply, except the full-table GP19
         // kernel (w axis longer than the profiles hold), left to the FP64 redo
-        const bool skip = MIX && L.use_brem && !b32 && L.brem_impl == 2 && !prof;
+        const bool skip = L.use_brem && !b32 && L.brem_impl == 2 && !prof;
 
         for (int e0 = 0; e0 < ne; e0 += kEChunk)
         {
             const int nec     = (ne - e0) < kEChunk ? (ne - e0) : kEChunk;
-            const uint32_t cm = (uint32_t)(emask >> e0) &
-                                (nec == 32 ? 0xffffffffu : ((1u << nec) - 1u));
-            if (cm == 0u)
-                continue;
             __syncwarp();
             for (int c = lane; c < nec; c += 32)
             {
-                if (!((cm >> c) & 1u))
-                    continue;
-                const double y = L.energies[e0 + c] / T;
-                if (L.use_pair && !skip && !MIX)
+                const double y   = L.energies[e0 + c] / T;
+                const dfm::df yd = dfm::from_double(y);
+                X.yeh[c] = yd.hi;
+                X.yel[c] = yd.lo;
+                if (L.use_pair)
                 {
-                    if (low && L.energies[e0 + c] < kPairLowEnergy * T)
-                    {
-                        fdi_rational<1, 5>(eta_e - y, W.fmy[c]);
-                        fdi_rational<1, 5>(eta_e + y, W.fpy[c]);
-                    }
-                    else
-                    {
-                        fdi_orders<1, 5>(eta_e - y, W.fmy[c]);
-                        fdi_orders<1, 5>(eta_e + y, W.fpy[c]);
-                    }
-                }
-                if (MIX)
-                {
-                    const dfm::df yd = dfm::from_double(y);
-                    X.yeh[c] = yd.hi;
-                    X.yel[c] = yd.lo;
-                    if (L.use_pair)
-                    {
-                        X.ehy[c] = fx::exp(y - 0.5 * fabs(eta_e));
-                        X.dny[c] = fx::exp(-y);
-                    }
+                    X.ehy[c] = fx::exp(y - 0.5 * fabs(eta_e));
+                    X.dny[c] = fx::exp(-y);
                 }
             }
             __syncwarp();
-            const int nt = __popc(cm);
-            for (int r0 = 0; r0 < nt; r0 += per_round)
+            for (int r0 = 0; r0 < nec; r0 += per_round)
             {
-                const int kq    = r0 + lane / Gq;
-                const bool act  = kq < nt;
-                const int c     = act ? nth_bit(cm, kq) : 0;
+                const bool act  = r0 + lane / G < nec;
+                const int c     = act ? r0 + lane / G : 0;
                 const double nu = act ? L.energies[e0 + c] : 1.;
                 const double w  = nu / T;
                 double acc[8];
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)
                     acc[kk] = 0.;
-                float gl[8]; // mixed: sum|t| / 1.25 + 1e9 x dropped
-                double gp[8]; // mixed: sum|t| of the FP32 pair terms
+                float gl[8]; // sum|t| / 1.25 + 1e9 x dropped
+                double gp[8]; // sum|t| of the FP32 pair terms
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)
                 {
@@ -493,20 +723,15 @@ __global__ void __launch_bounds__(kWarps * 32)
                     gp[kk] = 0.;
                 }
                 const double sbe = sb * fx::exp(-w); // brem emission carries e^{-nu/T}
-                const double inu2 = MIX ? 1. / (nu * nu) : 0.;
+                const double inu2 = 1. / (nu * nu);
                 if (act && !skip)
                 {
-                    for (int a = grp; a < M; a += Gq)
+                    for (int a = grp; a < M; a += G)
                     {
                         const double wa  = S.B1[a];
                         const double nub = W.nb[a];
                         const double* gb = W.gb[a];
-                        double pe[4] = {0., 0., 0., 0.}, pa[4] = {0., 0., 0., 0.};
                         double be = 0., ba = 0.;
-                        if (L.use_pair && !MIX)
-                            pair_kernel(T, eta_e, nu, nub, w, W.zb[a], W.fmy[c], W.fpy[c],
-                                        W.fmz[a], W.fpz[a], W.fe3, W.fe4, pe, pa,
-                                        low && nu < kPairLowEnergy * T);
                         if (L.use_brem && !b32)
                         {
                             if (L.brem_impl == 0)
@@ -516,22 +741,17 @@ __global__ void __launch_bounds__(kWarps * 32)
                             else if (prof)
                                 gp19_profile_node(W.gp, W.gpp, S.lw, G19.d3, wmin, wmax, nu,
                                                   nub, &be, &ba);
-                            else if (!MIX)
-                                gp19_kernel(G19, nbar, ye, T, nu, nub, &be, &ba);
-                        }
-                        const double nb2 = nub * nub;
-                        if (!MIX || (L.use_brem && !b32))
-                        {
+                            const double nb2 = nub * nub;
 #pragma unroll
                             for (int s = 0; s < 4; ++s)
                             {
                                 const int ps    = s ^ 1;
                                 const double bf = nbb ? 1. : 1. - gb[ps];
-                                acc[s] += wa * (nb2 * ((pe[s] + be) * bf));
-                                acc[4 + s] += wa * (nb2 * ((pa[s] + ba) * gb[ps]));
+                                acc[s] += wa * (nb2 * (be * bf));
+                                acc[4 + s] += wa * (nb2 * (ba * gb[ps]));
                             }
                         }
-                        if (MIX && L.use_pair)
+                        if (L.use_pair)
                         {
                             // FP32 pair integral: (em, ab) (nu nubar)^2, positive
                             double qe[4], qa[4];
@@ -552,7 +772,7 @@ __global__ void __launch_bounds__(kWarps * 32)
                                 gp[4 + s] += fabs(ta);
                             }
                         }
-                        if (MIX && b32)
+                        if (b32)
                         {
                             // kernel shape at x = (nu + nubar) / T (hi + lo)
                             const dfm::df xs = dfm::add(dfm::df{X.yeh[c], X.yel[c]},
@@ -630,13 +850,10 @@ __global__ void __launch_bounds__(kWarps * 32)
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)
                 {
-                    acc[kk] = seg_sum(acc[kk], Gq);
-                    if (MIX)
-                    {
-                        gl[kk] = seg_sum(gl[kk], Gq);
-                        if (L.use_pair)
-                            gp[kk] = seg_sum(gp[kk], Gq);
-                    }
+                    acc[kk] = seg_sum(acc[kk], G);
+                    gl[kk]  = seg_sum(gl[kk], G);
+                    if (L.use_pair)
+                        gp[kk] = seg_sum(gp[kk], G);
                 }
                 if (act && grp == 0)
                 {
@@ -644,15 +861,11 @@ __global__ void __launch_bounds__(kWarps * 32)
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk)
                     {
-                        E.pb[kk] = acc[kk];
-                        if (MIX)
-                            E.bpb[kk] = skip ? INFINITY
-                                             : (b32 ? (kk < 4 ? sbe : sb) *
-                                                          ((double)gl[kk] + kSpecFloor)
-                                                    : 0.) +
-                                                   gp[kk] * (1. / kSpecCancelPair);
-                        else if (MODE == kSpecRedo)
-                            E.bpb[kk] = 0.;
+                        E.pb[kk]  = acc[kk];
+                        E.bpb[kk] = skip ? INFINITY
+                                         : (b32 ? (kk < 4 ? sbe : sb) * ((double)gl[kk] + kSpecFloor)
+                                                : 0.) +
+                                               gp[kk] * (1. / kSpecCancelPair);
                     }
                 }
             }
@@ -666,41 +879,234 @@ __global__ void __launch_bounds__(kWarps * 32)
 struct NesWarp
 {
     Distr d;
-    double fe[2][6];
-    double fd0[2];
-    int same_cf;
-    double fw[kEChunk][2][6];
-};
-
-struct NesWarpMixed
-{
-    NepsMixed Q; // eta and F_k(eta) of e-, e+
+    double fe[2][6], fd0[2];
+    double fw[kEChunk][2][5]; // Fermi integrals at eta_e - nu/T (nes_spec_node)
     NesSpec Z;
-    dfm::df rw[kEChunk][2][5]; // unreflected F_1..F_5 at eta_e - nu/T per energy and lepton
-    dfm::df aw[kEChunk][2];
+    NesDf Q;
     dfm::df lnu[kEChunk];
 };
 
-template <int MODE>
 struct NesShared
 {
     double x[kMaxQ], xinv[kMaxQ], B1[kMaxM];
     dfm::df lxd[kMaxQ];
     dfm::FdiTab ftab;
     NesWarp w[kWarps];
-    NesWarpMixed m[(MODE == kSpecMixed || MODE == kSpecAcc) ? kWarps : 1];
 };
 
-template <int MODE>
-__global__ void __launch_bounds__(kWarps * 32, MODE == kSpecMixed ? 4 : 1)
-    spec_nes_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
-                    const double* __restrict__ dsc, EnergyRec* __restrict__ rec,
-                    const uint64_t* __restrict__ flags, int G)
+// NES/NPS in FP64: every energy, or (flags) the ones the mixed path's checks
+// flagged.  A CTA takes a point; groups of G consecutive lanes take an energy and
+// split its nodes.  An energy w = nu/T enters its nodes (w x_i, w / x_i) only
+// through one bracket per lepton (nes_bracket): the couplings of the four species,
+// the factors 1 / (1 - e) of NEPSExpFunc and the occupations follow from it, and the
+// node's weight nubar^2 cancels the bracket's 1 / w'^2.  Bound by the FP64 pipe beside
+// the integer work of its Fermi integrals and exponentials.
+struct Nes64Smem
 {
-    constexpr bool ACC = MODE == kSpecAcc;
-    constexpr bool MIX = MODE == kSpecMixed || ACC;
+    double x[kMaxQ], xinv[kMaxQ], xc[kMaxQ], xci[kMaxQ]; // nodes, x^0.6 and inverses
+    double m[kMaxM];                                     // 24 x weight
+    Occ64 occ[4];
+    double fe[2][6], fd0[2];
+    double w[kEChunk], wc[kEChunk];     // nu/T and its 0.6th power
+    double fw[kEChunk][2][5];           // phi_1..phi_5 at eta_e - nu/T
+    int eid[kEChunk];
+    int twin;     // heavy-lepton neutrinos evolved as one species
+    double steep; // T over the lowest temperature of the point
+};
+
+// 1 - e^{-d} for e = e^{-d}, d >= 0: by its series below d = 1/4 (2^-53 relative).
+__device__ __forceinline__ double one_minus_exp(double d, double e)
+{
+    if (d >= 0.25)
+        return 1. - e;
+    double t = 1. / 479001600.;
+    t = fma(t, -d, 1. / 39916800.);
+    t = fma(t, -d, 1. / 3628800.);
+    t = fma(t, -d, 1. / 362880.);
+    t = fma(t, -d, 1. / 40320.);
+    t = fma(t, -d, 1. / 5040.);
+    t = fma(t, -d, 1. / 720.);
+    t = fma(t, -d, 1. / 120.);
+    t = fma(t, -d, 1. / 24.);
+    t = fma(t, -d, 1. / 6.);
+    t = fma(t, -d, 0.5);
+    return fma(d * d, -t, d);
+}
+
+// Emission term of species s at a node of an energy so high that everything it emits
+// is next to 0: the reference clamps its exponentials at e^-700 and the products
+// round in the denormal range, so they are taken in its order.  A0, B0
+// and A1, B1: the brackets of e- and e+; m = 24 x weight; f: the NEPSExpFunc factor.
+__device__ __noinline__ double nes64_far(int s, double A0, double B0, double A1, double B1,
+                                         double w, double wp, double T, double m, double f,
+                                         double g)
+{
+    const double P = w * wp, nub = wp * T;
+    const double h = 24. * k::NepsConst * (T * T) / (P * P);
+    const double b = s < 2 ? k::NepsBPlus : k::NepsBMinus, z = k::NepsBZero;
+    const double r0 = s & 1 ? z * A0 + b * B0 : b * A0 + z * B0;
+    const double r1 = s & 1 ? b * A1 + z * B1 : z * A1 + b * B1;
+    const double em = __dadd_rn(__dmul_rn(h * r0, f), __dmul_rn(h * r1, f));
+    return m * (1. / 24.) * (nub * nub * __dmul_rn(em, g));
+}
+
+__global__ void __launch_bounds__(kWarps * 32, 4)
+    spec_nes64_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0,
+                      const double* __restrict__ dsc, EnergyRec* __restrict__ rec,
+                      const uint64_t* __restrict__ flags)
+{
+    constexpr int NT = kWarps * 32;
+    const int64_t q  = blockIdx.x;
+    const int n = L.n1, M = 2 * n, ne = L.n_energies, tid = threadIdx.x;
+    const uint64_t emask = energy_mask(flags, q, ne);
+    if (emask == 0ull)
+        return;
+    __shared__ Nes64Smem S;
+    const int64_t p  = p0 + q;
+    const double T   = L.eos[1][p], eta_e = L.eos[7][p] / T;
+    const bool nbb   = L.neglect_blocking != 0;
+    const double sc  = k::NepsConst * (T * T) * (T * T);
+    if (tid < n)
+    {
+        const double x = L.x1[tid], xi = 1. / x;
+        S.x[tid]    = x;
+        S.xinv[tid] = xi;
+        S.xc[tid]   = fx::pow(x, k::CF);
+        S.xci[tid]  = fx::pow(xi, k::CF);
+    }
+    if (tid >= 64 && tid < 64 + M)
+        S.m[tid - 64] = 24. * L.B1[tid - 64];
+    const Distr& d = *(const Distr*)(dsc + q * 28);
+    if (tid >= 32 && tid < 36)
+        occ64_from(d, tid - 32, T, &S.occ[tid - 32]);
+    if (tid == 64 || tid == 65)
+    {
+        const double et = tid == 65 ? -eta_e : eta_e;
+        fdi_orders<0, 5>(et, S.fe[tid - 64]);
+        S.fd0[tid - 64] = fermi_distr(0., 1., et);
+    }
+    if (tid == 96)
+    {
+        S.twin   = species_twins(d);
+        double t = fmin(T, fmin(d.temp_t[0], d.temp_f[0]));
+        for (int s = 1; s < 4; ++s)
+            t = fmin(t, fmin(d.temp_t[s], d.temp_f[s]));
+        S.steep = T / t;
+    }
+    const int nt = __popcll(emask);
+    const int G  = pick_groups(nt < kEChunk ? nt : kEChunk, M, NT);
+    const int grp = tid % G, per_round = NT / G;
+    const int chunks = (nt + kEChunk - 1) / kEChunk, per = (nt + chunks - 1) / chunks;
+#pragma unroll 1
+    for (int k0 = 0; k0 < nt; k0 += per)
+    {
+        const int nc = nt - k0 < per ? nt - k0 : per;
+        __syncthreads(); // the last chunk's readers are done
+        for (int t = tid; t < 2 * nc; t += NT)
+        {
+            const int c = t >> 1, e = nth_bit(emask, k0 + c);
+            const double w = L.energies[e] / T;
+            if ((t & 1) == 0)
+            {
+                S.eid[c] = e;
+                S.w[c]   = w;
+                S.wc[c]  = fx::pow(w, k::CF);
+            }
+            fx::fd_orders<1, 5, true>((t & 1 ? -eta_e : eta_e) - w, S.fw[c][t & 1]);
+        }
+        __syncthreads();
+        const Occ64* occ  = S.occ;
+        const bool common = occ[0].cf == k::CF && occ[1].cf == k::CF && occ[2].cf == k::CF &&
+                            occ[3].cf == k::CF;
+        const int nocc = S.twin ? 3 : 4;
+#pragma unroll 1
+        for (int r0 = 0; r0 < nc; r0 += per_round)
+        {
+            const bool act = r0 + tid / G < nc;
+            const int c    = act ? r0 + tid / G : 0;
+            const double w = S.w[c];
+            const bool tiny = !(w * S.steep < 500.); // e^-500: emission near the denormals
+            double acc[8];
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+                acc[kk] = 0.;
+#pragma unroll 1
+            for (int a = act ? grp : M; a < M; a += G)
+            {
+                const bool down = a < n; // w' < w: the neutrino loses energy
+                const int i     = down ? a : a - n;
+                const double wp = w * (down ? S.x[i] : S.xinv[i]);
+                const double x = down ? w : wp, y = down ? wp : w, dl = x - y;
+                double U = 0., V = 0.; // A of e- + B of e+, B of e- + A of e+
+                double A = 0., B = 0.; // at the end those of e+
+#pragma unroll 1
+                for (int e = 0; e < 2; ++e)
+                {
+                    const double eta = e ? -eta_e : eta_e;
+                    const double* fe = S.fe[e];
+                    if (y > eta * 1e-3)
+                    {
+                        double f[5];
+                        const double* g = S.fw[c][e];
+                        fx::fd_orders<1, 5, true>(eta - wp, f);
+                        nes_bracket(eta, x, y, dl, down ? g : f, down ? f : g, fe, &A, &B);
+                    }
+                    else
+                        nes_bracket_taylor(eta, x, y, dl, fe, S.fd0[e], &A, &B);
+                    U += e ? B : A;
+                    V += e ? A : B;
+                }
+                constexpr double bp = k::NepsBPlus, bm = k::NepsBMinus, bz = k::NepsBZero;
+                const double zU = bz * U, zV = bz * V;
+                const double r[4] = {fma(bp, U, zV), fma(bp, V, zU), fma(bm, U, zV),
+                                     fma(bm, V, zU)};
+                // NEPSExpFunc: e / (1 - e) up and 1 / (1 - e) down in energy
+                const double ex = safe_exp(-dl);
+                const double kb = S.m[a] * fx::rcp(one_minus_exp(dl, ex) + (dl == 0.));
+                const double ka = kb * ex;
+                const double ke = down ? ka : kb, kk = down ? kb : ka;
+                const double pc = common ? S.wc[c] * (down ? S.xc[i] : S.xci[i]) : 0.;
+                double g = 0.;
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                {
+                    if (s < nocc)
+                        g = occ64_one(occ[s], wp, common ? pc : fx::pow(wp, occ[s].cf));
+                    if (tiny)
+                        acc[s] += nes64_far(s, U - B, V - A, A, B, w, wp, T, S.m[a],
+                                            ke / S.m[a], g) * (w * w / sc);
+                    else
+                        acc[s] = fma(ke * r[s], g, acc[s]);
+                    acc[4 + s] = fma(kk * r[s], nbb ? 1. : 1. - g, acc[4 + s]);
+                }
+            }
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+                acc[kk] = seg_sum(acc[kk], G);
+            if (act && grp == 0)
+            {
+                EnergyRec& E   = rec[q * ne + S.eid[c]];
+                const double f = sc * fx::rcp(w * w);
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk)
+                {
+                    E.nes[kk]  = f * acc[kk];
+                    // -inf: the first check saw the other parts alone and stands
+                    E.bnes[kk] = flags && isinf(E.bnes[kk]) ? -INFINITY : 0.;
+                }
+            }
+        }
+    }
+}
+
+// NES/NPS of the mixed path.
+template <bool LOW>
+__global__ void __launch_bounds__(kWarps * 32, 4)
+    spec_nes_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
+                    const double* __restrict__ dsc, EnergyRec* __restrict__ rec)
+{
     extern __shared__ __align__(16) unsigned char s_raw[];
-    NesShared<MODE>& S = *reinterpret_cast<NesShared<MODE>*>(s_raw);
+    NesShared& S = *reinterpret_cast<NesShared*>(s_raw);
     for (int k = threadIdx.x; k < kMaxQ; k += blockDim.x)
     {
         S.x[k]    = L.x1[k];
@@ -709,30 +1115,30 @@ __global__ void __launch_bounds__(kWarps * 32, MODE == kSpecMixed ? 4 : 1)
     }
     for (int k = threadIdx.x; k < kMaxM; k += blockDim.x)
         S.B1[k] = L.B1[k];
-    if (MIX)
-        for (int k = threadIdx.x; k < (int)(sizeof(dfm::FdiTab) / sizeof(float)); k += blockDim.x)
-            ((float*)&S.ftab)[k] = ((const float*)&dfm::kFdiTab)[k];
+    for (int k = threadIdx.x; LOW && k < (int)(sizeof(dfm::FdiTab) / sizeof(float)); k += blockDim.x)
+        ((float*)&S.ftab)[k] = ((const float*)&dfm::kFdiTab)[k];
     __syncthreads();
 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    NesWarp& W      = S.w[wid];
-    NesWarpMixed& X = S.m[MIX ? wid : 0];
+    NesWarp& W     = S.w[wid];
     const int n = L.n1, M = 2 * n, ne = L.n_energies;
     const bool nbb      = L.neglect_blocking != 0;
     const int64_t nwarp = (int64_t)gridDim.x * kWarps;
 
     for (int64_t q = (int64_t)blockIdx.x * kWarps + wid; q < np; q += nwarp)
     {
-        const uint64_t emask = energy_mask(MODE, flags, q, ne);
-        if (emask == 0ull)
-            continue;
-        const int Gq        = (MODE == kSpecRedo || ACC) ? pick_groups(__popcll(emask), M) : G;
-        const int grp       = lane % Gq;
-        const int per_round = 32 / Gq;
         const int64_t p     = p0 + q;
         const double T = L.eos[1][p], mu_e = L.eos[7][p];
         const double eta_e = mu_e / T, invT = 1. / T;
         EnergyRec* R       = rec + q * ne;
+        if (LOW)
+        {
+            bool any = false;
+            for (int e = lane; e < ne; e += 32)
+                any = any || !(L.energies[e] / T >= kSpecNesDfW);
+            if (!__any_sync(0xffffffffu, any))
+                continue;
+        }
         __syncwarp();
         load_distr(dsc, q, &W.d, lane);
         if (lane == 28 || lane == 29)
@@ -743,8 +1149,6 @@ __global__ void __launch_bounds__(kWarps * 32, MODE == kSpecMixed ? 4 : 1)
             W.fd0[e] = fermi_distr(0., 1., et);
         }
         __syncwarp();
-        if (lane == 0)
-            W.same_cf = same_cf_of(W.d);
         NepsPoint NP;
         NP.T    = T;
         NP.pre  = k::NepsConst * (T * T);
@@ -754,68 +1158,63 @@ __global__ void __launch_bounds__(kWarps * 32, MODE == kSpecMixed ? 4 : 1)
         NP.fd01 = W.fd0[1];
         NP.fe0  = W.fe[0];
         NP.fe1  = W.fe[1];
-        bool m32  = false;
-        double sn = 0.;
-        if (MIX)
+        const bool m32  = fp32_envelope(W.d, eta_e);
+        const double sn = (T * T) * NP.pre;
+        if (lane < 4)
+            nes_spec_species(W.d, lane, &W.Z);
+        else if (lane == 8)
+            nes_spec_masks(W.d, &W.Z);
+        else if (LOW && lane >= 16 && lane < 18)
         {
-            m32 = fp32_envelope(W.d, eta_e);
-            if (m32)
-            {
-                if (lane < 2)
-                {
-                    X.Q.eta[lane] = dfm::from_double(lane ? NP.eta1 : NP.eta0);
-                    dfm::fdi_raw15(X.Q.eta[lane], X.Q.reta[lane], 1, &S.ftab);
-                }
-                else if (lane >= 8 && lane < 12)
-                    nes_spec_species(W.d, lane - 8, &X.Z);
-                else if (lane == 12)
-                    nes_spec_masks(W.d, &X.Z);
-            }
-            sn = (T * T) * NP.pre;
+            W.Q.eta[lane - 16] = dfm::from_double(lane == 17 ? -eta_e : eta_e);
+            dfm::fdi_raw15(W.Q.eta[lane - 16], W.Q.reta[lane - 16], 1, &S.ftab);
         }
         __syncwarp();
-        const bool same_cf = W.same_cf != 0;
 
         for (int e0 = 0; e0 < ne; e0 += kEChunk)
         {
             const int nec     = (ne - e0) < kEChunk ? (ne - e0) : kEChunk;
-            const uint32_t cm = (uint32_t)(emask >> e0) &
-                                (nec == 32 ? 0xffffffffu : ((1u << nec) - 1u));
-            if (cm == 0u)
-                continue;
             __syncwarp();
-            for (int c = lane; c < nec; c += 32)
+            // this kernel's energies of the chunk; LOW: those below kSpecNesDfW, and
+            // the ones left to the FP64 pass (bound = inf)
+            const double wl = lane < nec ? L.energies[e0 + lane] / T : 0.;
+            const bool runl = m32 && wl >= kSpecNesMinW, lowl = !(wl >= kSpecNesDfW);
+            const uint32_t mask = __ballot_sync(0xffffffffu, runl && lowl == LOW);
+            if (lane < nec)
             {
-                if (!((cm >> c) & 1u))
-                    continue;
-                const double nu = L.energies[e0 + c];
-                const double y  = nu / T;
-                if (!MIX)
+                W.lnu[lane] = dfm::from_double(log(L.energies[e0 + lane]));
+                if (!runl && lowl == LOW)
                 {
-                    fdi_orders<0, 5>(eta_e - y, W.fw[c][0]);
-                    fdi_orders<0, 5>(NP.eta1 - y, W.fw[c][1]);
-                }
-                else if (m32 && y >= kSpecNesMinW)
-                {
-                    X.lnu[c] = dfm::from_double(log(nu));
-#pragma unroll 1
-                    for (int e = 0; e < 2; ++e)
+                    EnergyRec& E = R[e0 + lane];
+#pragma unroll
+                    for (int kk = 0; kk < 8; ++kk)
                     {
-                        X.aw[c][e] = dfm::from_double((e ? NP.eta1 : NP.eta0) - y);
-                        dfm::fdi_raw15(X.aw[c][e], X.rw[c][e], 1, &S.ftab);
+                        E.nes[kk]  = 0.;
+                        E.bnes[kk] = INFINITY;
                     }
                 }
             }
-            __syncwarp();
-            const int nt = __popc(cm);
-            for (int r0 = 0; r0 < nt; r0 += per_round)
+            for (int t = lane; t < 2 * nec; t += 32)
             {
-                const int kq    = r0 + lane / Gq;
+                const int c = t >> 1, e = t & 1;
+                if (!((mask >> c) & 1u))
+                    continue;
+                const double a = (e ? NP.eta1 : NP.eta0) - L.energies[e0 + c] / T;
+                if (LOW)
+                    dfm::fdi_raw15(dfm::from_double(a), (dfm::df*)W.fw[c][e], 1, &S.ftab);
+                else
+                    fx::fd_orders<1, 5, true>(a, W.fw[c][e]);
+            }
+            __syncwarp();
+            // G lanes an energy
+            const int nt = __popc(mask), G = pick_groups(nt, M, 32), grp = lane & (G - 1);
+            for (int r0 = 0; r0 * 32 < nt * G; ++r0)
+            {
+                const int kq    = (r0 * 32 + lane) / G;
                 const bool act  = kq < nt;
-                const int c     = act ? nth_bit(cm, kq) : 0;
+                const int c     = act ? nth_bit(mask, kq) : 0;
                 const double nu = act ? L.energies[e0 + c] : 1.;
                 const double w  = nu / T;
-                const bool run  = act && (!MIX || (m32 && w >= kSpecNesMinW));
                 double acc[8];
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)
@@ -825,90 +1224,49 @@ __global__ void __launch_bounds__(kWarps * 32, MODE == kSpecMixed ? 4 : 1)
                 for (int kk = 0; kk < 8; ++kk)
                     gl[kk] = 0.f;
                 float sig[2] = {0.f, 0.f};
-                double sne = 0., sna = 0.;
-                if (MIX)
+                // scale of this energy: group-wide maximum of the lanes' scans
+                nes_spec_scan(W.Z, (float)w, (float)nu, W.lnu[c].hi, S.x, S.lxd, n,
+                              act ? grp : M, G, nbb, sig);
+                for (int o = 1; o < G; o <<= 1)
                 {
-                    // scale of this energy: group-wide maximum of the lanes' scans
-                    nes_spec_scan(X.Z, (float)w, (float)nu, X.lnu[run ? c : 0].hi, S.x, S.lxd,
-                                  n, run ? grp : M, Gq, nbb, sig);
-                    for (int o = 1; o < Gq; o <<= 1)
-                    {
-                        sig[0] = fmaxf(sig[0], __shfl_xor_sync(0xffffffffu, sig[0], o));
-                        sig[1] = fmaxf(sig[1], __shfl_xor_sync(0xffffffffu, sig[1], o));
-                    }
-                    sig[0] = isfinite(sig[0]) ? sig[0] : 0.f;
-                    sig[1] = isfinite(sig[1]) ? sig[1] : 0.f;
-                    sne    = sn * fx::exp((double)sig[0]);
-                    sna    = sn * fx::exp((double)sig[1]);
+                    sig[0] = fmaxf(sig[0], __shfl_xor_sync(0xffffffffu, sig[0], o));
+                    sig[1] = fmaxf(sig[1], __shfl_xor_sync(0xffffffffu, sig[1], o));
                 }
+                sig[0] = isfinite(sig[0]) ? sig[0] : 0.f;
+                sig[1] = isfinite(sig[1]) ? sig[1] : 0.f;
+                const double sne = sn * fx::exp((double)sig[0]);
+                const double sna = sn * fx::exp((double)sig[1]);
                 const dfm::df Wd = dfm::from_double(w);
-                if (run)
+                if (act)
                 {
-                    for (int a = grp; a < M; a += Gq)
+                    for (int a = grp; a < M; a += G)
                     {
-                        const int i      = a < n ? a : a - n;
-                        const double wa  = S.B1[a];
-                        const double nub =
-                            a < n ? nu * S.x[i] : (MIX ? nu * S.xinv[i] : nu / S.x[i]);
-                        // mixed passes: nubar/T and log nubar without divisions
-                        const double wp  = MIX ? nub * invT : nub / T;
+                        const int i = a < n ? a : a - n;
+                        // nubar/T and log nubar without divisions
+                        const double nub = nu * (a < n ? S.x[i] : S.xinv[i]);
+                        const double wp  = nub * invT;
                         const dfm::df NB = dfm::from_double(nub), WPd = dfm::from_double(wp);
                         const dfm::df LB =
-                            dfm::add(X.lnu[c], a < n ? S.lxd[i] : dfm::neg(S.lxd[i]));
-                        if (ACC)
-                        {
-                            double te[4], ta[4];
-                            float de[4], da[4];
-                            nes_spec_node_df(NP, X.Q, X.Z, &S.ftab, w, wp, Wd, WPd, NB, LB, wa,
-                                             sig[0], sig[1], nbb, X.rw[c], X.aw[c], te, ta, de,
-                                             da);
+                            dfm::add(W.lnu[c], a < n ? S.lxd[i] : dfm::neg(S.lxd[i]));
+                        float te[4], ta[4], de[4], da[4];
+                        nes_spec_node(NP, W.Z, w, wp, Wd, WPd, NB, LB, (float)S.B1[a], sig[0],
+                                      sig[1], nbb, W.fw[c], LOW ? &W.Q : nullptr, &S.ftab, te, ta, de, da);
 #pragma unroll
-                            for (int s = 0; s < 4; ++s)
-                            {
-                                acc[s]     = fma(sne, te[s], acc[s]);
-                                acc[4 + s] = fma(sna, ta[s], acc[4 + s]);
-                                gl[s] += (float)(fabs(te[s]) * (1. / kSpecCancelDf)) + 1e9f * de[s];
-                                gl[4 + s] +=
-                                    (float)(fabs(ta[s]) * (1. / kSpecCancelDf)) + 1e9f * da[s];
-                            }
-                        }
-                        else if (MIX)
+                        for (int s = 0; s < 4; ++s)
                         {
-                            float te[4], ta[4], de[4], da[4];
-                            nes_spec_node(NP, X.Q, X.Z, &S.ftab, w, wp, Wd, WPd, NB, LB, (float)wa,
-                                          sig[0], sig[1], nbb, X.rw[c], X.aw[c], te, ta, de, da);
-#pragma unroll
-                            for (int s = 0; s < 4; ++s)
-                            {
-                                acc[s]     = fma(sne, (double)te[s], acc[s]);
-                                acc[4 + s] = fma(sna, (double)ta[s], acc[4 + s]);
-                                gl[s] += fabsf(te[s]) * (float)(1. / kSpecCancelNes) + 1e9f * de[s];
-                                gl[4 + s] +=
-                                    fabsf(ta[s]) * (float)(1. / kSpecCancelNes) + 1e9f * da[s];
-                            }
-                        }
-                        else
-                        {
-                            double gb[4], em[4], ab[4];
-                            total_nu_f4(nub, W.d, same_cf, gb);
-                            neps_one(NP, nu, nub, W.fw[c][0], W.fw[c][1], em, ab);
-                            const double nb2 = nub * nub;
-#pragma unroll
-                            for (int s = 0; s < 4; ++s)
-                            {
-                                const double bf = nbb ? 1. : 1. - gb[s];
-                                acc[s] += wa * (nb2 * (em[s] * gb[s]));
-                                acc[4 + s] += wa * (nb2 * (ab[s] * bf));
-                            }
+                            acc[s]     = fma(sne, (double)te[s], acc[s]);
+                            acc[4 + s] = fma(sna, (double)ta[s], acc[4 + s]);
+                            gl[s] += fabsf(te[s]) * (float)(1. / kSpecCancelNes) + 1e9f * de[s];
+                            gl[4 + s] +=
+                                fabsf(ta[s]) * (float)(1. / kSpecCancelNes) + 1e9f * da[s];
                         }
                     }
                 }
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)
                 {
-                    acc[kk] = seg_sum(acc[kk], Gq);
-                    if (MIX)
-                        gl[kk] = seg_sum(gl[kk], Gq);
+                    acc[kk] = seg_sum(acc[kk], G);
+                    gl[kk]  = seg_sum(gl[kk], G);
                 }
                 if (act && grp == 0)
                 {
@@ -916,12 +1274,8 @@ __global__ void __launch_bounds__(kWarps * 32, MODE == kSpecMixed ? 4 : 1)
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk)
                     {
-                        E.nes[kk] = acc[kk];
-                        if (MIX)
-                            E.bnes[kk] = run ? (kk < 4 ? sne : sna) * ((double)gl[kk] + kSpecFloor)
-                                             : INFINITY;
-                        else if (MODE == kSpecRedo)
-                            E.bnes[kk] = 0.;
+                        E.nes[kk]  = acc[kk];
+                        E.bnes[kk] = (kk < 4 ? sne : sna) * ((double)gl[kk] + kSpecFloor);
                     }
                 }
             }
@@ -1107,34 +1461,62 @@ cudaError_t grid_of(K kernel, size_t smem, bool* attr_set, int num_sms, int64_t 
     return cudaSuccess;
 }
 
-template <int MODE>
-cudaError_t launch_pb(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
-                      EnergyRec* rec, const uint64_t* flags, int G, cudaStream_t st, int sms)
+cudaError_t launch_pb_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
+                            EnergyRec* rec, int G, cudaStream_t st, int sms)
 {
     static bool attr  = false;
-    const size_t smem = sizeof(PbShared<MODE>);
+    const size_t smem = sizeof(PbShared);
     int grid          = 0;
-    cudaError_t err   = grid_of(spec_pb_kernel<MODE>, smem, &attr, sms, np, &grid);
+    cudaError_t err   = grid_of(spec_pb_kernel, smem, &attr, sms, np, &grid);
     if (err != cudaSuccess || grid == 0)
         return err;
     phase_mark(kPhSpectral, 0, st);
-    spec_pb_kernel<MODE><<<grid, kWarps * 32, smem, st>>>(L, p0, np, dsc, rec, flags, G);
+    spec_pb_kernel<<<grid, kWarps * 32, smem, st>>>(L, p0, np, dsc, rec, G);
     phase_mark(kPhSpectral, 1, st);
     return cudaGetLastError();
 }
 
-template <int MODE>
-cudaError_t launch_nes(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
-                       EnergyRec* rec, const uint64_t* flags, int G, cudaStream_t st, int sms)
+cudaError_t launch_nes_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
+                             EnergyRec* rec, cudaStream_t st, int sms)
 {
-    static bool attr  = false;
-    const size_t smem = sizeof(NesShared<MODE>);
-    int grid          = 0;
-    cudaError_t err   = grid_of(spec_nes_kernel<MODE>, smem, &attr, sms, np, &grid);
+    static bool attr[2] = {false, false};
+    const size_t smem   = sizeof(NesShared);
+    int grid = 0, low = 0;
+    cudaError_t err = grid_of(spec_nes_kernel<false>, smem, &attr[0], sms, np, &grid);
+    if (err == cudaSuccess)
+        err = grid_of(spec_nes_kernel<true>, smem, &attr[1], sms, np, &low);
     if (err != cudaSuccess || grid == 0)
         return err;
     phase_mark(kPhSpectral, 0, st);
-    spec_nes_kernel<MODE><<<grid, kWarps * 32, smem, st>>>(L, p0, np, dsc, rec, flags, G);
+    spec_nes_kernel<false><<<grid, kWarps * 32, smem, st>>>(L, p0, np, dsc, rec);
+    phase_mark(kPhSpectral, 1, st);
+    phase_mark(kPhSpectral, 0, st);
+    spec_nes_kernel<true><<<low, kWarps * 32, smem, st>>>(L, p0, np, dsc, rec);
+    phase_mark(kPhSpectral, 1, st);
+    return cudaGetLastError();
+}
+
+// FP64 passes: every energy (flags null) or the flagged ones.
+cudaError_t launch_pb64(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
+                        EnergyRec* rec, const uint64_t* flags, cudaStream_t st)
+{
+    phase_mark(kPhSpectral, 0, st);
+    const int impl = L.use_brem ? L.brem_impl : 1;
+    if (impl == 0)
+        spec_pb64_kernel<0><<<(int)np, kWarps * 32, 0, st>>>(L, p0, dsc, rec, flags);
+    else if (impl == 1)
+        spec_pb64_kernel<1><<<(int)np, kWarps * 32, 0, st>>>(L, p0, dsc, rec, flags);
+    else
+        spec_pb64_kernel<2><<<(int)np, kWarps * 32, 0, st>>>(L, p0, dsc, rec, flags);
+    phase_mark(kPhSpectral, 1, st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_nes64(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
+                         EnergyRec* rec, const uint64_t* flags, cudaStream_t st)
+{
+    phase_mark(kPhSpectral, 0, st);
+    spec_nes64_kernel<<<(int)np, kWarps * 32, 0, st>>>(L, p0, dsc, rec, flags);
     phase_mark(kPhSpectral, 1, st);
     return cudaGetLastError();
 }
@@ -1198,7 +1580,7 @@ cudaError_t launch_spectral(const OpacityLaunch& L, cudaStream_t st0, int sms, v
     if (L.npts <= 0 || L.n_energies <= 0)
         return cudaSuccess;
     const int ne     = L.n_energies;
-    const int G      = pick_groups(ne < kEChunk ? ne : kEChunk, 2 * L.n1);
+    const int G      = pick_groups(ne < kEChunk ? ne : kEChunk, 2 * L.n1, 32);
     const bool pb    = L.use_pair || L.use_brem;
     const bool inel  = L.use_inel != 0;
     // With an auxiliary stream and scratch, consecutive chunks alternate
@@ -1241,28 +1623,24 @@ cudaError_t launch_spectral(const OpacityLaunch& L, cudaStream_t st0, int sms, v
             break;
         if (!L.mixed)
         {
-            if (pb && (err = launch_pb<kSpecFp64>(L, p0, np, dsc, rec, nullptr, G, st, sms)))
+            if (pb && (err = launch_pb64(L, p0, np, dsc, rec, nullptr, st)))
                 break;
-            if (inel && (err = launch_nes<kSpecFp64>(L, p0, np, dsc, rec, nullptr, G, st, sms)))
+            if (inel && (err = launch_nes64(L, p0, np, dsc, rec, nullptr, st)))
                 break;
             err = launch_assemble<kSpecFp64>(L, p0, np, dsc, rec, fl_pb, fl_nes, st, sms);
             continue;
         }
-        if (pb && (err = launch_pb<kSpecMixed>(L, p0, np, dsc, rec, nullptr, G, st, sms)))
+        if (pb && (err = launch_pb_mixed(L, p0, np, dsc, rec, G, st, sms)))
             break;
-        if (inel && (err = launch_nes<kSpecMixed>(L, p0, np, dsc, rec, nullptr, G, st, sms)))
+        if (inel && (err = launch_nes_mixed(L, p0, np, dsc, rec, st, sms)))
             break;
         if ((err = launch_assemble<kSpecMixed>(L, p0, np, dsc, rec, fl_pb, fl_nes, st, sms)))
             break;
         for (int round = 0; round < 2 && err == cudaSuccess; ++round)
         {
-            if (pb && (err = launch_pb<kSpecRedo>(L, p0, np, dsc, rec, fl_pb, G, st, sms)))
+            if (pb && (err = launch_pb64(L, p0, np, dsc, rec, fl_pb, st)))
                 break;
-            // NES: double-float products first, FP64 for what still fails
-            if (inel && (err = round == 0 ? launch_nes<kSpecAcc>(L, p0, np, dsc, rec, fl_nes, G,
-                                                                 st, sms)
-                                          : launch_nes<kSpecRedo>(L, p0, np, dsc, rec, fl_nes,
-                                                                  G, st, sms)))
+            if (inel && (err = launch_nes64(L, p0, np, dsc, rec, fl_nes, st)))
                 break;
             err = round == 0
                       ? launch_assemble<kSpecRedo>(L, p0, np, dsc, rec, fl_pb, fl_nes, st, sms)
