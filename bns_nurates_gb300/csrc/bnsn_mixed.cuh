@@ -334,7 +334,7 @@ __device__ __forceinline__ void neps_r_mixed(const NepsPoint& P, double w, doubl
 }
 
 // What neps_r_df needs of a point: eta and the unreflected F_1..F_5 of e- and e+.
-struct NesDf
+struct alignas(8) NesDf
 {
     dfm::df reta[2][5], eta[2];
 };
@@ -431,7 +431,7 @@ namespace {
 constexpr float kNesDrop    = 7.52316385e-37f; // 2^-120
 constexpr float kNesDropArg = -83.1777f;       // log 2^-120
 
-struct NesSpec
+struct alignas(8) NesSpec
 {
     dfm::df invTt[4], etat[4], invTf[4], cf[4], lbf[4], lwt[4], lwf[4];
     int has_t;  // bit s: w_t of species s nonzero

@@ -6,7 +6,8 @@
 // Phases per chunk of points (the phase split keeps every kernel's code small enough
 // for the instruction cache; a single fused kernel spent most cycles waiting on
 // instruction fetch):
-//   prelude   NuDistributionParams of each point -> chunk scratch;
+//   prelude   the constants of each point (distribution parameters, brem, beta and
+//             iso constants, Fermi integrals at eta_e) -> chunk scratch;
 //   pb        pair + brem sums of every (point, energy) -> records;
 //   nes       NES/NPS sums -> records;
 //   assemble  beta, iso, the outer factors and the stimulated-absorption
@@ -38,8 +39,8 @@
 // remaining bounds, and a last round finishes what is left.  (A double-float pass over
 // the flagged NES parts before the FP64 one took 2.2 ms of 10.8 per 4,096 points at
 // 5% occupancy, and the FP64 kernels are as fast per energy.)
-// 4,096 points x 24 energies: FP64 n = 10 HR98 without NES 9.1 -> 1.7 ms, n = 20 GP19
-// with NES 17.0 -> 4.1 ms; mixed n = 20 GP19 with NES 12.8 -> 5.8 ms.
+// 4,096 points x 24 energies: FP64 n = 10 HR98 without NES 9.1 -> 1.3 ms, n = 20 GP19
+// with NES 17.0 -> 3.9 ms; mixed n = 20 GP19 with NES 12.8 -> 5.5 ms.
 
 #include <cuda_runtime.h>
 
@@ -136,13 +137,6 @@ __device__ __forceinline__ int nth_bit(uint64_t m, int kq)
     return __ffsll((long long)m) - 1;
 }
 
-// Distribution of a point from the chunk scratch into shared memory.
-__device__ __forceinline__ void load_distr(const double* dsc, int64_t q, Distr* d, int lane)
-{
-    if (lane < 28)
-        (&d->w_t[0])[lane] = dsc[q * 28 + lane];
-}
-
 __device__ __forceinline__ bool same_cf_of(const Distr& d)
 {
     const double c0 = d.c_f[0];
@@ -173,27 +167,137 @@ __device__ __forceinline__ uint64_t energy_mask(const uint64_t* flags, int64_t q
 }
 
 // ---------------------------------------------------------------------------
-// prelude: NuDistributionParams per point (distribution.hpp:51-243)
+// prelude: the constants of each point
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128)
-    spec_prelude_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
-                        double* __restrict__ dsc)
+
+// Per point of the chunk scratch.
+struct SpecPoint
 {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= np * 4)
-        return;
-    const int64_t q = t >> 2;
-    const int s     = (int)(t & 3);
-    const int64_t p = p0 + q;
-    double* d       = dsc + q * 28;
-    if (L.has_distr)
+    Distr d;                 // distribution.hpp:51-243
+    Occ64 occ[4], occT[4];   // occupations of an energy in MeV, and in units of T
+    double fe[2][6], fd0[2]; // F_0..F_5 and FermiDistr(0, 1, .) at +-eta_e
+    BetaPoint beta;
+    double eta_pp, eta_nn;
+    Hr98Point hr;
+    Hr98Cell hc;
+    double brt06_pre;
+    Gp19Point pt;
+    Gp19Corners cor[2];
+    fp32::Hr98Mixed hm; // mixed path
+    NesSpec Z;
+    NesDf Q;
+    double steep; // T over the lowest temperature of the point
+    int twin;     // heavy-lepton neutrinos evolved as one species
+    int same_cf, env;
+};
+static_assert(sizeof(SpecPoint) % sizeof(double) == 0, "SpecPoint must be double words");
+
+// n doubles of a record into shared memory, by threads t, t + nt, ...
+template <class T>
+__device__ __forceinline__ void copy_in(T* dst, const T& src, int t, int nt)
+{
+    static_assert(sizeof(T) % sizeof(double) == 0 && alignof(T) % sizeof(double) == 0,
+                  "copied by double words");
+    for (int k = t; k < (int)(sizeof(T) / sizeof(double)); k += nt)
+        ((double*)dst)[k] = ((const double*)&src)[k];
+}
+
+// A CTA takes 32 points, a warp one task of all of them, so every lane works and no
+// warp diverges; the second set of tasks needs the first's results.  With the tasks in
+// single lanes of the pb and nes kernels, and the beta constants in every lane of
+// assemble, they took half the time of 24 energies at n = 10: 4,096 points FP64 HR98
+// 1.72 -> 1.27 ms, mixed 2.27 -> 1.97 ms; n = 20 GP19 with NES mixed 5.87 -> 5.5 ms.
+constexpr int kPreTasks = 15;
+
+__global__ void __launch_bounds__(kPreTasks * 32)
+    spec_prelude_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
+                        SpecPoint* __restrict__ pts)
+{
+    const int64_t q  = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
+    const int task   = threadIdx.x >> 5;
+    const bool in    = q < np;
+    const int64_t p  = p0 + (in ? q : 0);
+    SpecPoint& P     = pts[in ? q : 0];
+    const bool hr98  = L.use_brem && L.brem_impl == 0;
+    const bool prof  = L.use_brem && L.brem_impl == 2 && L.gp19.d3 <= kGp19MaxW;
+    const double T   = L.eos[1][p], mu_e = L.eos[7][p], nbar = L.eos[0][p];
+    const double yp = L.eos[3][p], yn = L.eos[4][p], eta = mu_e / T;
+    if (in)
     {
-        for (int k = 0; k < 7; ++k)
-            d[k * 4 + s] = L.distr[k * 4 + s][p];
-        return;
+        if (task < 4)
+        {
+            Distr& d    = P.d;
+            const int s = task;
+            if (L.has_distr)
+                for (int k = 0; k < 7; ++k)
+                    (&d.w_t[0])[k * 4 + s] = L.distr[k * 4 + s][p];
+            else
+                distr_species(L.m1[s][p], L.m1[4 + s][p], L.m1[8 + s][p], L.gamma36, &d.w_t[s],
+                              &d.temp_t[s], &d.eta_t[s], &d.w_f[s], &d.temp_f[s], &d.c_f[s],
+                              &d.beta_f[s]);
+        }
+        else if (task < 7 && hr98)
+            P.hr.ch[task - 4] = hr98_channel(nbar, yn, yp, T, task - 4);
+        else if (task == 7 && hr98)
+            hr98_point_common(nbar, T, L.use_medium != 0, &P.hr);
+        else if (task == 8 && L.use_brem && L.brem_impl == 1)
+            P.brt06_pre = brt06_point(nbar, T, yn, yp);
+        else if (task == 8 && prof)
+            gp19_point(gp19_table(L), nbar, L.eos[2][p], T, &P.pt);
+        else if (task == 9 && L.use_abs_em)
+            P.beta = beta_point(nbar, T, yp, yn, L.eos[5][p], L.eos[6][p], mu_e, L.eos[9][p],
+                                L.eos[10][p], L.use_dU, L.use_dm_eff, L.use_WM_ab, L.use_decay);
+        else if (task == 10)
+        {
+            P.eta_pp = L.use_iso ? eta_nn_sc(nbar, T, yp) : 0.;
+            P.eta_nn = L.use_iso ? eta_nn_sc(nbar, T, yn) : 0.;
+        }
+        else if (task == 11 || task == 12)
+        {
+            const double e = task == 12 ? -eta : eta;
+            fdi_orders<0, 5>(e, P.fe[task - 11]);
+            P.fd0[task - 11] = fermi_distr(0., 1., e);
+        }
+        else if (task >= 13 && L.mixed && L.use_inel)
+        {
+            const int e  = task - 13;
+            P.Q.eta[e]   = dfm::from_double(e ? -eta : eta);
+            dfm::fdi_raw15(P.Q.eta[e], P.Q.reta[e], 1, &dfm::kFdiTab);
+        }
     }
-    distr_species(L.m1[s][p], L.m1[4 + s][p], L.m1[8 + s][p], L.gamma36, &d[s], &d[4 + s],
-                  &d[8 + s], &d[12 + s], &d[16 + s], &d[20 + s], &d[24 + s]);
+    __syncthreads();
+    if (!in)
+        return;
+    const Distr& d = P.d;
+    if (task < 4)
+    {
+        occ64_from(d, task, 1., &P.occ[task]);
+        occ64_from(d, task, T, &P.occT[task]);
+        if (L.mixed)
+            nes_spec_species(d, task, &P.Z);
+    }
+    else if (task < 8 && hr98)
+        hr98_cell_from(P.hr, task - 4, &P.hc);
+    else if (task >= 8 && task < 12 && hr98 && L.mixed)
+        fp32::hr98_mixed_part(P.hr, task - 8, &P.hm);
+    else if (task >= 12 && task < 14 && prof)
+    {
+        const int k = task - 12;
+        if (k == 0 || P.pt.regime >= 2)
+            gp19_profile_corners(gp19_table(L), P.pt.nbp, P.pt.yep, P.pt.pT[k], &P.cor[k]);
+    }
+    else if (task == 14)
+    {
+        P.twin    = species_twins(d);
+        P.same_cf = same_cf_of(d);
+        P.env     = fp32_envelope(d, eta);
+        if (L.mixed)
+            nes_spec_masks(d, &P.Z);
+        double t = T;
+        for (int s = 0; s < 4; ++s)
+            t = fmin(t, fmin(d.temp_t[s], d.temp_f[s]));
+        P.steep = T / t;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -203,8 +307,6 @@ struct PbWarp
 {
     Distr d;
     Hr98Point hr;
-    double brt06_pre;
-    int same_cf;
     double nb[kMaxM], zb[kMaxM]; // nubar and nubar / T
     double gb[kMaxM][4];
     Gp19Point gp;
@@ -268,13 +370,7 @@ struct Pb64Brem
 template <>
 struct Pb64Brem<0>
 {
-    Hr98Point hr;
     Hr98Cell hc;
-};
-template <>
-struct Pb64Brem<1>
-{
-    double pre;
 };
 template <>
 struct Pb64Brem<2>
@@ -316,7 +412,7 @@ __device__ __noinline__ double pb64_far(double psi, double Kbrem, double T, doub
 template <int IMPL>
 __global__ void __launch_bounds__(kWarps * 32, 4)
     spec_pb64_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0,
-                     const double* __restrict__ dsc, EnergyRec* __restrict__ rec,
+                     const SpecPoint* __restrict__ pts, EnergyRec* __restrict__ rec,
                      const uint64_t* __restrict__ flags)
 {
     constexpr int NT = kWarps * 32;
@@ -326,33 +422,28 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
     if (emask == 0ull)
         return;
     __shared__ Pb64Smem<IMPL> S;
-    const int64_t p   = p0 + q;
-    const double nbar = L.eos[0][p], T = L.eos[1][p], ye = L.eos[2][p];
-    const double yp = L.eos[3][p], yn = L.eos[4][p];
-    const double eta = L.eos[7][p] / T;
+    const SpecPoint& P = pts[q];
+    const int64_t p    = p0 + q;
+    const double T = L.eos[1][p], eta = L.eos[7][p] / T;
     const bool pair = L.use_pair != 0, brem = L.use_brem != 0;
     const bool nbb  = L.neglect_blocking != 0;
     const Gp19Table G19 = gp19_table(L);
     const bool prof     = IMPL == 2 && brem && G19.d3 <= kGp19MaxW;
     if (tid < n)
         S.x[tid] = L.x1[tid];
-    if (tid >= 32 && tid < 36)
-        occ64_from(*(const Distr*)(dsc + q * 28), tid - 32, 1., &S.occ[tid - 32]);
+    if (tid >= 32 && tid < 64)
+        copy_in(&S.occ, P.occ, tid - 32, 32);
     if constexpr (IMPL == 0)
-    {
-        if (brem && tid >= 64 && tid < 67)
-            S.X.hr.ch[tid - 64] = hr98_channel(nbar, yn, yp, T, tid - 64);
-        if (brem && tid == 96)
-            hr98_point_common(nbar, T, L.use_medium != 0, &S.X.hr);
-    }
-    if constexpr (IMPL == 1)
-        if (brem && tid == 64)
-            S.X.pre = brt06_point(nbar, T, yn, yp);
+        if (brem && tid >= 64 && tid < 96)
+            copy_in(&S.X.hc, P.hc, tid - 64, 32);
     if constexpr (IMPL == 2)
         if (prof)
         {
-            if (tid == 64)
-                gp19_point(G19, nbar, ye, T, &S.X.pt);
+            if (tid >= 64 && tid < 96)
+            {
+                copy_in(&S.X.pt, P.pt, tid - 64, 32);
+                copy_in(&S.X.gc, P.cor, tid - 64, 32);
+            }
             if (tid >= 96)
                 for (int k = tid - 96; k < G19.d3; k += 32)
                     gp19_axis_entry(S.X.axis, G19.logw, G19.d3, k);
@@ -379,27 +470,16 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
             S.dnz[a] = dz;
         }
     }
-    bool fast = false;
-    if constexpr (IMPL == 0)
-    {
-        if (brem && tid >= 64 && tid < 68)
-            hr98_cell_from(S.X.hr, tid - 64, &S.X.hc);
-    }
     if constexpr (IMPL == 2)
-    {
         if (prof)
         {
             const int np19 = S.X.pt.regime >= 2 ? 2 : 1;
-            if (tid < np19)
-                gp19_profile_corners(G19, S.X.pt.nbp, S.X.pt.yep, S.X.pt.pT[tid], &S.X.gc[tid]);
-            __syncthreads();
             for (int e = tid; e < np19 * G19.d3; e += NT)
             {
                 const int pr = e / G19.d3, l = e - pr * G19.d3;
                 S.X.p[pr][l] = gp19_profile_eval(G19, S.X.gc[pr], l);
             }
         }
-    }
     uint64_t low = 0ull;
     if (pair)
         for (int e = 0; e < ne; ++e)
@@ -423,7 +503,10 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                     if (pass)
                         fdi_rational<3, 4>(eta, S.fe);
                     else
-                        fdi_orders<3, 4>(eta, S.fe);
+                    {
+                        S.fe[0] = P.fe[0][3];
+                        S.fe[1] = P.fe[0][4];
+                    }
                     continue;
                 }
                 const int a = t >> 1;
@@ -471,8 +554,6 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                 }
             }
             __syncthreads();
-            if constexpr (IMPL == 0)
-                fast = S.X.hc.fast;
             const double f40 = 40. * S.fe[0], f20 = 20. * S.fe[1];
             for (int t = tid; t < nc * M; t += NT)
             {
@@ -502,13 +583,13 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                     if constexpr (IMPL == 0)
                     {
                         double b;
-                        if (fast && y > 1e-6 && y < 4e4)
+                        if (S.X.hc.fast && y > 1e-6 && y < 4e4)
                             Kb = hr98_absorption(S.X.hc, y + z, ex);
                         else
-                            hr98_kernel(S.X.hr, S.nu[c], S.nb[a], &b, &Kb);
+                            hr98_kernel(P.hr, S.nu[c], S.nb[a], &b, &Kb);
                     }
                     else if constexpr (IMPL == 1)
-                        Kb = S.X.pre * brt06_shape(0.5 * (y + z));
+                        Kb = P.brt06_pre * brt06_shape(0.5 * (y + z));
                     else
                     {
                         double b;
@@ -517,7 +598,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                                 S.X.pt, S.X.p, S.X.axis, G19.d3,
                                 fmax(fmin(S.nu[c] + S.nb[a], G19.w[G19.d3 - 1]), G19.w[0]));
                         else
-                            gp19_kernel(G19, nbar, ye, T, S.nu[c], S.nb[a], &b, &Kb);
+                            gp19_kernel(G19, L.eos[0][p], L.eos[2][p], T, S.nu[c], S.nb[a], &b, &Kb);
                     }
                 }
                 const int o = c * Ms + a;
@@ -561,7 +642,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 // Pair + brem of the mixed path.
 __global__ void __launch_bounds__(kWarps * 32)
     spec_pb_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
-                   const double* __restrict__ dsc, EnergyRec* __restrict__ rec, int G)
+                   const SpecPoint* __restrict__ pts, EnergyRec* __restrict__ rec, int G)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     PbShared& S         = *reinterpret_cast<PbShared*>(s_raw);
@@ -597,36 +678,22 @@ __global__ void __launch_bounds__(kWarps * 32)
     for (int64_t q = (int64_t)blockIdx.x * kWarps + wid; q < np; q += nwarp)
     {
         const int64_t p     = p0 + q;
-        const double nbar = L.eos[0][p], T = L.eos[1][p], ye = L.eos[2][p];
-        const double yp = L.eos[3][p], yn = L.eos[4][p], mu_e = L.eos[7][p];
-        const double eta_e = mu_e / T;
+        const double T = L.eos[1][p], eta_e = L.eos[7][p] / T;
         EnergyRec* R       = rec + q * ne;
+        const SpecPoint& P = pts[q];
         __syncwarp();
-        load_distr(dsc, q, &W.d, lane);
+        copy_in(&W.d, P.d, lane, 32);
         if (L.use_brem && L.brem_impl == 0)
         {
-            if (lane >= 6 && lane < 9)
-                W.hr.ch[lane - 6] = hr98_channel(nbar, yn, yp, T, lane - 6);
-            if (lane == 29)
-                hr98_point_common(nbar, T, L.use_medium != 0, &W.hr);
-        }
-        if (lane == 30 && L.use_brem && L.brem_impl == 1)
-            W.brt06_pre = brt06_point(nbar, T, yn, yp);
-        if (lane == 31 && prof)
-            gp19_point(G19, nbar, ye, T, &W.gp);
-        __syncwarp();
-        if (lane == 0)
-        {
-            W.same_cf = same_cf_of(W.d);
-            if (L.use_brem && L.brem_impl == 0)
-                fp32::hr98_mixed_from(W.hr, &X.hm);
+            copy_in(&W.hr, P.hr, lane, 32);
+            copy_in(&X.hm, P.hm, lane, 32);
         }
         if (prof)
         {
-            const int np19 = (W.gp.regime >= 2) ? 2 : 1;
-            if (lane < np19)
-                gp19_profile_corners(G19, W.gp.nbp, W.gp.yep, W.gp.pT[lane], &W.gc[lane]);
+            copy_in(&W.gp, P.pt, lane, 32);
+            copy_in(&W.gc, P.cor, lane, 32);
             __syncwarp();
+            const int np19 = (W.gp.regime >= 2) ? 2 : 1;
             for (int e = lane; e < np19 * G19.d3; e += 32)
             {
                 const int pr = e / G19.d3, l = e - pr * G19.d3;
@@ -636,7 +703,7 @@ __global__ void __launch_bounds__(kWarps * 32)
             }
         }
         __syncwarp();
-        const bool same_cf = W.same_cf != 0;
+        const bool same_cf = P.same_cf != 0;
         // mixed pair: eta and the point's factor (Phi T^2 / 2) T^4 / 15
         const dfm::df ETA = dfm::from_double(eta_e);
         const double T2   = T * T;
@@ -673,7 +740,7 @@ __global__ void __launch_bounds__(kWarps * 32)
         if (L.use_brem)
         {
             b32 = (L.brem_impl == 0 || (prof && W.gp.regime != 3 && W.gp.regime != 5)) &&
-                  fp32_envelope(W.d, eta_e);
+                  P.env;
             if (L.brem_impl == 0)
                 sb = (T * T) * X.hm.outer;
             else if (prof)
@@ -737,7 +804,7 @@ __global__ void __launch_bounds__(kWarps * 32)
                             if (L.brem_impl == 0)
                                 hr98_kernel(W.hr, nu, nub, &be, &ba);
                             else if (L.brem_impl == 1)
-                                brt06_kernel(W.brt06_pre, T, nu, nub, &be, &ba);
+                                brt06_kernel(P.brt06_pre, T, nu, nub, &be, &ba);
                             else if (prof)
                                 gp19_profile_node(W.gp, W.gpp, S.lw, G19.d3, wmin, wmax, nu,
                                                   nub, &be, &ba);
@@ -878,8 +945,7 @@ __global__ void __launch_bounds__(kWarps * 32)
 // ---------------------------------------------------------------------------
 struct NesWarp
 {
-    Distr d;
-    double fe[2][6], fd0[2];
+    double fe[2][6];
     double fw[kEChunk][2][5]; // Fermi integrals at eta_e - nu/T (nes_spec_node)
     NesSpec Z;
     NesDf Q;
@@ -910,8 +976,6 @@ struct Nes64Smem
     double w[kEChunk], wc[kEChunk];     // nu/T and its 0.6th power
     double fw[kEChunk][2][5];           // phi_1..phi_5 at eta_e - nu/T
     int eid[kEChunk];
-    int twin;     // heavy-lepton neutrinos evolved as one species
-    double steep; // T over the lowest temperature of the point
 };
 
 // 1 - e^{-d} for e = e^{-d}, d >= 0: by its series below d = 1/4 (2^-53 relative).
@@ -952,7 +1016,7 @@ __device__ __noinline__ double nes64_far(int s, double A0, double B0, double A1,
 
 __global__ void __launch_bounds__(kWarps * 32, 4)
     spec_nes64_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0,
-                      const double* __restrict__ dsc, EnergyRec* __restrict__ rec,
+                      const SpecPoint* __restrict__ pts, EnergyRec* __restrict__ rec,
                       const uint64_t* __restrict__ flags)
 {
     constexpr int NT = kWarps * 32;
@@ -976,22 +1040,12 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
     }
     if (tid >= 64 && tid < 64 + M)
         S.m[tid - 64] = 24. * L.B1[tid - 64];
-    const Distr& d = *(const Distr*)(dsc + q * 28);
-    if (tid >= 32 && tid < 36)
-        occ64_from(d, tid - 32, T, &S.occ[tid - 32]);
-    if (tid == 64 || tid == 65)
+    const SpecPoint& P = pts[q];
+    if (tid >= 32 && tid < 64)
     {
-        const double et = tid == 65 ? -eta_e : eta_e;
-        fdi_orders<0, 5>(et, S.fe[tid - 64]);
-        S.fd0[tid - 64] = fermi_distr(0., 1., et);
-    }
-    if (tid == 96)
-    {
-        S.twin   = species_twins(d);
-        double t = fmin(T, fmin(d.temp_t[0], d.temp_f[0]));
-        for (int s = 1; s < 4; ++s)
-            t = fmin(t, fmin(d.temp_t[s], d.temp_f[s]));
-        S.steep = T / t;
+        copy_in(&S.occ, P.occT, tid - 32, 32);
+        copy_in(&S.fe, P.fe, tid - 32, 32);
+        copy_in(&S.fd0, P.fd0, tid - 32, 32);
     }
     const int nt = __popcll(emask);
     const int G  = pick_groups(nt < kEChunk ? nt : kEChunk, M, NT);
@@ -1018,14 +1072,14 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
         const Occ64* occ  = S.occ;
         const bool common = occ[0].cf == k::CF && occ[1].cf == k::CF && occ[2].cf == k::CF &&
                             occ[3].cf == k::CF;
-        const int nocc = S.twin ? 3 : 4;
+        const int nocc = P.twin ? 3 : 4;
 #pragma unroll 1
         for (int r0 = 0; r0 < nc; r0 += per_round)
         {
             const bool act = r0 + tid / G < nc;
             const int c    = act ? r0 + tid / G : 0;
             const double w = S.w[c];
-            const bool tiny = !(w * S.steep < 500.); // e^-500: emission near the denormals
+            const bool tiny = !(w * P.steep < 500.); // e^-500: emission near the denormals
             double acc[8];
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
@@ -1103,7 +1157,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 template <bool LOW>
 __global__ void __launch_bounds__(kWarps * 32, 4)
     spec_nes_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
-                    const double* __restrict__ dsc, EnergyRec* __restrict__ rec)
+                    const SpecPoint* __restrict__ pts, EnergyRec* __restrict__ rec)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     NesShared& S = *reinterpret_cast<NesShared*>(s_raw);
@@ -1140,36 +1194,23 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                 continue;
         }
         __syncwarp();
-        load_distr(dsc, q, &W.d, lane);
-        if (lane == 28 || lane == 29)
-        {
-            const int e     = lane - 28;
-            const double et = e ? -eta_e : eta_e;
-            fdi_orders<0, 5>(et, W.fe[e]);
-            W.fd0[e] = fermi_distr(0., 1., et);
-        }
+        const SpecPoint& P = pts[q];
+        copy_in(&W.fe, P.fe, lane, 32);
+        copy_in(&W.Z, P.Z, lane, 32);
+        if (LOW)
+            copy_in(&W.Q, P.Q, lane, 32);
         __syncwarp();
         NepsPoint NP;
         NP.T    = T;
         NP.pre  = k::NepsConst * (T * T);
         NP.eta0 = eta_e;
         NP.eta1 = -eta_e;
-        NP.fd00 = W.fd0[0];
-        NP.fd01 = W.fd0[1];
+        NP.fd00 = P.fd0[0];
+        NP.fd01 = P.fd0[1];
         NP.fe0  = W.fe[0];
         NP.fe1  = W.fe[1];
-        const bool m32  = fp32_envelope(W.d, eta_e);
+        const bool m32  = P.env != 0;
         const double sn = (T * T) * NP.pre;
-        if (lane < 4)
-            nes_spec_species(W.d, lane, &W.Z);
-        else if (lane == 8)
-            nes_spec_masks(W.d, &W.Z);
-        else if (LOW && lane >= 16 && lane < 18)
-        {
-            W.Q.eta[lane - 16] = dfm::from_double(lane == 17 ? -eta_e : eta_e);
-            dfm::fdi_raw15(W.Q.eta[lane - 16], W.Q.reta[lane - 16], 1, &S.ftab);
-        }
-        __syncwarp();
 
         for (int e0 = 0; e0 < ne; e0 += kEChunk)
         {
@@ -1289,7 +1330,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 template <int MODE>
 __global__ void __launch_bounds__(kWarps * 32)
     spec_assemble_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
-                         const double* __restrict__ dsc, const EnergyRec* __restrict__ rec,
+                         const SpecPoint* __restrict__ pts, const EnergyRec* __restrict__ rec,
                          uint64_t* __restrict__ fl_pb, uint64_t* __restrict__ fl_nes)
 {
     constexpr bool GUARD = MODE == kSpecMixed || MODE == kSpecRedo;
@@ -1308,25 +1349,15 @@ __global__ void __launch_bounds__(kWarps * 32)
             if (emask == 0ull)
                 continue;
         }
-        const int64_t p   = p0 + q;
-        const double nbar = L.eos[0][p], T = L.eos[1][p];
-        const double yp = L.eos[3][p], yn = L.eos[4][p];
-        const double mu_p = L.eos[5][p], mu_n = L.eos[6][p], mu_e = L.eos[7][p];
-        const double dU = L.eos[9][p], dm_eff = L.eos[10][p];
+        const int64_t p    = p0 + q;
+        const double T     = L.eos[1][p];
+        const SpecPoint& P = pts[q];
         __syncwarp();
-        load_distr(dsc, q, &D, lane);
+        copy_in(&D, P.d, lane, 32);
         __syncwarp();
-        const bool same_cf = same_cf_of(D);
-        BetaPoint bp;
-        if (L.use_abs_em)
-            bp = beta_point(nbar, T, yp, yn, mu_p, mu_n, mu_e, dU, dm_eff, L.use_dU, L.use_dm_eff,
-                            L.use_WM_ab, L.use_decay);
-        double eta_pp = 0., eta_nn = 0.;
-        if (L.use_iso)
-        {
-            eta_pp = eta_nn_sc(nbar, T, yp);
-            eta_nn = eta_nn_sc(nbar, T, yn);
-        }
+        const bool same_cf  = P.same_cf != 0;
+        const BetaPoint& bp = P.beta;
+        const double eta_pp = P.eta_pp, eta_nn = P.eta_nn;
         const double ts = k::TempMultiple * T;
         uint64_t bad_pb = 0ull, bad_nes = 0ull;
         for (int e0 = 0; e0 < ne; e0 += 32)
@@ -1461,7 +1492,7 @@ cudaError_t grid_of(K kernel, size_t smem, bool* attr_set, int num_sms, int64_t 
     return cudaSuccess;
 }
 
-cudaError_t launch_pb_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
+cudaError_t launch_pb_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
                             EnergyRec* rec, int G, cudaStream_t st, int sms)
 {
     static bool attr  = false;
@@ -1471,12 +1502,12 @@ cudaError_t launch_pb_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, cons
     if (err != cudaSuccess || grid == 0)
         return err;
     phase_mark(kPhSpectral, 0, st);
-    spec_pb_kernel<<<grid, kWarps * 32, smem, st>>>(L, p0, np, dsc, rec, G);
+    spec_pb_kernel<<<grid, kWarps * 32, smem, st>>>(L, p0, np, pts, rec, G);
     phase_mark(kPhSpectral, 1, st);
     return cudaGetLastError();
 }
 
-cudaError_t launch_nes_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
+cudaError_t launch_nes_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
                              EnergyRec* rec, cudaStream_t st, int sms)
 {
     static bool attr[2] = {false, false};
@@ -1488,41 +1519,41 @@ cudaError_t launch_nes_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, con
     if (err != cudaSuccess || grid == 0)
         return err;
     phase_mark(kPhSpectral, 0, st);
-    spec_nes_kernel<false><<<grid, kWarps * 32, smem, st>>>(L, p0, np, dsc, rec);
+    spec_nes_kernel<false><<<grid, kWarps * 32, smem, st>>>(L, p0, np, pts, rec);
     phase_mark(kPhSpectral, 1, st);
     phase_mark(kPhSpectral, 0, st);
-    spec_nes_kernel<true><<<low, kWarps * 32, smem, st>>>(L, p0, np, dsc, rec);
+    spec_nes_kernel<true><<<low, kWarps * 32, smem, st>>>(L, p0, np, pts, rec);
     phase_mark(kPhSpectral, 1, st);
     return cudaGetLastError();
 }
 
 // FP64 passes: every energy (flags null) or the flagged ones.
-cudaError_t launch_pb64(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
+cudaError_t launch_pb64(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
                         EnergyRec* rec, const uint64_t* flags, cudaStream_t st)
 {
     phase_mark(kPhSpectral, 0, st);
     const int impl = L.use_brem ? L.brem_impl : 1;
     if (impl == 0)
-        spec_pb64_kernel<0><<<(int)np, kWarps * 32, 0, st>>>(L, p0, dsc, rec, flags);
+        spec_pb64_kernel<0><<<(int)np, kWarps * 32, 0, st>>>(L, p0, pts, rec, flags);
     else if (impl == 1)
-        spec_pb64_kernel<1><<<(int)np, kWarps * 32, 0, st>>>(L, p0, dsc, rec, flags);
+        spec_pb64_kernel<1><<<(int)np, kWarps * 32, 0, st>>>(L, p0, pts, rec, flags);
     else
-        spec_pb64_kernel<2><<<(int)np, kWarps * 32, 0, st>>>(L, p0, dsc, rec, flags);
+        spec_pb64_kernel<2><<<(int)np, kWarps * 32, 0, st>>>(L, p0, pts, rec, flags);
     phase_mark(kPhSpectral, 1, st);
     return cudaGetLastError();
 }
 
-cudaError_t launch_nes64(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
+cudaError_t launch_nes64(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
                          EnergyRec* rec, const uint64_t* flags, cudaStream_t st)
 {
     phase_mark(kPhSpectral, 0, st);
-    spec_nes64_kernel<<<(int)np, kWarps * 32, 0, st>>>(L, p0, dsc, rec, flags);
+    spec_nes64_kernel<<<(int)np, kWarps * 32, 0, st>>>(L, p0, pts, rec, flags);
     phase_mark(kPhSpectral, 1, st);
     return cudaGetLastError();
 }
 
 template <int MODE>
-cudaError_t launch_assemble(const OpacityLaunch& L, int64_t p0, int64_t np, const double* dsc,
+cudaError_t launch_assemble(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
                             const EnergyRec* rec, uint64_t* fl_pb, uint64_t* fl_nes,
                             cudaStream_t st, int sms)
 {
@@ -1532,7 +1563,7 @@ cudaError_t launch_assemble(const OpacityLaunch& L, int64_t p0, int64_t np, cons
     if (err != cudaSuccess || grid == 0)
         return err;
     phase_mark(kPhSpectral, 0, st);
-    spec_assemble_kernel<MODE><<<grid, kWarps * 32, 0, st>>>(L, p0, np, dsc, rec, fl_pb, fl_nes);
+    spec_assemble_kernel<MODE><<<grid, kWarps * 32, 0, st>>>(L, p0, np, pts, rec, fl_pb, fl_nes);
     phase_mark(kPhSpectral, 1, st);
     return cudaGetLastError();
 }
@@ -1549,7 +1580,7 @@ int64_t spectral_chunk_points(int n_energies)
 size_t spectral_scratch_bytes(int64_t chunk_points, int n_energies)
 {
     return (size_t)chunk_points *
-           (28 * sizeof(double) + 2 * sizeof(uint64_t) + (size_t)n_energies * sizeof(EnergyRec));
+           (sizeof(SpecPoint) + 2 * sizeof(uint64_t) + (size_t)n_energies * sizeof(EnergyRec));
 }
 
 cudaError_t spectral_mixed_counts(unsigned long long* counts, bool reset)
@@ -1610,41 +1641,40 @@ cudaError_t launch_spectral(const OpacityLaunch& L, cudaStream_t st0, int sms, v
     {
         const bool odd        = two && (k & 1);
         const cudaStream_t st = odd ? aux : st0;
-        double* dsc           = (double*)(odd ? scratch1 : scratch);
-        uint64_t* fl_pb       = (uint64_t*)(dsc + chunk_points * 28);
+        SpecPoint* pts        = (SpecPoint*)(odd ? scratch1 : scratch);
+        uint64_t* fl_pb       = (uint64_t*)(pts + chunk_points);
         uint64_t* fl_nes      = fl_pb + chunk_points;
         EnergyRec* rec        = (EnergyRec*)(fl_nes + chunk_points);
         const int64_t np  = (L.npts - p0) < chunk_points ? (L.npts - p0) : chunk_points;
-        const int64_t nth = np * 4;
         phase_mark(kPhSpectral, 0, st);
-        spec_prelude_kernel<<<(int)((nth + 127) / 128), 128, 0, st>>>(L, p0, np, dsc);
+        spec_prelude_kernel<<<(int)((np + 31) / 32), kPreTasks * 32, 0, st>>>(L, p0, np, pts);
         phase_mark(kPhSpectral, 1, st);
         if ((err = cudaGetLastError()) != cudaSuccess)
             break;
         if (!L.mixed)
         {
-            if (pb && (err = launch_pb64(L, p0, np, dsc, rec, nullptr, st)))
+            if (pb && (err = launch_pb64(L, p0, np, pts, rec, nullptr, st)))
                 break;
-            if (inel && (err = launch_nes64(L, p0, np, dsc, rec, nullptr, st)))
+            if (inel && (err = launch_nes64(L, p0, np, pts, rec, nullptr, st)))
                 break;
-            err = launch_assemble<kSpecFp64>(L, p0, np, dsc, rec, fl_pb, fl_nes, st, sms);
+            err = launch_assemble<kSpecFp64>(L, p0, np, pts, rec, fl_pb, fl_nes, st, sms);
             continue;
         }
-        if (pb && (err = launch_pb_mixed(L, p0, np, dsc, rec, G, st, sms)))
+        if (pb && (err = launch_pb_mixed(L, p0, np, pts, rec, G, st, sms)))
             break;
-        if (inel && (err = launch_nes_mixed(L, p0, np, dsc, rec, st, sms)))
+        if (inel && (err = launch_nes_mixed(L, p0, np, pts, rec, st, sms)))
             break;
-        if ((err = launch_assemble<kSpecMixed>(L, p0, np, dsc, rec, fl_pb, fl_nes, st, sms)))
+        if ((err = launch_assemble<kSpecMixed>(L, p0, np, pts, rec, fl_pb, fl_nes, st, sms)))
             break;
         for (int round = 0; round < 2 && err == cudaSuccess; ++round)
         {
-            if (pb && (err = launch_pb64(L, p0, np, dsc, rec, fl_pb, st)))
+            if (pb && (err = launch_pb64(L, p0, np, pts, rec, fl_pb, st)))
                 break;
-            if (inel && (err = launch_nes64(L, p0, np, dsc, rec, fl_nes, st)))
+            if (inel && (err = launch_nes64(L, p0, np, pts, rec, fl_nes, st)))
                 break;
             err = round == 0
-                      ? launch_assemble<kSpecRedo>(L, p0, np, dsc, rec, fl_pb, fl_nes, st, sms)
-                      : launch_assemble<kSpecFinal>(L, p0, np, dsc, rec, fl_pb, fl_nes, st, sms);
+                      ? launch_assemble<kSpecRedo>(L, p0, np, pts, rec, fl_pb, fl_nes, st, sms)
+                      : launch_assemble<kSpecFinal>(L, p0, np, pts, rec, fl_pb, fl_nes, st, sms);
         }
     }
     if (two)
