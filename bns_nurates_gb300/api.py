@@ -423,7 +423,9 @@ def spectral_mixed_stats(reset=False):
 
 def grey_mixed_stats(reset=False):
     """Mixed grey path on the current device since the last reset:
-    {"evaluated", "nes_df", "nes_fp64", "pair_fp64", "brem_fp64"} point counts."""
+    {"evaluated", "nes_df", "nes_fp64", "pair_fp64", "brem_fp64"} point counts.
+    nes_df: points whose FP32 NES sums cancel, nes_fp64: points outside the FP32
+    range; the NES sums of both are computed in FP64."""
     c = (ctypes.c_int64 * 5)()
     _check(C.load().bnsn_grey_mixed_stats(c, int(reset)))
     return dict(zip(("evaluated", "nes_df", "nes_fp64", "pair_fp64", "brem_fp64"),

@@ -77,8 +77,8 @@ enum Phase
     kPhFinal,
     kPhSpectral,
     kPhAux,
-    kPhNepsAccurate, // mixed path: df pass over the points the fast pass flagged
-    kPhNepsFp64,     // mixed path: FP64 pass over the points flagged again
+    kPhNepsAccurate, // mixed path: list of the points the fast pass flagged
+    kPhNepsFp64,     // mixed path: FP64 pass over them
     kNumPhases
 };
 

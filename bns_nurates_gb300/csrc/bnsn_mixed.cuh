@@ -225,14 +225,6 @@ __device__ __forceinline__ int gp19_bracket32(double w, const float* lwf, const 
     return l;
 }
 
-// Per-point data of the mixed item loop.
-struct NepsMixed
-{
-    dfm::df reta[2][5]; // unreflected F_1..F_5 at eta for e- (0) and e+ (1)
-    dfm::df eta[2];
-    double invTt[4], etat[4], lbf[4], invTf[4], cf[4]; // exponent arguments in FP64
-};
-
 // NEPSExpFunc (functions.hpp:4401-4413) in FP32 for the FP64 argument d;
 // e^{-|d|} takes the FP32 exponential of the rounded argument times the
 // first-order correction for its remainder, expm1 keeps 1 - e^{-|d|}

@@ -68,7 +68,7 @@ struct PointTab
     double siso[4];      // iso per species
     double sbrem[16];    // brem alone (its part of s2d)
     double bmag[16];     // mixed path: sum of |term| of FP32 brem cells (s2d units), else 0
-    double neps_fp64;    // mixed path: 1 if the NES sums of the point must be FP64
+    double neps_fp64;    // mixed path: not 0 if the NES sums of the point must be FP64
     double bredo;        // mixed path: 1 if the brem sums must be recomputed in FP64
 };
 static_assert(sizeof(PointTab) % sizeof(double) == 0, "PointTab must be double words");
@@ -85,8 +85,8 @@ struct PairMixed
     double predo;     // 1 if the point's pair sums must be recomputed in FP64
 };
 static_assert(sizeof(PairMixed) <= sizeof(((PointTab*)nullptr)->fm), "PairMixed overlay");
-// Mixed path: points evaluated, NES handed to the double-float pass, NES in
-// FP64, pair sums redone in FP64, brem sums redone in FP64 (read by
+// Mixed path: points evaluated, points whose FP32 NES sums cancel and those outside
+// the FP32 range (NES in FP64), pair sums redone in FP64, brem sums redone in FP64 (read by
 // grey_mixed_counts).
 __device__ unsigned long long g_grey_mixed[5];
 
@@ -114,14 +114,6 @@ size_t grey_point_scratch_bytes() { return sizeof(PointTab); }
 namespace {
 
 constexpr int kWarps = 4; // warps per CTA in the per-point kernels
-
-__device__ __forceinline__ double warp_sum(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 // Sums the 16 values of the warp's lanes: lane l returns the total of value
 // sum_index(l).  Each round halves the values a lane carries, 16 additions in
@@ -155,28 +147,7 @@ __device__ __forceinline__ void warp_copy(double* __restrict__ dst,
         dst[k] = src[k];
 }
 
-// s_beta of m1_opacities.hpp:1093-1110 from F_4, F_5 at +-eta_e.
-__device__ __forceinline__ void beta_scales(double T, double eta_e, const double (&fe)[2][6],
-                                            double* sb)
-{
-    if (eta_e > -30. && eta_e < 30.)
-    {
-        sb[0] = T * fe[0][5] / fe[0][4];
-        sb[1] = T * fe[1][5] / fe[1][4];
-    }
-    else if (eta_e > 30.)
-    {
-        sb[0] = T * eta_e * 0.8333333333333333;
-        sb[1] = T * 5.;
-    }
-    else
-    {
-        sb[0] = T * 5.;
-        sb[1] = T * eta_e * 0.8333333333333333;
-    }
-}
-
-// The scale of species s alone, from its F_4, F_5.
+// s_beta of m1_opacities.hpp:1093-1110 of species s (0, 1) from F_4, F_5 at +-eta_e.
 __device__ __forceinline__ double beta_scale(double f4, double f5, double T, double eta_e, int s)
 {
     if (eta_e > -30. && eta_e < 30.)
@@ -639,93 +610,10 @@ struct Acc32
     }
 };
 
-// Largest error amplification over the 16 moments of a point (number and
-// energy, emission and absorption, 4 species): the sum of |term| over
-// |total|, where the total adds the other reactions' sums of the same output
-// (`other`, in the units of scale x acc: the pair, brem or NES sums already
-// computed and the beta rates, which cancel the brem or NES sums where the
-// reconstructed occupation exceeds 1).  Terms are those of this lane (acc,
-// mag, unscaled; moments 8..15 scaled by scale_e); the result is
-// warp-reduced and 1 when every contribution has one sign.
-// The same from the totals (already summed over the point's lanes).
-__device__ __forceinline__ double cancel_factor_tot(const double* acc, const double* mag,
-                                                    double scale, double scale_e,
-                                                    const double* other)
-{
-    double amp = 1.;
-#pragma unroll
-    for (int s = 0; s < 16; ++s)
-    {
-        const double sc  = s < 8 ? scale : scale_e;
-        const double m   = mag[s] * sc;
-        const double tot = fabs(acc[s] * sc + other[s]);
-        amp = fmax(amp, m > 0. ? m / tot : 1.);
-    }
-    return amp;
-}
-
-// v[0..16) summed over the CTA's NW warps in a fixed order; every thread
-// receives the totals.  red: NW x 32 doubles of shared memory, columns
-// col .. col + 15 used.
-template <int NW>
-__device__ __forceinline__ void block_sum(double* v, double (*red)[32], int col)
-{
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk)
-        v[kk] = warp_sum(v[kk]);
-    if (lane == 0)
-    {
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk)
-            red[wid][col + kk] = v[kk];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk)
-    {
-        double t = 0.;
-        for (int w = 0; w < NW; ++w)
-            t += red[w][col + kk];
-        v[kk] = t;
-    }
-    __syncthreads();
-}
-
-// The beta rates of a point in the units of the pair/brem sums (s2d, unit
-// t2 = (2.182 T)^2 for number and t2d t2 for energy moments) or, with
+// The beta rate of element idx of a point's 16 sums in the units of the pair/brem
+// sums (s2d, unit t2 = (2.182 T)^2 for number and t2d t2 for energy moments) or, with
 // to_nes, of the NES sums (unit hn = 8 t2, times T for energy moments), as
 // the final assembly combines them (m1_opacities.hpp:1172-1294).
-__device__ __forceinline__ void beta_in_sum_units(const PointTab* P, double T, double eta_e,
-                                                  bool use_abs_em, bool to_nes, double* b)
-{
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk)
-        b[kk] = 0.;
-    if (!use_abs_em)
-        return;
-    double fe[2][6];
-#pragma unroll
-    for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int kk = 0; kk < 6; ++kk)
-            fe[e][kk] = P->fe[e][kk];
-    double sb[2];
-    beta_scales(T, eta_e, fe, sb);
-    const double t2d = k::TempMultiple * T, t2 = t2d * t2d;
-    const double un  = k::FourPiHc3 * (to_nes ? 8. * t2 : t2);
-    const double ue  = to_nes ? un : un * t2d;
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-    {
-        b[s]      = P->sbeta[s] * sb[s] / un;     // number emission
-        b[4 + s]  = P->sbeta[4 + s] * sb[s] / un; // number absorption
-        b[8 + s]  = P->sbeta[2 + s] * sb[s] / ue; // energy emission
-        b[12 + s] = P->sbeta[6 + s] * sb[s] / ue; // energy absorption
-    }
-}
-
-// Element idx of the same (each lane of a warp takes its own).
 __device__ __forceinline__ double beta_in_sum_unit(const PointTab* P, double T, double eta_e,
                                                    bool use_abs_em, bool to_nes, int idx)
 {
@@ -746,8 +634,6 @@ constexpr double kMaxCancel = 2.0;
 constexpr double kMaxCancelBrem = 1.25;
 // FP32 pair integrals carry up to ~3e-7 per cell.
 constexpr double kMaxCancelPair = 1.5;
-// The accurate (all-df) pass keeps ~1e-13 per term.
-constexpr double kMaxCancelDf = 1e5;
 
 // add_cell in FP32 for a species-independent kernel (brem): K_em, K_ab are
 // dimensionless; P1 = (y_a y_b)^2 W1 and P2 = (y_a y_b)^2 W2 are the cell's
@@ -1608,368 +1494,50 @@ struct NepsTab
     double same_cf;
 };
 
-// Energies of NES item (r, i, j) (m1_opacities.hpp:880-905).
-__device__ __forceinline__ void neps_energies(int r, double xi, double xj, double tn, double* nu,
-                                              double* nub)
-{
-    if (!r)
-    {
-        *nu  = 0.5 * tn * xi * (1. - xj);
-        *nub = 0.5 * tn * xi * (1. + xj);
-    }
-    else
-    {
-        *nu  = 0.5 * tn * (1. - xj) / xi;
-        *nub = 0.5 * tn * (1. + xj) / xi;
-    }
-}
-
-// TotalNuF and 1 - TotalNuF in df (the accurate pass of the mixed path).
-__device__ __forceinline__ void total_nu_df(double omega, double lw, const NepsMixed& Q,
-                                            const double* wt, const double* wf, dfm::df* g,
-                                            dfm::df* gm)
-{
-    using namespace dfm;
-#pragma unroll 1
-    for (int s = 0; s < 4; ++s)
-    {
-        const double arg = fma(omega, Q.invTt[s], -Q.etat[s]);
-        const df t       = exp_df(from_double(-fabs(arg)));
-        const df inv     = div(mk(1.f), add(t, 1.f));
-        const df ti      = mul(t, inv);
-        const df ft = arg > 0. ? ti : inv, ftm = arg > 0. ? inv : ti;
-        const df fn = exp_df(from_double(fma(Q.cf[s], lw, fma(-omega, Q.invTf[s], Q.lbf[s]))));
-        const df Wt = from_double(wt[s]), Wf = from_double(wf[s]);
-        g[s]  = add(mul(Wt, ft), mul(Wf, fn));
-        gm[s] = add(mul(Wt, ftm), mul(Wf, add(neg(fn), 1.f)));
-    }
-}
-
-// NEPSExpFunc in df.
-__device__ __forceinline__ dfm::df neps_exp_df(double d, bool negd)
-{
-    using namespace dfm;
-    const df e  = exp_df(from_double(-fabs(d)));
-    const df dn = add(add(neg(e), 1.f), d == 0. ? 1.f : 0.f);
-    return div(negd ? mk(1.f) : neg(e), dn);
-}
-
-// neps_item_mixed with every product after the Fermi integrals in df.
-__device__ __forceinline__ void neps_item_df(const NepsPoint& P, const NepsMixed& Q,
-                                             const dfm::FdiTab* ftab, double w, double wp,
-                                             dfm::df* em1, dfm::df* ab1, dfm::df* em2,
-                                             dfm::df* ab2)
-{
-    using namespace dfm;
-    const double x = (w > wp) ? w : wp;
-    const double y = (w < wp) ? w : wp;
-    const double d1 = wp - w, d2 = w - wp;
-    const bool n1 = signbit(d1) != 0, n2 = signbit(d2) != 0;
-    const df efa = neps_exp_df(d1, n1);
-    const df efb = neps_exp_df(d2, n2);
-    const float sign1 = n1 ? 1.f : -1.f;
-    const float sign2 = n2 ? 1.f : -1.f;
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-        em1[s] = ab1[s] = em2[s] = ab2[s] = {0.f, 0.f};
-    const df W  = from_double(w), WP = from_double(wp);
-    const df S  = add(W, WP);
-    const df Pp = mul(W, WP);
-    const df Dn = mul(Pp, Pp);
-    const df iDn = div(mk(1.f), Dn); // the four brackets per lepton share 1 / Dn
-    const df X  = from_double(x), Y = from_double(y);
-    // e+ terms scale as e^{-eta_e}: below 1e-13 of the e- terms for eta_e > 30
-    const int nlep = P.eta0 > 30. ? 1 : 2;
-#pragma unroll 1
-    for (int e = 0; e < nlep; ++e)
-    {
-        const double eta = e ? P.eta1 : P.eta0;
-        df r1[4], r2[4];
-        if (y > eta * 1e-3)
-        {
-            const df aw = from_double(eta - w), awp = from_double(eta - wp);
-            const double adw = fabs(w - wp);
-            const df aab = from_double(eta - adw);
-            df rw[5], rwp[5], rab[5];
-            fdi_raw15(aw, rw, 1, ftab);
-            fdi_raw15(awp, rwp, 1, ftab);
-            fdi_raw15(aab, rab, 3, ftab); // only F_3..F_5 enter through |w - w'|
-            rab[0] = rab[1] = Q.reta[e][0]; // unused orders: keep the arrays defined
-            df dw[5], d5[5];
-            fdi_diff15(rw, rwp, aw, awp, from_double(w - wp), dw);
-            fdi_diff15(rab, Q.reta[e], aab, Q.eta[e], from_double(adw), d5);
-            const df dabs[3] = {d5[2], d5[3], d5[4]};
-            const df T1 = add(dw[3], mul(add(mul(S, dw[2]), mul(mul(Pp, 3.f), dw[1])), 2.f));
-            const df U  = add(mul(X, dabs[1]), mul(mul(mul(X, X), 2.f), dabs[0]));
-            const df V  = add(neg(mul(Y, dabs[1])), mul(mul(mul(Y, Y), 2.f), dabs[0]));
-            const df ST = mul(S, T1);
-            constexpr dfc kFifth(0.2);
-            const df dd2 = mul(dabs[2], mk(kFifth)), dw4 = mul(dw[4], mk(kFifth));
-            const df c1 = sub(mul(dd2, sign1), dw4);
-            const df c2 = add(mul(dd2, sign2), dw4);
-            const df s6 = mul(dw[0], 6.f);
-            const df A1 = sub(mul(add(sub(c1, ST), mul(U, sign1)), iDn), s6);
-            const df B1 = mul(add(c1, mul(V, sign1)), iDn);
-            const df A2 = add(mul(add(add(c2, ST), mul(U, sign2)), iDn), s6);
-            const df B2 = mul(add(c2, mul(V, sign2)), iDn);
-            constexpr dfc kBp(k::NepsBPlus), kBm(k::NepsBMinus), kBz(k::NepsBZero);
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                const df bo      = (s < 2) ? mk(kBp) : mk(kBm);
-                const bool first = ((s & 1) == 0) != (e == 1);
-                r1[s] = first ? add(mul(A1, bo), mul(B1, mk(kBz))) : add(mul(A1, mk(kBz)), mul(B1, bo));
-                r2[s] = first ? add(mul(A2, bo), mul(B2, mk(kBz))) : add(mul(A2, mk(kBz)), mul(B2, bo));
-            }
-        }
-        else
-        {
-            double t1[4], t2[4];
-            neps_taylor(P, e, w, wp, x, y, (int)sign1, (int)sign2, t1, t2);
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-            {
-                r1[s] = from_double(t1[s]);
-                r2[s] = from_double(t2[s]);
-            }
-        }
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-        {
-            em1[s] = sub(em1[s], mul(r1[s], efb));
-            ab1[s] = add(ab1[s], mul(r1[s], efa));
-            em2[s] = sub(em2[s], mul(r2[s], efa));
-            ab2[s] = add(ab2[s], mul(r2[s], efb));
-        }
-    }
-}
-
-// The mixed path's NES runs three launches per chunk, each over all points but
-// working only on its own:
+// The mixed path's NES runs three launches per chunk:
 //   grey_nes_fast_kernel  FP32 kernel integrals (bnsn_nes32.cuh); flags a
 //                 point 1 when its sums cancel (terms of both signs, or
 //                 negative pair + brem sums) and 2 when it leaves the FP32
 //                 range envelope;
-//   grey_neps_kernel      flag 1: every product in df (cancellation up to
-//                 ~1e5); beyond that the point is flagged 2;
-//   grey_nes64_kernel     flag 2: FP64 items (the plain path runs it over
-//                 every point).
-// The passes over the few flagged points run a point per CTA, its items over
-// all the CTA's threads (one warp alone would leave the pass as long as a
-// point's whole item loop).
-constexpr int kNesAccWarps = 8;
+//   grey_nes_list_kernel  the flagged points' list;
+//   grey_nes64_kernel     FP64 items of the listed points, a point per CTA (the plain
+//                 path runs it over every point).
+// A pass with every product in double-float over the points flagged 1, with FP64 for
+// the sums that cancel beyond 1e5, took 128 us of 1,001 points at n = 6 (one CTA per point
+// running long chains), now 38, and 0.42 ms of 8,192 at n = 20, now 0.13.
+
+// The list in the mixed path's record words of F_k(eta + nu/T), which it leaves free:
+// word 0 of record 0 its length, then its entries, 400 a record.
+__device__ __forceinline__ int* nes_list(double* scratch, int64_t k)
+{
+    constexpr int per = 2 * 5 * kMaxM;
+    return (int*)&((PointTab*)(scratch + k / per * kTabWords))->fp[0][0] + k % per;
+}
 
 template <bool MULTI = false>
-__global__ void __launch_bounds__(kNesAccWarps * 32, 2)
-    grey_neps_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
-                     int64_t np, double* __restrict__ scratch)
+__global__ void __launch_bounds__(256)
+    grey_nes_list_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t np,
+                         double* __restrict__ scratch)
 {
-    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
     if (MULTI)
     {
-        const GroupChunk& gcz = GA.gc[blockIdx.z];
-        p0      = gcz.p0;
-        np      = gcz.np;
-        scratch = gcz.ws;
+        if (!GA.Ls[blockIdx.z].use_inel)
+            return;
+        np      = GA.gc[blockIdx.z].np;
+        scratch = GA.gc[blockIdx.z].ws;
     }
-    if (MULTI && !L.use_inel)
+    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in   = q < np && ((PointTab*)(scratch + q * kTabWords))->neps_fp64 != 0.;
+    const uint32_t m = __ballot_sync(0xffffffffu, in);
+    if (m == 0u)
         return;
-    constexpr int NW = kNesAccWarps;
-    __shared__ double s_x2[kMaxQ], s_w2[kMaxQ], s_wx[kMaxQ], s_wx3[kMaxQ];
-    __shared__ NepsTab N;
-    __shared__ NepsMixed Q;
-    __shared__ dfm::FdiTab s_ftab;
-    __shared__ double s_red[NW][32];
-    for (int k = threadIdx.x; k < kMaxQ; k += blockDim.x)
-    {
-        s_x2[k]  = L.x2[k];
-        s_w2[k]  = L.w2[k];
-        s_wx[k]  = L.wx[k];
-        s_wx3[k] = L.wx3[k];
-    }
-    for (int k = threadIdx.x; k < (int)(sizeof(dfm::FdiTab) / sizeof(float)); k += blockDim.x)
-        ((float*)&s_ftab)[k] = ((const float*)&dfm::kFdiTab)[k];
-    __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int wid  = threadIdx.x >> 5;
-    const int n2   = L.n2;
-    const bool nbb = L.neglect_blocking != 0;
-    // items of a point: thread t0, t0 + stride, ...
-    const int t0     = (int)threadIdx.x;
-    const int stride = NW * 32;
-
-    for (int64_t q = blockIdx.x; q < np; q += gridDim.x)
-    {
-        const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
-        PointTab* P     = (PointTab*)(scratch + q * kTabWords);
-        if (P->neps_fp64 != 1.)
-            continue;
-        const double T = L.eos[1][p], mu_e = L.eos[7][p];
-        __syncthreads(); // the previous point's readers are done
-        if (wid == 0)
-        {
-            warp_copy((double*)&N.d, (const double*)&P->d, 28 + 12 + 2, lane);
-            if (lane == 0)
-                N.same_cf = P->same_cf;
-        }
-        __syncthreads();
-        NepsPoint NP;
-        NP.T    = T;
-        NP.pre  = k::NepsConst * (T * T);
-        NP.eta0 = mu_e / T;
-        NP.eta1 = -mu_e / T;
-        NP.fd00 = N.fd0[0];
-        NP.fd01 = N.fd0[1];
-        NP.fe0  = N.fe[0];
-        NP.fe1  = N.fe[1];
-        const double tn = 4. * (k::TempMultiple * T);
-        double acc[16];
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk)
-            acc[kk] = 0.;
-        {
-            int flag = 0;
-            {
-                if (wid == 0 && lane < 2)
-                {
-                    Q.eta[lane] = dfm::from_double(lane ? NP.eta1 : NP.eta0);
-                    dfm::fdi_raw15(Q.eta[lane], Q.reta[lane], 1, &s_ftab);
-                }
-                else if (wid == 0 && lane >= 8 && lane < 12)
-                {
-                    const int s    = lane - 8;
-                    const Distr& d = N.d;
-                    Q.invTt[s] = 1. / d.temp_t[s];
-                    Q.etat[s]  = d.eta_t[s];
-                    Q.lbf[s]   = d.beta_f[s] > 0. ? log(d.beta_f[s]) : -INFINITY;
-                    Q.invTf[s] = 1. / d.temp_f[s];
-                    Q.cf[s]    = d.c_f[s];
-                }
-                __syncthreads();
-                const double invT = 1. / T;
-                const double lhtn = log(0.5 * tn);
-                dfm::df dacc[16];
-#pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                    dacc[kk] = {0.f, 0.f};
-                float mag[16];
-#pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                    mag[kk] = 0.f;
-                const int nn2 = n2 * n2;
-                for (int it = t0; it < 2 * nn2; it += stride)
-                {
-                    const int r   = it >= nn2;
-                    const int rem = it - r * nn2;
-                    const int i = rem / n2, j = rem - (rem / n2) * n2;
-                    double nu, nub;
-                    neps_energies(r, s_x2[i], s_x2[j], tn, &nu, &nub);
-                    const double w = nu * invT, wp = nub * invT;
-                    // log nu, log nubar from the node logarithms
-                    const double lx = L.lx2[i], lm = L.l1m[j], lp = L.l1p[j];
-                    const double lnu  = lhtn + (r ? lm - lx : lx + lm);
-                    const double lnub = lhtn + (r ? lp - lx : lx + lp);
-                    const double Wr   = (r ? s_wx3[i] : s_wx[i]) * s_w2[j];
-                    {
-                        using namespace dfm;
-                        df em1[4], ab1[4], em2[4], ab2[4];
-                        neps_item_df(NP, Q, &s_ftab, w, wp, em1, ab1, em2, ab2);
-                        double wt[4], wfd[4];
-#pragma unroll
-                        for (int s = 0; s < 4; ++s)
-                        {
-                            wt[s]  = N.d.w_t[s];
-                            wfd[s] = N.d.w_f[s];
-                        }
-                        df g[4], gm[4], gb[4], gbm[4];
-                        total_nu_df(nu, lnu, Q, wt, wfd, g, gm);
-                        total_nu_df(nub, lnub, Q, wt, wfd, gb, gbm);
-                        const df W = from_double(w), WP = from_double(wp);
-                        const df ww = mul(W, WP), w4 = mul(ww, ww), Wd = from_double(Wr);
-#pragma unroll
-                        for (int s = 0; s < 4; ++s)
-                        {
-                            const df e1 = mul(em1[s], gb[s]);
-                            const df a1 = nbb ? ab1[s] : mul(ab1[s], gbm[s]);
-                            const df e2 = mul(em2[s], g[s]);
-                            const df a2 = nbb ? ab2[s] : mul(ab2[s], gm[s]);
-                            df EM1, AB1, EM2, AB2;
-                            if (L.stim)
-                            {
-                                AB1 = mul(mul(w4, g[s]), add(e1, a1));
-                                EM1 = mul(w4, e1);
-                                AB2 = mul(mul(w4, gb[s]), add(e2, a2));
-                                EM2 = mul(w4, e2);
-                            }
-                            else
-                            {
-                                AB1 = mul(mul(w4, g[s]), a1);
-                                EM1 = mul(mul(w4, gm[s]), e1);
-                                AB2 = mul(mul(w4, gb[s]), a2);
-                                EM2 = mul(mul(w4, gbm[s]), e2);
-                            }
-                            const df tem = mul(Wd, add(EM1, EM2)), tab = mul(Wd, add(AB1, AB2));
-                            const df tee = mul(Wd, add(mul(W, EM1), mul(WP, EM2)));
-                            const df tae = mul(Wd, add(mul(W, AB1), mul(WP, AB2)));
-                            dacc[s]      = add(dacc[s], tem);
-                            dacc[4 + s]  = add(dacc[4 + s], tab);
-                            dacc[8 + s]  = add(dacc[8 + s], tee);
-                            dacc[12 + s] = add(dacc[12 + s], tae);
-                            mag[s] += fabsf(tem.hi);
-                            mag[4 + s] += fabsf(tab.hi);
-                            mag[8 + s] += fabsf(tee.hi);
-                            mag[12 + s] += fabsf(tae.hi);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                    acc[kk] = dfm::to_double(dacc[kk]);
-                // terms of both signs (occupation above 1), or NES sums
-                // cancelling the pair + brem sums of the same output (those enter
-                // the assembly with t2d^2 = hn / 8, times t2d for energy moments)
-                // or the beta rates: the fast pass hands the point to the
-                // accurate pass, the accurate pass to FP64
-                const double T4 = (T * T) * (T * T);
-                double other[16];
-                beta_in_sum_units(P, T, NP.eta0, L.use_abs_em, true, other);
-                const double t2d = k::TempMultiple * T;
-#pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                    other[kk] += (L.use_pair || L.use_brem)
-                                     ? 0.125 * P->s2d[kk] * (kk >= 8 ? t2d : 1.)
-                                     : 0.;
-                double macc[16];
-#pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                    macc[kk] = (double)mag[kk];
-                block_sum<NW>(acc, s_red, 0);
-                block_sum<NW>(macc, s_red, 16);
-                const double amp =
-                    cancel_factor_tot(acc, macc, NP.pre * T4, NP.pre * T4 * T, other);
-                if (amp > kMaxCancelDf)
-                    flag = 2;
-#pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                    acc[kk] *= NP.pre * T4 * (kk >= 8 ? T : 1.);
-            }
-            if (flag != 0)
-            {
-                if (threadIdx.x == 0)
-                {
-                    P->neps_fp64 = (double)flag;
-                    atomicAdd(&g_grey_mixed[2], 1ull);
-                }
-                continue; // a later launch writes this point's sums
-            }
-        }
-        if (threadIdx.x == 0)
-        {
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
-                P->snes[kk] = acc[kk];
-        }
-    }
+    int first      = 0;
+    if (lane == 0)
+        first = atomicAdd(nes_list(scratch, 0), __popc(m));
+    first = __shfl_sync(0xffffffffu, first, 0);
+    if (in)
+        *nes_list(scratch, 1 + first + __popc(m & ((1u << lane) - 1u))) = (int)q;
 }
 
 
@@ -2072,13 +1640,14 @@ __global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
         make_table();
         __syncthreads();
     }
-    for (int64_t q = (int64_t)blockIdx.x * Smem::kPts + slot; q < np;
-         q += (int64_t)gridDim.x * Smem::kPts)
+    const bool listed = WIDE && flagged; // the list's points, else all
+    const int64_t nw  = listed ? *nes_list(scratch, 0) : np;
+    for (int64_t k = (int64_t)blockIdx.x * Smem::kPts + slot; k < nw;
+         k += (int64_t)gridDim.x * Smem::kPts)
     {
+        const int64_t q = listed ? *nes_list(scratch, 1 + k) : k;
         const int64_t p = L.pidx ? L.pidx[p0 + q] : p0 + q;
         PointTab* P     = (PointTab*)(scratch + q * kTabWords);
-        if (WIDE && flagged && P->neps_fp64 != 2.)
-            continue; // uniform: a point per CTA
         if (!table)
         {
             make_table(); // before the point's first barrier below
@@ -2371,6 +1940,8 @@ __global__ void __launch_bounds__(kNesWarps * 32, 2)
     }
     if (MULTI && !L.use_inel)
         return;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *nes_list(scratch, 0) = 0; // grey_nes_list_kernel fills it
     extern __shared__ __align__(16) unsigned char nes_smem_raw[];
     using Smem   = NesSmem<WIDE>;
     Smem& S      = *reinterpret_cast<Smem*>(nes_smem_raw);
@@ -2655,7 +2226,7 @@ __global__ void __launch_bounds__(kNesWarps * 32, 2)
             // terms of both signs (occupation above 1), or NES sums cancelling
             // the pair + brem sums of the same output (those enter the assembly
             // with t2d^2 = hn / 8, times t2d for energy moments) or the beta
-            // rates: the point goes to the accurate pass
+            // rates: the point goes to the FP64 pass
             const double unit = NP.pre * ((T * T) * (T * T)) * (idx >= 8 ? T : 1.);
             tot *= unit;
             mtot *= unit;
@@ -2678,7 +2249,10 @@ __global__ void __launch_bounds__(kNesWarps * 32, 2)
 }
 
 // ---------------------------------------------------------------------------
-// assembly (m1_opacities.hpp:1172-1294), one thread per point
+// assembly (m1_opacities.hpp:1172-1294): a CTA takes 32 points, a warp a species of
+// them.  Bound by the latency of the record's words and ~12 divisions: with a thread per
+// point, all four species in turn, one point took 17 us and now 11, 8,192 points 20 and
+// 13.
 // ---------------------------------------------------------------------------
 
 // Points whose outputs hold a NaN or Inf (the reference propagates them from
@@ -2698,15 +2272,21 @@ __global__ void __launch_bounds__(128)
         np      = gcz.np;
         scratch = gcz.ws;
     }
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < np;
-         q += (int64_t)gridDim.x * blockDim.x)
+    __shared__ uint32_t s_bad[2][3]; // per point: brem, pair sums to redo; not finite
+    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
+    if (threadIdx.x < 6)
+        s_bad[threadIdx.x / 3][threadIdx.x % 3] = 0u;
+    __syncthreads();
+    int turn = 0;
+    for (int64_t q0 = blockIdx.x * (int64_t)32; q0 < np; q0 += (int64_t)gridDim.x * 32, turn ^= 1)
     {
+        const int64_t q     = q0 + lane;
+        uint32_t* bad       = s_bad[turn];
         bool nonfinite      = false;
-        const int64_t p     = L.pidx ? L.pidx[p0 + q] : p0 + q;
-        PointTab* P         = (PointTab*)(scratch + q * kTabWords);
         const bool pcheck   = L.mixed && L.use_pair;
-        if (redo_only && P->bredo != 1. && !(pcheck && pair_mixed(P)->predo == 1.))
-            continue;
+        PointTab* P         = (PointTab*)(scratch + (q < np ? q : q0) * kTabWords);
+        const bool run      = q < np && !(redo_only && P->bredo != 1. &&
+                                          !(pcheck && pair_mixed(P)->predo == 1.));
         // mixed path: FP32 brem terms whose sum the other reactions cancel
         // (the NES sums of the opposite sign where the occupation exceeds 1)
         // by more than kMaxCancelBrem are recomputed in FP64 (bredo = 1); the
@@ -2715,25 +2295,18 @@ __global__ void __launch_bounds__(128)
         const bool check_pair = !redo_only && pcheck;
         bool bredo       = false;
         bool predo       = false;
-        const double T      = L.eos[1][p];
-        const double eta_e  = L.eos[7][p] / T;
-        const double t2d    = k::TempMultiple * T;
-        const double t2     = t2d * t2d;
-        const double tn     = 4. * (k::TempMultiple * T);
-        const double hn     = 0.5 * (tn * tn);
-        const bool has2d    = L.use_pair || L.use_brem;
-        double sb[2];
-        double fe[2][6];
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-#pragma unroll
-            for (int kk = 0; kk < 6; ++kk)
-                fe[e][kk] = P->fe[e][kk];
-        beta_scales(T, eta_e, fe, sb);
-        const double F = k::FourPiHc3, F2 = k::FourPiHc3Sqr, c = k::Clight;
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
+        if (run)
         {
+            const int64_t p     = L.pidx ? L.pidx[p0 + q] : p0 + q;
+            const double T      = L.eos[1][p];
+            const double eta_e  = L.eos[7][p] / T;
+            const double t2d    = k::TempMultiple * T;
+            const double t2     = t2d * t2d;
+            const double tn     = 4. * (k::TempMultiple * T);
+            const double hn     = 0.5 * (tn * tn);
+            const bool has2d    = L.use_pair || L.use_brem;
+            const double sb = s < 2 ? beta_scale(P->fe[s & 1][4], P->fe[s & 1][5], T, eta_e, s) : 0.;
+            const double F = k::FourPiHc3, F2 = k::FourPiHc3Sqr, c = k::Clight;
             const double n = L.m1[s][p], J = L.m1[4 + s][p];
             const double s_iso = (n > k::ThresholdN) ? (J / n) : 1.5 * T;
             const double n2d_em = has2d ? P->s2d[s] * t2 : 0.;
@@ -2751,10 +2324,10 @@ __global__ void __launch_bounds__(128)
             {
                 if (L.use_abs_em)
                 {
-                    bne = P->sbeta[s] * sb[s];
-                    bje = P->sbeta[2 + s] * sb[s];
-                    bna = P->sbeta[4 + s] * sb[s];
-                    bja = P->sbeta[6 + s] * sb[s];
+                    bne = P->sbeta[s] * sb;
+                    bje = P->sbeta[2 + s] * sb;
+                    bna = P->sbeta[4 + s] * sb;
+                    bja = P->sbeta[6 + s] * sb;
                 }
                 o[0] = F * (F * (n2d_em + nne_em) + bne);
                 o[2] = F * (F * (e2d_em + ene_em) + bje);
@@ -2797,20 +2370,41 @@ __global__ void __launch_bounds__(128)
                 nonfinite = nonfinite || !isfinite(o[qq]);
             }
         }
-        if (!redo_only)
-            P->bredo = bredo ? 1. : 0.; // also where brem is off: scratch is reused
-        if (check_pair)
-            pair_mixed(P)->predo = predo ? 1. : 0.;
-        if (!redo_only && L.mixed)
+        const uint32_t mb = __ballot_sync(0xffffffffu, bredo), mp = __ballot_sync(0xffffffffu, predo);
+        const uint32_t mn = __ballot_sync(0xffffffffu, nonfinite);
+        if (lane == 0)
         {
-            atomicAdd(&g_grey_mixed[0], 1ull);
-            if (predo)
-                atomicAdd(&g_grey_mixed[3], 1ull);
-            if (bredo)
-                atomicAdd(&g_grey_mixed[4], 1ull);
+            if (mb)
+                atomicOr(&bad[0], mb);
+            if (mp)
+                atomicOr(&bad[1], mp);
+            if (mn)
+                atomicOr(&bad[2], mn);
         }
-        if (nonfinite && !redo_only)
-            atomicAdd(&g_grey_nonfinite, 1ull);
+        __syncthreads();
+        if (s == 0)
+        {
+            const uint32_t br = bad[0], pr = bad[1], nf = bad[2];
+            const uint32_t mr = __ballot_sync(0xffffffffu, run);
+            if (run && !redo_only)
+                P->bredo = (br >> lane) & 1u ? 1. : 0.; // also where brem is off: scratch is reused
+            if (run && check_pair)
+                pair_mixed(P)->predo = (pr >> lane) & 1u ? 1. : 0.;
+            if (lane == 0)
+            {
+                bad[0] = bad[1] = bad[2] = 0u; // for the turn after the next
+                if (!redo_only && L.mixed)
+                {
+                    atomicAdd(&g_grey_mixed[0], (unsigned long long)__popc(mr));
+                    if (pr)
+                        atomicAdd(&g_grey_mixed[3], (unsigned long long)__popc(pr));
+                    if (br)
+                        atomicAdd(&g_grey_mixed[4], (unsigned long long)__popc(br));
+                }
+                if (nf && !redo_only)
+                    atomicAdd(&g_grey_nonfinite, (unsigned long long)__popc(nf));
+            }
+        }
     }
 }
 
@@ -3004,10 +2598,8 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
                 return err;
             phase_mark(kPhNeps, 1, st);
             phase_mark(kPhNepsAccurate, 0, st);
-            constexpr int wa = kNesAccWarps * 32;
-            grey_neps_kernel<MULTI>
-                <<<dim3(grid_for(grey_neps_kernel<MULTI>, wa, np, sms), 1, gz), wa, 0, st>>>(
-                    L, S.GA, S.p0, np, S.ws);
+            grey_nes_list_kernel<MULTI><<<dim3((unsigned)((np + 255) / 256), 1, gz), 256, 0, st>>>(
+                L, S.GA, np, S.ws);
             phase_mark(kPhNepsAccurate, 1, st);
             phase_mark(kPhNepsFp64, 0, st);
             if ((err = launch_nes64<true, MULTI>(S, st, sms, 1)) != cudaSuccess)
@@ -3024,7 +2616,7 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
             phase_mark(kPhNeps, 1, st);
         }
     }
-    const dim3 fgrid(grid_for(grey_final_kernel<MULTI>, 128, (np + 127) / 128, sms), 1, gz);
+    const dim3 fgrid(grid_for(grey_final_kernel<MULTI>, 128, (np + 31) / 32, sms), 1, gz);
     phase_mark(kPhFinal, 0, st);
     grey_final_kernel<MULTI><<<fgrid, 128, 0, st>>>(L, S.GA, S.p0, np, S.ws, 0);
     phase_mark(kPhFinal, 1, st);
