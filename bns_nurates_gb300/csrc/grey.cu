@@ -713,7 +713,7 @@ __device__ __forceinline__ void fill_tab32(CellTab32& D, const CellTab& C, int M
 // and 4 rounds of cells at n = 20 and 10, 12 to 25 KB of shared memory per
 // point).
 // ---------------------------------------------------------------------------
-constexpr int kCellThreads = 64;
+constexpr int kCellThreads = 64, kCellWide = 256;
 
 template <int NT>
 struct CellNodes
@@ -862,13 +862,13 @@ __device__ __forceinline__ void cell_row_sums(const CellNodes<NT>& C, int M, boo
     }
 }
 
-// Totals over the CTA: lane l of a warp holds that of moment sum_index(l).
-template <int NT>
+// Totals over the first NT of a CTA's NTW threads: lane l of a warp holds that of moment sum_index(l).
+template <int NTW, int NT>
 __device__ __forceinline__ double cell_total(CellNodes<NT>& C, double* acc, int slot)
 {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double v = warp_sum16(acc, lane);
-    if (!(lane & 1))
+    if ((NTW == NT || wid < NT / 32) && !(lane & 1))
         C.red[slot][wid][sum_index(lane)] = v;
     __syncthreads();
     double t = C.red[slot][0][sum_index(lane)];
@@ -903,8 +903,8 @@ struct PairTab64
 // Fermi-integral tables itself.
 // 8,192 points, n = 20: FP64 2.95 -> 1.35 ms, mixed with its redo pass 2.46 ->
 // 1.52 ms; one point, n = 10: 74 -> 29 us.
-template <bool MIXED, bool MULTI = false>
-__global__ void __launch_bounds__(kCellThreads)
+template <bool MIXED, bool MULTI = false, int NTW = kCellThreads>
+__global__ void __launch_bounds__(NTW)
     grey_pair_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
                      int64_t np, double* __restrict__ scratch, int redo_only)
 {
@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(kCellThreads)
         }
         if (!MIXED)
         {
-            for (int qq = threadIdx.x; qq < 2 * M; qq += kCellThreads)
+            for (int qq = threadIdx.x; qq < 2 * M; qq += NTW)
             {
                 const int a = qq >> 1;
                 double f[5];
@@ -979,7 +979,7 @@ __global__ void __launch_bounds__(kCellThreads)
         // em = Phi T^2 / 2 (alpha1^2 Psi(y, z) + alpha2^2 Psi(z, y)) / (1 - e^s), ab = e^s em
         const double sc = MIXED ? 0.5 * k::PairPhi * T2 * (T2 * T2) / 15.
                                 : -0.5 * k::PairPhi * T2 / 15.;
-        for (int c = threadIdx.x; c < ncell; c += kCellThreads)
+        for (int c = threadIdx.x; c < ncell; c += NTW)
         {
             const uint32_t ab = C.cells[c];
             const int a = ab & 0xffu, b = ab >> 8;
@@ -1011,8 +1011,9 @@ __global__ void __launch_bounds__(kCellThreads)
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk)
             acc[kk] = 0.;
-        cell_row_sums<false, false>(C, M, stim, e0, e1, x0, x1, acc);
-        const double tot = cell_total(C, acc, 0);
+        if (NTW == kCellThreads || threadIdx.x < kCellThreads)
+            cell_row_sums<false, false>(C, M, stim, e0, e1, x0, x1, acc);
+        const double tot = cell_total<NTW>(C, acc, 0);
         double mag       = fabs(tot);
         if (MIXED && above)
         {
@@ -1020,7 +1021,7 @@ __global__ void __launch_bounds__(kCellThreads)
             for (int kk = 0; kk < 16; ++kk)
                 acc[kk] = 0.;
             cell_row_sums<false, true>(C, M, stim, e0, e1, x0, x1, acc);
-            const double m = cell_total(C, acc, 1);
+            const double m = cell_total<NTW>(C, acc, 1);
             if (!(sum_index(threadIdx.x & 31) & 4))
                 mag = m;
         }
@@ -1088,9 +1089,9 @@ __device__ __forceinline__ void brem64_constants(Brem64Smem<IMPL, NT>& S, const 
     }
 }
 
-// The brem sums of a point, by all NT threads: lane l of each warp returns the
+// The brem sums of a point, by the CTA's threads (the row sums by the first NT): lane l of each warp returns the
 // total of moment sum_index(l).
-template <int IMPL, int NT>
+template <int NTW, int IMPL, int NT>
 __device__ __forceinline__ double brem64_point(Brem64Smem<IMPL, NT>& S, const OpacityLaunch& L,
                                                PointTab* P, int64_t p)
 {
@@ -1102,7 +1103,7 @@ __device__ __forceinline__ double brem64_point(Brem64Smem<IMPL, NT>& S, const Op
     bool fast = true; // HR98: every cell within hr98_absorption's range
     if constexpr (IMPL == 0)
     {
-        for (int k = threadIdx.x; k < (int)(sizeof(Hr98Point) / sizeof(double)); k += NT)
+        for (int k = threadIdx.x; k < (int)(sizeof(Hr98Point) / sizeof(double)); k += NTW)
             ((double*)&S.X.hr)[k] = ((const double*)&P->hr)[k];
         __syncthreads();
         if (threadIdx.x < 4)
@@ -1118,12 +1119,12 @@ __device__ __forceinline__ double brem64_point(Brem64Smem<IMPL, NT>& S, const Op
         prof = L.gp19.d3 <= kGp19MaxW;
         if (prof)
         {
-            for (int k = threadIdx.x; k < (int)(sizeof(Gp19Record) / sizeof(double)); k += NT)
+            for (int k = threadIdx.x; k < (int)(sizeof(Gp19Record) / sizeof(double)); k += NTW)
                 ((double*)&S.X.r)[k] = ((const double*)gp19_record(P))[k];
             __syncthreads();
             const Gp19Table G = gp19_table(L);
             const int np19    = S.X.r.pt.regime >= 2 ? 2 : 1;
-            for (int e = threadIdx.x; e < np19 * G.d3; e += NT)
+            for (int e = threadIdx.x; e < np19 * G.d3; e += NTW)
             {
                 const int pr = e / G.d3, l = e - pr * G.d3;
                 S.X.p[pr][l] = gp19_profile_eval(G, S.X.r.cor[pr], l);
@@ -1131,7 +1132,7 @@ __device__ __forceinline__ double brem64_point(Brem64Smem<IMPL, NT>& S, const Op
         }
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < L.ncell; c += NT)
+    for (int c = threadIdx.x; c < L.ncell; c += NTW)
     {
         const uint32_t ab = C.cells[c];
         const int a = ab & 0xffu, b = ab >> 8;
@@ -1164,16 +1165,17 @@ __device__ __forceinline__ double brem64_point(Brem64Smem<IMPL, NT>& S, const Op
 #pragma unroll
     for (int kk = 0; kk < 16; ++kk)
         acc[kk] = 0.;
-    cell_row_sums<true, false>(C, M, L.stim != 0, 1., 0., 1., 0., acc);
-    return cell_total(C, acc, 0);
+    if (NTW == NT || threadIdx.x < NT)
+        cell_row_sums<true, false>(C, M, L.stim != 0, 1., 0., 1., 0., acc);
+    return cell_total<NTW>(C, acc, 0);
 }
 
 // Every point (the plain path), or with redo_only the points the mixed path's
 // final kernel marked (bredo = 1), whose brem part of s2d it replaces.
 // 8,192 points: HR98 n = 10 1.40 -> 0.44 ms, GP19 n = 20 2.66 -> 0.84 ms, BRT06 n = 10
 // 0.65 -> 0.26 ms.
-template <int IMPL, bool MULTI = false>
-__global__ void __launch_bounds__(kCellThreads)
+template <int IMPL, bool MULTI = false, int NTW = kCellThreads>
+__global__ void __launch_bounds__(NTW)
     grey_brem_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
                      int64_t np, double* __restrict__ scratch, int add, int redo_only)
 {
@@ -1201,7 +1203,7 @@ __global__ void __launch_bounds__(kCellThreads)
             brem64_constants(S, L);
             ready = true;
         }
-        const double tot = brem64_point(S, L, P, p);
+        const double tot = brem64_point<NTW>(S, L, P, p);
         if (threadIdx.x < 32 && !(threadIdx.x & 1))
         {
             const int idx     = sum_index(threadIdx.x);
@@ -1472,7 +1474,7 @@ __global__ void __launch_bounds__(kWarps * 32, 3)
                 brem64_constants(S64, L);
                 ready = true;
             }
-            const double tot = brem64_point(S64, L, P, L.pidx ? L.pidx[p0 + q] : p0 + q);
+            const double tot = brem64_point<kWarps * 32>(S64, L, P, L.pidx ? L.pidx[p0 + q] : p0 + q);
             if (threadIdx.x < 32 && !(threadIdx.x & 1))
             {
                 const int idx = sum_index(threadIdx.x);
@@ -2500,12 +2502,35 @@ cudaError_t launch_nes64(const Step& S, cudaStream_t st, int sms, int flagged)
     return cudaGetLastError();
 }
 
+// FP64 chunks of at most a point per SM take 256 threads a point in the cell kernels: a
+// point's cells in one round instead of four at n = 10.  The row sums stay with the first
+// 64 threads, so a point's results do not depend on it.  One point, pair and brem: n = 10
+// HR98 64 -> 48 us, n = 20 GP19 124 -> 89; 152 points 68 -> 49, 153 -> 108; 304 points at
+// n = 20 157 -> 179.
+template <bool MIXED, bool MULTI, int NTW>
+void launch_pair_of(const Step& S, cudaStream_t st, int sms, int redo_only)
+{
+    const auto kernel = grey_pair_kernel<MIXED, MULTI, NTW>;
+    kernel<<<dim3(grid_for(kernel, NTW, S.np, sms), 1, MULTI ? S.G : 1), NTW, 0, st>>>(
+        *S.L, S.GA, S.p0, S.np, S.ws, redo_only);
+}
+
 template <bool MIXED, bool MULTI>
 void launch_pair(const Step& S, cudaStream_t st, int sms, int redo_only)
 {
-    const auto kernel = grey_pair_kernel<MIXED, MULTI>;
-    kernel<<<dim3(grid_for(kernel, kCellThreads, S.np, sms), 1, MULTI ? S.G : 1), kCellThreads, 0,
-             st>>>(*S.L, S.GA, S.p0, S.np, S.ws, redo_only);
+    if (!MIXED && !MULTI && S.np <= sms)
+        launch_pair_of<MIXED, MULTI, MIXED || MULTI ? kCellThreads : kCellWide>(S, st, sms,
+                                                                                redo_only);
+    else
+        launch_pair_of<MIXED, MULTI, kCellThreads>(S, st, sms, redo_only);
+}
+
+template <int IMPL, bool MULTI, int NTW>
+void launch_brem64(const Step& S, cudaStream_t st, int sms, int add, bool redo)
+{
+    const auto k64 = grey_brem_kernel<IMPL, MULTI, NTW>;
+    k64<<<dim3(grid_for(k64, NTW, S.np, sms), 1, MULTI ? S.G : 1), NTW, 0, st>>>(
+        *S.L, S.GA, S.p0, S.np, S.ws, add, redo ? 1 : 0);
 }
 
 // Brem variant IMPL; redo is the FP64 pass over the points the mixed path's
@@ -2522,12 +2547,10 @@ void launch_brem_impl(const Step& S, cudaStream_t st, int sms, bool mixed, int a
         k32<<<dim3(grid_for(k32, kWarps * 32, work, sms), 1, gz), kWarps * 32, 0, st>>>(
             *S.L, S.GA, S.p0, S.np, S.ws, add);
     }
+    else if (!MULTI && S.np <= sms)
+        launch_brem64<IMPL, MULTI, MULTI ? kCellThreads : kCellWide>(S, st, sms, add, redo);
     else
-    {
-        const auto k64 = grey_brem_kernel<IMPL, MULTI>;
-        k64<<<dim3(grid_for(k64, kCellThreads, S.np, sms), 1, gz), kCellThreads, 0, st>>>(
-            *S.L, S.GA, S.p0, S.np, S.ws, add, redo ? 1 : 0);
-    }
+        launch_brem64<IMPL, MULTI, kCellThreads>(S, st, sms, add, redo);
     phase_mark(kPhBrem, 1, st);
 }
 
