@@ -893,6 +893,13 @@ struct PairTab64
     double m[kMaxM][5], p[kMaxM][5], iy2[kMaxM];
 };
 
+template <bool MIXED>
+struct PairSmem
+{
+    CellNodes<kCellThreads> C;
+    alignas(16) unsigned char tab[MIXED ? sizeof(PairTab32) : sizeof(PairTab64)];
+};
+
 // e+e- pair phase.  MIXED: cells from the FP32 integral (bnsn_pair32.cuh); the
 // sums and the magnitudes of their terms are written to the record (PairMixed).
 // The pair kernels are non-negative and so are the absorption terms (em + am =
@@ -903,24 +910,14 @@ struct PairTab64
 // Fermi-integral tables itself.
 // 8,192 points, n = 20: FP64 2.95 -> 1.35 ms, mixed with its redo pass 2.46 ->
 // 1.52 ms; one point, n = 10: 74 -> 29 us.
-template <bool MIXED, bool MULTI = false, int NTW = kCellThreads>
-__global__ void __launch_bounds__(NTW)
-    grey_pair_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
-                     int64_t np, double* __restrict__ scratch, int redo_only)
+template <bool MIXED, int NTW>
+__device__ __forceinline__ void pair_points(PairSmem<MIXED>& S, const OpacityLaunch& L,
+                                            int64_t p0, int64_t np, double* __restrict__ scratch,
+                                            int redo_only)
 {
-    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
-    if (MULTI)
-    {
-        const GroupChunk& gcz = GA.gc[blockIdx.z];
-        p0      = gcz.p0;
-        np      = gcz.np;
-        scratch = gcz.ws;
-    }
-    if (MULTI && !L.use_pair)
-        return; // a group without pair (uniform over the CTA)
-    __shared__ CellNodes<kCellThreads> C;
-    __shared__ PairTab32 X;
-    __shared__ PairTab64 W;
+    CellNodes<kCellThreads>& C = S.C;
+    PairTab32& X = *reinterpret_cast<PairTab32*>(S.tab); // MIXED
+    PairTab64& W = *reinterpret_cast<PairTab64*>(S.tab); // !MIXED
     const int M     = 2 * L.n2;
     const int ncell = L.ncell;
     const bool nbb = L.neglect_blocking != 0, stim = L.stim != 0;
@@ -1043,6 +1040,25 @@ __global__ void __launch_bounds__(NTW)
                 Y->predo = 0.;
         }
     }
+}
+
+template <bool MIXED, bool MULTI = false, int NTW = kCellThreads>
+__global__ void __launch_bounds__(NTW)
+    grey_pair_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
+                     int64_t np, double* __restrict__ scratch, int redo_only)
+{
+    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
+    if (MULTI)
+    {
+        const GroupChunk& gcz = GA.gc[blockIdx.z];
+        p0      = gcz.p0;
+        np      = gcz.np;
+        scratch = gcz.ws;
+    }
+    if (MULTI && !L.use_pair)
+        return; // a group without pair (uniform over the CTA)
+    __shared__ PairSmem<MIXED> S;
+    pair_points<MIXED, NTW>(S, L, p0, np, scratch, redo_only);
 }
 
 // ---------------------------------------------------------------------------
@@ -1174,23 +1190,11 @@ __device__ __forceinline__ double brem64_point(Brem64Smem<IMPL, NT>& S, const Op
 // final kernel marked (bredo = 1), whose brem part of s2d it replaces.
 // 8,192 points: HR98 n = 10 1.40 -> 0.44 ms, GP19 n = 20 2.66 -> 0.84 ms, BRT06 n = 10
 // 0.65 -> 0.26 ms.
-template <int IMPL, bool MULTI = false, int NTW = kCellThreads>
-__global__ void __launch_bounds__(NTW)
-    grey_brem_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
-                     int64_t np, double* __restrict__ scratch, int add, int redo_only)
+template <int NTW, int IMPL>
+__device__ __forceinline__ void brem_points(Brem64Smem<IMPL, kCellThreads>& S,
+                                            const OpacityLaunch& L, int64_t p0, int64_t np,
+                                            double* __restrict__ scratch, int add, int redo_only)
 {
-    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
-    if (MULTI)
-    {
-        const GroupChunk& gcz = GA.gc[blockIdx.z];
-        p0      = gcz.p0;
-        np      = gcz.np;
-        scratch = gcz.ws;
-        if (!L.use_brem || L.brem_impl != IMPL)
-            return; // another brem variant's launch serves this group
-        add = L.use_pair;
-    }
-    __shared__ Brem64Smem<IMPL, kCellThreads> S;
     bool ready = false;
     for (int64_t q = blockIdx.x; q < np; q += gridDim.x)
     {
@@ -1213,6 +1217,26 @@ __global__ void __launch_bounds__(NTW)
             P->bmag[idx]  = 0.;
         }
     }
+}
+
+template <int IMPL, bool MULTI = false, int NTW = kCellThreads>
+__global__ void __launch_bounds__(NTW)
+    grey_brem_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
+                     int64_t np, double* __restrict__ scratch, int add, int redo_only)
+{
+    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
+    if (MULTI)
+    {
+        const GroupChunk& gcz = GA.gc[blockIdx.z];
+        p0      = gcz.p0;
+        np      = gcz.np;
+        scratch = gcz.ws;
+        if (!L.use_brem || L.brem_impl != IMPL)
+            return; // another brem variant's launch serves this group
+        add = L.use_pair;
+    }
+    __shared__ Brem64Smem<IMPL, kCellThreads> S;
+    brem_points<NTW>(S, L, p0, np, scratch, add, redo_only);
 }
 
 // Per-warp GP19 state of the FP32 brem kernel.
@@ -1583,25 +1607,13 @@ struct Nes64Smem
     double terms[WIDE ? 16 : 1][WIDE ? kNW * 32 : 1]; // EM1, AB1, EM2, AB2 of a round's items
 };
 
-template <bool WIDE, bool MULTI = false>
-__global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
-    grey_nes64_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
-                      int64_t np, double* __restrict__ scratch, int flagged)
+template <bool WIDE>
+__device__ __forceinline__ void nes64_points(Nes64Smem<WIDE>& S, const OpacityLaunch& L,
+                                             int64_t p0, int64_t np,
+                                             double* __restrict__ scratch, int flagged)
 {
-    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
-    if (MULTI)
-    {
-        const GroupChunk& gcz = GA.gc[blockIdx.z];
-        p0      = gcz.p0;
-        np      = gcz.np;
-        scratch = gcz.ws;
-    }
-    if (MULTI && !L.use_inel)
-        return;
     using Smem = Nes64Smem<WIDE>;
     constexpr int kStride = Smem::kWPP * 32;
-    extern __shared__ __align__(16) unsigned char nes_smem_raw[];
-    Smem& S        = *reinterpret_cast<Smem*>(nes_smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int slot = wid / Smem::kWPP, wsub = wid - slot * Smem::kWPP;
     const int n2 = L.n2, nn2 = n2 * n2, nit = 2 * nn2;
@@ -1813,6 +1825,52 @@ __global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
             P->snes[idx] = t * (pre * ((T * T) * (T * T)) * (idx >= 8 ? T : 1.));
         }
     }
+}
+
+template <bool WIDE, bool MULTI = false>
+__global__ void __launch_bounds__(Nes64Smem<WIDE>::kNW * 32, WIDE ? 2 : 1)
+    grey_nes64_kernel(const __grid_constant__ OpacityLaunch L0, const GroupArgs GA, int64_t p0,
+                      int64_t np, double* __restrict__ scratch, int flagged)
+{
+    const OpacityLaunch& L = MULTI ? GA.Ls[blockIdx.z] : L0;
+    if (MULTI)
+    {
+        const GroupChunk& gcz = GA.gc[blockIdx.z];
+        p0      = gcz.p0;
+        np      = gcz.np;
+        scratch = gcz.ws;
+    }
+    if (MULTI && !L.use_inel)
+        return;
+    extern __shared__ __align__(16) unsigned char nes_smem_raw[];
+    nes64_points(*reinterpret_cast<Nes64Smem<WIDE>*>(nes_smem_raw), L, p0, np, scratch, flagged);
+}
+
+// Pair + brem (blockIdx.y = 0) and NES (1) of small FP64 calls in one launch, a point per
+// CTA: they need only the prelude's tables, and each alone leaves most of the chip and of
+// its own CTA's latency unused.  One point, n = 10 HR98: the three phases 83 -> 46 us.
+template <int IMPL>
+__global__ void __launch_bounds__(kCellWide, 2)
+    grey_small_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
+                      double* __restrict__ scratch)
+{
+    static_assert(Nes64Smem<true>::kNW * 32 == kCellWide, "one CTA size");
+    static_assert(sizeof(PairSmem<false>) <= sizeof(Nes64Smem<true>) &&
+                      sizeof(Brem64Smem<IMPL, kCellThreads>) <= sizeof(Nes64Smem<true>),
+                  "shared memory of the launch");
+    extern __shared__ __align__(16) unsigned char nes_smem_raw[];
+    if (blockIdx.y == 1)
+    {
+        nes64_points(*reinterpret_cast<Nes64Smem<true>*>(nes_smem_raw), L, p0, np, scratch, 0);
+        return;
+    }
+    if (L.use_pair)
+        pair_points<false, kCellWide>(*reinterpret_cast<PairSmem<false>*>(nes_smem_raw), L, p0, np,
+                                      scratch, 0);
+    __syncthreads(); // the pair tables' readers are done
+    if (L.use_brem)
+        brem_points<kCellWide>(*reinterpret_cast<Brem64Smem<IMPL, kCellThreads>*>(nes_smem_raw), L,
+                               p0, np, scratch, L.use_pair, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -2570,6 +2628,35 @@ cudaError_t launch_brem(const Step& S, cudaStream_t st, int sms, bool mixed, int
     return cudaGetLastError();
 }
 
+template <int IMPL>
+cudaError_t launch_small_impl(const Step& S, cudaStream_t st)
+{
+    constexpr int smem  = (int)sizeof(Nes64Smem<true>);
+    const auto kernel   = grey_small_kernel<IMPL>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               smem);
+    if (e != cudaSuccess)
+        return e;
+    phase_mark(kPhNeps, 0, st);
+    kernel<<<dim3((unsigned)S.np, S.L->use_inel ? 2 : 1), kCellWide, smem, st>>>(*S.L, S.p0, S.np, S.ws);
+    phase_mark(kPhNeps, 1, st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_small(const Step& S, cudaStream_t st)
+{
+    const int impl = S.L->use_brem ? S.L->brem_impl : 1;
+    return impl == 0 ? launch_small_impl<0>(S, st)
+                     : impl == 1 ? launch_small_impl<1>(S, st) : launch_small_impl<2>(S, st);
+}
+
+// FP64 calls of at most this many points per SM take grey_small_kernel for NES beside
+// pair or brem, and of at most one for pair and brem alone.  A call's time, each phase by
+// itself -> together: one point n = 10 HR98 173 -> 140 us, n = 20 GP19 304 -> 220; 304
+// points n = 6 152 -> 143, n = 10 229 -> 211, n = 20 466 -> 415; 456 points 185 -> 180, 280 ->
+// 267, 668 -> 611; 608 points 199 -> 208, 313 -> 319, 716 -> 708.
+constexpr int64_t kSmallPerSm = 3;
+
 // The phase kernels of one step on stream st: point constants, prelude, pair,
 // brem, NES, final, and on the mixed path the FP64 passes over the points the
 // final kernel marked, with a second final pass.
@@ -2595,7 +2682,12 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
         <<<dim3(grid_for(grey_prelude_kernel<MULTI>, kPreWarps * 32, np, sms), 1, gz),
            kPreWarps * 32, 0, st>>>(L, S.GA, S.p0, np, S.ws);
     phase_mark(kPhPrelude, 1, st);
-    if (L.use_pair)
+    const bool small = !MULTI && !L.mixed &&
+                       (L.use_inel ? (L.use_pair || L.use_brem) && np <= kSmallPerSm * sms
+                                   : L.use_pair && L.use_brem && np <= sms);
+    if (small && (err = launch_small(S, st)) != cudaSuccess)
+        return err;
+    if (L.use_pair && !small)
     {
         phase_mark(kPhPair, 0, st);
         if (L.mixed)
@@ -2604,13 +2696,13 @@ cudaError_t launch_step(const Step& S, cudaStream_t st, int sms)
             launch_pair<false, MULTI>(S, st, sms, 0);
         phase_mark(kPhPair, 1, st);
     }
-    if (L.use_brem)
+    if (L.use_brem && !small)
     {
         err = launch_brem<MULTI>(S, st, sms, L.mixed != 0, L.use_pair);
         if (err != cudaSuccess)
             return err;
     }
-    if (L.use_inel)
+    if (L.use_inel && !small)
     {
         if (L.mixed)
         {
