@@ -18,10 +18,12 @@
 // One thread per argument, grid-stride, the order's table (9 KB) in shared memory
 // per CTA.  Arguments come in any order, so a warp usually meets all three regimes:
 // they share the polynomial, and the factors (e^x, x^(j+1)) run on the integer
-// pipes (bnsn_fx.cuh).  FP64-pipe bound, ~30 operations per argument against 16 bytes of
-// traffic.  A loop per regime instead (16 + 25 Clenshaw + 12 terms, exp, sqrt and two
+// pipes (bnsn_fx.cuh).  The interval and the position in it come from the argument in
+// fixed point.  FP64-pipe bound, ~20 operations per argument against 16 bytes of traffic.  A loop per regime instead (16 + 25 Clenshaw + 12 terms, exp, sqrt and two
 // divisions) cost a mixed warp the sum of them: ~150.  4,000,037 arguments uniform in
-// [-50, 150), order 1/2: 978 -> 265 us.
+// [-50, 150), order 1/2: 978 -> 164 us (265 with
+// the interval in FP64).
+
 #include <cuda_runtime.h>
 
 #include "bnsn_fdi_tab.h"
@@ -75,34 +77,27 @@ __device__ __forceinline__ double fdi_table(const FdiShared& S, int h, int64_t P
                                             bool integer, double x)
 {
     using namespace fdit;
+    static_assert(kXlo == -4. && kXmid == 40. && kXhi == 100. && kWidth == 11. / 16. &&
+                      kWide == 10.,
+                  "the interval arithmetic below");
+    const uint64_t bits = fx::bits_of(x), mag = bits & 0x7fffffffffffffffull;
+    const bool neg      = (int64_t)bits < 0;
     double v, f = 1.;
     int row;
-    if (x < kXlo)
+    if (neg && mag > 0x4010000000000000ull) // x < -4, or NaN
     {
         f   = fx::exp(x);
         v   = -f;
         row = 0;
     }
-    else if (x < kXhi)
+    else if (!neg && mag >= 0x4059000000000000ull) // x >= 100, or NaN
     {
-        const bool narrow = x < kXmid;
-        const double lo   = narrow ? kXlo : kXmid;
-        int i = (int)((x - lo) * (narrow ? 1. / kWidth : 1. / kWide));
-        const int last = narrow ? kNarrow - 1 : kPieces - kNarrow - 1;
-        i   = i > last ? last : i;
-        v   = (x - (lo + (narrow ? kWidth : kWide) * ((double)i + 0.5))) *
-              (narrow ? 2. / kWidth : 2. / kWide);
-        row = 1 + i + (narrow ? 0 : kNarrow);
-    }
-    else
-    {
-        if (x != x) // NaN fails both regime tests above
-            return integer ? 0. : x;
         row = kPieces + 1;
-        if (x < 0x1p80)
+        if (mag < 0x44f0000000000000ull) // 2^80
         {
-            v = fx::rcp(x * x);
-            f = fx::pow_q(fx::log2_q56(x), P) * ij1;
+            const int64_t L = fx::log2_q56(x);
+            v = fx::pow_q(L, -2 * (1ll << 58));
+            f = fx::pow_q(L, P) * ij1;
         }
         else
         {
@@ -110,11 +105,27 @@ __device__ __forceinline__ double fdi_table(const FdiShared& S, int h, int64_t P
             f = pow_half(x, h) * ij1;
         }
     }
+    else
+    {
+        // y = x + 4 in 2^-56 (exact for |x| >= 1/8), its interval in sixteenths
+        const int sh     = 7 + 1023 - (int)(mag >> 52);
+        const uint64_t A = sh > 63 ? 0ull : ((mag << 11) | 0x8000000000000000ull) >> sh;
+        const int64_t Y  = (4ll << 56) + (neg ? -(int64_t)A : (int64_t)A);
+        const int y16    = (int)(Y >> 52);
+        const bool wide  = y16 >= 704;
+        const int i      = wide ? (y16 - 704) / 160 : y16 / 11;
+        const int w = wide ? 160 : 11, base = wide ? 704 + i * 160 : i * 11;
+        // 2 (y - start) - width over the width
+        const int64_t r = 2 * (Y - ((int64_t)base << 52)) - ((int64_t)w << 52);
+        v   = (double)r * (wide ? 0x1p-52 / 160. : 0x1p-52 / 11.);
+        row = 1 + i + (wide ? kNarrow : 0);
+    }
     double p = S.c[kDegree][row];
 #pragma unroll
     for (int m = kDegree - 1; m >= 0; --m)
         p = fma(p, v, S.c[m][row]);
-    return f * p;
+    // NaN: 0 for the integer orders, as the reference's regime tests give
+    return mag > 0x7ff0000000000000ull ? (integer ? 0. : x) : f * p;
 }
 
 template <int K>
