@@ -14,8 +14,8 @@
 // polynomial for e^r - 1 on |r| <= ln2/32, and four exact-ish squarings of
 // (1 + q) carried as q -> q (2 + q).
 //
-// fdi_df<KLO, KHI> evaluates the same Fukushima rational forms as
-// fdi_orders (bnsn_fp64.cuh) with df coefficients.
+// fdi_raw15 evaluates the reference's rational forms of F_1..F_5 (fdi_rational,
+// bnsn_fp64.cuh) with df coefficients.
 #pragma once
 
 #include <math.h>
@@ -86,7 +86,6 @@ BNSN_DI df add(df a, float b)
 }
 
 BNSN_DI df neg(df a) { return {-a.hi, -a.lo}; }
-BNSN_DI df neg_df(df a) { return {-a.hi, -a.lo}; }
 BNSN_DI df sub(df a, df b) { return add(a, neg(b)); }
 
 BNSN_DI df mul(df a, df b)
@@ -261,49 +260,6 @@ BNSN_DI df reflect(df f, df y)
         return add(f, mul(y, add(mk(r4a), mul(y2, add(mk(r4b), mul(y2, mk(r4c)))))));
     return add(neg(f),
                add(mk(r5a), mul(y2, add(mk(r5b), mul(y2, add(mk(r5c), mul(y2, mk(r5d))))))));
-}
-
-// F_K(y), K = KLO..KHI, into out[K - KLO]; regimes as fdi_orders (x = -|y|).
-template <int KLO, int KHI>
-BNSN_DI void fdi_df(df y, df* out)
-{
-    const df x = (y.hi > 0.f) ? neg(y) : y;
-    if (!(x.hi <= 0.f)) // NaN argument: 0, as fdi_orders
-    {
-#pragma unroll
-        for (int kk = 0; kk <= KHI - KLO; ++kk)
-            out[kk] = {0.f, 0.f};
-        return;
-    }
-    if (x.hi < -2.f)
-    {
-        constexpr dfc e2(7.38905609893065023);
-        const df ex = exp_df(x);
-        const df t  = mul(ex, mk(e2));
-#define BNSN_DF_LOW(K)                                                                             \
-    if (KLO <= K && K <= KHI)                                                                      \
-        out[K - KLO] = Fdi<K>::low(ex, t);
-        BNSN_DF_LOW(0) BNSN_DF_LOW(1) BNSN_DF_LOW(2) BNSN_DF_LOW(3) BNSN_DF_LOW(4) BNSN_DF_LOW(5)
-#undef BNSN_DF_LOW
-    }
-    else
-    {
-        const df s = {-0.5f * x.hi, -0.5f * x.lo};
-        const df t = add(neg(s), 1.f);
-#define BNSN_DF_MID(K)                                                                             \
-    if (KLO <= K && K <= KHI)                                                                      \
-        out[K - KLO] = Fdi<K>::mid(s, t);
-        BNSN_DF_MID(0) BNSN_DF_MID(1) BNSN_DF_MID(2) BNSN_DF_MID(3) BNSN_DF_MID(4) BNSN_DF_MID(5)
-#undef BNSN_DF_MID
-    }
-    if (y.hi > 0.f)
-    {
-#define BNSN_DF_REF(K)                                                                             \
-    if (KLO <= K && K <= KHI)                                                                      \
-        out[K - KLO] = reflect<K>(out[K - KLO], y);
-        BNSN_DF_REF(0) BNSN_DF_REF(1) BNSN_DF_REF(2) BNSN_DF_REF(3) BNSN_DF_REF(4) BNSN_DF_REF(5)
-#undef BNSN_DF_REF
-    }
 }
 
 // ---------------------------------------------------------------------------

@@ -61,12 +61,6 @@ BNSN_DI void hr98_mixed_part(const fp64::Hr98Point& P, int ch, Hr98Mixed* M)
     M->outer  = 3. * k::BremConst / P.mcorr;
 }
 
-BNSN_DI void hr98_mixed_from(const fp64::Hr98Point& P, Hr98Mixed* M)
-{
-    for (int ch = 0; ch < 4; ++ch)
-        hr98_mixed_part(P, ch, M);
-}
-
 // x^p for x > 0 to about 1 ulp: log2 x = k + log2 m with the binary exponent
 // k exact and m in [1, 2); p log2 x is carried as hi + lo (exact product of p
 // and k), split into an integer n and a fraction f, and x^p = 2^n exp2(f).

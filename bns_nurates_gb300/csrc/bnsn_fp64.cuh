@@ -578,12 +578,6 @@ BNSN_DI double iso_scatt_leg0(double omega, double eta_pp, double eta_nn, bool u
 // e+e- pair kernel (kernel_pair.hpp:16-198)
 // ---------------------------------------------------------------------------
 
-// Fermi integrals F_1..F_5 at eta - y (m) and eta + y (p) of one energy.
-struct PairEnergyFdi
-{
-    double m[5], p[5];
-};
-
 // Spectral energies y = nu / T below this take the reference's rational Fermi
 // integrals throughout.  Psi differences them over 15 y^2 z^2: at y = 0.01 (1
 // MeV at T = 100 MeV) an ulp moved kappa by up to 2e-7, at y = 0.025 by 2e-8, and

@@ -8,30 +8,29 @@
 // waiting on instruction fetch):
 //
 //   point   : per (point, task) (one thread): distribution parameters,
-//             Fermi integrals at +-eta_e, brem and iso constants, written to
+//             Fermi integrals at +-eta_e, brem, beta and iso constants, written to
 //             the header of the point's scratch record.
-//   prelude : per point (one warp): the 2n-energy tables of the double
+//   prelude : per point (four warps): the 2n-energy tables of the double
 //             integral (distribution values, F_k(eta +- w/T)) and the 1-D beta
-//             and iso-scattering integrals; the per-point record is staged in
-//             shared memory and written to the scratch arena.
-//   pair    : per point (one warp): the M(M+1)/2 unordered (w, w') cells of
-//             the pair kernel, one evaluation filling (w, w') and (w', w),
-//             weighted and summed into the number and energy moments.
-//   brem    : the same cells for the bremsstrahlung kernel (HR98, BRT06, GP19).
-//   neps    : per point (one warp): the 2 n^2 (nu, nubar) pairs of the NES/NPS
+//             and iso-scattering integrals.
+//   pair    : per point (64 threads): the M(M+1)/2 unordered (w, w') cells of the
+//             pair kernel, one evaluation filling (w, w') and (w', w) of a kernel
+//             matrix in shared memory, then its rows weighted and summed into the
+//             number and energy moments.
+//   brem    : the same for the bremsstrahlung kernel (HR98, BRT06, GP19).
+//   neps    : per point (two warps): the 2 n^2 (nu, nubar) pairs of the NES/NPS
 //             double integral, both directions from one set of Fermi integrals.
-//   final   : per point (one thread): assembly of the 20 outputs.
+//   final   : per (point, species) (one thread): assembly of the 20 outputs.
 //
-// The reference's 2n x 2n integrand matrices (m1_opacities.hpp:774-1057) are
-// never materialised: every cell is multiplied by its quadrature weight and
-// summed directly; lane sums are combined with warp shuffles.
+// Calls of few points take a point per wider CTA in pair, brem and neps, and run the
+// three in one launch; a point's results do not depend on the form.
 //
-// MIXED = false: every operation in FP64 (the plain path).
-// MIXED = true : the HR98 bremsstrahlung shape of each cell runs in FP32
-// (bnsn_fp32.cuh) and the pair kernel takes one expm1 instead of two
-// exponentials; Fermi-Dirac integrals, the pair Psi polynomial (catastrophic
-// cancellation), distribution reconstruction, detailed balance and the
-// distribution-weighted sums stay FP64.
+// FP64 path: every sum and weight in FP64; exponentials, logarithms, powers and the Fermi
+// integrals in 64-bit fixed point on the integer pipes (bnsn_fx.cuh), to an ulp.
+// Mixed path: FP32 pair (bnsn_pair32.cuh), NES (bnsn_nes32.cuh) and brem kernels
+// (bnsn_fp32.cuh) and occupations with double-float exponent arguments; the weights
+// and sums stay FP64 (brem and NES terms are summed in FP32 and double-float runs), and
+// sums that cancel are recomputed in FP64.
 
 #include <cuda_runtime.h>
 
@@ -56,7 +55,7 @@ struct PointTab
     Hr98Point hr;
     double brt06_pre;
     double eta_pp, eta_nn;
-    double same_cf;
+    double spare;
     double nu[kMaxM];    // energies of the double-integral grid
     double y[kMaxM];     // nu / T
     double g[kMaxM][4];  // TotalNuF at nu per species
@@ -448,8 +447,6 @@ __global__ void __launch_bounds__(kPreWarps * 32, 4)
         __syncthreads();
         const double c0    = S.occ[0].cf;
         const bool same_cf = S.occ[1].cf == c0 && S.occ[2].cf == c0 && S.occ[3].cf == c0;
-        if (threadIdx.x == 0)
-            P->same_cf = same_cf ? 1. : 0.;
         const double eta_pp = P->eta_pp, eta_nn = P->eta_nn;
         // a lane's species is fixed: lane & 1 in the beta units, lane & 3 in the iso units
         double bn_em = 0., bj_em = 0., bn_ab = 0., bj_ab = 0., iso_sum = 0.;
@@ -1514,10 +1511,8 @@ __global__ void __launch_bounds__(kWarps * 32, 3)
 // ---------------------------------------------------------------------------
 struct NepsTab
 {
-    Distr d;
     double fe[2][6];
     double fd0[2];
-    double same_cf;
 };
 
 // The mixed path's NES runs three launches per chunk:
