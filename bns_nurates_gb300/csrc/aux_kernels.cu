@@ -1,7 +1,7 @@
 // Small per-point kernels: distribution parameters from M1 moments and the
 // equilibrium distribution with its M1 densities.  One thread per point;
-// bound by the FP64 pipe (the reconstruction's rational fits, ~80 operations a
-// species) beside 336 bytes a point.  1,000,003 points, both: 2.65 -> 0.73 ms.
+// bound by the FP64 pipe (the reconstruction's rational fit and quotients, ~65 operations
+// a species) beside 336 bytes a point.  1,000,003 points, both: 2.65 -> 0.57 ms.
 
 #include <cuda_runtime.h>
 

@@ -285,6 +285,21 @@ struct Distr
     double w_t[4], temp_t[4], eta_t[4], w_f[4], temp_f[4], c_f[4], beta_f[4];
 };
 
+// Fits of the degeneracy (distribution.hpp:51-175) for y < 0.005, y <= 0.7 and y <
+// 0.79: numerator and denominator, ascending powers of y.  In memory, not as immediates:
+// the lanes of a warp take different rows through one evaluation.
+static __device__ const double kDegeneracyFit[3][14] = {
+    {1.60356108438235e-8, 1120.71610972194, 5750.1878570758, 14364.6331099737, 38865.0149220478,
+     0.19926987701997, 1., 83.0160130941424, 75.7101579899442, -171.874844843596,
+     -99.9009680656931, 38840.0743174942, 1., 1.},
+    {0.000660414331285249, 0.315360380575709, 14.4883415579211, 66.5726772426253,
+     -157.774993512235, 32.5515666786612, 41.3836568203438, 2.64160073447322e-5,
+     0.0113386564109086, 0.483128792035557, 1.94673781342617, -5.35488690539183, 1.8888797407042,
+     1.},
+    {586.406885304906, -1769.59868329086, 1732.89925128741, 1.54082262710661e-6, 1102.91561586553,
+     -5316.18895799799, 3852.81416018959, 143.849128123195, -89.0343496217014, -180.100197053091,
+     -81.2467063138386, 9.42360945627147e-5, 255.936658313629, 1.}};
+
 // distribution.hpp:51-175 and :206-243 for one species; gamma36 is
 // GammaStirling(3.6) (functions.hpp:4460-4471), evaluated on the host.
 BNSN_DI void distr_species(double n_in, double J_in, double chi, double gamma36,
@@ -297,45 +312,25 @@ BNSN_DI void distr_species(double n_in, double J_in, double chi, double gamma36,
     *w_t           = 1.5 * (1. - chi);
     const double q = fx::div(n, J);
     const double y = n * (q * q * q) * (1. / k::FourPiHc3);
-    double eta;
-    if (y < 0.005)
+    // the three fits are quotients of polynomials of degree 6, log, shifted or exp
+    const uint64_t yb = fx::bits_of(y); // y > 0, or NaN
+    const int fit     = yb < fx::bits_of(0.005)                   ? 0
+                        : yb <= fx::bits_of(0.7)                  ? 1
+                        : yb < fx::bits_of(0.7901234567745267)    ? 2
+                                                                  : 3;
+    double eta = 20.;
+    if (fit < 3)
     {
-        const double num =
-            y * (y * (y * (y * (y * (y + 0.19926987701997) + 38865.0149220478) +
-                           14364.6331099737) + 5750.1878570758) + 1120.71610972194) +
-            1.60356108438235e-8;
-        const double den =
-            y * (y * (y * (y * (y * (y + 1.0) + 38840.0743174942) - 99.9009680656931) -
-                      171.874844843596) + 75.7101579899442) + 83.0160130941424;
-        eta = fx::log(fx::div(num, den));
-    }
-    else if (y <= 0.7)
-    {
-        const double num =
-            y * (y * (y * (y * (y * (41.3836568203438 * y + 32.5515666786612) -
-                                157.774993512235) + 66.5726772426253) +
-                      14.4883415579211) + 0.315360380575709) + 0.000660414331285249;
-        const double den =
-            y * (y * (y * (y * (y * (y + 1.8888797407042) - 5.35488690539183) +
-                           1.94673781342617) + 0.483128792035557) +
-                 0.0113386564109086) + 2.64160073447322e-5;
-        eta = fx::div(num, den) - 30.;
-    }
-    else if (y > 0.7 && y < 0.7901234567745267)
-    {
-        const double num =
-            y * (y * (y * (y * (y * (3852.81416018959 * y - 5316.18895799799) +
-                                1102.91561586553) + 1.54082262710661e-6) +
-                      1732.89925128741) - 1769.59868329086) + 586.406885304906;
-        const double den =
-            y * (y * (y * (y * (y * (y + 255.936658313629) + 9.42360945627147e-5) -
-                           81.2467063138386) - 180.100197053091) - 89.0343496217014) +
-            143.849128123195;
-        eta = fx::exp(num / den);
-    }
-    else
-    {
-        eta = 20.;
+        const double* c = kDegeneracyFit[fit];
+        double num = c[6], den = c[13];
+#pragma unroll
+        for (int k = 5; k >= 0; --k)
+        {
+            num = fma(num, y, c[k]);
+            den = fma(den, y, c[7 + k]);
+        }
+        const double r = fx::div(num, den);
+        eta = fit == 0 ? fx::log(r) : fit == 1 ? r - 30. : fx::exp(r);
     }
     eta = (eta < 20.) ? eta : 20.;
     double f23[2];

@@ -19,10 +19,10 @@
 // per CTA.  Arguments come in any order, so a warp usually meets all three regimes:
 // they share the polynomial, and the factors (e^x, x^(j+1)) run on the integer
 // pipes (bnsn_fx.cuh).  The interval and the position in it come from the argument in
-// fixed point.  FP64-pipe bound, ~20 operations per argument against 16 bytes of traffic.  A loop per regime instead (16 + 25 Clenshaw + 12 terms, exp, sqrt and two
+// fixed point.  FP64-pipe bound, ~20 operations per argument against 16 bytes of traffic.
+// A loop per regime instead (16 + 25 Clenshaw + 12 terms, exp, sqrt and two
 // divisions) cost a mixed warp the sum of them: ~150.  4,000,037 arguments uniform in
-// [-50, 150), order 1/2: 978 -> 164 us (265 with
-// the interval in FP64).
+// [-50, 150), order 1/2: 978 -> 164 us (265 with the interval in FP64).
 
 #include <cuda_runtime.h>
 
