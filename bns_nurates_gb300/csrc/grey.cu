@@ -906,7 +906,7 @@ struct PairSmem
 // marked (predo), whose pair part of s2d it replaces; that pass computes its
 // Fermi-integral tables itself.
 // 8,192 points, n = 20: FP64 2.95 -> 1.35 ms, mixed with its redo pass 2.46 ->
-// 1.52 ms; one point, n = 10: 74 -> 29 us.
+// 1.52 ms; one point, n = 10: 74 -> 23 us.
 template <bool MIXED, int NTW>
 __device__ __forceinline__ void pair_points(PairSmem<MIXED>& S, const OpacityLaunch& L,
                                             int64_t p0, int64_t np, double* __restrict__ scratch,
@@ -1870,7 +1870,7 @@ __global__ void __launch_bounds__(kCellWide, 2)
 
 // ---------------------------------------------------------------------------
 // NES/NPS fast pass of the mixed path (InelasticScattKernels and the grey
-// item sums of m1_opacities.hpp:880-905): one warp per point, one item per
+// item sums of m1_opacities.hpp:880-905): two warps per point (or a CTA), one item per
 // lane, the kernel integrals of bnsn_nes32.cuh in FP32.
 // ---------------------------------------------------------------------------
 

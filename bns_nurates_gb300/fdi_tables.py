@@ -42,7 +42,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 HEADER = os.path.join(HERE, "csrc", "bnsn_fdi_tab.h")
 
 # Twice the order of each table slot: the half-integers -9/2 .. 21/2 and the
-# integers 6 .. 10 (0 .. 5 have their own rational approximations).
+# integers 6 .. 10 (0 .. 5 have the Taylor tables of fx_tables.py).
 ORDERS2 = (-9, -7, -5, -3, -1, 1, 3, 5, 7, 9, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21)
 # Every twice-order of the family (functions.hpp:442-4375).
 FAMILY2 = (-9, -7, -5, -3, -1) + tuple(range(0, 22))

@@ -548,8 +548,8 @@ int bnsn_synthetic_points(uint64_t seed, int64_t first, int64_t npts,
  * the FP64-pipe roofline of the opacity kernels.  A diagnostic with no
  * counterpart in the reference. */
 int bnsn_fp64_peak_probe(int64_t iters, double* tflops);
-/* The same for FP32 FMA chains (the pipe of the mixed path's double-float
- * arithmetic).  A diagnostic with no counterpart in the reference. */
+/* The same for FP32 FMA chains (the pipe of the mixed path's pair, NES and
+ * double-float arithmetic).  A diagnostic with no counterpart in the reference. */
 int bnsn_fp32_peak_probe(int64_t iters, double* tflops);
 
 /* Per-phase device timing of the library's own kernels (diagnostics with no
@@ -560,9 +560,9 @@ int bnsn_fp32_peak_probe(int64_t iters, double* tflops);
  * previous bnsn_phase_times call), and clears the record.  Phases:
  * 0 grey prelude, 1 pair cells, 2 brem cells, 3 NES/NPS pairs (mixed path:
  * the fast pass), 4 grey assembly, 5 spectral, 6 distribution/equilibrium,
- * 7 mixed NES double-float pass over flagged points, 8 mixed NES FP64 pass
- * over the points flagged again.  Timing one device at a time is
- * supported. */
+ * 7 list of the points the mixed NES pass flagged, 8 NES FP64 pass over them.
+ * FP64 calls of few points run pair, brem and NES in one launch, counted as
+ * phase 3.  Timing one device at a time is supported. */
 #define BNSN_NUM_PHASES 9
 int bnsn_phase_timing(int enable);
 int bnsn_phase_times(double* ms, int64_t* launches);
