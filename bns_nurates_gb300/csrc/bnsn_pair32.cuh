@@ -112,6 +112,23 @@ __device__ __forceinline__ void hpair(int k, const Cell& c, float x, float r, fl
     }
 }
 
+// The same for lanes in different pieces k: the outer two are one form.
+__device__ __forceinline__ void hpair_any(int k, const Cell& c, float x, float r, float& h0,
+                                          float& h1)
+{
+    const float m  = c.ylz ? c.y : c.z;
+    const float m3 = 4.f * m * m * m;
+    const float hs = m3 * fmaf(r, fmaf(10.f, r, 15.f * m), 6.f * m * m);
+    const float hb = m3 * fmaf(x, fmaf(10.f, x, -5.f * m), m * m);
+    const float v  = k == 0 ? x : r;
+    const float a = k == 0 ? c.z : c.y, b = k == 0 ? c.y : c.z;
+    const float v3 = 4.f * v * v * v;
+    const float o0 = v3 * fmaf(v, v - 5.f * a, 10.f * a * a);
+    const float o1 = v3 * fmaf(v, v - 5.f * b, 10.f * b * b);
+    h0 = k == 1 ? (c.ylz ? hs : hb) : o0;
+    h1 = k == 1 ? (c.ylz ? hb : hs) : o1;
+}
+
 // Edge-zone panel [pu, pv] of piece k (right end Q): 8 Gauss-Legendre nodes
 // with the full occupation factor.
 __device__ __forceinline__ void edge_panel(int k, const Cell& c, dfm::df pu, dfm::df pv,
@@ -138,7 +155,7 @@ __device__ __forceinline__ void edge_panel(int k, const Cell& c, dfm::df pu, dfm
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(corr));
         const float gh = __expf(arg) * rc;
         float h0, h1;
-        hpair(k, c, CM.hi + ht, rq - ht, h0, h1);
+        hpair_any(k, c, CM.hi + ht, rq - ht, h0, h1);
         const float w = kG8w[i >> 1] * gh;
         s0 = fmaf(w, h0, s0);
         s1 = fmaf(w, h1, s1);
@@ -238,28 +255,75 @@ __device__ __forceinline__ void cell_integrals(const Cell& c, double& Q0, double
                 q0 = hw * s0 * __expf(c.k00);
                 q1 = hw * s1 * __expf(c.k00);
             }
-            else
-            {
-                const int npan = max(1, (int)ceilf(len * (1.f / kPanel)));
-                const float h  = len / (float)npan;
-                dfm::df pu     = U;
-#pragma unroll 1
-                for (int pn = 0; pn < npan; ++pn)
-                {
-                    const dfm::df pv = pn == npan - 1 ? V : dfm::add(U, (float)(pn + 1) * h);
-                    float a0, a1;
-                    edge_panel(k, c, pu, pv, Q, a0, a1);
-                    q0 += a0;
-                    q1 += a1;
-                    pu = pv;
-                }
-            }
+            // edge zones follow below
             A0 = dfm::add(A0, q0);
             A1 = dfm::add(A1, q1);
             U = V;
             if (j == 4)
                 break;
         }
+    }
+    // The panels of the edge zones, a lane's own one after the other: with them inside the
+    // loop above, lanes at the same cut had other segments there or fewer panels (2.3
+    // panels issued per one needed at n = 10, now 1.4).  8,192 points, mixed pair phase:
+    // n = 10 0.62 -> 0.57 ms, n = 20 1.52 -> 1.44.
+    int k = -1, j = 5, pn = 0, npan = 0;
+    float q0 = 0.f, q1 = 0.f, h = 0.f;
+    dfm::df Q = dfm::mk(0.f), U = Q, S0 = Q, S1 = Q, pu = Q;
+#pragma unroll 1
+    for (;;)
+    {
+        if (pn == npan)
+        {
+            A0   = dfm::add(A0, q0);
+            A1   = dfm::add(A1, q1);
+            npan = 0;
+#pragma unroll 1
+            while (npan == 0)
+            {
+                if (j > 4)
+                {
+                    if (++k > 2)
+                        break;
+                    U = k == 0 ? dfm::mk(0.f) : (k == 1 ? c.A : c.B);
+                    Q = k == 0 ? c.A : (k == 1 ? c.B : c.S);
+                    j = dsub(Q, U) > 0.f ? 0 : 5;
+                    continue;
+                }
+                const float z = j == 0   ? c.e1
+                                : j == 1 ? fminf(c.e2, c.e3)
+                                : j == 2 ? fmaxf(c.e2, c.e3)
+                                         : c.e4;
+                const bool last = j++ == 4;
+                if (!last && !(z > U.hi && z < Q.hi))
+                    continue;
+                const dfm::df V = last ? Q : dfm::mk(z);
+                const float len = dsub(V, U);
+                const float mid = U.hi + 0.5f * len;
+                const float d1m = mid - c.ETA.hi, d2m = d1m - c.S.hi;
+                if (!(d1m < -kEdge && len >= kRamp) && !(d2m > kEdge && len >= kRamp) &&
+                    !(d1m > kEdge && d2m < -kEdge))
+                {
+                    npan = max(1, (int)ceilf(len * (1.f / kPanel)));
+                    h    = len / (float)npan;
+                    S0 = U;
+                    S1 = V;
+                    pu = U;
+                }
+                U = V;
+            }
+            if (npan == 0)
+                break;
+            pn = 0;
+            q0 = q1 = 0.f;
+        }
+        const dfm::df pv = pn == npan - 1 ? S1 : dfm::add(S0, (float)(pn + 1) * h);
+        float a0, a1;
+        edge_panel(k, c, pu, pv, Q, a0, a1);
+        q0 += a0;
+        q1 += a1;
+        pu = pv;
+        ++pn;
     }
     Q0 = dfm::to_double(A0);
     Q1 = dfm::to_double(A1);
