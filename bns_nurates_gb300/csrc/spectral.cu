@@ -1145,8 +1145,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                 for (int kk = 0; kk < 8; ++kk)
                 {
                     E.nes[kk]  = f * acc[kk];
-                    // -inf: the first check saw the other parts alone and stands
-                    E.bnes[kk] = flags && isinf(E.bnes[kk]) ? -INFINITY : 0.;
+                    E.bnes[kk] = 0.;
                 }
             }
         }
