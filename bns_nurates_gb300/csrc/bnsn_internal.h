@@ -129,11 +129,13 @@ cudaError_t launch_grey_multi(const OpacityLaunch& U, unsigned brem_set, const G
                               unsigned groups, int64_t np_max, cudaStream_t stream, int num_sms);
 // Spectral opacities (phase kernels over chunks of points).  The scratch of
 // one call holds spectral_scratch_bytes(chunk, n_energies) bytes for chunks of
-// spectral_chunk_points(n_energies) points (about kSpecChunkRecords
-// (point, energy) records of 256 bytes).  With aux and scratch1 (a second
-// scratch of the same size) consecutive chunks alternate between stream and
-// aux; stream waits for aux at the end.
-constexpr int64_t kSpecChunkRecords = 131072;
+// spectral_chunk_points(n_energies) points: 2,064 bytes of constants and flags
+// a point and 256 a (point, energy) record, at most kSpecChunkRecords records
+// (from 24 energies on) and kSpecChunkBytes bytes (below, where the points'
+// part is the larger one: 304 MB at one energy without it).  With aux and
+// scratch1 (a second scratch of the same size) consecutive chunks alternate
+// between stream and aux; stream waits for aux at the end.
+constexpr int64_t kSpecChunkRecords = 131072, kSpecChunkBytes = 45000000;
 int64_t spectral_chunk_points(int n_energies);
 size_t spectral_scratch_bytes(int64_t chunk_points, int n_energies);
 cudaError_t launch_spectral(const OpacityLaunch& L, cudaStream_t stream, int num_sms,

@@ -42,6 +42,8 @@
 // 4,096 points x 24 energies: FP64 n = 10 HR98 without NES 9.1 -> 1.3 ms, n = 20 GP19
 // with NES 17.0 -> 3.9 ms; mixed n = 20 GP19 with NES 12.8 -> 5.5 ms.
 
+#include <algorithm>
+
 #include <cuda_runtime.h>
 
 #include "bnsn_df.cuh"
@@ -190,7 +192,7 @@ struct SpecPoint
     int twin;     // heavy-lepton neutrinos evolved as one species
     int same_cf, env;
 };
-static_assert(sizeof(SpecPoint) % sizeof(double) == 0, "SpecPoint must be double words");
+static_assert(sizeof(SpecPoint) == 2048, "the documented scratch of a point");
 
 // n doubles of a record into shared memory, by threads t, t + nt, ...
 template <class T>
@@ -1572,7 +1574,8 @@ cudaError_t launch_assemble(const OpacityLaunch& L, int64_t p0, int64_t np, cons
 int64_t spectral_chunk_points(int n_energies)
 {
     const int64_t ne = n_energies < 1 ? 1 : n_energies;
-    const int64_t c  = kSpecChunkRecords / ne;
+    const int64_t c  = std::min(kSpecChunkRecords / ne,
+                                kSpecChunkBytes / (int64_t)spectral_scratch_bytes(1, (int)ne));
     return c < 32 ? 32 : c;
 }
 

@@ -196,8 +196,9 @@ typedef struct SpectralOpacities
  * per device, created on the first call), allocating and freeing it in order
  * on `stream`, so calls on different streams never share scratch.  The pool
  * keeps its memory for later calls.  bnsn_spectral_opacities takes its
- * scratch (256 B per (point, energy) record, about 131,072 records per chunk,
- * two chunks for larger batches) from the same pool; bnsn_m1_opacities_noalloc
+ * scratch (2,064 B per point and 256 B per (point, energy) record, at most
+ * 131,072 records and 45 MB per chunk, two chunks for larger batches) from the
+ * same pool; bnsn_m1_opacities_noalloc
  * uses a static device array; the host-buffer calls copy through a
  * library-owned staging buffer.  The other batched calls allocate nothing.
  * ====================================================================== */
