@@ -457,11 +457,12 @@ struct BetaPoint
     int use_WM_ab, use_decay;
 };
 
-// x / T from the stored reciprocal, with one correction of the quotient.
+// x / T from the stored reciprocal, with one correction of the quotient; where the
+// quotient, the reciprocal or T is infinite, the correction alone is NaN.
 BNSN_DI double over_T(const BetaPoint& b, double x)
 {
-    const double q = x * b.iT;
-    return fma(fma(-b.T, q, x), b.iT, q);
+    const double q = x * b.iT, c = fma(fma(-b.T, q, x), b.iT, q);
+    return ((uint32_t)__double2hiint(c) & 0x7fffffffu) >= 0x7ff00000u ? q : c;
 }
 
 BNSN_DI BetaPoint beta_point(double nb, double T, double yp, double yn,
