@@ -85,10 +85,16 @@ struct Occ64
     double rt, eta, rf, wt, kf, cf;
 };
 
+// The degeneracy for it; the reference's argument (omega - T eta) / T is NaN at T = inf.
+__device__ __forceinline__ double occ64_eta(const Distr& d, int s)
+{
+    return isinf(d.temp_t[s]) ? __longlong_as_double(0x7ff8000000000000LL) : d.eta_t[s];
+}
+
 __device__ __forceinline__ void occ64_from(const Distr& d, int s, double u, Occ64* o)
 {
     o->rt  = u / d.temp_t[s];
-    o->eta = d.eta_t[s];
+    o->eta = occ64_eta(d, s);
     o->rf  = u / d.temp_f[s];
     o->wt  = d.w_t[s];
     o->cf  = d.c_f[s];

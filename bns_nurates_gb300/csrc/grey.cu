@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kPreWarps * 32, 4)
         if (threadIdx.x >= 96 && threadIdx.x < 100)
         {
             const int s  = threadIdx.x - 96;
-            S.occ[s].eta = P->d.eta_t[s];
+            S.occ[s].eta = occ64_eta(P->d, s);
             S.occ[s].wt  = P->d.w_t[s];
             S.occ[s].cf  = P->d.c_f[s];
         }

@@ -1,5 +1,5 @@
 """States at the ends of the number range against the CPU oracle: temperatures of 0 and
-next to it, infinite chemical potentials.  What the reference makes
+next to it, infinite chemical potentials and energy densities.  What the reference makes
 of them is an accident of its clamped exponentials, but it is finite in many outputs, and
 the FP64 path follows it.  Tolerance: the plain path's 1e-12.
 """
@@ -51,3 +51,11 @@ def test_grey_beta_rates(cuda, port, row, values):
     eos, m1 = states(row, values)
     args = (m1, (1, 0, 0, 0, 0), DEFAULT, 6)
     assert_close(gpu_grey(cuda, eos, *args), oracle_grey(port, eos, *args), what="beta rates")
+
+
+@pytest.mark.parametrize("flags", [(1, 0, 0, 0, 0), (0, 0, 1, 0, 0), (0, 0, 0, 1, 0)])
+def test_grey_infinite_energy_density(cuda, port, flags):
+    eos, m1 = bn.synthetic_points(5, 8)
+    m1[4:8] = np.inf
+    args = (m1, flags, DEFAULT, 6)
+    assert_close(gpu_grey(cuda, eos, *args), oracle_grey(port, eos, *args), what="J = inf")
