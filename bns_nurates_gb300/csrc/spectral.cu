@@ -625,7 +625,13 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                     {
                         const double x = S.y[c] + S.z[a], Kp = fma(c0, K0[a], c1 * K1[a]);
                         const double wn = L.B1[a], nb2 = S.nb[a] * S.nb[a];
-                        const double g = ab ? v[a] / (wn * nb2) : nbb ? 1. : v[a] / (S.dnz[a] * (wn * nb2));
+                        // g, or 1 - g from the stored product unless that underflows (T < 1e-10)
+                        const double wnb = wn * nb2, den = ab ? wnb : S.dnz[a] * wnb;
+                        const double gp  = wnb > 0. ? S.vA[s][a] / wnb : 0.;
+                        const double g   = ab          ? gp
+                                           : nbb       ? 1.
+                                           : den > 1e-290 ? v[a] / den
+                                                          : 1. - gp;
                         const double K = x > k::ExpUpp ? pb64_far(Kp, Kb[a], T, x, ab)
                                                        : (Kp + Kb[a]) * (ab ? 1. : safe_exp(-x));
                         acc += wn * (nb2 * (K * g));

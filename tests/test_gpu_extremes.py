@@ -1,6 +1,6 @@
 """States at the ends of the number range against the CPU oracle: temperatures of 0 and
-next to it, infinite chemical potentials and energy densities.  What the reference makes
-of them is an accident of its clamped exponentials, but it is finite in many outputs, and
+next to it, infinite chemical potentials and energy densities.  What the reference makes of
+them is an accident of its clamped exponentials, but it is finite in many outputs, and
 the FP64 path follows it.  Tolerance: the plain path's 1e-12.
 """
 
@@ -59,3 +59,12 @@ def test_grey_infinite_energy_density(cuda, port, flags):
     m1[4:8] = np.inf
     args = (m1, flags, DEFAULT, 6)
     assert_close(gpu_grey(cuda, eos, *args), oracle_grey(port, eos, *args), what="J = inf")
+
+
+@pytest.mark.parametrize("nq", [6, 20])
+@pytest.mark.parametrize("flags,brem", [((0, 1, 0, 0, 0), 0), ((0, 0, 1, 0, 0), 2)])
+def test_spectral_pair_and_brem_next_to_zero_temperature(cuda, port, flags, brem, nq):
+    """Energies far above e^700 T, nodes whose weight underflows."""
+    eos, m1 = states(TEMP, [1e-310, 1e-200, 1e-100, 1e-30])
+    got, want = spectral_both(cuda, port, eos, m1, flags, DEFAULT[:5] + (brem,) + DEFAULT[6:], nq=nq)
+    assert_close(got, want, what="T next to 0")
