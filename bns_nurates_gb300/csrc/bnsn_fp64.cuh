@@ -903,7 +903,9 @@ BNSN_DI double brt06_point(double nb, double T, double yn, double yp)
 }
 
 // K_1(x) e^{x} / x, with the reference's clamp of e^{x} at x = 700 (its exp(-x)
-// keeps falling): the polynomial fits of bessi1 / bessk1.
+// keeps falling): the polynomial fits of bessi1 / bessk1.  The reference's
+// product underflows to 0 from x = 745, and from x = 500 at low densities (its prefactor
+// multiplies K_1 first); this one stays finite.
 BNSN_DI double brt06_shape(double x)
 {
     if (x <= 2.)
@@ -915,12 +917,20 @@ BNSN_DI double brt06_shape(double x)
     return x > k::ExpUpp ? r * fx::exp(k::ExpUpp - x) : r;
 }
 
+// The emission kernel, e^{-2x} of the absorption kernel.  The reference multiplies by e^{-x}
+// twice, so e^{-2x} is not clamped at 2x = 700.
+BNSN_DI double brt06_emission(double ab, double x)
+{
+    const double ex = fx::exp(x > 350. ? -x : -2. * x);
+    return x > 350. ? ab * ex * ex : ab * ex;
+}
+
 BNSN_DI void brt06_kernel(double pre, double T, double omega, double omega_p,
                           double* em, double* ab)
 {
     const double x = 0.5 * (omega + omega_p) / T;
     *ab            = pre * brt06_shape(x);
-    *em            = *ab * safe_exp(-2. * x);
+    *em            = brt06_emission(*ab, x);
 }
 
 // ---------------------------------------------------------------------------

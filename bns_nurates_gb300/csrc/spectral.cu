@@ -403,12 +403,13 @@ struct Pb64Smem
 // A cell with x = (nu + nubar) / T > 700 from the pair kernel's sum of Psi and the brem
 // absorption kernel.  There the reference clamps e^x at e^700, its emission kernel
 // rounds in the denormal range and the pair absorption kernel is e^700 times that,
-// so both are formed in its order.
+// so both are formed in its order.  BRT06's emission kernel is not clamped.
+template <int IMPL>
 __device__ __noinline__ double pb64_far(double psi, double Kbrem, double T, double x, int ab)
 {
     const double ex = safe_exp(x);
     const double em = 0.5 * (psi * (k::PairPhi * (T * T) / (1. - ex)));
-    return ab ? ex * em + Kbrem : em + Kbrem * safe_exp(-x);
+    return ab ? ex * em + Kbrem : em + (IMPL == 1 ? brt06_emission(Kbrem, 0.5 * x) : Kbrem * safe_exp(-x));
 }
 
 template <int IMPL>
@@ -632,7 +633,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                                            : nbb       ? 1.
                                            : den > 1e-290 ? v[a] / den
                                                           : 1. - gp;
-                        const double K = x > k::ExpUpp ? pb64_far(Kp, Kb[a], T, x, ab)
+                        const double K = x > k::ExpUpp ? pb64_far<IMPL>(Kp, Kb[a], T, x, ab)
                                                        : (Kp + Kb[a]) * (ab ? 1. : safe_exp(-x));
                         acc += wn * (nb2 * (K * g));
                     }

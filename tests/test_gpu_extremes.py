@@ -68,3 +68,15 @@ def test_spectral_pair_and_brem_next_to_zero_temperature(cuda, port, flags, brem
     eos, m1 = states(TEMP, [1e-310, 1e-200, 1e-100, 1e-30])
     got, want = spectral_both(cuda, port, eos, m1, flags, DEFAULT[:5] + (brem,) + DEFAULT[6:], nq=nq)
     assert_close(got, want, what="T next to 0")
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_spectral_brt06_emission_far_above_the_temperature(cuda, port, precision):
+    """K_1(x/2) e^{-x/2} at x = (nu + nubar) / T beyond 700, where a clamped e^{-x} would stay at
+    e^-700.  Densities far above nuclear ones lift the difference over the smallest doubles."""
+    eos, m1 = bn.synthetic_points(5, 4)
+    eos[0], eos[TEMP] = 1e39, [1., 1.4, 1.2, 0.7]
+    got, want = spectral_both(cuda, port, eos, m1, (0, 0, 1, 0, 0),
+                              DEFAULT[:5] + (1,) + DEFAULT[6:], precision, 0,
+                              np.array([400., 900., 960., 1100., 1400.]))
+    assert_close(got[:4], want[:4], what="BRT06 emission")
