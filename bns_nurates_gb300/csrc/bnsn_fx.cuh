@@ -414,5 +414,24 @@ BNSN_FX_HD void fd_orders(double y, double* out)
 #undef BNSN_FX_ORDER
 }
 
+// The interval of x in [-4, 100) among those of the Fermi-Dirac family (fdi.cu): 64 of width
+// 11/16 below 40, then 6 of width 10; the position in it, in [-1, 1), is returned.
+BNSN_FX_HD double fd_interval(double x, int* interval)
+{
+    const uint64_t bits = bits_of(x), mag = bits & 0x7fffffffffffffffull;
+    // y = x + 4 in 2^-56 (exact for |x| >= 1/8), its interval in sixteenths
+    const int sh     = 7 + 1023 - (int)(mag >> 52);
+    const uint64_t A = sh > 63 ? 0ull : ((mag << 11) | 0x8000000000000000ull) >> sh;
+    const int64_t Y  = (4ll << 56) + ((int64_t)bits < 0 ? -(int64_t)A : (int64_t)A);
+    const int y16    = (int)(Y >> 52);
+    const bool wide  = y16 >= 704;
+    const int i      = wide ? (y16 - 704) / 160 : y16 / 11;
+    const int w = wide ? 160 : 11, base = wide ? 704 + i * 160 : i * 11;
+    *interval = i + (wide ? 64 : 0);
+    // 2 (y - start) - width over the width
+    const int64_t r = 2 * (Y - ((int64_t)base << 52)) - ((int64_t)w << 52);
+    return (double)r * (wide ? 0x1p-52 / 160. : 0x1p-52 / 11.);
+}
+
 } // namespace fx
 } // namespace bnsn

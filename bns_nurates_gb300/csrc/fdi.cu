@@ -78,8 +78,8 @@ __device__ __forceinline__ double fdi_table(const FdiShared& S, int h, int64_t P
 {
     using namespace fdit;
     static_assert(kXlo == -4. && kXmid == 40. && kXhi == 100. && kWidth == 11. / 16. &&
-                      kWide == 10.,
-                  "the interval arithmetic below");
+                      kWide == 10. && kNarrow == 64,
+                  "fx::fd_interval");
     const uint64_t bits = fx::bits_of(x), mag = bits & 0x7fffffffffffffffull;
     const bool neg      = (int64_t)bits < 0;
     double v, f = 1.;
@@ -107,18 +107,8 @@ __device__ __forceinline__ double fdi_table(const FdiShared& S, int h, int64_t P
     }
     else
     {
-        // y = x + 4 in 2^-56 (exact for |x| >= 1/8), its interval in sixteenths
-        const int sh     = 7 + 1023 - (int)(mag >> 52);
-        const uint64_t A = sh > 63 ? 0ull : ((mag << 11) | 0x8000000000000000ull) >> sh;
-        const int64_t Y  = (4ll << 56) + (neg ? -(int64_t)A : (int64_t)A);
-        const int y16    = (int)(Y >> 52);
-        const bool wide  = y16 >= 704;
-        const int i      = wide ? (y16 - 704) / 160 : y16 / 11;
-        const int w = wide ? 160 : 11, base = wide ? 704 + i * 160 : i * 11;
-        // 2 (y - start) - width over the width
-        const int64_t r = 2 * (Y - ((int64_t)base << 52)) - ((int64_t)w << 52);
-        v   = (double)r * (wide ? 0x1p-52 / 160. : 0x1p-52 / 11.);
-        row = 1 + i + (wide ? kNarrow : 0);
+        v = fx::fd_interval(x, &row);
+        ++row;
     }
     double p = S.c[kDegree][row];
 #pragma unroll

@@ -224,7 +224,9 @@ def pow_half(x, h):
 
 
 def evaluate(k2, x, tabs):
-    """F_{k2/2}(x) for a table order, in FP64 with the kernel's operation order."""
+    """F_{k2/2}(x) for a table order, in FP64 from the kernel's tables.  The kernel finds
+    the interval and the position in it in fixed point (fd_interval of bnsn_fx.cuh)
+    and takes its exponentials and powers from there; here they are numpy's."""
     slot = ORDERS2.index(k2)
     x = np.asarray(x, dtype=np.float64)
     j1 = 0.5 * k2 + 1.0
