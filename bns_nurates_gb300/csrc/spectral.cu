@@ -70,6 +70,7 @@ constexpr double kSpecCancelNes  = 2.0;     // same for the NES/NPS terms
 constexpr double kSpecNesMinW    = 0.05;    // NES in FP64 below nu/T = 0.05
 constexpr double kSpecNesDfW     = 0.2;    // NES brackets in double-float below nu/T = 0.2
 constexpr double kSpecFloor      = 7.2e-34; // 1e9 x the denormal floor of a sum
+constexpr double kKeepPb         = -1.;     // bpb: an output the last FP64 pass leaves as it is
 
 // Per (point, energy) record of the chunk scratch.
 struct EnergyRec
@@ -641,6 +642,8 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                     for (int a = 0; a < M; ++a)
                         acc = fma(fma(c0, K0[a], fma(c1, K1[a], Kb[a])), v[a], acc);
                 EnergyRec& E       = rec[q * ne + S.eid[c]];
+                if (flags && E.bpb[4 * ab + s] == kKeepPb)
+                    continue;
                 E.pb[4 * ab + s]  = ab || S.far[c] ? acc : acc * S.dny[c];
                 E.bpb[4 * ab + s] = 0.;
             }
@@ -1338,7 +1341,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 template <int MODE>
 __global__ void __launch_bounds__(kWarps * 32)
     spec_assemble_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
-                         const SpecPoint* __restrict__ pts, const EnergyRec* __restrict__ rec,
+                         const SpecPoint* __restrict__ pts, EnergyRec* __restrict__ rec,
                          uint64_t* __restrict__ fl_pb, uint64_t* __restrict__ fl_nes)
 {
     constexpr bool GUARD = MODE == kSpecMixed || MODE == kSpecRedo;
@@ -1394,6 +1397,7 @@ __global__ void __launch_bounds__(kWarps * 32)
                 if (GUARD)
                 {
                     // FP32 error bounds against each output's total
+                    uint32_t pb_of = 0u; // outputs whose pair + brem part is flagged
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk)
                     {
@@ -1417,10 +1421,16 @@ __global__ void __launch_bounds__(kWarps * 32)
                                 xp = hp;
                                 xn = hn;
                             }
-                            fpb  = fpb || xp;
+                            pb_of |= (uint32_t)xp << kk;
                             fnes = fnes || xn;
                         }
                     }
+                    fpb = pb_of != 0u;
+                    // the second check keeps the outputs that passed
+                    if (MODE == kSpecRedo && fpb)
+                        for (int kk = 0; kk < 8; ++kk)
+                            if (!((pb_of >> kk) & 1u))
+                                rec[q * ne + e].bpb[kk] = kKeepPb;
                 }
                 if (!fpb && !fnes)
                 {
@@ -1562,7 +1572,7 @@ cudaError_t launch_nes64(const OpacityLaunch& L, int64_t p0, int64_t np, const S
 
 template <int MODE>
 cudaError_t launch_assemble(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
-                            const EnergyRec* rec, uint64_t* fl_pb, uint64_t* fl_nes,
+                            EnergyRec* rec, uint64_t* fl_pb, uint64_t* fl_nes,
                             cudaStream_t st, int sms)
 {
     static bool attr = false;
