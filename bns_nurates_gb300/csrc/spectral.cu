@@ -651,10 +651,19 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
     }
 }
 
-// Pair + brem of the mixed path.
+// Launches of fewer points than this many per SM share a point's energies between warps. A
+// pair cell is a chain of ~10 us, and a warp's slowest lane sets its time: 16 points x 40
+// energies, pair alone, n = 20: a warp per point 1.57 ms, shared 0.6; 16 x 24 with HR98
+// 0.81 -> 0.44. 304 points x 24, n = 10: 0.48 -> 0.41, 608: no difference. With 8 per SM
+// instead of 4, 456 points x 40 with HR98 at n = 20 took 2.38 ms instead of 2.22 (the node tables
+// are made by every warp).
+constexpr int64_t kPbWarpsPerSm = 4;
+
+// Pair + brem of the mixed path: a warp takes a point, or (parts > 1) every parts-th
+// energy of one; an energy's sums do not depend on it.
 __global__ void __launch_bounds__(kWarps * 32)
     spec_pb_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
-                   const SpecPoint* __restrict__ pts, EnergyRec* __restrict__ rec, int G)
+                   const SpecPoint* __restrict__ pts, EnergyRec* __restrict__ rec, int G, int parts)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     PbShared& S         = *reinterpret_cast<PbShared*>(s_raw);
@@ -687,8 +696,10 @@ __global__ void __launch_bounds__(kWarps * 32)
     const int64_t nwarp = (int64_t)gridDim.x * kWarps;
     const int grp = lane % G, per_round = 32 / G;
 
-    for (int64_t q = (int64_t)blockIdx.x * kWarps + wid; q < np; q += nwarp)
+    for (int64_t t = (int64_t)blockIdx.x * kWarps + wid; t < np * parts; t += nwarp)
     {
+        const int64_t q     = t / parts;
+        const int part      = (int)(t - q * parts);
         const int64_t p     = p0 + q;
         const double T = L.eos[1][p], eta_e = L.eos[7][p] / T;
         EnergyRec* R       = rec + q * ne;
@@ -783,10 +794,13 @@ __global__ void __launch_bounds__(kWarps * 32)
                 }
             }
             __syncwarp();
-            for (int r0 = 0; r0 < nec; r0 += per_round)
+            // the part's energies: e = part, part + parts, ...
+            const int first = (part + parts - e0 % parts) % parts;
+            const int own   = first < nec ? (nec - first + parts - 1) / parts : 0;
+            for (int r0 = 0; r0 < own; r0 += per_round)
             {
-                const bool act  = r0 + lane / G < nec;
-                const int c     = act ? r0 + lane / G : 0;
+                const bool act  = r0 + lane / G < own;
+                const int c     = act ? (r0 + lane / G) * parts + first : 0;
                 const double nu = act ? L.energies[e0 + c] : 1.;
                 const double w  = nu / T;
                 double acc[8];
@@ -1515,12 +1529,14 @@ cudaError_t launch_pb_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, cons
 {
     static bool attr  = false;
     const size_t smem = sizeof(PbShared);
+    const int parts   = (int)std::max<int64_t>(
+        1, std::min<int64_t>(sms * kPbWarpsPerSm / np, L.n_energies));
     int grid          = 0;
-    cudaError_t err   = grid_of(spec_pb_kernel, smem, &attr, sms, np, &grid);
+    cudaError_t err   = grid_of(spec_pb_kernel, smem, &attr, sms, np * parts, &grid);
     if (err != cudaSuccess || grid == 0)
         return err;
     phase_mark(kPhSpectral, 0, st);
-    spec_pb_kernel<<<grid, kWarps * 32, smem, st>>>(L, p0, np, pts, rec, G);
+    spec_pb_kernel<<<grid, kWarps * 32, smem, st>>>(L, p0, np, pts, rec, G, parts);
     phase_mark(kPhSpectral, 1, st);
     return cudaGetLastError();
 }
