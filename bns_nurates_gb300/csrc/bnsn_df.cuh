@@ -10,7 +10,7 @@
 // the compiler keeps every addition below in IEEE order (FMA contraction only
 // merges a product with an addition, and the sums below contain no products).
 //
-// df_exp uses Cody-Waite range reduction with a three-part ln 2, a Taylor
+// exp_df uses Cody-Waite range reduction with a three-part ln 2, a Taylor
 // polynomial for e^r - 1 on |r| <= ln2/32, and four exact-ish squarings of
 // (1 + q) carried as q -> q (2 + q).
 //
@@ -144,17 +144,6 @@ BNSN_DI df fma_df(df t, df p, df c)
 // a * 2^k for integer k (exact unless the result leaves the normal range).
 BNSN_DI df ldexp_df(df a, int k) { return {ldexpf(a.hi, k), ldexpf(a.lo, k)}; }
 
-// Horner evaluation with df coefficients: c[0] + t c[1] + ... + t^{N-1} c[N-1].
-template <int N>
-BNSN_DI df horner(const dfc (&c)[N], df t)
-{
-    df p = mk(c[N - 1]);
-#pragma unroll
-    for (int i = N - 2; i >= 0; --i)
-        p = add(mk(c[i]), mul(t, p));
-    return p;
-}
-
 // e^x.  Results below the FP32 normal range lose precision (and are 0 for
 // x < -104); callers only use them as negligible contributions.
 BNSN_DI df exp_df(df x)
@@ -190,54 +179,9 @@ BNSN_DI df exp_df(df x)
 }
 
 // ---------------------------------------------------------------------------
-// Fermi-Dirac integrals F_K, K = KLO..KHI, in df (the forms of fdi_orders).
+// Fermi-Dirac integrals F_1..F_5 in df.
 // ---------------------------------------------------------------------------
-__device__ constexpr dfc kAN0[5] = {22696.2126132366633, 5222.0667923565138, 357.623326425354522, 6.9167792879948140, 0.00200096064827815813};
-__device__ constexpr dfc kAD0[5] = {45392.4252264733267, 14539.5980679273792, 1611.36476693109675, 71.072178562726798, 1.0};
-__device__ constexpr dfc kBN0[9] = {159.601717762460980, 23.7193942338278703, 0.377783268730614356, 10.5181677709577503, 3.78181326142271599, -0.441998676614933572, -0.450072959113928254, -0.0734798777056723512, 0.000915454570009894267};
-__device__ constexpr dfc kBD0[8] = {284.26032127745967, 315.2592651624449, 310.2713981221035, 206.21640678892182, 96.77898293084927, 35.456591489081173, 8.1762315442738975, 1.0};
-__device__ constexpr dfc kAN1[5] = {22189.1070807945062, 4915.92700908746777, 322.901386168881348, 5.9897442965804548, 0.00397641173774375092};
-__device__ constexpr dfc kAD1[5] = {88756.428323178025, 25002.3197546553836, 2389.06277237306633, 88.376214553692756, 1.0};
-__device__ constexpr dfc kBN1[9] = {145.488167182330098, 251.392824471576922, 56.6537141912783024, 17.9918985363509694, 20.1369115558099802, 7.09659390228556164, 0.199701180197912643, -0.403173132925886253, -0.0792966701498222697};
-__device__ constexpr dfc kBD1[9] = {606.0757707716040, 374.1806357435014, 252.1367051536344, 27.2746245830016, -61.57766112137513, -53.72117554363975, -25.678454878692950, -7.1995819520154718, -1.0};
-__device__ constexpr dfc kAN2[4] = {1914.06748184935743, 273.085756700981399, 8.5861610217850095, 0.0161890243763741414};
-__device__ constexpr dfc kAD2[4] = {7656.2699273974454, 1399.35442210906621, 72.929152915475392, 1.0};
-__device__ constexpr dfc kBN2[9] = {2711.49678259128843, 1299.85460914884154, 222.606134197895041, 172.881855215582924, 112.951038040682055, 24.0376482128898634, -2.68393549333878715, -2.14077421411719935, -0.326188299771397236};
-__device__ constexpr dfc kBD2[9] = {2517.1726659917047, 3038.7689794575778, 2541.7823512372631, 1428.0589853413436, 531.62378035996132, 122.54595216479181, 8.395768655115050, -3.9142702096919080, -1.0};
-__device__ constexpr dfc kAN3[4] = {5121.6401850302408, 664.28706260743472, 19.0856927562699544, 0.0410982603688952131};
-__device__ constexpr dfc kAD3[4] = {13657.7071600806539, 2136.54222460571183, 92.376788603062645, 1.0};
-__device__ constexpr dfc kBN3[8] = {7881.24597452900838, 4323.07526636309661, 1260.13125873282465, 653.359212389160499, 354.630774329461644, 113.373708671587772, 19.9559488532742796, 1.59407954898394322};
-__device__ constexpr dfc kBD3[8] = {2570.7250703533430, 2972.7443644211129, 2393.9995533270879, 1259.0724833462608, 459.86413596901097, 112.60906419590854, 16.468882811659000, 1.0};
-__device__ constexpr dfc kAN4[4] = {18247.2542465629199, 2120.56302902849207, 54.659507299984584, 0.121876197098273914};
-__device__ constexpr dfc kAD4[4] = {24329.6723287505678, 3261.01909656925521, 117.071576489684022, 1.0};
-__device__ constexpr dfc kBN4[8] = {33093.9102025608137, 19031.4783357798975, 5431.08357152245897, 2393.94262931609398, 1268.40017257978070, 418.662172475927160, 77.4108960876508190, 6.67374311450268357};
-__device__ constexpr dfc kBD4[8] = {2645.4885670047153, 3236.2237702166948, 2500.5977847175497, 1278.0109577275445, 448.99020896813485, 105.86020755838874, 15.216887271751039, 1.0};
-__device__ constexpr dfc kAN5[4] = {81190.938912603315, 8368.4990332049831, 190.753830813273698, 0.413800735538960261};
-__device__ constexpr dfc kAD5[4] = {43301.8340867217726, 4977.68099709243407, 148.484432990224213, 1.0};
-__device__ constexpr dfc kBN5[8] = {159651.547840031111, 96307.2005742063042, 26923.5693307648389, 9274.54751848368696, 4445.76333033698006, 1461.45267097859337, 272.164427980501432, 23.6526046298891619};
-__device__ constexpr dfc kBD5[8] = {2522.7839609396783, 3244.5527999477567, 2403.0532924519756, 1176.7202478443275, 397.7596246691212, 91.84661231161838, 13.491911254479298, 1.0};
-
-template <int K> struct Fdi;
-
-#define BNSN_DF_FDI(K, A0)                                                                         \
-    template <> struct Fdi<K>                                                                      \
-    {                                                                                              \
-        static constexpr float a0 = A0;                                                            \
-        BNSN_DI static df low(df ex, df t)                                                         \
-        {                                                                                          \
-            return mul(ex, sub(mk(a0), mul(ex, div(horner(kAN##K, t), horner(kAD##K, t)))));       \
-        }                                                                                          \
-        BNSN_DI static df mid(df s, df t) { return div(horner(kBN##K, t), horner(kBD##K, s)); }   \
-    };
-BNSN_DF_FDI(0, 1.f)
-BNSN_DF_FDI(1, 1.f)
-BNSN_DF_FDI(2, 2.f)
-BNSN_DF_FDI(3, 6.f)
-BNSN_DF_FDI(4, 24.f)
-BNSN_DF_FDI(5, 120.f)
-#undef BNSN_DF_FDI
-
-// Reflection for y > 0 (the polynomials of FdiCoef<K>::reflect).
+// Reflection for y > 0 (the polynomials of FdiCoef<K>::reflect), K = 1..5.
 template <int K>
 BNSN_DI df reflect(df f, df y)
 {
@@ -247,8 +191,6 @@ BNSN_DI df reflect(df f, df y)
     constexpr dfc r4a(45.4575758158678040), r4b(6.57973626739290575), r4c(0.2);
     constexpr dfc r5a(236.532261911384425), r5b(113.643939539669510), r5c(8.22467033424113218),
         r5d(0.166666666666666667);
-    if (K == 0)
-        return add(f, y);
     const df y2 = mul(y, y);
     if (K == 1)
         return add(neg(f), add(mk(r1a), mul(y2, 0.5f)));

@@ -110,10 +110,6 @@ BNSN_DI double horner(const double (&c)[N], double t)
 
 // Coefficient tables (functions.hpp:1550-2838), numerator/denominator of
 // the x < -2 (an, ad) and -2 <= x <= 0 (bn, bd) rational forms.
-__device__ constexpr double kAN0[5] = {22696.2126132366633, 5222.0667923565138, 357.623326425354522, 6.9167792879948140, 0.00200096064827815813};
-__device__ constexpr double kAD0[5] = {45392.4252264733267, 14539.5980679273792, 1611.36476693109675, 71.072178562726798, 1.0};
-__device__ constexpr double kBN0[9] = {159.601717762460980, 23.7193942338278703, 0.377783268730614356, 10.5181677709577503, 3.78181326142271599, -0.441998676614933572, -0.450072959113928254, -0.0734798777056723512, 0.000915454570009894267};
-__device__ constexpr double kBD0[8] = {284.26032127745967, 315.2592651624449, 310.2713981221035, 206.21640678892182, 96.77898293084927, 35.456591489081173, 8.1762315442738975, 1.0};
 __device__ constexpr double kAN1[5] = {22189.1070807945062, 4915.92700908746777, 322.901386168881348, 5.9897442965804548, 0.00397641173774375092};
 __device__ constexpr double kAD1[5] = {88756.428323178025, 25002.3197546553836, 2389.06277237306633, 88.376214553692756, 1.0};
 __device__ constexpr double kBN1[9] = {145.488167182330098, 251.392824471576922, 56.6537141912783024, 17.9918985363509694, 20.1369115558099802, 7.09659390228556164, 0.199701180197912643, -0.403173132925886253, -0.0792966701498222697};
@@ -136,16 +132,6 @@ __device__ constexpr double kBN5[8] = {159651.547840031111, 96307.2005742063042,
 __device__ constexpr double kBD5[8] = {2522.7839609396783, 3244.5527999477567, 2403.0532924519756, 1176.7202478443275, 397.7596246691212, 91.84661231161838, 13.491911254479298, 1.0};
 
 template <int K> struct FdiCoef;
-
-template <> struct FdiCoef<0>
-{
-    static constexpr double a0 = 1.;
-    BNSN_DI static const double (&an())[5] { return kAN0; }
-    BNSN_DI static const double (&ad())[5] { return kAD0; }
-    BNSN_DI static const double (&bn())[9] { return kBN0; }
-    BNSN_DI static const double (&bd())[8] { return kBD0; }
-    BNSN_DI static double reflect(double fd, double y) { return fd + y; }
-};
 
 template <> struct FdiCoef<1>
 {
@@ -221,9 +207,9 @@ template <> struct FdiCoef<5>
 // The same integrals from the reference's own approximations in its operation
 // order (Fukushima's piecewise minimax rational forms in x = -|y|: x < -2 a
 // series in e^x, -2 <= x <= 0 rational in s = -x/2, the reflection polynomial
-// for y > 0).  Six times the cost of fdi_orders, with which it agrees to an
-// ulp; for the cells of the pair kernel whose cancellation magnifies an ulp of
-// a Fermi integral by 10^8 and more (pair_low_energy).
+// for y > 0), 1 <= KLO.  150 FP64 operations for F_1..F_5 against 9 of fdi_orders, with
+// which it agrees to an ulp; for the cells of the pair kernel whose cancellation magnifies an
+// ulp of a Fermi integral by 10^8 and more (kPairLowEnergy).
 template <int KLO, int KHI>
 __device__ __noinline__ void fdi_rational(double y, double* out)
 {
@@ -236,8 +222,7 @@ __device__ __noinline__ void fdi_rational(double y, double* out)
     if (KLO <= K && K <= KHI)                                                    \
         out[K - KLO] = ex * (FdiCoef<K>::a0 -                                    \
                              ex * horner(FdiCoef<K>::an(), t) / horner(FdiCoef<K>::ad(), t));
-        BNSN_FDI_LOW(0) BNSN_FDI_LOW(1) BNSN_FDI_LOW(2)
-        BNSN_FDI_LOW(3) BNSN_FDI_LOW(4) BNSN_FDI_LOW(5)
+        BNSN_FDI_LOW(1) BNSN_FDI_LOW(2) BNSN_FDI_LOW(3) BNSN_FDI_LOW(4) BNSN_FDI_LOW(5)
 #undef BNSN_FDI_LOW
     }
     else if (x <= 0.)
@@ -247,8 +232,7 @@ __device__ __noinline__ void fdi_rational(double y, double* out)
 #define BNSN_FDI_MID(K)                                                          \
     if (KLO <= K && K <= KHI)                                                    \
         out[K - KLO] = horner(FdiCoef<K>::bn(), t) / horner(FdiCoef<K>::bd(), s);
-        BNSN_FDI_MID(0) BNSN_FDI_MID(1) BNSN_FDI_MID(2)
-        BNSN_FDI_MID(3) BNSN_FDI_MID(4) BNSN_FDI_MID(5)
+        BNSN_FDI_MID(1) BNSN_FDI_MID(2) BNSN_FDI_MID(3) BNSN_FDI_MID(4) BNSN_FDI_MID(5)
 #undef BNSN_FDI_MID
     }
     else
@@ -262,8 +246,7 @@ __device__ __noinline__ void fdi_rational(double y, double* out)
 #define BNSN_FDI_REF(K)                                                          \
     if (KLO <= K && K <= KHI)                                                    \
         out[K - KLO] = FdiCoef<K>::reflect(out[K - KLO], y);
-        BNSN_FDI_REF(0) BNSN_FDI_REF(1) BNSN_FDI_REF(2)
-        BNSN_FDI_REF(3) BNSN_FDI_REF(4) BNSN_FDI_REF(5)
+        BNSN_FDI_REF(1) BNSN_FDI_REF(2) BNSN_FDI_REF(3) BNSN_FDI_REF(4) BNSN_FDI_REF(5)
 #undef BNSN_FDI_REF
     }
 }
@@ -844,7 +827,8 @@ BNSN_DI double hr98_absorption(const Hr98Cell& M, double x, double ex)
     return tot;
 }
 
-// The same at any argument, with the library's powers.
+// The same at any argument, in the reference's order, with the powers of fx::pow (the
+// library's outside its range).
 BNSN_DI void hr98_kernel(const Hr98Point& P, double omega, double omega_p,
                          double* em, double* ab)
 {
