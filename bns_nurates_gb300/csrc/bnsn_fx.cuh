@@ -9,9 +9,10 @@
 // log 33, pow 100, a division 5-7, the rational Fermi integrals F_1..F_5 150.
 // The functions below work on 64-bit fixed-point numbers, which hold 11 bits
 // more than a double's mantissa: 2^x and log2 x take ~35 clocks (2.2 FMA) per
-// warp and F_1..F_5 ~150 clocks (9 FMA), at errors of at most one ulp of
-// the exact value (tests/test_fx.py measures them on the host, the same
-// source compiled by g++).
+// warp and F_1..F_5 ~150 clocks (9 FMA).  Error bounds (tests/test_fx.py measures them on
+// the host, the same source compiled by g++): e^x one ulp (2^-52); F_k 2^-51; x^p 2^-52 + |p|
+// 2^-55, since log2 x carries 2^-56; log and log2 an absolute 2^-56, so near x = 1 they
+// are not relatively accurate; quotients 2^-51.
 //
 // Methods: table-driven exponential and logarithm (P. T. P. Tang, ACM TOMS 15
 // (1989) 144 and 16 (1990) 378) carried out in fixed point; Fermi integrals by
@@ -254,7 +255,8 @@ BNSN_FX_HD bool log2_range(double x)
     return ((uint32_t)(bits_of(x) >> 52) - (1023u - 120u)) < 240u;
 }
 
-// log2(x) and log(x) for any x (absolute error 2^-57 near x = 1).
+// log2(x) and log(x) for any x, to an absolute 2^-56: not relatively accurate near x = 1
+// (log(1 + 2^-30) holds 28 bits).
 BNSN_FX_HD double log2(double x)
 {
     return log2_range(x) ? (double)log2_q56(x) * 1.3877787807814457e-17
@@ -381,7 +383,9 @@ BNSN_FX_HD void fd_orders(double y, double* out)
         else
         {
             const double ex = y < 0. ? exp(y) : 0.;
-#define BNSN_FX_ORDER(K)                                                                               if (KLO <= K && K <= KHI)                                                                              out[K - KLO < 0 ? 0 : K - KLO] = (NORM ? 1. : fd_factorial<K>()) * ex;
+#define BNSN_FX_ORDER(K)                                                                           \
+    if (KLO <= K && K <= KHI)                                                                      \
+        out[K - KLO < 0 ? 0 : K - KLO] = (NORM ? 1. : fd_factorial<K>()) * ex;
             BNSN_FX_ORDER(0) BNSN_FX_ORDER(1) BNSN_FX_ORDER(2)
             BNSN_FX_ORDER(3) BNSN_FX_ORDER(4) BNSN_FX_ORDER(5)
 #undef BNSN_FX_ORDER
@@ -408,7 +412,9 @@ BNSN_FX_HD void fd_orders(double y, double* out)
     S.h8  = (int32_t)(h >> 3);
     S.h9  = (int32_t)umulhi(h, 477218589u);
     S.h10 = (int32_t)umulhi(h, 429496730u);
-#define BNSN_FX_ORDER(K)                                                                               if (KLO <= K && K <= KHI)                                                                              out[K - KLO < 0 ? 0 : K - KLO] = fd_one<K, NORM>(r, S, scale, d);
+#define BNSN_FX_ORDER(K)                                                                           \
+    if (KLO <= K && K <= KHI)                                                                      \
+        out[K - KLO < 0 ? 0 : K - KLO] = fd_one<K, NORM>(r, S, scale, d);
     BNSN_FX_ORDER(0) BNSN_FX_ORDER(1) BNSN_FX_ORDER(2)
     BNSN_FX_ORDER(3) BNSN_FX_ORDER(4) BNSN_FX_ORDER(5)
 #undef BNSN_FX_ORDER

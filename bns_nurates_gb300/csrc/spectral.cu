@@ -653,10 +653,10 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 
 // Launches of fewer points than this many per SM share a point's energies between warps. A
 // pair cell is a chain of ~10 us, and a warp's slowest lane sets its time: 16 points x 40
-// energies, pair alone, n = 20: a warp per point 1.57 ms, shared 0.6; 16 x 24 with HR98
-// 0.81 -> 0.44. 304 points x 24, n = 10: 0.48 -> 0.41, 608: no difference. With 8 per SM
-// instead of 4, 456 points x 40 with HR98 at n = 20 took 2.38 ms instead of 2.22 (the node tables
-// are made by every warp).
+// energies, pair alone, n = 20: a warp per point 1.57 ms, shared 0.74; 16 x 24 with HR98
+// 0.81 -> 0.43. 304 points x 24, n = 10, pair: 0.48 -> 0.41; 608: no difference. With 8 per SM
+// 456 points x 40 with HR98 at n = 20 take 2.38 ms instead of 2.22 (every warp makes the node
+// tables).
 constexpr int64_t kPbWarpsPerSm = 4;
 
 // Pair + brem of the mixed path: a warp takes a point, or (parts > 1) every parts-th
