@@ -43,6 +43,7 @@
 // with NES 17.0 -> 3.9 ms; mixed n = 20 GP19 with NES 12.8 -> 5.5 ms.
 
 #include <algorithm>
+#include <type_traits>
 
 #include <cuda_runtime.h>
 
@@ -70,7 +71,6 @@ constexpr double kSpecCancelNes  = 2.0;     // same for the NES/NPS terms
 constexpr double kSpecNesMinW    = 0.05;    // NES in FP64 below nu/T = 0.05
 constexpr double kSpecNesDfW     = 0.2;    // NES brackets in double-float below nu/T = 0.2
 constexpr double kSpecFloor      = 7.2e-34; // 1e9 x the denormal floor of a sum
-constexpr double kKeepPb         = -1.;     // bpb: an output the last FP64 pass leaves as it is
 
 // Per (point, energy) record of the chunk scratch.
 struct EnergyRec
@@ -642,8 +642,6 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                     for (int a = 0; a < M; ++a)
                         acc = fma(fma(c0, K0[a], fma(c1, K1[a], Kb[a])), v[a], acc);
                 EnergyRec& E       = rec[q * ne + S.eid[c]];
-                if (flags && E.bpb[4 * ab + s] == kKeepPb)
-                    continue;
                 E.pb[4 * ab + s]  = ab || S.far[c] ? acc : acc * S.dny[c];
                 E.bpb[4 * ab + s] = 0.;
             }
@@ -1352,10 +1350,14 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 // ---------------------------------------------------------------------------
 // assemble (m1_opacities.hpp:1571-1660)
 // ---------------------------------------------------------------------------
+// Only the second check marks records; in the other modes they are read-only.
+template <int MODE>
+using AssembleRec = std::conditional_t<MODE == kSpecRedo, EnergyRec, const EnergyRec>;
+
 template <int MODE>
 __global__ void __launch_bounds__(kWarps * 32)
     spec_assemble_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
-                         const SpecPoint* __restrict__ pts, EnergyRec* __restrict__ rec,
+                         const SpecPoint* __restrict__ pts, AssembleRec<MODE>* __restrict__ rec,
                          uint64_t* __restrict__ fl_pb, uint64_t* __restrict__ fl_nes)
 {
     constexpr bool GUARD = MODE == kSpecMixed || MODE == kSpecRedo;
@@ -1401,11 +1403,17 @@ __global__ void __launch_bounds__(kWarps * 32)
                     beta_rates(bp, nu, 1, &b_ab[1], &b_em[1]);
                 }
                 const double F = k::FourPiHc3, c = k::Clight;
+                // the second round's pair + brem outputs that were not flagged
+                const bool keep =
+                    MODE == kSpecFinal && ((fl_pb[q] >> e) & 1ull) && !((fl_nes[q] >> e) & 1ull);
                 double ip[8], in[8];
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)
                 {
-                    ip[kk] = pb ? ts * E.pb[kk] : 0.;
+                    double v = E.pb[kk];
+                    if (MODE == kSpecFinal && keep && !isnan(E.bnes[kk]))
+                        v = E.bnes[kk];
+                    ip[kk] = pb ? ts * v : 0.;
                     in[kk] = L.use_inel ? nu * E.nes[kk] : 0.;
                 }
                 if (GUARD)
@@ -1440,11 +1448,14 @@ __global__ void __launch_bounds__(kWarps * 32)
                         }
                     }
                     fpb = pb_of != 0u;
-                    // the second check keeps the outputs that passed
-                    if (MODE == kSpecRedo && fpb)
-                        for (int kk = 0; kk < 8; ++kk)
-                            if (!((pb_of >> kk) & 1u))
-                                rec[q * ne + e].bpb[kk] = kKeepPb;
+                    // the outputs that pass the second check keep their sums: set aside
+                    // (NaN where flagged) in words that are free once NES has passed
+                    if constexpr (MODE == kSpecRedo)
+                        if (fpb && !fnes)
+                            for (int kk = 0; kk < 8; ++kk)
+                                rec[q * ne + e].bnes[kk] =
+                                    (pb_of >> kk) & 1u ? __longlong_as_double(0x7ff8000000000000LL)
+                                                       : E.pb[kk];
                 }
                 if (!fpb && !fnes)
                 {
