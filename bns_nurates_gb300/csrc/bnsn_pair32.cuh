@@ -263,7 +263,8 @@ __device__ __forceinline__ void cell_integrals(const Cell& c, double& Q0, double
                 break;
         }
     }
-    // The panels of the edge zones, a lane's own one after the other: with them inside the
+    // The panels of the edge zones, a lane's own one after the other and after all the other
+    // segments' sums: with them inside the
     // loop above, lanes at the same cut had other segments there or fewer panels (2.3
     // panels issued per one needed at n = 10, now 1.4).  8,192 points, mixed pair phase:
     // n = 10 0.62 -> 0.57 ms, n = 20 1.52 -> 1.44.

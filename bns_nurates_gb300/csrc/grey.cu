@@ -1582,7 +1582,7 @@ __global__ void __launch_bounds__(256)
 // (the 38 KB item table serves 8 points; one warp per point left the last of
 // 3.4 waves over 8,192 points 60% empty), or (WIDE) eight in 8-warp CTAs: the
 // mixed path's few flagged points, and launches with fewer points than the chip
-// has warps to fill.  8,192 points, n = 20: 5.55 -> 3.69 ms.
+// has warps to fill.  8,192 points, n = 20: 5.41 -> 3.69 ms.
 // ---------------------------------------------------------------------------
 
 template <bool WIDE>

@@ -35,8 +35,9 @@
 // exceeds it (terms that cancel), or where a part could not run in FP32
 // (bound = inf: occupations outside the FP32 range, NES at nu/T < 0.05), it flags the
 // part whose bound exceeds half the total.  Flagged parts are recomputed by the FP64
-// kernels over the flagged energies of a point; assemble checks again with the
-// remaining bounds, and a last round finishes what is left.  (A double-float pass over
+// kernels over the flagged energies of a point; assemble checks the remaining bounds
+// against the totals that now hold the FP64 sums, and a last pass recomputes the outputs
+// that fail (pair and brem sums that FP64 NES sums cancel).  (A double-float pass over
 // the flagged NES parts before the FP64 one took 2.2 ms of 10.8 per 4,096 points at
 // 5% occupancy, and the FP64 kernels are as fast per energy.)
 // 4,096 points x 24 energies: FP64 n = 10 HR98 without NES 9.1 -> 1.3 ms, n = 20 GP19

@@ -419,7 +419,9 @@ int bnsn_blocks_plan_destroy(bnsn_blocks_plan_t plan);
  * (`energies` is a host array, MeV).  Replaces
  * ComputeSpectralOpacitiesStimulatedAbs (stimulated = 1,
  * m1_opacities.hpp:1641-1660) and ComputeSpectralOpacitiesNotStimulatedAbs
- * (stimulated = 0, m1_opacities.hpp:1506-1637) called per (point, energy). */
+ * (stimulated = 0, m1_opacities.hpp:1506-1637) called per (point, energy).
+ * BNSN_FP64 is nearly always faster than BNSN_MIXED here (262,144 points x 24
+ * energies, n = 20, all reactions: 238 against 322 ms). */
 int bnsn_spectral_opacities(const MyQuadrature* quad_1d,
                             const OpacityFlags* flags,
                             const OpacityParams* params,
