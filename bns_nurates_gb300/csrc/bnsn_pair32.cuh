@@ -407,8 +407,8 @@ __device__ __forceinline__ void absorption_q(dfm::df Y, dfm::df Z, double ehy, d
 // The pair kernel of one cell for the four species: em and ab of
 // kernel_pair.hpp:135-198 times (nu nubar)^2, from the FP32 integral:
 // ab = (Phi T^2 / 2) alpha . (Psi / (1 - e^s)) e^{s}, em = ab / SafeExp(s).
-// Y, Z: nu / T and nubar / T as double-float; eh = e^{y - |eta| / 2} and
-// dn = e^{-y} of each side (e^{Lref} = eh_y eh_z where Lref != 0, e^{-s} =
+// Y, Z: nu / T and nubar / T as double-float; eh = e^{y - c_y}, e^{z - c_z} with c_y +
+// c_z = |eta| (e^{Lref} = eh_y eh_z where Lref != 0) and dn = e^{-y} of each side (e^{-s} =
 // dn_y dn_z for s <= 700); sc = (Phi T^2 / 2) T^4 / 15, the point's factor.
 __device__ __forceinline__ void kernel_q(dfm::df Y, dfm::df Z, double ehy, double ehz,
                                          double dny, double dnz, dfm::df ETA, double sc,

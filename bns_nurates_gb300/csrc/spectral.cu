@@ -323,7 +323,7 @@ struct PbWarpMixed
     fp32::Hr98Mixed hm;
     float yeh[kEChunk], yel[kEChunk]; // nu / T as hi + lo
     float ybh[kMaxM], ybl[kMaxM];     // nubar / T as hi + lo
-    double ehy[kEChunk], dny[kEChunk]; // pair: e^{y - |eta|/2}, e^{-y} of the energies
+    double ehy[kEChunk], dny[kEChunk]; // pair: e^{y - cy}, e^{-y} of the energies
     double ehz[kMaxM], dnz[kMaxM];     // the same of the nodes
     float gb32[kMaxM][4], gbm32[kMaxM][4];
     float gp32[2][kGp19MaxW];
@@ -730,6 +730,9 @@ __global__ void __launch_bounds__(kWarps * 32)
         const dfm::df ETA = dfm::from_double(eta_e);
         const double T2   = T * T;
         const double scq  = 0.5 * k::PairPhi * T2 * (T2 * T2) / 15.;
+        // shares of |eta| in e^{Lref} = e^{y - cy} e^{z - cz}, used where y + z <= |eta|: halves,
+        // or beyond 1,400, where those leave the double range, 300 on the node's side (z < 640)
+        const double aeta = fabs(eta_e), cz = aeta <= 1400. ? 0.5 * aeta : 300., cy = aeta - cz;
         // antineutrino grid of the pair/brem integral (m1_opacities.hpp:1542)
         const double ts = k::TempMultiple * T;
         for (int a = lane; a < M; a += 32)
@@ -744,7 +747,7 @@ __global__ void __launch_bounds__(kWarps * 32)
             X.ybl[a] = yd.lo;
             if (L.use_pair)
             {
-                X.ehz[a] = fx::exp(W.zb[a] - 0.5 * fabs(eta_e));
+                X.ehz[a] = fx::exp(W.zb[a] - cz);
                 X.dnz[a] = fx::exp(-W.zb[a]);
             }
 #pragma unroll
@@ -788,7 +791,7 @@ __global__ void __launch_bounds__(kWarps * 32)
                 X.yel[c] = yd.lo;
                 if (L.use_pair)
                 {
-                    X.ehy[c] = fx::exp(y - 0.5 * fabs(eta_e));
+                    X.ehy[c] = fx::exp(y - cy);
                     X.dny[c] = fx::exp(-y);
                 }
             }

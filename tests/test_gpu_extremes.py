@@ -8,7 +8,9 @@ import numpy as np
 import pytest
 
 import bns_nurates_gb300 as bn
-from test_gpu_parity import DEFAULT, F, P, assert_close, gpu_grey, oracle_grey
+from test_gpu_mixed import _check, _spec_oracle_with_sens
+from test_gpu_parity import (DEFAULT, F, P, assert_close, gpu_grey, oracle_grey,
+                             port_fma)  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +82,17 @@ def test_spectral_brt06_emission_far_above_the_temperature(cuda, port, precision
                               DEFAULT[:5] + (1,) + DEFAULT[6:], precision, 0,
                               np.array([400., 900., 960., 1100., 1400.]))
     assert_close(got[:4], want[:4], what="BRT06 emission")
+
+
+@pytest.mark.parametrize("nq", [6, 20])
+def test_mixed_spectral_energies_at_the_fermi_edge_of_cold_electrons(cuda, port, port_fma, nq):
+    """eta_e of thousands and energies just below mu_e: the FP32 pair integral's scale
+    e^{(nu + nubar - mu_e) / T} is a product of two numbers outside the double range there."""
+    eos, m1 = bn.synthetic_points(23, 8)
+    eos[TEMP] = np.tile([0.05, 0.07, 0.1, 0.12], 2)
+    eos[MU_E] = np.repeat([170., 140.], 4)
+    energies = np.array([128., 131., 136., 139.5, 150., 161., 166., 169.5])
+    flags, pars = (1, 1, 1, 1, 1), DEFAULT
+    got, _ = spectral_both(cuda, port, eos, m1, flags, pars, "mixed", 1, energies, nq)
+    want, sens = _spec_oracle_with_sens(port, port_fma, eos, m1, flags, pars, nq, energies)
+    _check(got, want, sens, "cold electrons")
