@@ -903,10 +903,16 @@ BNSN_DI double brt06_shape(double x)
 
 // The emission kernel, e^{-2x} of the absorption kernel.  The reference multiplies by e^{-x}
 // twice, so e^{-2x} is not clamped at 2x = 700.
+static __device__ __noinline__ double brt06_emission_far(double ab, double x)
+{
+    const double ex = fx::exp(-x);
+    return ab * ex * ex;
+}
 BNSN_DI double brt06_emission(double ab, double x)
 {
-    const double ex = fx::exp(x > 350. ? -x : -2. * x);
-    return x > 350. ? ab * ex * ex : ab * ex;
+    return __double2hiint(x) >= 0x4075e000 // x >= 350 (x > 0), or NaN
+               ? brt06_emission_far(ab, x)
+               : ab * safe_exp(-2. * x);
 }
 
 BNSN_DI void brt06_kernel(double pre, double T, double omega, double omega_p,

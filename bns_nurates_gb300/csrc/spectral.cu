@@ -628,13 +628,9 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                     {
                         const double x = S.y[c] + S.z[a], Kp = fma(c0, K0[a], c1 * K1[a]);
                         const double wn = L.B1[a], nb2 = S.nb[a] * S.nb[a];
-                        // g, or 1 - g from the stored product unless that underflows (T < 1e-10)
-                        const double wnb = wn * nb2, den = ab ? wnb : S.dnz[a] * wnb;
-                        const double gp  = wnb > 0. ? S.vA[s][a] / wnb : 0.;
-                        const double g   = ab          ? gp
-                                           : nbb       ? 1.
-                                           : den > 1e-290 ? v[a] / den
-                                                          : 1. - gp;
+                        // a weight that underflows (T < 1e-10) belongs to a term that does
+                        const double den = fmax((ab ? 1. : S.dnz[a]) * (wn * nb2), 2.3e-308);
+                        const double g   = !ab && nbb ? 1. : v[a] / den;
                         const double K = x > k::ExpUpp ? pb64_far<IMPL>(Kp, Kb[a], T, x, ab)
                                                        : (Kp + Kb[a]) * (ab ? 1. : safe_exp(-x));
                         acc += wn * (nb2 * (K * g));
@@ -658,8 +654,10 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 // tables).
 constexpr int64_t kPbWarpsPerSm = 4;
 
-// Pair + brem of the mixed path: a warp takes a point, or (parts > 1) every parts-th
-// energy of one; an energy's sums do not depend on it.
+// Pair + brem of the mixed path: a warp takes a point, or (SHARED) every parts-th energy of
+// one; an energy's sums do not depend on it.  (One kernel for both, with parts = 1, was 2%
+// slower on large calls.)
+template <bool SHARED>
 __global__ void __launch_bounds__(kWarps * 32)
     spec_pb_kernel(const __grid_constant__ OpacityLaunch L, int64_t p0, int64_t np,
                    const SpecPoint* __restrict__ pts, EnergyRec* __restrict__ rec, int G, int parts)
@@ -695,10 +693,11 @@ __global__ void __launch_bounds__(kWarps * 32)
     const int64_t nwarp = (int64_t)gridDim.x * kWarps;
     const int grp = lane % G, per_round = 32 / G;
 
-    for (int64_t t = (int64_t)blockIdx.x * kWarps + wid; t < np * parts; t += nwarp)
+    const int64_t tasks = SHARED ? np * parts : np;
+    for (int64_t t = (int64_t)blockIdx.x * kWarps + wid; t < tasks; t += nwarp)
     {
-        const int64_t q     = t / parts;
-        const int part      = (int)(t - q * parts);
+        const int64_t q     = SHARED ? t / parts : t;
+        const int part      = SHARED ? (int)(t - q * parts) : 0;
         const int64_t p     = p0 + q;
         const double T = L.eos[1][p], eta_e = L.eos[7][p] / T;
         EnergyRec* R       = rec + q * ne;
@@ -797,12 +796,13 @@ __global__ void __launch_bounds__(kWarps * 32)
             }
             __syncwarp();
             // the part's energies: e = part, part + parts, ...
-            const int first = (part + parts - e0 % parts) % parts;
-            const int own   = first < nec ? (nec - first + parts - 1) / parts : 0;
+            const int first = SHARED ? (part + parts - e0 % parts) % parts : 0;
+            const int own   = !SHARED ? nec : first < nec ? (nec - first + parts - 1) / parts : 0;
             for (int r0 = 0; r0 < own; r0 += per_round)
             {
                 const bool act  = r0 + lane / G < own;
-                const int c     = act ? (r0 + lane / G) * parts + first : 0;
+                const int k     = act ? r0 + lane / G : 0;
+                const int c     = SHARED ? (act ? k * parts + first : 0) : k;
                 const double nu = act ? L.energies[e0 + c] : 1.;
                 const double w  = nu / T;
                 double acc[8];
@@ -1407,19 +1407,18 @@ __global__ void __launch_bounds__(kWarps * 32)
                     beta_rates(bp, nu, 1, &b_ab[1], &b_em[1]);
                 }
                 const double F = k::FourPiHc3, c = k::Clight;
-                // the second round's pair + brem outputs that were not flagged
-                const bool keep =
-                    MODE == kSpecFinal && ((fl_pb[q] >> e) & 1ull) && !((fl_nes[q] >> e) & 1ull);
                 double ip[8], in[8];
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)
                 {
-                    double v = E.pb[kk];
-                    if (MODE == kSpecFinal && keep && !isnan(E.bnes[kk]))
-                        v = E.bnes[kk];
-                    ip[kk] = pb ? ts * v : 0.;
+                    ip[kk] = pb ? ts * E.pb[kk] : 0.;
                     in[kk] = L.use_inel ? nu * E.nes[kk] : 0.;
                 }
+                if constexpr (MODE == kSpecFinal)
+                    if (((fl_pb[q] >> e) & 1ull) && !((fl_nes[q] >> e) & 1ull))
+                        for (int kk = 0; kk < 8; ++kk)
+                            if (!isnan(E.bnes[kk])) // not flagged by the second check
+                                ip[kk] = ts * E.bnes[kk];
                 if (GUARD)
                 {
                     // FP32 error bounds against each output's total
@@ -1539,21 +1538,28 @@ cudaError_t grid_of(K kernel, size_t smem, bool* attr_set, int num_sms, int64_t 
     return cudaSuccess;
 }
 
-cudaError_t launch_pb_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
-                            EnergyRec* rec, int G, cudaStream_t st, int sms)
+template <bool SHARED>
+cudaError_t launch_pb_form(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
+                           EnergyRec* rec, int G, int parts, cudaStream_t st, int sms)
 {
     static bool attr  = false;
     const size_t smem = sizeof(PbShared);
-    const int parts   = (int)std::max<int64_t>(
-        1, std::min<int64_t>(sms * kPbWarpsPerSm / np, L.n_energies));
     int grid          = 0;
-    cudaError_t err   = grid_of(spec_pb_kernel, smem, &attr, sms, np * parts, &grid);
+    cudaError_t err   = grid_of(spec_pb_kernel<SHARED>, smem, &attr, sms, np * parts, &grid);
     if (err != cudaSuccess || grid == 0)
         return err;
     phase_mark(kPhSpectral, 0, st);
-    spec_pb_kernel<<<grid, kWarps * 32, smem, st>>>(L, p0, np, pts, rec, G, parts);
+    spec_pb_kernel<SHARED><<<grid, kWarps * 32, smem, st>>>(L, p0, np, pts, rec, G, parts);
     phase_mark(kPhSpectral, 1, st);
     return cudaGetLastError();
+}
+
+cudaError_t launch_pb_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
+                            EnergyRec* rec, int G, cudaStream_t st, int sms)
+{
+    const int64_t parts = std::min<int64_t>(sms * kPbWarpsPerSm / np, L.n_energies);
+    return parts > 1 ? launch_pb_form<true>(L, p0, np, pts, rec, G, (int)parts, st, sms)
+                     : launch_pb_form<false>(L, p0, np, pts, rec, G, 1, st, sms);
 }
 
 cudaError_t launch_nes_mixed(const OpacityLaunch& L, int64_t p0, int64_t np, const SpecPoint* pts,
