@@ -421,7 +421,7 @@ int bnsn_blocks_plan_destroy(bnsn_blocks_plan_t plan);
  * m1_opacities.hpp:1641-1660) and ComputeSpectralOpacitiesNotStimulatedAbs
  * (stimulated = 0, m1_opacities.hpp:1506-1637) called per (point, energy).
  * BNSN_FP64 is nearly always faster than BNSN_MIXED here (262,144 points x 24
- * energies, n = 20, all reactions: 238 against 322 ms). */
+ * energies, n = 20, all reactions: 234 against 320 ms). */
 int bnsn_spectral_opacities(const MyQuadrature* quad_1d,
                             const OpacityFlags* flags,
                             const OpacityParams* params,
